@@ -78,8 +78,8 @@ struct Rec<double> {
 // than 7 standard deviations above the mean tile occupancy at density 10; an
 // over-full tile takes the global-memory path.  Every shape gives the same
 // results bit for bit (the tile size changes only which block handles a
-// cell); the shape in use is chosen per precision, by default the first one,
-// or by rmpcd_bulk_autotune.
+// cell); the shape in use is chosen per precision by rmpcd_bulk_set_shape or
+// rmpcd_bulk_autotune, or else by the size of the box (pick_shape).
 template <int SL_, int CAP_, int MINB_>
 struct Shape {
     static constexpr int kSlots = SL_;
@@ -668,21 +668,17 @@ template <typename R>
 struct Shapes;
 template <>
 struct Shapes<float> {
-    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<128, 1792, 4>>(),
-                                                  entry<float, Shape<128, 1792, 5>>(),
-                                                  entry<float, Shape<96, 1408, 5>>(),
-                                                  entry<float, Shape<64, 1024, 6>>(),
-                                                  entry<float, Shape<160, 2176, 4>>(),
-                                                  entry<float, Shape<192, 2560, 3>>()};
+    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<128, 1792, 4>>(), entry<float, Shape<32, 512, 4>>(),
+                                                  entry<float, Shape<96, 1408, 5>>(), entry<float, Shape<64, 1024, 6>>(),
+                                                  entry<float, Shape<160, 2176, 4>>(), entry<float, Shape<16, 288, 4>>()};
+    static constexpr int by_size[] = {0, 3, 1, 5};  // widest first (pick_shape)
 };
 template <>
 struct Shapes<double> {
-    static constexpr ShapeEntry<double> list[] = {entry<double, Shape<96, 1408, 4>>(),
-                                                   entry<double, Shape<112, 1600, 3>>(),
-                                                   entry<double, Shape<128, 1792, 3>>(),
-                                                   entry<double, Shape<160, 2176, 2>>(),
-                                                   entry<double, Shape<192, 2560, 2>>(),
-                                                   entry<double, Shape<96, 1408, 3>>()};
+    static constexpr ShapeEntry<double> list[] = {entry<double, Shape<64, 1024, 4>>(), entry<double, Shape<112, 1600, 3>>(),
+                                                   entry<double, Shape<32, 512, 4>>(), entry<double, Shape<16, 288, 4>>(),
+                                                   entry<double, Shape<160, 2176, 2>>(), entry<double, Shape<96, 1408, 3>>()};
+    static constexpr int by_size[] = {0, 2, 3};
 };
 template <typename R>
 constexpr int n_shapes()
@@ -690,12 +686,33 @@ constexpr int n_shapes()
     return (int)(sizeof(Shapes<R>::list) / sizeof(Shapes<R>::list[0]));
 }
 
-static int g_shape[2] = {0, 0};  // shape in use: [0] FP32, [1] FP64
+static int g_shape[2] = {-1, -1};  // shape set: [0] FP32, [1] FP64; -1 = by the size of the box
+
+// The shape of a run: the one set, or the widest of by_size whose tiles, over
+// the cells of the box, number at least kMinTiles (about two per SM); a box
+// with fewer takes the narrowest.  A tile's block is a chain of latencies
+// (index copy, gather, collision, streaming) about as long as its passes over
+// the particles, so a small box wants every SM busy with short blocks and a
+// large one wants tiles wide enough to hide the chain.  us per interval
+// (slots per tile x blocks per SM): 16^3 FP32 20.7 (16 x 4), 24.7 (64 x 6),
+// 28.6 (128 x 4), FP64 22.3 (16 x 4), 25.7 (64 x 4), 28.6 (96 x 3); 24^3 FP64
+// 30.8 (32 x 4), 37.6 (64 x 4); 32^3 FP32 31.9 (64 x 6), 33.3 (128 x 4); 128^3
+// FP32 682 (128 x 4), 713 (64 x 6), FP64 1153 (64 x 4), 1177 (96 x 3), 1431
+// (96 x 4).
+constexpr int kMinTiles = 260;
 
 template <typename R>
-static const ShapeEntry<R> &shape_in_use()
+static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c)
 {
-    return Shapes<R>::list[g_shape[sizeof(R) == 8]];
+    const int set = g_shape[sizeof(R) == 8];
+    if (set >= 0) return Shapes<R>::list[set];
+    const long long cells = (long long)c->L[0] * c->L[1] * c->L[2];
+    int pick = 0;
+    for (int k : Shapes<R>::by_size) {
+        pick = k;
+        if (cells / Shapes<R>::list[k].slots >= kMinTiles) break;
+    }
+    return Shapes<R>::list[pick];
 }
 
 template <typename R>
@@ -733,7 +750,7 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
     cudaStream_t st = stream();
     int rc = prepare_shapes<R>();
     if (rc) return rc;
-    const ShapeEntry<R> &shape = shape_in_use<R>();
+    const ShapeEntry<R> &shape = pick_shape<R>(c);
     rc = ensure_records<R>(p);
     if (rc) return rc;
     double sin_a = 1, cos_a = 0;
@@ -878,7 +895,7 @@ static int autotune_t(const int L[3], double tau, int n_intervals, int *best, fl
             rc = fail(RMPCD_ERR_CUDA, "rmpcd_bulk_autotune: event creation failed");
         const int keep = g_shape[sizeof(R) == 8];
         float best_ms = 0;
-        int best_k = keep;
+        int best_k = 0;
         for (int k = 0; !rc && k < n_shapes<R>(); k++) {
             g_shape[sizeof(R) == 8] = k;
             rc = bulk_run_fused<R>(p, c, &r, tau, 0, 0.0, 1);
@@ -896,7 +913,7 @@ static int autotune_t(const int L[3], double tau, int n_intervals, int *best, fl
             }
         }
         g_shape[sizeof(R) == 8] = rc ? keep : best_k;
-        if (best) *best = g_shape[sizeof(R) == 8];
+        if (best) *best = best_k;
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -931,7 +948,7 @@ extern "C" int rmpcd_bulk_get_shape(int precision, int *shape)
 {
     RMPCD_ARG(shape, "null argument");
     RMPCD_ARG(precision == RMPCD_FP32 || precision == RMPCD_FP64, "precision must be 32 or 64");
-    *shape = g_shape[precision == RMPCD_FP64];
+    *shape = g_shape[precision == RMPCD_FP64] < 0 ? 0 : g_shape[precision == RMPCD_FP64];
     return RMPCD_OK;
 }
 

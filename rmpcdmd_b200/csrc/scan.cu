@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_totals(const int *__
 }
 
 // Launch 2: each block adds up the totals of the tiles before it (a few
-// loads per thread, from L2) and scans its own tile.
+// loads per thread, from L2) and scans its own tile.  Without tile_total (at
+// most kScanDirectTiles tiles) it adds up those tiles' elements instead.
 __global__ void __launch_bounds__(kScanThreads)
     k_scan_tiles(const int *__restrict__ in, int n, const int *__restrict__ tile_total, int *__restrict__ out,
                  int *__restrict__ out2, int *__restrict__ clear)
@@ -112,7 +113,16 @@ __global__ void __launch_bounds__(kScanThreads)
     __shared__ int s_part[kWarps];
     const int tile = blockIdx.x;
     int pre = 0;
-    for (int j = threadIdx.x; j < tile; j += kScanThreads) pre += tile_total[j];
+    if (tile_total) {
+        for (int j = threadIdx.x; j < tile; j += kScanThreads) pre += tile_total[j];
+    } else {
+        const int4 *q4 = reinterpret_cast<const int4 *>(in);
+#pragma unroll 4
+        for (int j = threadIdx.x; j < tile * (kScanTile / 4); j += kScanThreads) {
+            const int4 v = q4[j];
+            pre += v.x + v.y + v.z + v.w;
+        }
+    }
     const long long tile0 = (long long)tile * kScanTile;
     const bool whole = tile0 + kScanTile <= n;
     int4 q[kRows];
@@ -153,8 +163,9 @@ int exclusive_scan(const int *in, int *out, int *out2, int n, int *tile_total, i
     const int nb = scan_blocks_for(n);
     if (nb > kScanMaxTiles)
         return fail(RMPCD_ERR_CAPACITY, "slot scan: %d slots above the supported maximum", n);
-    k_scan_tile_totals<<<nb, kScanThreads, 0, s>>>(in, n, tile_total);
-    k_scan_tiles<<<nb, kScanThreads, 0, s>>>(in, n, tile_total, out, out2, clear);
+    const bool direct = nb <= kScanDirectTiles;
+    if (!direct) k_scan_tile_totals<<<nb, kScanThreads, 0, s>>>(in, n, tile_total);
+    k_scan_tiles<<<nb, kScanThreads, 0, s>>>(in, n, direct ? nullptr : tile_total, out, out2, clear);
     RMPCD_CHECK_LAUNCH();
     return RMPCD_OK;
 }

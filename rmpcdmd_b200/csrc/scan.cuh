@@ -14,6 +14,11 @@ constexpr int kScanTile = kScanThreads * kScanPerThread;
 // loads per thread at the maximum, 2^27 slots: the largest cell system)
 constexpr int kScanMaxTiles = 128 * kScanThreads;
 
+// up to this many tiles the second launch adds up the elements before a tile
+// itself, which saves the first: the last tile then reads 7 x 16 KB more (2.5
+// us) where the launch and its boundary take ~4
+constexpr int kScanDirectTiles = 8;
+
 inline int scan_blocks_for(int n) { return (n + kScanTile - 1) / kScanTile; }
 
 // Writes the exclusive scan of in[0..n) to out (and out2 when not null) and,
