@@ -1,7 +1,8 @@
 // MPCD on the GPU (src/mpcd.f90): SRD and MPC-AT collisions, the Lamura wall
 // rule, temperature, cell rescaling, streaming with periodic and wall
 // boundaries, and bulk reactions.  Collisions run one thread per Hilbert
-// slot over the sorted particle ranges (cells hold ~10 particles).
+// slot over the sorted particle ranges (cells hold ~10 particles), staged in
+// shared memory tile by tile.
 #include <cmath>
 
 #include "cellops.cuh"
@@ -13,17 +14,86 @@
 
 namespace rmpcd {
 
-// simple_mpcd_step, src/mpcd.f90:71-183
-template <typename R>
-__global__ void k_simple_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S,
-                              R *vx, R *vy, R *vz, const int *__restrict__ species, SrdParams q)
+// The collision kernels below work on tiles of kCellTile consecutive slots,
+// whose particles are one contiguous range: the block brings the range's
+// velocities and species into shared memory with coalesced loads, one thread
+// per slot runs the cell's sequential sums and updates there, and the block
+// writes the velocities back coalesced.  A thread per slot on global memory
+// touches 32 cells' ranges per warp load (64^3 at density 10: 79 us FP64 for
+// the SRD step against 30 us of HBM traffic); the cell's own chain of adds
+// then sets its pace.  64 slots per 128-thread block leave 8 (FP64) or 16
+// (FP32) blocks per SM, so that one block's loads overlap another's sums.  A
+// tile of more than kCellCap particles (7 standard deviations above the mean
+// at density 10) takes the same cell bodies on global memory.
+constexpr int kCellTile = 64;
+constexpr int kCellThreads = 128;
+constexpr int kCellCap = 832;
+
+struct CellRange {
+    int n, a;          // this thread's cell: particles, first particle (n = 0: no cell)
+    int a0, np;        // the tile's particles
+    __device__ CellRange(const int *__restrict__ count, const int *__restrict__ start, int S)
+    {
+        const int s0 = blockIdx.x * kCellTile, last = min(s0 + kCellTile, S) - 1;
+        const int s = s0 + (int)threadIdx.x;
+        n = 0;
+        a = 0;
+        if (threadIdx.x < kCellTile && s < S) {
+            n = count[s];
+            a = start[s];
+        }
+        a0 = start[s0];
+        np = start[last] + count[last] - a0;
+    }
+};
+
+inline int cell_blocks(int S) { return (S + kCellTile - 1) / kCellTile; }
+
+// K arrays src[k][a0 .. a0 + np) to or from rows of kCellCap of shared memory
+template <typename T, int K>
+__device__ __forceinline__ void tile_in(T (*dst)[kCellCap], const T *const (&src)[K], int a0, int np)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x)
-        srd_slot<R>(count[s], start[s], s, 0, vx, vy, vz, species, q);
+#pragma unroll 2
+    for (int j = threadIdx.x; j < np; j += kCellThreads) {
+#pragma unroll
+        for (int k = 0; k < K; k++) dst[k][j] = src[k][a0 + j];
+    }
+}
+template <typename T, int K>
+__device__ __forceinline__ void tile_out(T *const (&dst)[K], T (*src)[kCellCap], int a0, int np)
+{
+#pragma unroll 2
+    for (int j = threadIdx.x; j < np; j += kCellThreads) {
+#pragma unroll
+        for (int k = 0; k < K; k++) dst[k][a0 + j] = src[k][j];
+    }
 }
 
-// The MPC-AT normals of simple_mpcd_step (src/mpcd.f90:144-160): for every
-// particle i with species > 0, (R)(rng::normal(seed, step, i, k) * t_factor)
+// simple_mpcd_step, src/mpcd.f90:71-183
+template <typename R>
+__global__ void __launch_bounds__(kCellThreads)
+    k_simple_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+                  const int *__restrict__ species, SrdParams q)
+{
+    __shared__ R sv[3][kCellCap];
+    __shared__ int ss[1][kCellCap];
+    const CellRange c(count, start, S);
+    const long long slot = (long long)blockIdx.x * kCellTile + threadIdx.x;
+    if (c.np > kCellCap) {
+        srd_slot<R>(c.n, c.a, slot, 0, vx, vy, vz, species, q);
+        return;
+    }
+    tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
+    tile_in<int, 1>(ss, {species}, c.a0, c.np);
+    __syncthreads();
+    srd_slot<R>(c.n, c.a - c.a0, slot, -(long long)c.a0, sv[0], sv[1], sv[2], ss[0], q);
+    __syncthreads();
+    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
+}
+
+// The MPC-AT normals of simple_mpcd_step (src/mpcd.f90:144-160) and
+// wall_mpcd_step (:268-290): for every particle i with species > 0 (for every
+// particle when species is null), (R)(rng::normal(seed, step, i, k) * t_factor)
 // for k = 0, 1, 2 into n[k][i].  Each deviate is the first accepted of the
 // attempts t = 0, 1, ... of rng::normal, so the values are rng::normal's.  A
 // warp takes kAtChunks chunks of 32 particles at a time and deals the
@@ -56,7 +126,7 @@ __global__ void __launch_bounds__(kAtThreads) k_at_normals(const int *__restrict
         int tail = 0;
         for (int c = 0; c < kAtChunks; c++) {
             const long long i = base + c * 32 + lane;
-            const bool act = i < N && species[i] > 0;
+            const bool act = i < N && (!species || species[i] > 0);
             for (int k = 0; k < 3; k++) {
                 double z = 0;
                 const bool ok = act && rng::normal_attempt(q.seed, q.step, (uint32_t)i, (uint32_t)k, 0u, &z);
@@ -94,233 +164,314 @@ __global__ void __launch_bounds__(kAtThreads) k_at_normals(const int *__restrict
     }
 }
 
-// simple_mpcd_step with the MPC-AT thermostat given the normals of
-// k_at_normals: the thermostat branch of srd_slot (src/mpcd.f90:126-160) with
-// each normal read instead of drawn; vel = normal + dv (hydro) or the normal,
-// as srd_slot's store and later add.
+// the thermostat branch of srd_slot (src/mpcd.f90:126-160) for the n
+// particles from a, with each normal read instead of drawn; vel = normal + dv
+// (hydro) or the normal, as srd_slot's store and later add
 template <typename R>
-__global__ void k_at_cells(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
-                           const int *__restrict__ species, int hydro, const R *__restrict__ nx,
-                           const R *__restrict__ ny, const R *__restrict__ nz)
+__device__ __forceinline__ void at_cell(int n, int a, R *vx, R *vy, R *vz, const int *species, int hydro,
+                                        const R *nx, const R *ny, const R *nz)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-        const int n = count[s];
-        if (n <= 1) continue;
-        const long long a = start[s];
-        int n_eff = 0;
-        CellSum<R> sx, sy, sz, wx, wy, wz;
-        for (long long i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                sx.add(vx[i]);
-                sy.add(vy[i]);
-                sz.add(vz[i]);
+    if (n <= 1) return;
+    int n_eff = 0;
+    CellSum<R> sx, sy, sz, wx, wy, wz;
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            sx.add(vx[i]);
+            sy.add(vy[i]);
+            sz.add(vz[i]);
+            wx.add(nx[i]);
+            wy.add(ny[i]);
+            wz.add(nz[i]);
+            n_eff++;
+        }
+    }
+    if (n_eff <= 1) return;
+    const R lv[3] = {sx.value() / n_eff, sy.value() / n_eff, sz.value() / n_eff};
+    const R dv[3] = {lv[0] - wx.value() / n_eff, lv[1] - wy.value() / n_eff, lv[2] - wz.value() / n_eff};
+    for (int i = a; i < a + n; i++) {
+        if (species[i] <= 0) continue;
+        vx[i] = hydro ? nx[i] + dv[0] : nx[i];
+        vy[i] = hydro ? ny[i] + dv[1] : ny[i];
+        vz[i] = hydro ? nz[i] + dv[2] : nz[i];
+    }
+}
+
+// simple_mpcd_step with the MPC-AT thermostat given the normals of
+// k_at_normals
+template <typename R>
+__global__ void __launch_bounds__(kCellThreads)
+    k_at_cells(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+               const int *__restrict__ species, int hydro, const R *__restrict__ nx, const R *__restrict__ ny,
+               const R *__restrict__ nz)
+{
+    __shared__ R sv[6][kCellCap];
+    __shared__ int ss[1][kCellCap];
+    const CellRange c(count, start, S);
+    if (c.np > kCellCap) {
+        at_cell<R>(c.n, c.a, vx, vy, vz, species, hydro, nx, ny, nz);
+        return;
+    }
+    tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, c.a0, c.np);
+    tile_in<int, 1>(ss, {species}, c.a0, c.np);
+    __syncthreads();
+    at_cell<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0], hydro, sv[3], sv[4], sv[5]);
+    __syncthreads();
+    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
+}
+
+struct WallArgs {
+    int M0, M1, M2, L2;
+    int has_wall;
+    double wt0, wt1;
+    int wn0, wn1;
+    int do_cell_v;
+};
+
+// wall_mpcd_step of slot s (src/mpcd.f90:193-337), its n particles from a;
+// with the thermostat, nx, ny, nz hold the particles' normals
+template <typename R>
+__device__ __forceinline__ void wall_cell(int n, int a, int s, R *vx, R *vy, R *vz, const R *nx, const R *ny,
+                                          const R *nz, const SrdParams &q, const WallArgs &w)
+{
+    if (n <= 1) return;
+    const int M[3] = {w.M0, w.M1, w.M2};
+    int cell[3];
+    hilbert::compact_point(s, M, cell);
+    int wall_idx = -1;
+    if (w.has_wall && cell[2] + 1 == 1) wall_idx = 0;
+    else if (w.has_wall && cell[2] + 1 == w.L2) wall_idx = 1;
+    int n_virtual = 0;
+    double vv[3] = {0, 0, 0};
+    int wn = wall_idx == 0 ? w.wn0 : w.wn1;
+    if (wall_idx >= 0 && n < wn) {
+        n_virtual = wn - n;
+        for (int k = 0; k < 3; k++) vv[k] = rng::normal(q.seed, q.step, (uint32_t)s, (uint32_t)(3 + k));
+        double f = sqrt(n_virtual * (wall_idx == 0 ? w.wt0 : w.wt1));
+        for (int k = 0; k < 3; k++) vv[k] = vv[k] * f;
+    }
+    CellSum<R> sx, sy, sz;
+    for (int i = a; i < a + n; i++) {
+        sx.add(vx[i]);
+        sy.add(vy[i]);
+        sz.add(vz[i]);
+    }
+    R lv[3];
+    if (n_virtual > 0) {
+        lv[0] = (R)(((double)sx.value() + vv[0]) / wn);
+        lv[1] = (R)(((double)sy.value() + vv[1]) / wn);
+        lv[2] = (R)(((double)sz.value() + vv[2]) / wn);
+    } else {
+        lv[0] = sx.value() / n;
+        lv[1] = sy.value() / n;
+        lv[2] = sz.value() / n;
+    }
+    if (q.thermostat) {
+        R dv[3] = {0, 0, 0};
+        if (w.do_cell_v) {
+            CellSum<R> wx, wy, wz;
+            for (int i = a; i < a + n; i++) {
                 wx.add(nx[i]);
                 wy.add(ny[i]);
                 wz.add(nz[i]);
-                n_eff++;
             }
+            dv[0] = lv[0] - wx.value() / (R)n;
+            dv[1] = lv[1] - wy.value() / (R)n;
+            dv[2] = lv[2] - wz.value() / (R)n;
         }
-        if (n_eff <= 1) continue;
-        const R lv[3] = {sx.value() / n_eff, sy.value() / n_eff, sz.value() / n_eff};
-        const R dv[3] = {lv[0] - wx.value() / n_eff, lv[1] - wy.value() / n_eff, lv[2] - wz.value() / n_eff};
-        for (long long i = a; i < a + n; i++) {
-            if (species[i] <= 0) continue;
-            if (hydro) {
-                vx[i] = nx[i] + dv[0];
-                vy[i] = ny[i] + dv[1];
-                vz[i] = nz[i] + dv[2];
-            } else {
-                vx[i] = nx[i];
-                vy[i] = ny[i];
-                vz[i] = nz[i];
-            }
+        for (int i = a; i < a + n; i++) {
+            vx[i] = w.do_cell_v ? nx[i] + dv[0] : nx[i];
+            vy[i] = w.do_cell_v ? ny[i] + dv[1] : ny[i];
+            vz[i] = w.do_cell_v ? nz[i] + dv[2] : nz[i];
+        }
+    } else {
+        double n0, n1, n2;
+        rng::sphere(q.seed, q.step, (uint32_t)s, n0, n1, n2);
+        Rot o = srd_matrix(n0, n1, n2, q.sin_a, q.cos_a);
+        for (int i = a; i < a + n; i++) {
+            R x = vx[i], y = vy[i], z = vz[i];
+            srd_rotate(x, y, z, lv, o);
+            vx[i] = x;
+            vy[i] = y;
+            vz[i] = z;
         }
     }
 }
 
-// wall_mpcd_step, src/mpcd.f90:193-337
-template <typename R>
-__global__ void k_wall_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S,
-                            int M0, int M1, int M2, int L2, R *vx, R *vy, R *vz, SrdParams q,
-                            int has_wall, double wt0, double wt1, int wn0, int wn1, int do_cell_v)
+// wall_mpcd_step, src/mpcd.f90:193-337.  kAT: the thermostat's normals come
+// from k_at_normals, which deals the rejection attempts of a whole warp to its
+// lanes; drawn inside the cell loop they took a 1.2 M particle channel (FP64)
+// 148 us, one thread per cell.
+template <typename R, bool kAT>
+__global__ void __launch_bounds__(kCellThreads)
+    k_wall_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+                const R *__restrict__ nx, const R *__restrict__ ny, const R *__restrict__ nz, SrdParams q, WallArgs w)
 {
-    int M[3] = {M0, M1, M2};
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-        int n = count[s];
-        if (n <= 1) continue;
-        int a = start[s];
-        int cell[3];
-        hilbert::compact_point(s, M, cell);
-        int wall_idx = -1;
-        if (has_wall && cell[2] + 1 == 1) wall_idx = 0;
-        else if (has_wall && cell[2] + 1 == L2) wall_idx = 1;
-        int n_virtual = 0;
-        double vv[3] = {0, 0, 0};
-        int wn = wall_idx == 0 ? wn0 : wn1;
-        if (wall_idx >= 0 && n < wn) {
-            n_virtual = wn - n;
-            for (int k = 0; k < 3; k++) vv[k] = rng::normal(q.seed, q.step, (uint32_t)s, (uint32_t)(3 + k));
-            double f = sqrt(n_virtual * (wall_idx == 0 ? wt0 : wt1));
-            for (int k = 0; k < 3; k++) vv[k] = vv[k] * f;
-        }
-        CellSum<R> sx, sy, sz;
-        for (int i = a; i < a + n; i++) {
-            sx.add(vx[i]);
-            sy.add(vy[i]);
-            sz.add(vz[i]);
-        }
-        R lv[3];
-        if (n_virtual > 0) {
-            lv[0] = (R)(((double)sx.value() + vv[0]) / wn);
-            lv[1] = (R)(((double)sy.value() + vv[1]) / wn);
-            lv[2] = (R)(((double)sz.value() + vv[2]) / wn);
-        } else {
-            lv[0] = sx.value() / n;
-            lv[1] = sy.value() / n;
-            lv[2] = sz.value() / n;
-        }
-        if (q.thermostat) {
-            CellSum<R> wx, wy, wz;
-            for (int i = a; i < a + n; i++) {
-                R nx = (R)(rng::normal(q.seed, q.step, (uint32_t)i, 0) * q.t_factor);
-                R ny = (R)(rng::normal(q.seed, q.step, (uint32_t)i, 1) * q.t_factor);
-                R nz = (R)(rng::normal(q.seed, q.step, (uint32_t)i, 2) * q.t_factor);
-                vx[i] = nx;
-                vy[i] = ny;
-                vz[i] = nz;
-                wx.add(nx);
-                wy.add(ny);
-                wz.add(nz);
-            }
-            if (do_cell_v) {
-                R dv[3] = {lv[0] - wx.value() / (R)n, lv[1] - wy.value() / (R)n, lv[2] - wz.value() / (R)n};
-                for (int i = a; i < a + n; i++) {
-                    vx[i] = vx[i] + dv[0];
-                    vy[i] = vy[i] + dv[1];
-                    vz[i] = vz[i] + dv[2];
-                }
-            }
-        } else {
-            double n0, n1, n2;
-            rng::sphere(q.seed, q.step, (uint32_t)s, n0, n1, n2);
-            Rot o = srd_matrix(n0, n1, n2, q.sin_a, q.cos_a);
-            for (int i = a; i < a + n; i++) {
-                R x = vx[i], y = vy[i], z = vz[i];
-                srd_rotate(x, y, z, lv, o);
-                vx[i] = x;
-                vy[i] = y;
-                vz[i] = z;
-            }
-        }
+    __shared__ R sv[kAT ? 6 : 3][kCellCap];
+    const CellRange c(count, start, S);
+    const int slot = blockIdx.x * kCellTile + (int)threadIdx.x;
+    if (c.np > kCellCap) {
+        wall_cell<R>(c.n, c.a, slot, vx, vy, vz, nx, ny, nz, q, w);
+        return;
     }
+    if constexpr (kAT) tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, c.a0, c.np);
+    else tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
+    __syncthreads();
+    wall_cell<R>(c.n, c.a - c.a0, slot, sv[0], sv[1], sv[2], sv[kAT ? 3 : 0], sv[kAT ? 4 : 1], sv[kAT ? 5 : 2], q, w);
+    __syncthreads();
+    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
 
 constexpr int kRedBlocks = 1024;
 
-// compute_temperature, src/mpcd.f90:342-407: per-block partial (te, count),
-// then a fixed-order final sum
+// compute_temperature, src/mpcd.f90:342-407, of the n particles from a: the
+// cell's contribution to the sum of temperatures (0 for cells that add none)
 template <typename R>
-__global__ void k_temperature(const int *__restrict__ count, const int *__restrict__ start, int S,
-                              const R *vx, const R *vy, const R *vz, const int *__restrict__ species,
-                              double *part)
+__device__ __forceinline__ double cell_temperature(int n, int a, const R *vx, const R *vy, const R *vz,
+                                                   const int *species)
 {
-    double te = 0, cnt = 0;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-        int n = count[s];
-        if (n <= 1) continue;
-        int a = start[s];
-        cnt += 1;
-        int n_eff = 0;
-        CellSum<R> sx, sy, sz;
-        for (int i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                sx.add(vx[i]);
-                sy.add(vy[i]);
-                sz.add(vz[i]);
-                n_eff++;
-            }
+    if (n <= 1) return 0;
+    int n_eff = 0;
+    CellSum<R> sx, sy, sz;
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            sx.add(vx[i]);
+            sy.add(vy[i]);
+            sz.add(vz[i]);
+            n_eff++;
         }
-        if (n_eff <= 1) continue;
-        // local_v = local_v / n  (divides by n, not n_effective, as written)
-        double l0 = (double)(sx.value() / (R)n), l1 = (double)(sy.value() / (R)n),
-               l2 = (double)(sz.value() / (R)n);
-        double kin = 0;
-        for (int i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                double d0 = (double)vx[i] - l0, d1 = (double)vy[i] - l1, d2 = (double)vz[i] - l2;
-                kin = kin + (d0 * d0 + d1 * d1 + d2 * d2);
-            }
-        }
-        kin = kin / (double)(3 * (n_eff - 1));
-        te = te + kin;
     }
-    __shared__ double ste[256], sc[256];
-    ste[threadIdx.x] = te;
-    sc[threadIdx.x] = cnt;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            ste[threadIdx.x] += ste[threadIdx.x + o];
-            sc[threadIdx.x] += sc[threadIdx.x + o];
+    if (n_eff <= 1) return 0;
+    // local_v = local_v / n  (divides by n, not n_effective, as written)
+    double l0 = (double)(sx.value() / (R)n), l1 = (double)(sy.value() / (R)n), l2 = (double)(sz.value() / (R)n);
+    double kin = 0;
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            double d0 = (double)vx[i] - l0, d1 = (double)vy[i] - l1, d2 = (double)vz[i] - l2;
+            kin = kin + (d0 * d0 + d1 * d1 + d2 * d2);
         }
+    }
+    return kin / (double)(3 * (n_eff - 1));
+}
+
+// per-block partial sums (te, count) over the cells of one tile, for the
+// fixed-order sum of k_temperature_final
+template <typename R>
+__global__ void __launch_bounds__(kCellThreads)
+    k_temperature(const int *__restrict__ count, const int *__restrict__ start, int S, const R *vx, const R *vy,
+                  const R *vz, const int *__restrict__ species, double *part)
+{
+    __shared__ R sv[3][kCellCap];
+    __shared__ int ss[1][kCellCap];
+    const CellRange c(count, start, S);
+    double te;
+    if (c.np > kCellCap) {
+        te = cell_temperature<R>(c.n, c.a, vx, vy, vz, species);
+    } else {
+        tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
+        tile_in<int, 1>(ss, {species}, c.a0, c.np);
         __syncthreads();
+        te = cell_temperature<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0]);
     }
+    // kCellTile = 64 slots: two warps hold values
+    __shared__ double s_te[2];
+    double cnt = c.n > 1 ? 1 : 0;
+    for (int o = 16; o > 0; o >>= 1) {
+        te += __shfl_xor_sync(0xffffffffu, te, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    __shared__ double s_cnt[2];
+    if ((threadIdx.x & 31) == 0 && threadIdx.x < kCellTile) {
+        s_te[threadIdx.x >> 5] = te;
+        s_cnt[threadIdx.x >> 5] = cnt;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-        part[2 * blockIdx.x] = ste[0];
-        part[2 * blockIdx.x + 1] = sc[0];
+        part[2 * (size_t)blockIdx.x] = s_te[0] + s_te[1];
+        part[2 * (size_t)blockIdx.x + 1] = s_cnt[0] + s_cnt[1];
     }
 }
 
-__global__ void k_temperature_final(const double *part, int nb, double *out)
+// one block: the partials by a fixed tree (thread t adds t, t + 1024, ...)
+__global__ void __launch_bounds__(1024) k_temperature_final(const double *part, int nb, double *out)
 {
-    if (threadIdx.x == 0) {
-        double te = 0, cnt = 0;
-        for (int b = 0; b < nb; b++) {
-            te = te + part[2 * b];
-            cnt = cnt + part[2 * b + 1];
+    __shared__ double ste[32], sc[32];
+    double te = 0, cnt = 0;
+    for (int b = threadIdx.x; b < nb; b += 1024) {
+        te += part[2 * (size_t)b];
+        cnt += part[2 * (size_t)b + 1];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        te += __shfl_xor_sync(0xffffffffu, te, o);
+        cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        ste[threadIdx.x >> 5] = te;
+        sc[threadIdx.x >> 5] = cnt;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        te = ste[threadIdx.x];
+        cnt = sc[threadIdx.x];
+        for (int o = 16; o > 0; o >>= 1) {
+            te += __shfl_xor_sync(0xffffffffu, te, o);
+            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
         }
-        out[0] = te / cnt;
+        if (threadIdx.x == 0) out[0] = te / cnt;
     }
 }
 
-// rescale_cells, src/mpcd.f90:748-801
+// rescale_cells, src/mpcd.f90:748-801, of the n particles from a
 template <typename R>
-__global__ void k_rescale(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx,
-                          R *vy, R *vz, const int *__restrict__ species, double T)
+__device__ __forceinline__ void rescale_cell(int n, int a, R *vx, R *vy, R *vz, const int *species, double T)
 {
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
-        int n = count[s];
-        if (n <= 1) continue;
-        int a = start[s];
-        int n_eff = 0;
-        CellSum<R> sx, sy, sz;
-        for (int i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                sx.add(vx[i]);
-                sy.add(vy[i]);
-                sz.add(vz[i]);
-                n_eff++;
-            }
-        }
-        if (n_eff <= 1) continue;
-        R lv[3] = {sx.value() / n_eff, sy.value() / n_eff, sz.value() / n_eff};
-        double kin = 0;
-        for (int i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                double d0 = (double)(vx[i] - lv[0]), d1 = (double)(vy[i] - lv[1]),
-                       d2 = (double)(vz[i] - lv[2]);
-                kin = kin + (d0 * d0 + d1 * d1 + d2 * d2);
-            }
-        }
-        R tf = (R)sqrt((3 * (n_eff - 1)) * T / kin);
-        for (int i = a; i < a + n; i++) {
-            if (species[i] > 0) {
-                vx[i] = lv[0] + tf * (vx[i] - lv[0]);
-                vy[i] = lv[1] + tf * (vy[i] - lv[1]);
-                vz[i] = lv[2] + tf * (vz[i] - lv[2]);
-            }
+    if (n <= 1) return;
+    int n_eff = 0;
+    CellSum<R> sx, sy, sz;
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            sx.add(vx[i]);
+            sy.add(vy[i]);
+            sz.add(vz[i]);
+            n_eff++;
         }
     }
+    if (n_eff <= 1) return;
+    R lv[3] = {sx.value() / n_eff, sy.value() / n_eff, sz.value() / n_eff};
+    double kin = 0;
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            double d0 = (double)(vx[i] - lv[0]), d1 = (double)(vy[i] - lv[1]), d2 = (double)(vz[i] - lv[2]);
+            kin = kin + (d0 * d0 + d1 * d1 + d2 * d2);
+        }
+    }
+    R tf = (R)sqrt((3 * (n_eff - 1)) * T / kin);
+    for (int i = a; i < a + n; i++) {
+        if (species[i] > 0) {
+            vx[i] = lv[0] + tf * (vx[i] - lv[0]);
+            vy[i] = lv[1] + tf * (vy[i] - lv[1]);
+            vz[i] = lv[2] + tf * (vz[i] - lv[2]);
+        }
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(kCellThreads)
+    k_rescale(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+              const int *__restrict__ species, double T)
+{
+    __shared__ R sv[3][kCellCap];
+    __shared__ int ss[1][kCellCap];
+    const CellRange c(count, start, S);
+    if (c.np > kCellCap) {
+        rescale_cell<R>(c.n, c.a, vx, vy, vz, species, T);
+        return;
+    }
+    tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
+    tile_in<int, 1>(ss, {species}, c.a0, c.np);
+    __syncthreads();
+    rescale_cell<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0], T);
+    __syncthreads();
+    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
 
 // mpcd_stream_periodic, src/mpcd.f90:440-457
@@ -558,6 +709,26 @@ static SrdParams srd_params(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, in
     return q;
 }
 
+static int at_blocks(long long N) { return grid_full((N + 32 * kAtChunks - 1) / (32 * kAtChunks) * 32, kAtThreads); }
+
+// with the thermostat, the normals go into the sort target's velocity arrays
+// (free between sorts) first
+template <typename R>
+static void wall_launches(rmpcd_particles *p, rmpcd_cells *c, const SrdParams &q, const WallArgs &w)
+{
+    cudaStream_t s = stream();
+    const int g = cell_blocks(c->S);
+    PView<R> v = cur<R>(p), t = alt<R>(p);
+    if (q.thermostat && p->N > 0) {
+        k_at_normals<R><<<at_blocks(p->N), kAtThreads, 0, s>>>(nullptr, p->N, q, t.vel.x, t.vel.y, t.vel.z);
+        k_wall_mpcd<R, true><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, t.vel.x,
+                                                       t.vel.y, t.vel.z, q, w);
+    } else {
+        k_wall_mpcd<R, false><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, nullptr,
+                                                        nullptr, nullptr, q, w);
+    }
+}
+
 }  // namespace rmpcd
 
 using namespace rmpcd;
@@ -582,26 +753,26 @@ int rmpcd_simple_mpcd_step(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, int
     PhaseTimer t("step");
     SrdParams q = srd_params(p, c, r, has_alpha, alpha, thermostat, T, hydro);
     cudaStream_t s = stream();
-    int g = grid_full(c->S, 128);
+    const int g = cell_blocks(c->S);
     if (thermostat && !q.gauss && p->N > 0) {
         // the normals first, into the sort target's velocity arrays (free
         // between sorts), then the cells
-        const int gn = grid_full(((long long)p->N + 32 * kAtChunks - 1) / (32 * kAtChunks) * 32, kAtThreads);
+        const int gn = at_blocks(p->N);
         DISPATCH_R(p,
                    ({ PView<float> v = cur<float>(p), t = alt<float>(p);
                       k_at_normals<float><<<gn, kAtThreads, 0, s>>>(v.species, p->N, q, t.vel.x, t.vel.y, t.vel.z);
-                      k_at_cells<float><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
+                      k_at_cells<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
                                                           v.species, q.hydro, t.vel.x, t.vel.y, t.vel.z); }),
                    ({ PView<double> v = cur<double>(p), t = alt<double>(p);
                       k_at_normals<double><<<gn, kAtThreads, 0, s>>>(v.species, p->N, q, t.vel.x, t.vel.y, t.vel.z);
-                      k_at_cells<double><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
+                      k_at_cells<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
                                                            v.species, q.hydro, t.vel.x, t.vel.y, t.vel.z); }));
     } else {
         DISPATCH_R(p,
                    ({ PView<float> v = cur<float>(p);
-                      k_simple_mpcd<float><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }),
+                      k_simple_mpcd<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }),
                    ({ PView<double> v = cur<double>(p);
-                      k_simple_mpcd<double><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }));
+                      k_simple_mpcd<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }));
     }
     RMPCD_CHECK_LAUNCH();
     r->step++;
@@ -621,18 +792,11 @@ int rmpcd_wall_mpcd_step(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r,
     if (!keep_cell_v && !thermostat)
         return fail(RMPCD_ERR_STOP, "requiring .not. keep_cell_v and .not. thermostat in wall_mpcd_step");
     SrdParams q = srd_params(p, c, r, has_alpha, alpha, thermostat, bulk_temperature, 1);
-    double wt0 = all_present ? wall_temperature[0] : 0, wt1 = all_present ? wall_temperature[1] : 0;
-    int wn0 = all_present ? wall_n[0] : 0, wn1 = all_present ? wall_n[1] : 0;
-    cudaStream_t s = stream();
-    int g = grid_full(c->S, 128);
+    const WallArgs w{c->M[0], c->M[1], c->M[2], c->L[2], all_present ? 1 : 0, all_present ? wall_temperature[0] : 0,
+                     all_present ? wall_temperature[1] : 0, all_present ? wall_n[0] : 0, all_present ? wall_n[1] : 0,
+                     keep_cell_v ? 1 : 0};
     PhaseTimer t("step");
-    DISPATCH_R(p,
-               ({ PView<float> v = cur<float>(p);
-                  k_wall_mpcd<float><<<g, 128, 0, s>>>(c->count, c->start, c->S, c->M[0], c->M[1], c->M[2], c->L[2],
-                                                       v.vel.x, v.vel.y, v.vel.z, q, all_present, wt0, wt1, wn0, wn1, keep_cell_v ? 1 : 0); }),
-               ({ PView<double> v = cur<double>(p);
-                  k_wall_mpcd<double><<<g, 128, 0, s>>>(c->count, c->start, c->S, c->M[0], c->M[1], c->M[2], c->L[2],
-                                                        v.vel.x, v.vel.y, v.vel.z, q, all_present, wt0, wt1, wn0, wn1, keep_cell_v ? 1 : 0); }));
+    DISPATCH_R(p, wall_launches<float>(p, c, q, w), wall_launches<double>(p, c, q, w));
     RMPCD_CHECK_LAUNCH();
     r->step++;
     return RMPCD_OK;
@@ -643,15 +807,18 @@ int rmpcd_compute_temperature(rmpcd_particles *p, rmpcd_cells *c, double *te)
     RMPCD_ARG(p && c && te, "null argument");
     PhaseTimer t("compute_temperature");
     cudaStream_t s = stream();
-    double *part = c->d_red;
+    // two doubles per tile of slots, in the slots' scatter cursors (rewritten by
+    // the next count_particles or sort before they are read)
+    double *part = (double *)c->cursor, *out = c->d_red;
+    const int nb = cell_blocks(c->S);
     DISPATCH_R(p,
                ({ PView<float> v = cur<float>(p);
-                  k_temperature<float><<<kRedBlocks, 256, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }),
+                  k_temperature<float><<<nb, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }),
                ({ PView<double> v = cur<double>(p);
-                  k_temperature<double><<<kRedBlocks, 256, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }));
-    k_temperature_final<<<1, 32, 0, s>>>(part, kRedBlocks, part + 2 * kRedBlocks);
+                  k_temperature<double><<<nb, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }));
+    k_temperature_final<<<1, 1024, 0, s>>>(part, nb, out);
     RMPCD_CHECK_LAUNCH();
-    RMPCD_CUDA_TRY(cudaMemcpyAsync(te, part + 2 * kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, s));
+    RMPCD_CUDA_TRY(cudaMemcpyAsync(te, out, sizeof(double), cudaMemcpyDeviceToHost, s));
     return sync();
 }
 
@@ -660,12 +827,12 @@ int rmpcd_rescale_cells(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *, double 
     RMPCD_ARG(p && c, "null argument");
     PhaseTimer t("step");
     cudaStream_t s = stream();
-    int g = grid_full(c->S, 128);
+    const int g = cell_blocks(c->S);
     DISPATCH_R(p,
                ({ PView<float> v = cur<float>(p);
-                  k_rescale<float><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }),
+                  k_rescale<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }),
                ({ PView<double> v = cur<double>(p);
-                  k_rescale<double><<<g, 128, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }));
+                  k_rescale<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }));
     RMPCD_CHECK_LAUNCH();
     return RMPCD_OK;
 }

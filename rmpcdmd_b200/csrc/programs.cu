@@ -115,13 +115,21 @@ __global__ void k_vel_sums(PView<R> v, double *part)
         for (int k = 0; k < 4; k++) part[4 * blockIdx.x + k] = sh[k][0];
 }
 
-__global__ void k_vel_sums_final(const double *part, int nb, double *out)
+// one block: component k's partials by a fixed tree in warps 8k .. 8k + 7
+__global__ void __launch_bounds__(1024) k_vel_sums_final(const double *part, int nb, double *out)
 {
-    if (threadIdx.x != 0) return;
-    double a[4] = {0, 0, 0, 0};
-    for (int b = 0; b < nb; b++)
-        for (int k = 0; k < 4; k++) a[k] = a[k] + part[4 * b + k];
-    for (int k = 0; k < 4; k++) out[k] = a[k];
+    __shared__ double sh[32];
+    const int k = threadIdx.x >> 8, t = threadIdx.x & 255;
+    double a = 0;
+    for (int b = t; b < nb; b += 256) a += part[4 * b + k];
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
+    __syncthreads();
+    if (t == 0) {
+        double r = 0;
+        for (int w = 0; w < 8; w++) r += sh[8 * k + w];
+        out[k] = r;
+    }
 }
 
 }  // namespace rmpcd
@@ -254,7 +262,7 @@ int rmpcd_velocity_sums(rmpcd_particles *p, double out[4])
     if (p->N > 0) {
         DISPATCH_R(p, (k_vel_sums<float><<<nb, 256, 0, stream()>>>(cur<float>(p), part)),
                    (k_vel_sums<double><<<nb, 256, 0, stream()>>>(cur<double>(p), part)));
-        k_vel_sums_final<<<1, 32, 0, stream()>>>(part, nb, part + 4 * nb);
+        k_vel_sums_final<<<1, 1024, 0, stream()>>>(part, nb, part + 4 * nb);
         RMPCD_CHECK_LAUNCH();
         RMPCD_CUDA_TRY(cudaMemcpyAsync(out, part + 4 * nb, 4 * sizeof(double), cudaMemcpyDeviceToHost, stream()));
         return sync();
