@@ -493,22 +493,23 @@ int rmpcd_dimer_batch_scatter(rmpcd_dimer_batch *batch, int replica, rmpcd_parti
  * (the program's n_extra_sorting; array of n_replicas, may be NULL) */
 int rmpcd_dimer_batch_info(const rmpcd_dimer_batch *batch, int *n_replicas, long long *n_solvent,
                            int *n_extra_sorting);
-/* Engine shapes (no counterpart in the reference): particles per tile of
- * the solvent kernels, particles per thread and pass of the MD step's
- * begin / end halves, the blocks per SM they are compiled for, the list
- * entries per thread of the list kernels (pair forces, their application,
- * the contribution reset), and whether the colloid half of the step begin
- * runs in an extra first block while the solvent streams (1) or in the block
- * that finishes last (0).  Every shape gives the same results
- * bit for bit.  A batch starts on 1024-particle tiles (smaller when that
- * gives fewer than ~2 tiles per SM) and one list entry per thread. */
+/* Engine shapes (no counterpart in the reference): particles per tile of the
+ * sort's particle kernels, the blocks that run a replica's MD steps
+ * (blocks_per_sm; 0: chosen by the number of replicas, one block per SM), the
+ * solvent particles of the MD steps that each of their threads keeps in
+ * registers (per_thread_begin = per_thread_end), the list entries per thread
+ * of the kernels that list those particles, and colloid_block_first = 1 (the
+ * colloids' turn belongs to a replica's first block).  Every shape gives the
+ * same results bit for bit.  A batch starts on 1024-particle tiles (smaller
+ * when that gives fewer than ~2 tiles per SM), blocks by the number of
+ * replicas and one list entry per thread. */
 int rmpcd_dimer_batch_shapes(int precision, int *n_shapes);
 int rmpcd_dimer_batch_shape_info(int precision, int shape, int *particles_per_tile, int *per_thread_begin,
                                  int *per_thread_end, int *blocks_per_sm, int *list_entries_per_thread,
                                  int *colloid_block_first);
 int rmpcd_dimer_batch_set_shape(rmpcd_dimer_batch *batch, int shape);
 int rmpcd_dimer_batch_get_shape(const rmpcd_dimer_batch *batch, int *shape);
-/* The engine's autotuner: every tile size and kernel variant with one list
+/* The engine's autotuner: every tile size and block count with one list
  * entry per thread, then the fastest of them with each other list setting,
  * runs one interval (capture and warm-up) and n_intervals timed intervals of
  * the batch itself -- real intervals of the run, since every shape gives the

@@ -8,23 +8,39 @@
 // Hilbert order stays inside its own range, so the sort kernels of a single
 // system apply to every replica at once.
 //
-// One MD step is three kernels plus a conditional re-sort: the step-begin
-// kernel (md_pos, flag roll, displacement; its last block runs every
-// replica's colloid half and the program's re-sort test,
-// programs/single_dimer_pbc.f90:306-330), the pair-force kernel, the kernel
-// applying the pair forces, and the step-end kernel (md_vel, change_species,
-// colloid velocity half).  The re-sort is decided on the device: one flag per
-// replica, and in a captured graph an IF node whose body (the re-sort
-// kernels, which skip the tiles of unflagged replicas) runs only when some
-// replica needs it.  The re-sort gathers into the alternate buffers and
-// copies back, so the arrays never change place and a whole interval (N_MD MD
-// steps + shift + sort + collision + refuel) is captured once and replayed:
-// the RNG step and the grid origins are read from device memory, never baked
-// into the graph.
+// MD steps touch only the solvent that can interact.  A particle that is in
+// neither bead's neighbor list and carries no MD, PAST_MD, REAC or WALL flag
+// flies freely until the next re-sort: no force can reach it before the list
+// is rebuilt, so its md_pos steps depend on nothing but its own position and
+// velocity.  Such particles stay where they are in memory; the re-sort (or the
+// interval's end) advances each by its pending md_pos steps in one pass, adding
+// dt * v once per step so that every rounding is that of the steps one by one.
+// The others -- the active particles, ~6,000 per dimer at sigma = 2 -- are
+// advanced by kb_md, one thread-block cluster per replica, which runs the MD
+// steps one after another without leaving the kernel: pair forces, md_vel,
+// change_species, the colloid sums, velocity-Verlet and RATTLE, the next
+// step's md_pos, until the program's re-sort test
+// (programs/single_dimer_pbc.f90:323-330) fires or the interval's MD steps are
+// done.  The test needs the largest solvent displacement: of the active
+// particles the cluster has it, of the free ones kb_classify has computed the
+// first step at which any of them reaches the threshold, by the same additions
+// and the same comparison.  Replicas re-sort at steps of their own: a launch of
+// kb_md ends when each of its replicas waits for a re-sort or is done, then one
+// re-sort serves all that wait (a WHILE node of the captured interval graph).
+// The re-sort gathers into the other buffer of the particle system; which one
+// is current is kept per replica on the device (BRep::cur), as are the RNG
+// step and the grid origins, so one captured interval graph serves every
+// interval.
+//
+// Moving every particle in every MD step costs 56 B (FP32) per particle and
+// step: 121 us per step at 96^3 (4.1 TB/s) and 237 us for 48 replicas in boxes
+// of 16..48 cells, against 5 us per step for kb_md.
 //
 // Arithmetic per particle is that of the single-system kernels
 // (stepops.cuh, nlist_ops.cuh), so replica r reproduces, bit for bit, the
 // same program run alone through the C ABI with its own seed.
+#include <cooperative_groups.h>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -47,44 +63,22 @@ namespace rmpcd {
 constexpr int kTile = 1024;  // slots per slot tile
 constexpr int kBT = 256;     // threads per tile block
 
-// Engine shapes (rmpcd_dimer_batch_autotune): the particles a thread of the
-// step-begin / step-end kernel handles per pass, the blocks per SM they are
-// compiled for, and (at run time) the particles per tile.  Every shape gives
-// the same results bit for bit: tiles and passes only decide which thread
-// handles which particle, and every per-particle result, the maximum
-// displacement and the re-sort decision are independent of that.
-template <int KB_, int KE_, int MINB_, int FIRST_>
-struct BVar {
-    static constexpr int KB = KB_;      // particles per thread and pass, step begin
-    static constexpr int KE = KE_;      // the same, step end
-    static constexpr int MINB = MINB_;  // resident blocks per SM (launch bound)
-    // the colloid half of the step begin in an extra block 0 that runs while
-    // the solvent streams (1), or in the block that finishes last (0)
-    static constexpr bool FIRST = FIRST_ != 0;
-};
-template <typename R, int V>
-struct BVarOf;
-template <> struct BVarOf<float, 0> { using T = BVar<4, 4, 4, 0>; };
-template <> struct BVarOf<float, 1> { using T = BVar<2, 4, 4, 0>; };
-template <> struct BVarOf<float, 2> { using T = BVar<4, 2, 4, 0>; };
-template <> struct BVarOf<float, 3> { using T = BVar<4, 16, 4, 0>; };
-template <> struct BVarOf<float, 4> { using T = BVar<4, 4, 4, 1>; };
-template <> struct BVarOf<double, 0> { using T = BVar<2, 4, 4, 1>; };
-template <> struct BVarOf<double, 1> { using T = BVar<1, 4, 4, 1>; };
-template <> struct BVarOf<double, 2> { using T = BVar<2, 2, 4, 1>; };
-template <> struct BVarOf<double, 3> { using T = BVar<2, 8, 4, 1>; };
-template <> struct BVarOf<double, 4> { using T = BVar<2, 4, 4, 0>; };
+// Engine shapes (rmpcd_dimer_batch_autotune): the particles per tile of the
+// sort's particle kernels, the blocks a replica's MD steps run on (the cluster
+// of kb_md; 0: chosen by the number of replicas) and the list entries per
+// thread of the kernels that make the active list.  Every shape gives the same
+// results bit for bit: they only decide which thread handles which particle.
+constexpr int kClusters[] = {0, 8, 4, 2, 1};
 constexpr int kBVars = 5;
 constexpr long long kPTiles[] = {256, 512, 1024, 2048, 4096};  // particles per tile
 constexpr int kNPTiles = 5;
-// list entries per thread of the list kernels (pair forces, their
-// application, the contribution reset): their blocks per colloid are
-// ceil(capacity / (256 x this)), at most 64
+// list entries per thread: blocks per colloid are ceil(capacity / (256 x
+// this)), at most 64
 constexpr int kListPer[] = {1, 4};
 constexpr int kNListPer = 2;
 constexpr int kBShapes = kNListPer * kBVars * kNPTiles;
-// shape s: particle tile kPTiles[s % kNPTiles], kernel variant
-// (s / kNPTiles) % kBVars, list entries per thread kListPer[s / (kNPTiles * kBVars)]
+// shape s: particle tile kPTiles[s % kNPTiles], cluster kClusters[(s /
+// kNPTiles) % kBVars], list entries per thread kListPer[s / (kNPTiles * kBVars)]
 __host__ __device__ inline int shape_tile(int s) { return s % kNPTiles; }
 __host__ __device__ inline int shape_var(int s) { return (s / kNPTiles) % kBVars; }
 __host__ __device__ inline int shape_list(int s) { return s / (kNPTiles * kBVars); }
@@ -101,7 +95,7 @@ struct BRep {
     int n;          // its solvent particles
     int soff;       // first slot
     int S;          // its slots
-    int serial;     // the list stencil wraps this box: ordered single-thread force application
+    int cur;        // buffer holding the replica's current solvent arrays
     uint64_t seed;
     double far;     // refuel distance (single-precision expression of the program)
     Grid g;         // cells; origin rewritten on the device by the grid shift
@@ -135,12 +129,19 @@ struct rmpcd_dimer_batch {
     int n_stencil = 0;
     int Nmax = 0;
     int *list = nullptr, *nn = nullptr;
-    double *pair_f = nullptr, *pair_e = nullptr;
-    unsigned char *contrib = nullptr;
-    int *ncontrib = nullptr, *max_contrib = nullptr, *clist = nullptr, *cn = nullptr;
-    unsigned long long *so_max = nullptr;
-    double *co_max = nullptr;  // per replica: the colloids' displacement of this MD step
-    double *csnap = nullptr;   // colloid positions at the step's force evaluation, 3 per colloid
+    // active particles (kb_claim, kb_classify), in the replica's range of act:
+    // nl[r] of the neighbor lists first, then nx[r] flagged ones outside them
+    int *act = nullptr, *nl = nullptr, *nx = nullptr;
+    int *aidx = nullptr;       // per particle: its place in act, -1 when it flies freely
+    int *amap = nullptr;       // per list entry: the place in act of its particle
+    int *mult = nullptr;       // per listed active particle: entries in list 0 | entries in list 1 << 16
+    double *pf = nullptr;      // per listed active particle: pair forces from beads 0 and 1 (6 doubles)
+    unsigned char *cf = nullptr;  // ... and which of the two act on it (particles beyond kb_md's shared flags)
+    int *nf = nullptr;         // per replica: flagged particles, listed in sol->key from the replica's first place
+    int *s_free = nullptr;     // per replica: first MD step at which a free particle forces a re-sort
+    int *adv = nullptr, *base = nullptr;  // per replica: md_pos steps done this interval, and those in memory
+    int *fresh = nullptr;      // per replica: pos_old is the caller's (no sort yet)
+    bool ran = false;          // an interval has been run
     // whether some solvent species was negative at creation; species change
     // only to 1 or 2 inside the batch, so otherwise every particle passes
     // maximum_displacement's species >= 0 test and species need not be read
@@ -152,17 +153,13 @@ struct rmpcd_dimer_batch {
     uint64_t step = 0;  // host copy of every replica's RNG step
     rmpcd::Masses ms{};
     rmpcd::LJDev lj_sc{}, lj_cc{};
-    int parity = 0;  // 0: force = buffer force[0], force_old = force_old[0]; swapped by each MD step
-    unsigned *done = nullptr;   // blocks finished in the current step kernel (last-block hand-off)
+    unsigned *done = nullptr;   // replicas finished in the current kb_md launch (last-block hand-off)
     bool use_graph = true;
     bool capturing = false;
     cudaError_t cap_err = cudaSuccess;
-    cudaStream_t body = nullptr;  // captures the bodies of the re-sort IF nodes
-    cudaGraphConditionalHandle cond_next = 0;  // re-sort condition of the next MD step, while capturing
-    cudaStream_t side = nullptr;   // captures the speculative force branch beside each re-sort IF node
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    int *any = nullptr;  // 1 when the last MD-step beginning decided to re-sort some replica
-    cudaGraphExec_t exec[2] = {nullptr, nullptr};
+    cudaStream_t body = nullptr;  // captures the body of the re-sort WHILE node
+    int *any = nullptr;  // 1 when the last kb_md launch left some replica waiting for a re-sort
+    cudaGraphExec_t exec = nullptr;
 };
 
 namespace rmpcd {
@@ -175,34 +172,11 @@ static PView<R> phys(const rmpcd_particles *p, int b)
     return view<R>(p, b);
 }
 
-// current arrays with force / force_old as the MD-step parity says
+// buffer 0 or 1
 template <typename R>
-static PView<R> live(const rmpcd_particles *p, int parity)
+__device__ __forceinline__ PView<R> pick(const PView<R> &v0, const PView<R> &v1, int which)
 {
-    PView<R> v = view<R>(p, 0);
-    if (parity) {
-        Vec3<R> t = v.force;
-        v.force = v.force_old;
-        v.force_old = t;
-    }
-    return v;
-}
-
-template <typename R>
-__device__ inline PView<R> shifted(PView<R> v, long long off, int n)
-{
-    v.N = n;
-    v.pos = {v.pos.x + off, v.pos.y + off, v.pos.z + off};
-    v.vel = {v.vel.x + off, v.vel.y + off, v.vel.z + off};
-    v.force = {v.force.x + off, v.force.y + off, v.force.z + off};
-    v.force_old = {v.force_old.x + off, v.force_old.y + off, v.force_old.z + off};
-    v.ix += off;
-    v.iy += off;
-    v.iz += off;
-    v.id += off;
-    v.species += off;
-    v.flags += off;
-    return v;
+    return which ? v1 : v0;
 }
 
 // the tiles a re-sort kernel visits: tiles[ids[k]] for k < *n (every tile
@@ -216,96 +190,25 @@ struct TileSet {
 // ------------------------------------------------------------ MD step
 //
 // Force entries that can be non-zero are known from the flags: MD set means
-// the particle received a contribution in the last force evaluation (its
-// `force` entry), PAST_MD in the one before (`force_old`).  Every other entry
-// is exactly zero, so the MD-step kernels neither read nor clear it; the
-// arithmetic uses a zero in its place and stays that of md_pos / md_vel.
+// the particle received a contribution in the last force evaluation, PAST_MD
+// in the one before.  Every other entry is exactly zero.  In memory `force` is
+// the last evaluation's force of particles with MD or PAST_MD set and zero
+// elsewhere; `force_old` is written by an interval's last MD step only.
+
+constexpr int kActiveBits = (1 << WALL_BIT) | (1 << MD_BIT) | (1 << PAST_MD_BIT) | (1 << REAC_BIT);
 
 __device__ inline bool same_bits(float a, float b) { return __float_as_int(a) == __float_as_int(b); }
 __device__ inline bool same_bits(double a, double b) { return __double_as_longlong(a) == __double_as_longlong(b); }
 
+// md_vel of a particle without force turns a -0 velocity component into +0 in
+// the FP64 form, as the reference's does; the FP32 form leaves such
+// velocities untouched (a -0 component, which an SRD rotation product can
+// round to, stays: equal in value, not in bits)
 template <typename R>
-__device__ inline R flagged(const R *a, long long i, bool set)
+__device__ __forceinline__ R md_vel_free(R v, R dt)
 {
-    return set ? a[i] : (R)0;
-}
-
-// colloid position half, RATTLE and colloid displacement of replica r
-// (programs/single_dimer_pbc.f90:311-322); clears the colloid force entries
-// that become `force` after switch_force; returns the displacement.  Touches
-// no solvent data.
-__device__ inline double colloid_begin(int r, const BRep *rep, const PView<double> &c, const Vec3<double> &cold,
-                                       const Vec3<double> &c_next, double *const rat[3], const double *mass,
-                                       const Masses &ms, double d, double dt, unsigned *err)
-{
-    PView<double> cr = shifted(c, 2 * (long long)r, 2);
-    for (int k = 0; k < 2; k++) {
-        rat[0][2 * r + k] = cr.pos.x[k];
-        rat[1][2 * r + k] = cr.pos.y[k];
-        rat[2][2 * r + k] = cr.pos.z[k];
-    }
-    colloid_vv_pos_one(cr, 0, mass[2 * r], dt);
-    colloid_vv_pos_one(cr, 1, mass[2 * r + 1], dt);
-    E3 L{{rep[r].g.edges[0], rep[r].g.edges[1], rep[r].g.edges[2]}};
-    rattle_pos_dimer(cr, rat[0] + 2 * r, rat[1] + 2 * r, rat[2] + 2 * r, ms, d, dt, L, err);
-    Vec3<double> o = {cold.x + 2 * r, cold.y + 2 * r, cold.z + 2 * r};
-    double m0 = disp_sq_one(cr.pos, o, cr.species, 0), m1 = disp_sq_one(cr.pos, o, cr.species, 1);
-    for (int k = 2 * r; k < 2 * r + 2; k++) c_next.x[k] = c_next.y[k] = c_next.z[k] = 0;
-    return sqrt(m0 > m1 ? m0 : m1);
-}
-
-// the re-sort decision of replica r (programs/single_dimer_pbc.f90:323-330),
-// given its colloid displacement co, once the solvent's maximum displacement
-// of the step is complete
-__device__ inline int resort_decision(int r, double skin, double co, unsigned long long *so_max, int *resort,
-                                      int *n_extra)
-{
-    double so = sqrt(__longlong_as_double((long long)__ldcg(so_max + r)));
-    int need = (co >= skin * 0.1) || (so >= skin * 0.89);
-    resort[r] = need;
-    if (need) n_extra[r] += 1;
-    so_max[r] = 0;
-    return need;
-}
-
-struct ColloidStep {
-    PView<double> c;       // colloids, force/force_old of this step
-    Vec3<double> cold;     // colloid pos_old
-    Vec3<double> c_next;   // colloid force entries cleared for the next evaluation
-    double *rat[3];        // pos_rattle
-    const double *mass;    // velocity-Verlet masses, 2 per replica
-    Masses ms;
-    double d, dt, skin;
-    int R;
-    double *co_max;        // per replica: the colloids' displacement of this step
-};
-
-// exclusive block scan of one int per thread; *total gets the block's sum
-// (ws: kBT / 32 + 1 ints of shared memory)
-__device__ inline int block_excl_scan(int v, int *ws, int *total)
-{
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int inc = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) ws[w] = inc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int k = 0; k < kBT / 32; k++) {
-            int y = ws[k];
-            ws[k] = acc;
-            acc += y;
-        }
-        ws[kBT / 32] = acc;
-    }
-    __syncthreads();
-    int ex = ws[w] + inc - v;
-    *total = ws[kBT / 32];
-    __syncthreads();
-    return ex;
+    const R z = 0;
+    return sizeof(R) == 8 ? v + dt * (z + z) / 2 : v;
 }
 
 // the tile lists of the replicas flagged for a re-sort
@@ -315,499 +218,752 @@ struct ResortLists {
     int *n;                                        // out: n[0] particle tiles, n[1] slot tiles
 };
 
-// md_pos over the particle tile t (the solvent half of the MD step's
-// beginning): returns this thread's largest squared displacement from pos_old
-// among particles of species >= 0.  K particles per thread and pass, all
-// loads issued before any use.
-template <typename R, int K>
-__device__ __forceinline__ double begin_tile(const BTile &t, const PView<R> &v, const Vec3<R> &old,
-                                             const Vec3<R> &next, R dt, R dt_sq, int read_species)
+// exclusive block scan of one int per thread (blocks of up to 1024 threads, a
+// multiple of 32); *total gets the block's sum (ws: 33 ints of shared memory)
+__device__ inline int block_excl_scan(int v, int *ws, int *total)
 {
-    double m = 0;
-    for (long long base = t.begin + threadIdx.x; base < t.end; base += (long long)K * blockDim.x) {
-        int f[K], sp[K];
-        R px[K], py[K], pz[K], vx[K], vy[K], vz[K], ox[K], oy[K], oz[K];
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const long long i = base + (long long)k * blockDim.x;
-            if (i < t.end) {
-                f[k] = v.flags[i];
-                sp[k] = read_species ? v.species[i] : 0;
-                px[k] = v.pos.x[i];
-                py[k] = v.pos.y[i];
-                pz[k] = v.pos.z[i];
-                vx[k] = v.vel.x[i];
-                vy[k] = v.vel.y[i];
-                vz[k] = v.vel.z[i];
-                ox[k] = old.x[i];
-                oy[k] = old.y[i];
-                oz[k] = old.z[i];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            const long long i = base + (long long)k * blockDim.x;
-            if (i >= t.end) continue;
-            const bool md = (f[k] >> MD_BIT) & 1, past = (f[k] >> PAST_MD_BIT) & 1;
-            const R fx = flagged(v.force.x, i, md), fy = flagged(v.force.y, i, md), fz = flagged(v.force.z, i, md);
-            const R qx = px[k] + dt * vx[k] + dt_sq * fx;
-            const R qy = py[k] + dt * vy[k] + dt_sq * fy;
-            const R qz = pz[k] + dt * vz[k] + dt_sq * fz;
-            v.pos.x[i] = qx;
-            v.pos.y[i] = qy;
-            v.pos.z[i] = qz;
-            if (past) next.x[i] = next.y[i] = next.z[i] = 0;
-            if (md || past) flag_roll_one(v.flags, i);
-            if (sp[k] >= 0) {
-                double d0 = (double)qx - (double)ox[k], d1 = (double)qy - (double)oy[k],
-                       d2 = (double)qz - (double)oz[k];
-                double r = d0 * d0 + d1 * d1 + d2 * d2;
-                m = m > r ? m : r;
-            }
-        }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
     }
-    return m;
-}
-
-// the block's maximum displacement (m, one value per thread) into its
-// replica's so_max (r_tile < 0: a block without particles), then the
-// last-block hand-off: true in the one block of the grid that finishes last
-__device__ __forceinline__ bool block_done(double m, int r_tile, unsigned long long *so_max, unsigned *done,
-                                           double *s_max, int *s_last)
-{
-    m = warp_max(m);
-    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
+    if (lane == 31) ws[w] = inc;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < kBT / 32; w++) m = m > s_max[w] ? m : s_max[w];
-        // one atomic per block, skipped when it cannot raise the maximum
-        if (r_tile >= 0 && m > __longlong_as_double((long long)__ldcg(so_max + r_tile)))
-            atomic_max_nonneg(so_max + r_tile, m);
-        __threadfence();
-        *s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+        int acc = 0;
+        for (int k = 0; k < nw; k++) {
+            int y = ws[k];
+            ws[k] = acc;
+            acc += y;
+        }
+        ws[32] = acc;
     }
     __syncthreads();
-    return *s_last;
+    int ex = ws[w] + inc - v;
+    *total = ws[32];
+    __syncthreads();
+    return ex;
 }
 
-// the last block's part of an MD step's beginning: the colloid half of every
-// replica unless an earlier block did it (kFirst), the re-sort decisions, the
-// tile lists of the replicas to re-sort and the graph's re-sort condition
-// (any_out, if given, receives whether some replica re-sorts)
-template <bool kFirst>
-__device__ __forceinline__ void begin_tail(const BRep *rep, unsigned long long *so_max, unsigned *done, int *resort,
-                                           int *n_extra, const ColloidStep &cs, const ResortLists &rl,
-                                           cudaGraphConditionalHandle cond, int use_cond, unsigned *err, int *ws,
-                                           int *any_out = nullptr)
+// Flagged particles of the replicas at creation (later the re-sort's gather
+// lists them); force entries that the flags say are zero are made so.
+template <typename R>
+__global__ void kb_collect_flagged(TileSet ts, const BRep *rep, PView<R> v, int *key, int *nf)
 {
+    for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
+        const BTile t = ts.tiles[ts.ids[kt]];
+        for (long long i = t.begin + threadIdx.x; i < t.end; i += blockDim.x) {
+            const int f = v.flags[i];
+            if (f & kActiveBits) key[rep[t.r].off + atomicAdd(nf + t.r, 1)] = (int)i;
+            if (!((f >> MD_BIT) & 1)) v.force.x[i] = v.force.y[i] = v.force.z[i] = 0;
+            if (!((f >> PAST_MD_BIT) & 1)) v.force_old.x[i] = v.force_old.y[i] = v.force_old.z[i] = 0;
+        }
+    }
+}
+
+// The listed particles of the replicas in flag (every one when null) become
+// active, each once: its place in act goes to aidx.
+__global__ void kb_claim(const int *flag, const BRep *rep, const int *list, const int *n, int Nmax, int *aidx, int *act,
+                         int *nl, int *mult)
+{
+    const int i = blockIdx.y, r = i >> 1;
+    if (flag && !flag[r]) return;
+    const long long off = rep[r].off;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n[i]; e += gridDim.x * blockDim.x) {
+        const int idx = list[(size_t)i * Nmax + e];
+        if (atomicCAS(aidx + idx, -1, -2) != -1) continue;
+        const int a = atomicAdd(nl + r, 1);
+        act[off + a] = idx;
+        aidx[idx] = a;
+        mult[(size_t)2 * r * Nmax + a] = 0;
+    }
+}
+
+// steps[r] <- the first MD step at whose test some free particle of replica r
+// has moved sqrt(d2) >= thr from pos_old (programs/single_dimer_pbc.f90:324-329,
+// src/particle_system.f90:357-378).  A particle's earliest possible step
+// follows from its speed (with a margin for the rounding of each addition);
+// only the particles that could be first -- a few per replica -- go through
+// their additions one by one.
+template <typename R>
+__device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &old, long long i, int fresh, R dt,
+                                              double thr, int base, int n_rem, double slack, int read_species,
+                                              int *steps)
+{
+    if (read_species && v.species[i] < 0) return;
+    const R vx = v.vel.x[i], vy = v.vel.y[i], vz = v.vel.z[i];
+    const float ux = (float)vx, uy = (float)vy, uz = (float)vz;
+    float reach = (float)dt * sqrtf(ux * ux + uy * uy + uz * uz) * 1.001f + (float)slack;
+    float left = (float)thr;
+    if (fresh) {
+        // positions and pos_old are the caller's: any distance, any place
+        const double d0 = (double)v.pos.x[i] - (double)old.x[i], d1 = (double)v.pos.y[i] - (double)old.y[i],
+                     d2 = (double)v.pos.z[i] - (double)old.z[i];
+        left = (float)(thr - sqrt(d0 * d0 + d1 * d1 + d2 * d2)) - 1e-3f * (float)thr;
+        reach += (sizeof(R) == 4 ? 2.4e-7f : 4.4e-16f) *
+                 (fabsf((float)v.pos.x[i]) + fabsf((float)v.pos.y[i]) + fabsf((float)v.pos.z[i]));
+    }
+    if (!(reach * (float)n_rem >= left)) return;
+    int lo = left > 0 ? (int)fminf(left / reach, 1e9f) - 1 : 1;  // no crossing before the lo-th addition
+    if (lo < 1) lo = 1;
+    if (base + lo - 1 >= *(volatile int *)steps) return;
+    const R hx = dt * vx, hy = dt * vy, hz = dt * vz;
+    R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
+    const double ox = fresh ? (double)old.x[i] : (double)x, oy = fresh ? (double)old.y[i] : (double)y,
+                 oz = fresh ? (double)old.z[i] : (double)z;
+    for (int j = 1; j <= n_rem; j++) {
+        x = x + hx;
+        y = y + hy;
+        z = z + hz;
+        if (j < lo) continue;
+        const double d0 = (double)x - ox, d1 = (double)y - oy, d2 = (double)z - oz;
+        if (sqrt(d0 * d0 + d1 * d1 + d2 * d2) >= thr) {
+            atomicMin(steps, base + j - 1);
+            return;
+        }
+        if (base + j - 1 >= *(volatile int *)steps) return;
+    }
+}
+
+// After kb_claim: the first step at which a free particle forces a re-sort
+// (particle tiles), the places of the list entries and their multiplicities
+// (gx blocks per bead), and the flagged particles outside the lists, which
+// become active behind the listed ones (one block per replica).
+template <typename R>
+__global__ void __launch_bounds__(kBT)
+    kb_classify(TileSet ts, int n_tile_blocks, int gx, int R_, const int *flag, const BRep *rep, PView<R> v0,
+                PView<R> v1, R dt, double thr, int N_MD, int read_species, const int *base, const int *fresh,
+                int *s_free, const int *list, const int *n, int Nmax, int *aidx, int *act, const int *nl, int *nx,
+                int *mult, int *amap, const int *key, const int *nf)
+{
+    int b = blockIdx.x;
+    if (b < n_tile_blocks) {
+        for (int kt = b; kt < *ts.n; kt += n_tile_blocks) {
+            const BTile t = ts.tiles[ts.ids[kt]];
+            const BRep &rp = rep[t.r];
+            const PView<R> v = pick(v0, v1, rp.cur);
+            const Vec3<R> old = rp.cur ? v0.pos : v1.pos;
+            const int b0 = base[t.r], fr = fresh[t.r];
+            // three components, each rounded by at most half an ulp of a
+            // position inside twice the box
+            const double slack = (sizeof(R) == 4 ? 2.4e-7 : 4.4e-16) * (rp.g.edges[0] + rp.g.edges[1] + rp.g.edges[2]);
+            for (long long i = t.begin + threadIdx.x; i < t.end; i += blockDim.x)
+                if (!(v.flags[i] & kActiveBits) && aidx[i] < 0)
+                    free_crossing<R>(v, old, i, fr, dt, thr, b0, N_MD - b0, slack, read_species, s_free + t.r);
+        }
+        return;
+    }
+    b -= n_tile_blocks;
+    if (b < gx * 2 * R_) {
+        const int i = b / gx, r = i >> 1;
+        if (flag && !flag[r]) return;
+        for (int e = (b % gx) * blockDim.x + threadIdx.x; e < n[i]; e += gx * blockDim.x) {
+            const size_t q = (size_t)i * Nmax + e;
+            const int a = aidx[list[q]];
+            amap[q] = a;
+            atomicAdd(mult + (size_t)2 * r * Nmax + a, (i & 1) ? 1 << 16 : 1);
+        }
+        return;
+    }
+    const int r = b - gx * 2 * R_;
+    if (flag && !flag[r]) return;
+    const long long off = rep[r].off;
+    for (int k = threadIdx.x; k < nf[r]; k += blockDim.x) {
+        const int idx = key[off + k];
+        if (atomicCAS(aidx + idx, -1, -2) != -1) continue;
+        const int a = nl[r] + atomicAdd(nx + r, 1);
+        act[off + a] = idx;
+        aidx[idx] = a;
+    }
+}
+
+// kb_md: threads per block, active particles per thread kept in registers
+// (the others go through memory in every step), list entries per bead whose
+// places are kept in shared memory, and particles whose force flags are
+constexpr int kMdThreads = 512;
+constexpr int kMdPer = 2;
+constexpr int kMdMap = 4096;
+constexpr int kMdFlags = 8192;
+constexpr int kMdList = 1024;  // contributing entries compacted at a time (FP64 colloid sums)
+
+template <typename R>
+struct MdArgs {
+    const BRep *rep;
+    PView<R> v0, v1;      // solvent, buffers 0 and 1
+    PView<double> c;      // colloids
+    Vec3<double> cold;    // colloid pos_old
+    double *rat[3];       // pos_rattle
+    const double *mass;   // velocity-Verlet masses, 2 per replica
+    Masses ms;
+    double bond, dt, skin;
+    R dt_r, dt_sq_r;
+    double cut_c, cut_n, prob;
+    LJDev lj_sc, lj_cc;
+    int R_, N_MD, Nmax, start, read_species;
+    const uint64_t *d_step;
+    const int *n, *amap, *act, *nl, *nx, *mult;
+    double *pf;
+    unsigned char *cf;
+    const int *s_free, *fresh;
+    int *adv, *resort, *n_extra;
+    ResortLists rl;
+    unsigned *done;
+    int *any;
+    cudaGraphConditionalHandle cond;
+    int use_cond;
+    unsigned *err;
+};
+
+// one active solvent particle
+template <typename R>
+struct Part {
+    int idx;
+    int f, sp, m;       // flags, species, multiplicity in the two lists
+    R p[3], v[3], o[3]; // position, velocity, pos_old
+    R g[3];             // the last evaluation's force (zero without MD and PAST_MD)
+};
+
+struct MdShared {
+    double pos[3][2], vel[3][2], force[3][2], fold[3][2], old[3][2], rat[3][2];  // the beads (block 0)
+    double x[6];                 // bead positions of the current step
+    double wmax[8 * (kMdThreads / 32)];  // every warp's largest squared displacement (block 0)
+    double wsum[2][3][kMdThreads / 64];
+    double val[2][3][256];
+    int lst[2][kMdList];
+    int wcnt[2][kMdThreads / 64];
+    int map[2][kMdMap];
+    unsigned char cf[kMdFlags];  // which beads act on the particle (block 0)
+    int species[2];
+    int ws[33];
+    int stop, last;
+};
+
+template <typename R>
+__device__ __forceinline__ void md_load(Part<R> &q, const MdArgs<R> &A, const PView<R> &v, const Vec3<R> &old,
+                                        long long off, int r, int a, int nl, bool fresh)
+{
+    const int i = A.act[off + a];
+    q.idx = i;
+    q.f = v.flags[i];
+    q.sp = v.species[i];
+    q.m = a < nl ? A.mult[(size_t)2 * r * A.Nmax + a] : 0;
+    const bool forced = q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT));
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        q.p[k] = v.pos[k][i];
+        q.v[k] = v.vel[k][i];
+        q.o[k] = fresh ? old[k][i] : q.p[k];
+        q.g[k] = forced ? v.force[k][i] : (R)0;
+    }
+}
+
+template <typename R>
+__device__ __forceinline__ void md_store(const Part<R> &q, const PView<R> &v)
+{
+    const int i = q.idx;
+    v.flags[i] = q.f;
+    v.species[i] = q.sp;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        v.pos[k][i] = q.p[k];
+        v.vel[k][i] = q.v[k];
+        v.force[k][i] = q.g[k];
+    }
+}
+
+// md_pos (src/md.f90:61-77), the PAST_MD / MD roll (src/neighbor_list.f90:180-188)
+// and the squared displacement of maximum_displacement (0 for species < 0)
+template <typename R>
+__device__ __forceinline__ double md_begin(Part<R> &q, R dt, R dt_sq, int read_species)
+{
+    const bool md = (q.f >> MD_BIT) & 1;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (!md) q.g[k] = 0;
+        q.p[k] = q.p[k] + dt * q.v[k] + dt_sq * q.g[k];
+    }
+    q.f = md ? q.f | (1 << PAST_MD_BIT) : q.f & ~(1 << PAST_MD_BIT);
+    q.f &= ~(1 << MD_BIT);
+    if (read_species && q.sp < 0) return 0;
+    const double d0 = (double)q.p[0] - (double)q.o[0], d1 = (double)q.p[1] - (double)q.o[1],
+                 d2 = (double)q.p[2] - (double)q.o[2];
+    return d0 * d0 + d1 * d1 + d2 * d2;
+}
+
+// pair forces of the particle's list entries (src/neighbor_list.f90:198-219, in
+// (bead, entry) order), flag_particles_nl of the catalytic bead
+// (programs/single_dimer_pbc.f90:493-509), md_vel (src/md.f90:219-237) and
+// change_species (programs/single_dimer_pbc.f90:511-542).  Returns which beads
+// act on it; their forces go to pf[0..5].
+template <typename R>
+__device__ __forceinline__ int md_forces_end(Part<R> &q, const MdArgs<R> &A, const double X[6], const int cs[2],
+                                             const double L[3], double *pf, uint64_t seed, uint64_t step,
+                                             long long off)
+{
+    int acts = 0;
+    R nf[3] = {0, 0, 0};
+    double r_sq[2];
+    const double px = (double)q.p[0], py = (double)q.p[1], pz = (double)q.p[2];
+    const int sp0 = q.sp;
+    if (q.m && sp0 > 0) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int times = i ? q.m >> 16 : q.m & 0xffff;
+            if (!times) continue;
+            const double d0 = min_image_d(X[3 * i] - px, L[0]), d1 = min_image_d(X[3 * i + 1] - py, L[1]),
+                         d2 = min_image_d(X[3 * i + 2] - pz, L[2]);
+            r_sq[i] = d0 * d0 + d1 * d1 + d2 * d2;
+            const int tt = (sp0 - 1) + A.lj_sc.n1 * (cs[i] - 1);
+            if (r_sq[i] <= A.lj_sc.cut_sq[tt]) {
+                const double fr = lj_force_over_r(r_sq[i], A.lj_sc.epsilon[tt], A.lj_sc.sigma[tt]);
+                const double f0 = fr * d0, f1 = fr * d1, f2 = fr * d2;
+                pf[3 * i] = f0;
+                pf[3 * i + 1] = f1;
+                pf[3 * i + 2] = f2;
+                for (int t = 0; t < times; t++) {
+                    nf[0] = nf[0] - (R)f0;
+                    nf[1] = nf[1] - (R)f1;
+                    nf[2] = nf[2] - (R)f2;
+                }
+                acts |= 1 << i;
+                q.f |= (1 << MD_BIT) | (cs[i] == 1 ? (1 << CATALYZED_BIT) : 0);
+            }
+            if (i == 0 && sp0 == 1 && r_sq[0] < A.cut_c) q.f |= 1 << REAC_BIT;
+        }
+    }
+    const R dt = A.dt_r;
+    if (!((q.f >> WALL_BIT) & 1)) {
+        if (q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) q.v[k] = q.v[k] + dt * (nf[k] + q.g[k]) / 2;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 3; k++) q.v[k] = md_vel_free(q.v[k], dt);
+        }
+    } else {
+        q.f &= ~(1 << WALL_BIT);
+    }
+    if ((q.f >> REAC_BIT) & 1) {
+        double d[2];
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const double d0 = min_image_d(X[3 * i] - px, L[0]), d1 = min_image_d(X[3 * i + 1] - py, L[1]),
+                         d2 = min_image_d(X[3 * i + 2] - pz, L[2]);
+            d[i] = d0 * d0 + d1 * d1 + d2 * d2;
+        }
+        if ((d[0] > A.cut_c) && (d[1] > A.cut_n)) {
+            double u0, u1;
+            rng::uniform2(seed, step, (uint32_t)(q.idx - off), rng::REACT, 0, u0, u1);
+            if (u0 <= A.prob) q.sp = 2;
+            q.f &= ~(1 << REAC_BIT);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) q.g[k] = nf[k];
+    return acts;
+}
+
+// the place in act of entry e of bead h's list, and whether the bead acts on it
+__device__ __forceinline__ int md_place(const MdShared &sh, const int *amap, int h, int e)
+{
+    return e < kMdMap ? sh.map[h][e] : amap[e];
+}
+__device__ __forceinline__ bool md_acts(const MdShared &sh, const unsigned char *cf, int h, int a)
+{
+    const int c = a < kMdFlags ? sh.cf[a] : __ldcg(cf + a);
+    return (c >> h) & 1;
+}
+
+// Bead h's force += the sum of its pair forces, one half of the block per bead
+// (src/neighbor_list.f90:214-218): in list order in the FP64 form -- the
+// contributing entries are compacted in order and three threads add them one
+// by one -- and in the FP32 form by colloid_tree_block's fixed tree.
+template <typename R>
+__device__ __forceinline__ void md_colloid_sums(MdShared &sh, const MdArgs<R> &A, int r)
+{
+    constexpr int H = kMdThreads / 2, NW = H / 32;
+    const int h = threadIdx.x / H, t = threadIdx.x % H, lane = t & 31, w = t >> 5;
+    const int ni = A.n[2 * r + h];
+    const int *amap = A.amap + (size_t)(2 * r + h) * A.Nmax;
+    const double *pf = A.pf + (size_t)2 * r * A.Nmax * 6 + 3 * h;
+    const unsigned char *cf = A.cf + (size_t)2 * r * A.Nmax;
+    if constexpr (sizeof(R) == 4) {
+        static_assert(H == kNlBlockThreads, "colloid_tree_block's order");
+        double a0 = 0, a1 = 0, a2 = 0;
+        for (int e0 = t; e0 < ni; e0 += 32 * H) {
+            unsigned mask = 0;
+            for (int u = 0; u < 32; u++) {
+                const int e = e0 + u * H;
+                if (e >= ni) break;
+                if (md_acts(sh, cf, h, md_place(sh, amap, h, e))) mask |= 1u << u;
+            }
+            while (mask) {
+                double f[4][3];
+                unsigned got = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (mask) {
+                        const double *q = pf + 6 * (size_t)md_place(sh, amap, h, e0 + (__ffs(mask) - 1) * H);
+                        mask &= mask - 1;
+                        f[k][0] = __ldcg(q);
+                        f[k][1] = __ldcg(q + 1);
+                        f[k][2] = __ldcg(q + 2);
+                        got |= 1u << k;
+                    }
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if ((got >> k) & 1) {
+                        a0 = a0 + f[k][0];
+                        a1 = a1 + f[k][1];
+                        a2 = a2 + f[k][2];
+                    }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            a0 = a0 + __shfl_xor_sync(0xffffffffu, a0, o);
+            a1 = a1 + __shfl_xor_sync(0xffffffffu, a1, o);
+            a2 = a2 + __shfl_xor_sync(0xffffffffu, a2, o);
+        }
+        if (lane == 0) {
+            sh.wsum[h][0][w] = a0;
+            sh.wsum[h][1][w] = a1;
+            sh.wsum[h][2][w] = a2;
+        }
+        __syncthreads();
+        if (w == 0) {
+            double b0 = lane < NW ? sh.wsum[h][0][lane] : 0.0, b1 = lane < NW ? sh.wsum[h][1][lane] : 0.0,
+                   b2 = lane < NW ? sh.wsum[h][2][lane] : 0.0;
+#pragma unroll
+            for (int o = NW / 2; o > 0; o >>= 1) {
+                b0 = b0 + __shfl_xor_sync(0xffffffffu, b0, o);
+                b1 = b1 + __shfl_xor_sync(0xffffffffu, b1, o);
+                b2 = b2 + __shfl_xor_sync(0xffffffffu, b2, o);
+            }
+            if (lane == 0) {
+                sh.force[0][h] = sh.force[0][h] + b0;
+                sh.force[1][h] = sh.force[1][h] + b1;
+                sh.force[2][h] = sh.force[2][h] + b2;
+            }
+        }
+        __syncthreads();
+    } else {
+        // each warp takes a contiguous run of the list
+        const int per = (ni + 32 * NW - 1) / (32 * NW) * 32;
+        const int e_lo = w * per, e_hi = min(ni, e_lo + per);
+        int cnt = 0;
+        for (int e = e_lo + lane; e - lane < e_hi; e += 32) {
+            const bool on = e < e_hi && md_acts(sh, cf, h, md_place(sh, amap, h, e));
+            cnt += __popc(__ballot_sync(0xffffffffu, on));
+        }
+        if (lane == 0) sh.wcnt[h][w] = cnt;
+        __syncthreads();
+        int before = 0, tot[2] = {0, 0};
+        for (int k = 0; k < NW; k++) {
+            if (k < w) before += sh.wcnt[h][k];
+            tot[0] += sh.wcnt[0][k];
+            tot[1] += sh.wcnt[1][k];
+        }
+        const int most = max(tot[0], tot[1]), mine = tot[h];
+        double acc = 0;  // thread c < 3 of the half adds component c
+        for (int c0 = 0; c0 < most; c0 += kMdList) {
+            int at = before;
+            for (int e = e_lo + lane; e - lane < e_hi; e += 32) {
+                const int a = e < e_hi ? md_place(sh, amap, h, e) : 0;
+                const bool on = e < e_hi && md_acts(sh, cf, h, a);
+                const unsigned bal = __ballot_sync(0xffffffffu, on);
+                const int k = at + __popc(bal & ((1u << lane) - 1u));
+                if (on && k >= c0 && k < c0 + kMdList) sh.lst[h][k - c0] = a;
+                at += __popc(bal);
+            }
+            __syncthreads();
+            for (int v0 = 0; v0 < kMdList && c0 + v0 < most; v0 += H) {
+                const int m = min(H, mine - c0 - v0);
+                if (t < m) {
+                    const double *q = pf + 6 * (size_t)sh.lst[h][v0 + t];
+                    sh.val[h][0][t] = __ldcg(q);
+                    sh.val[h][1][t] = __ldcg(q + 1);
+                    sh.val[h][2][t] = __ldcg(q + 2);
+                }
+                __syncthreads();
+                if (t < 3) {
+#pragma unroll 8
+                    for (int k = 0; k < m; k++) acc = acc + sh.val[h][t][k];
+                }
+                __syncthreads();
+            }
+        }
+        if (t < 3) sh.force[t][h] = sh.force[t][h] + acc;
+        __syncthreads();
+    }
+}
+
+__device__ inline PView<double> md_beads(MdShared &sh)
+{
+    PView<double> c{};
+    c.N = 2;
+    c.pos = {sh.pos[0], sh.pos[1], sh.pos[2]};
+    c.vel = {sh.vel[0], sh.vel[1], sh.vel[2]};
+    c.force = {sh.force[0], sh.force[1], sh.force[2]};
+    c.force_old = {sh.fold[0], sh.fold[1], sh.fold[2]};
+    c.species = sh.species;
+    return c;
+}
+
+// compute_force_n2, the colloid velocity half and RATTLE's velocity correction
+// (src/neighbor_list.f90:227-264, programs/single_dimer_pbc.f90:356-359,
+// src/md.f90:298-319)
+template <typename R>
+__device__ __forceinline__ void md_colloid_end(MdShared &sh, const MdArgs<R> &A, int r, const double e[3])
+{
+    PView<double> c = md_beads(sh);
+    for (int m = 0; m < 2; m++)
+        force_n2_one(m, c.pos.x, c.pos.y, c.pos.z, c.species, 2, e[0], e[1], e[2], A.lj_cc, c.force.x, c.force.y,
+                     c.force.z);
+    colloid_vv_vel_one(c, 0, A.mass[2 * r], A.dt);
+    colloid_vv_vel_one(c, 1, A.mass[2 * r + 1], A.dt);
+    rattle_vel_dimer(c, A.ms, A.bond, E3{{e[0], e[1], e[2]}}, A.err);
+}
+
+// the colloid position half, RATTLE and switch_force
+// (programs/single_dimer_pbc.f90:311-322); returns the beads' displacement
+template <typename R>
+__device__ __forceinline__ double md_colloid_begin(MdShared &sh, const MdArgs<R> &A, int r, const double e[3])
+{
+    PView<double> c = md_beads(sh);
+    for (int k = 0; k < 3; k++)
+        for (int i = 0; i < 2; i++) sh.rat[k][i] = sh.pos[k][i];
+    colloid_vv_pos_one(c, 0, A.mass[2 * r], A.dt);
+    colloid_vv_pos_one(c, 1, A.mass[2 * r + 1], A.dt);
+    rattle_pos_dimer(c, sh.rat[0], sh.rat[1], sh.rat[2], A.ms, A.bond, A.dt, E3{{e[0], e[1], e[2]}}, A.err);
+    Vec3<double> o = {sh.old[0], sh.old[1], sh.old[2]};
+    const double m0 = disp_sq_one(c.pos, o, c.species, 0), m1 = disp_sq_one(c.pos, o, c.species, 1);
+    for (int k = 0; k < 3; k++)
+        for (int i = 0; i < 2; i++) {
+            sh.fold[k][i] = sh.force[k][i];
+            sh.force[k][i] = 0;
+        }
+    return sqrt(m0 > m1 ? m0 : m1);
+}
+
+// warp 0 of block 0: with the displacements of MD step k's beginning complete,
+// the colloid position half and the re-sort test of step k
+// (programs/single_dimer_pbc.f90:311-330), then the bead positions and the
+// decision to every block of the cluster
+template <typename R>
+__device__ __forceinline__ void md_turn(MdShared &sh, const MdArgs<R> &A, int r, const double e[3], int k, int blocks,
+                                        bool end, bool begin)
+{
+    namespace cg = cooperative_groups;
+    const int lane = threadIdx.x;
+    if (end && lane == 0) md_colloid_end<R>(sh, A, r, e);
+    if (begin) {
+        double m = 0;
+        for (int w = lane; w < blocks * (kMdThreads / 32); w += 32) m = m > sh.wmax[w] ? m : sh.wmax[w];
+        m = warp_max(m);
+        if (lane == 0) {
+            const double co = md_colloid_begin<R>(sh, A, r, e);
+            const double so = sqrt(m);
+            sh.stop = (co >= A.skin * 0.1) || (so >= A.skin * 0.89) || k >= A.s_free[r];
+        }
+        __syncwarp();
+        if (lane < blocks) {
+            MdShared *to = cg::this_cluster().map_shared_rank(&sh, lane);
+            for (int q = 0; q < 6; q++) to->x[q] = sh.pos[q % 3][q / 3];
+            if (lane > 0) to->stop = sh.stop;
+        }
+    }
+}
+
+// The MD steps of every replica (start) or of those that were re-sorted
+// (resort[r]), one cluster per replica, each until its next re-sort or the
+// interval's end.  Per step two cluster barriers: after every particle's
+// forces, velocity and next position (the bead sums and the re-sort test need
+// them), and after the beads' turn (the particles need their positions).
+// Latency bound: a step is this chain of barriers, L2 round trips of the pair
+// forces to block 0 and one thread's bead arithmetic.
+template <typename R>
+__global__ void __launch_bounds__(kMdThreads, 1) kb_md(MdArgs<R> A)
+{
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char md_smem[];
+    MdShared &sh = *reinterpret_cast<MdShared *>(md_smem);
+    cg::cluster_group cl = cg::this_cluster();
+    const int blocks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int r = blockIdx.x / blocks;
+    const int t = threadIdx.x;
+    int need = 0;
+    if (A.start || A.resort[r]) {
+        const BRep &rp = A.rep[r];
+        const long long off = rp.off;
+        const uint64_t seed = rp.seed, step0 = *A.d_step;
+        const double L[3] = {rp.g.edges[0], rp.g.edges[1], rp.g.edges[2]};
+        const PView<R> v = pick(A.v0, A.v1, rp.cur);
+        const Vec3<R> old = rp.cur ? A.v0.pos : A.v1.pos;
+        const bool fresh = A.fresh[r] != 0;
+        const int nl = A.nl[r], na = nl + A.nx[r];
+        const int nthr = blocks * kMdThreads, tid = rank * kMdThreads + t;
+        double *pf = A.pf + (size_t)2 * r * A.Nmax * 6;
+        unsigned char *cf = A.cf + (size_t)2 * r * A.Nmax;
+        MdShared *sh0 = cl.map_shared_rank(&sh, 0);
+        cl.sync();  // every block runs before its shared memory is written from another
+        int k = A.start ? 0 : A.adv[r] - 1;
+        const int cs[2] = {A.c.species[2 * r], A.c.species[2 * r + 1]};
+        // this thread's particles: kMdPer in registers, the rest in place
+        Part<R> q[kMdPer];
+#pragma unroll
+        for (int u = 0; u < kMdPer; u++)
+            if (tid + u * nthr < na) md_load(q[u], A, v, old, off, r, tid + u * nthr, nl, fresh);
+        double m = 0;
+        if (A.start) {
+            // force_old of the last interval's end is no longer current
+            auto clear_old = [&](const Part<R> &p) {
+                if ((p.f >> PAST_MD_BIT) & 1) v.force_old.x[p.idx] = v.force_old.y[p.idx] = v.force_old.z[p.idx] = 0;
+            };
+#pragma unroll
+            for (int u = 0; u < kMdPer; u++)
+                if (tid + u * nthr < na) {
+                    clear_old(q[u]);
+                    const double d = md_begin(q[u], A.dt_r, A.dt_sq_r, A.read_species);
+                    m = m > d ? m : d;
+                }
+        }
+        for (int a = tid + kMdPer * nthr; a < na; a += nthr) {
+            Part<R> p;
+            md_load(p, A, v, old, off, r, a, nl, fresh);
+            if (!fresh)
+                for (int c = 0; c < 3; c++) old[c][p.idx] = p.o[c];
+            if (A.start) {
+                if ((p.f >> PAST_MD_BIT) & 1) v.force_old.x[p.idx] = v.force_old.y[p.idx] = v.force_old.z[p.idx] = 0;
+                const double d = md_begin(p, A.dt_r, A.dt_sq_r, A.read_species);
+                m = m > d ? m : d;
+                md_store(p, v);
+            }
+        }
+        if (rank == 0) {
+            for (int h = 0; h < 2; h++)
+                for (int e = t; e < min(A.n[2 * r + h], kMdMap); e += kMdThreads)
+                    sh.map[h][e] = A.amap[(size_t)(2 * r + h) * A.Nmax + e];
+            if (t < 6) {
+                const int c = t % 3, i = t / 3;
+                sh.pos[c][i] = A.c.pos[c][2 * r + i];
+                sh.vel[c][i] = A.c.vel[c][2 * r + i];
+                sh.force[c][i] = A.c.force[c][2 * r + i];
+                sh.fold[c][i] = A.c.force_old[c][2 * r + i];
+                sh.old[c][i] = A.cold[c][2 * r + i];
+                sh.rat[c][i] = A.rat[c][2 * r + i];
+                if (c == 0) sh.species[i] = cs[i];
+            }
+        }
+        m = warp_max(m);
+        if ((t & 31) == 0) sh0->wmax[rank * (kMdThreads / 32) + (t >> 5)] = m;
+        cl.sync();
+        if (rank == 0 && t < 32) {
+            if (A.start) {
+                md_turn<R>(sh, A, r, L, k, blocks, false, true);
+            } else if (t < blocks) {
+                // resumed after a re-sort: the step's forces come next
+                MdShared *to = cl.map_shared_rank(&sh, t);
+                for (int c = 0; c < 6; c++) to->x[c] = sh.pos[c % 3][c / 3];
+                to->stop = 0;
+            }
+        }
+        cl.sync();
+        while (!sh.stop) {
+            const bool last = k + 1 == A.N_MD;
+            const double X[6] = {sh.x[0], sh.x[1], sh.x[2], sh.x[3], sh.x[4], sh.x[5]};
+            m = 0;
+            // one particle's forces and end of step k, then its beginning of step k + 1
+            auto one = [&](Part<R> &p, int a) {
+                if (last) {
+                    // the interval's last step leaves force_old behind
+                    const bool past = (p.f >> PAST_MD_BIT) & 1;
+                    for (int c = 0; c < 3; c++) v.force_old[c][p.idx] = past ? p.g[c] : (R)0;
+                }
+                const int acts = md_forces_end(p, A, X, cs, L, pf + 6 * (size_t)a, seed, step0 + (uint64_t)k, off);
+                if (a < nl) {
+                    if (a < kMdFlags) sh0->cf[a] = (unsigned char)acts;
+                    else cf[a] = (unsigned char)acts;
+                }
+                if (!last) {
+                    const double d = md_begin(p, A.dt_r, A.dt_sq_r, A.read_species);
+                    m = m > d ? m : d;
+                }
+            };
+#pragma unroll
+            for (int u = 0; u < kMdPer; u++)
+                if (tid + u * nthr < na) one(q[u], tid + u * nthr);
+            for (int a = tid + kMdPer * nthr; a < na; a += nthr) {
+                Part<R> p;
+                md_load(p, A, v, old, off, r, a, nl, true);
+                one(p, a);
+                md_store(p, v);
+            }
+            m = warp_max(m);
+            if ((t & 31) == 0) sh0->wmax[rank * (kMdThreads / 32) + (t >> 5)] = m;
+            cl.sync();
+            if (rank == 0) {
+                md_colloid_sums<R>(sh, A, r);
+                if (t < 32) md_turn<R>(sh, A, r, L, k + 1, blocks, true, !last);
+            }
+            cl.sync();
+            k++;
+            if (last) break;
+        }
+        need = k < A.N_MD;  // stopped in front of step k's forces
+#pragma unroll
+        for (int u = 0; u < kMdPer; u++)
+            if (tid + u * nthr < na) md_store(q[u], v);
+        if (rank == 0) {
+            if (t < 6) {
+                const int c = t % 3, i = t / 3;
+                A.c.pos[c][2 * r + i] = sh.pos[c][i];
+                A.c.vel[c][2 * r + i] = sh.vel[c][i];
+                A.c.force[c][2 * r + i] = sh.force[c][i];
+                A.c.force_old[c][2 * r + i] = sh.fold[c][i];
+                A.rat[c][2 * r + i] = sh.rat[c][i];
+            }
+            if (t == 0) {
+                A.adv[r] = need ? k + 1 : A.N_MD;
+                A.resort[r] = need;
+                if (need) A.n_extra[r] += 1;
+            }
+        }
+    }
+    if (rank != 0) return;
+    // the last replica to finish lists the tiles of those to re-sort and sets
+    // the graph's loop condition
+    if (t == 0) {
+        __threadfence();
+        sh.last = atomicAdd(A.done, 1u) == (unsigned)A.R_ - 1u;
+    }
+    __syncthreads();
+    if (!sh.last) return;
     __threadfence();
     int any = 0, base_p = 0, base_s = 0;
-    for (int r0 = 0; r0 < cs.R; r0 += blockDim.x) {
-        const int r = r0 + threadIdx.x;
-        int need = 0;
-        if (r < cs.R) {
-            const double co = kFirst ? __ldcg(cs.co_max + r)
-                                     : colloid_begin(r, rep, cs.c, cs.cold, cs.c_next, cs.rat, cs.mass, cs.ms, cs.d,
-                                                     cs.dt, err);
-            need = resort_decision(r, cs.skin, co, so_max, resort, n_extra);
-        }
-        any |= need;
-        const int np = need ? rl.pcount[r] : 0, ns = need ? rl.scount[r] : 0;
+    for (int r0 = 0; r0 < A.R_; r0 += kMdThreads) {
+        const int q = r0 + t;
+        const int nd = q < A.R_ ? __ldcg(A.resort + q) : 0;
+        any |= nd;
+        const int np = nd ? A.rl.pcount[q] : 0, ns = nd ? A.rl.scount[q] : 0;
         int tp, ts;
-        const int ep = base_p + block_excl_scan(np, ws, &tp);
-        const int es = base_s + block_excl_scan(ns, ws, &ts);
-        for (int k = 0; k < np; k++) rl.pids[ep + k] = rl.pfirst[r] + k;
-        for (int k = 0; k < ns; k++) rl.sids[es + k] = rl.sfirst[r] + k;
+        const int ep = base_p + block_excl_scan(np, sh.ws, &tp);
+        const int es = base_s + block_excl_scan(ns, sh.ws, &ts);
+        for (int c = 0; c < np; c++) A.rl.pids[ep + c] = A.rl.pfirst[q] + c;
+        for (int c = 0; c < ns; c++) A.rl.sids[es + c] = A.rl.sfirst[q] + c;
         base_p += tp;
         base_s += ts;
     }
     any = __syncthreads_or(any);
-    if (threadIdx.x == 0) {
-        rl.n[0] = base_p;
-        rl.n[1] = base_s;
-        if (use_cond && any) cudaGraphSetConditional(cond, 1);
-        if (any_out) *any_out = any;
-        *done = 0;
+    if (t == 0) {
+        A.rl.n[0] = base_p;
+        A.rl.n[1] = base_s;
+        *A.any = any;
+        *A.done = 0;
+        if (A.use_cond) cudaGraphSetConditional(A.cond, any ? 1u : 0u);
         __threadfence();
     }
-}
-
-// md_pos of every solvent particle, the PAST_MD/MD roll of compute_force,
-// clearing of the entries that become `force` after switch_force and the
-// solvent's maximum displacement (src/md.f90:61-77,
-// src/neighbor_list.f90:180-188, src/particle_system.f90:357-378), one block
-// per particle tile; the last block to finish takes the program's re-sort
-// decision, lists the tiles of the replicas to re-sort and raises the graph's
-// re-sort condition when there are any.  The colloid half of every replica
-// runs either in that last block or in an extra block 0 while the solvent
-// streams (V::FIRST, a choice of the engine shape: the extra block's registers
-// make the FP32 streaming path spill, which costs the large FP32 batches more
-// than the overlap gains, and the autotuner weighs the two).
-template <typename R, typename V>
-__global__ void __launch_bounds__(kBT, V::MINB)
-    kb_step_begin(const BTile *tiles, const BRep *rep, PView<R> v, Vec3<R> old, Vec3<R> next, R dt, R dt_sq,
-                  unsigned long long *so_max, unsigned *done, int *resort, int *n_extra, ColloidStep cs,
-                  ResortLists rl, cudaGraphConditionalHandle cond, int use_cond, int read_species, unsigned *err,
-                  int *any_out)
-{
-    __shared__ int s_last;
-    __shared__ int ws[kBT / 32 + 1];
-    __shared__ double s_max[kBT / 32];
-    constexpr bool kFirst = V::FIRST;
-    double m = 0;
-    int r_tile = -1;
-    if (kFirst && blockIdx.x == 0) {
-        for (int r = threadIdx.x; r < cs.R; r += blockDim.x)
-            cs.co_max[r] = colloid_begin(r, rep, cs.c, cs.cold, cs.c_next, cs.rat, cs.mass, cs.ms, cs.d, cs.dt, err);
-    } else {
-        const BTile t = tiles[blockIdx.x - (kFirst ? 1 : 0)];
-        r_tile = t.r;
-        m = begin_tile<R, V::KB>(t, v, old, next, dt, dt_sq, read_species);
-    }
-    if (!block_done(m, r_tile, so_max, done, s_max, &s_last)) return;
-    begin_tail<kFirst>(rep, so_max, done, resort, n_extra, cs, rl, cond, use_cond, err, ws, any_out);
-}
-
-// list pair forces (src/neighbor_list.f90:198-219) fused with
-// flag_particles_nl of the catalytic bead (programs/single_dimer_pbc.f90:493-509):
-// both only read positions and species and OR bits into flags.  Block (0, i)
-// also copies colloid i's position to csnap[3 i ..], the positions that the
-// step's change_species uses.  skip (if given): the MD step's beginning
-// decided to re-sort, so this launch is the graph's speculative one and the
-// re-sort branch evaluates the forces instead.
-template <typename R>
-__global__ void kb_pair_forces(const BRep *rep, PView<double> c, PView<R> s, const int *list, const int *n, int Nmax,
-                               LJDev lj, double *pf, double *pe, unsigned char *contrib, int *ncontrib,
-                               int *max_contrib, double flag_cut_sq, double *csnap, const int *skip)
-{
-    if (skip && *(const volatile int *)skip) return;
-    const int i = blockIdx.y;
-    const int r = i >> 1;
-    const int ni = n[i];
-    const double x[3] = {c.pos.x[i], c.pos.y[i], c.pos.z[i]};
-    if (blockIdx.x == 0 && threadIdx.x < 3) csnap[3 * i + threadIdx.x] = x[threadIdx.x];
-    const int s1 = c.species[i];
-    const double L0 = rep[r].g.edges[0], L1 = rep[r].g.edges[1], L2 = rep[r].g.edges[2];
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ni; e += gridDim.x * blockDim.x) {
-        size_t q = (size_t)i * Nmax + e;
-        pair_force_entry(q, x, s1, s.pos.x, s.pos.y, s.pos.z, s.species, s.flags, list, L0, L1, L2, lj, pf, pe,
-                         contrib, ncontrib, max_contrib + r);
-        if ((i & 1) == 0)
-            flag_nl_one(list[q], x, s.pos.x, s.pos.y, s.pos.z, s.species, s.flags, L0, L1, L2, flag_cut_sq);
-    }
-}
-
-// the three consumers of the pair forces, on disjoint data: solvent
-// particles with one contribution, those with several (per replica, in
-// order), and the colloid sums (list order in the FP64 form, a fixed tree in
-// the FP32 form); skip: as kb_pair_forces
-template <typename R>
-__global__ void kb_apply_sum(const BRep *rep, int R_, int gx, const int *list, const int *n, int Nmax,
-                             const unsigned char *contrib, const double *pf, const int *ncontrib,
-                             const int *max_contrib, R *fx, R *fy, R *fz, double *cfx, double *cfy, double *cfz,
-                             int *clist, int *cn, const int *skip)
-{
-    if (skip && *(const volatile int *)skip) return;
-    const int b = blockIdx.x;
-    const int n_single = gx * 2 * R_;
-    if (b < n_single) {
-        const int i = b / gx, bx = b % gx;
-        for (int e = bx * blockDim.x + threadIdx.x; e < n[i]; e += gx * blockDim.x)
-            apply_single_entry((size_t)i * Nmax + e, list, contrib, pf, ncontrib, fx, fy, fz);
-    } else if (b < n_single + R_) {
-        const int r = b - n_single;
-        if (max_contrib[r] < 2) return;
-        const size_t q0 = (size_t)2 * r * Nmax;
-        apply_multi_block(list + q0, n + 2 * r, 2, Nmax, contrib + q0, pf + 3 * q0, ncontrib, rep[r].serial, fx, fy,
-                          fz);
-    } else if constexpr (sizeof(R) == 8) {
-        colloid_sum_block(b - n_single - R_, n, Nmax, contrib, pf, cfx, cfy, cfz, clist, cn);
-    } else {
-        colloid_tree_block(b - n_single - R_, n, Nmax, contrib, pf, cfx, cfy, cfz);
-    }
-}
-
-// the solvent half over the particle tile t of replica rp, whose colloid
-// positions are a and bb; step is the random-number step of change_species
-template <typename R, int K>
-__device__ __forceinline__ void end_tile(const BTile &t, const BRep &rp, const PView<R> &v, const double a[3],
-                                         const double bb[3], R dt, double cut_c, double cut_n, double prob,
-                                         uint64_t step)
-{
-    const double L0 = rp.g.edges[0], L1 = rp.g.edges[1], L2 = rp.g.edges[2];
-    const uint64_t seed = rp.seed;
-    const long long off = rp.off;
-    // The FP64 form reads every velocity: a zero-force update turns a -0
-    // component into +0, as the reference's does.  The FP32 form reads
-    // velocities only for particles with a force and leaves the others'
-    // bits untouched, so it keeps a -0 component (an SRD rotation product
-    // can round to one) where the reference would store +0: equal in
-    // value, not in bits, which is why FP32 results are compared by value.
-    constexpr bool kAllVel = sizeof(R) == 8;
-    if constexpr (!kAllVel) {
-        // FP32: only particles with a WALL, MD, PAST_MD or REAC bit do
-        // anything, so the flags are read four at a time (one 16-byte
-        // load; the arrays are allocated to a multiple of 4) and a group
-        // of four without such a bit is skipped whole
-        constexpr int kBits = (1 << WALL_BIT) | (1 << MD_BIT) | (1 << PAST_MD_BIT) | (1 << REAC_BIT);
-        auto one = [&](long long i, int f) {
-            if (!(f & kBits)) return;
-            if (!((f >> WALL_BIT) & 1)) {
-                const bool md = (f >> MD_BIT) & 1, past = (f >> PAST_MD_BIT) & 1;
-                if (md || past) {
-                    const R vx = v.vel.x[i], vy = v.vel.y[i], vz = v.vel.z[i];
-                    R f0 = flagged(v.force.x, i, md), f1 = flagged(v.force.y, i, md),
-                      f2 = flagged(v.force.z, i, md);
-                    R g0 = flagged(v.force_old.x, i, past), g1 = flagged(v.force_old.y, i, past),
-                      g2 = flagged(v.force_old.z, i, past);
-                    v.vel.x[i] = vx + dt * (f0 + g0) / 2;
-                    v.vel.y[i] = vy + dt * (f1 + g1) / 2;
-                    v.vel.z[i] = vz + dt * (f2 + g2) / 2;
-                }
-            } else {
-                v.flags[i] = f & ~(1 << WALL_BIT);
-                f = f & ~(1 << WALL_BIT);
-            }
-            if ((f >> REAC_BIT) & 1)
-                change_species_one(v, i, i - off, a, bb, L0, L1, L2, cut_c, cut_n, prob, seed, step);
-        };
-        const long long a4 = (t.begin + 3) & ~3LL, e4 = t.end & ~3LL;
-        const long long h_end = a4 < t.end ? a4 : t.end;
-        for (long long i = t.begin + threadIdx.x; i < h_end; i += blockDim.x) one(i, v.flags[i]);
-        if (a4 < e4) {
-            const int4 *f4 = (const int4 *)v.flags;
-            constexpr int U = 4;
-            for (long long q0 = a4 / 4 + threadIdx.x; q0 < e4 / 4; q0 += (long long)U * blockDim.x) {
-                int4 g[U];
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    const long long q = q0 + (long long)u * blockDim.x;
-                    g[u] = q < e4 / 4 ? f4[q] : make_int4(0, 0, 0, 0);
-                }
-#pragma unroll
-                for (int u = 0; u < U; u++) {
-                    if (!((g[u].x | g[u].y | g[u].z | g[u].w) & kBits)) continue;
-                    const long long i = 4 * (q0 + (long long)u * blockDim.x);
-                    one(i, g[u].x);
-                    one(i + 1, g[u].y);
-                    one(i + 2, g[u].z);
-                    one(i + 3, g[u].w);
-                }
-            }
-        }
-        const long long t_begin = e4 > h_end ? e4 : h_end;
-        for (long long i = t_begin + threadIdx.x; i < t.end; i += blockDim.x) one(i, v.flags[i]);
-        return;
-    }
-    for (long long base = t.begin + threadIdx.x; base < t.end; base += (long long)K * blockDim.x) {
-      int fk[K];
-      R vxk[K] = {}, vyk[K] = {}, vzk[K] = {};
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const long long i = base + (long long)k * blockDim.x;
-        if (i < t.end) {
-            fk[k] = v.flags[i];
-            if (kAllVel) {
-                vxk[k] = v.vel.x[i];
-                vyk[k] = v.vel.y[i];
-                vzk[k] = v.vel.z[i];
-            }
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < K; k++) {
-        const long long i = base + (long long)k * blockDim.x;
-        if (i >= t.end) continue;
-        int f = fk[k];
-        if (!kAllVel && !((f >> WALL_BIT) & 1) && (((f >> MD_BIT) & 1) || ((f >> PAST_MD_BIT) & 1))) {
-            vxk[k] = v.vel.x[i];
-            vyk[k] = v.vel.y[i];
-            vzk[k] = v.vel.z[i];
-        }
-        const R vx = vxk[k], vy = vyk[k], vz = vzk[k];
-        if (!((f >> WALL_BIT) & 1)) {
-            const bool md = (f >> MD_BIT) & 1, past = (f >> PAST_MD_BIT) & 1;
-            if (md || past) {
-                R f0 = flagged(v.force.x, i, md), f1 = flagged(v.force.y, i, md), f2 = flagged(v.force.z, i, md);
-                R g0 = flagged(v.force_old.x, i, past), g1 = flagged(v.force_old.y, i, past),
-                  g2 = flagged(v.force_old.z, i, past);
-                v.vel.x[i] = vx + dt * (f0 + g0) / 2;
-                v.vel.y[i] = vy + dt * (f1 + g1) / 2;
-                v.vel.z[i] = vz + dt * (f2 + g2) / 2;
-            } else if (kAllVel) {
-                // both forces are zero: the update changes a velocity
-                // only if it is -0, so the store is kept for that case
-                const R z = 0;
-                const R nx = vx + dt * (z + z) / 2, ny = vy + dt * (z + z) / 2, nz = vz + dt * (z + z) / 2;
-                if (!same_bits(nx, vx) || !same_bits(ny, vy) || !same_bits(nz, vz)) {
-                    v.vel.x[i] = nx;
-                    v.vel.y[i] = ny;
-                    v.vel.z[i] = nz;
-                }
-            }
-        } else {
-            v.flags[i] = f & ~(1 << WALL_BIT);
-            f = f & ~(1 << WALL_BIT);
-        }
-        if ((f >> REAC_BIT) & 1)
-            change_species_one(v, i, i - off, a, bb, L0, L1, L2, cut_c, cut_n, prob, seed, step);
-      }
-    }
-}
-
-// clearing of the contribution counters over entries [bx * blockDim.x, ...)
-// of list i, strided by gx blocks
-__device__ __forceinline__ void end_reset(int i, int bx, int gx, const int *list, const int *n, int Nmax,
-                                          const unsigned char *contrib, int *ncontrib, int *max_contrib)
-{
-    for (int e = bx * blockDim.x + threadIdx.x; e < n[i]; e += gx * blockDim.x) {
-        size_t qq = (size_t)i * Nmax + e;
-        if (contrib[qq]) ncontrib[list[qq]] = 0;
-    }
-    if (bx == 0 && threadIdx.x == 0 && (i & 1) == 0) max_contrib[i >> 1] = 0;
-}
-
-// compute_force_n2, the colloid velocity half and RATTLE's velocity
-// correction of replica r
-__device__ __forceinline__ void end_colloid(int r, const BRep *rep, const PView<double> &c, const ColloidStep &cs,
-                                            const LJDev &lj_cc, unsigned *err)
-{
-    PView<double> cr = shifted(c, 2 * (long long)r, 2);
-    const double *e = rep[r].g.edges;
-    for (int m = 0; m < 2; m++)
-        force_n2_one(m, cr.pos.x, cr.pos.y, cr.pos.z, cr.species, 2, e[0], e[1], e[2], lj_cc, cr.force.x,
-                     cr.force.y, cr.force.z);
-    colloid_vv_vel_one(cr, 0, cs.mass[2 * r], cs.dt);
-    colloid_vv_vel_one(cr, 1, cs.mass[2 * r + 1], cs.dt);
-    E3 L{{e[0], e[1], e[2]}};
-    rattle_vel_dimer(cr, cs.ms, cs.d, L, err);
-}
-
-// md_vel then change_species of every solvent particle (src/md.f90:219-237,
-// programs/single_dimer_pbc.f90:511-542), one block per particle tile;
-// clearing of the per-particle contribution counters; compute_force_n2, the
-// colloid velocity half and RATTLE's velocity correction per replica
-// (src/neighbor_list.f90:227-264, programs/single_dimer_pbc.f90:356-359,
-// src/md.f90:298-319).  The last MD step of an interval ends with this
-// kernel; the others end inside kb_step_end_begin.
-template <typename R, typename V>
-__global__ void __launch_bounds__(kBT, V::MINB)
-    kb_step_end(const BTile *tiles, int n_tiles, int gx, const BRep *rep, PView<R> v, PView<double> c, R dt,
-                double cut_c, double cut_n, double prob, const uint64_t *d_step, int step_off, const int *list,
-                const int *n, int Nmax, const unsigned char *contrib, int *ncontrib, int *max_contrib,
-                ColloidStep cs, LJDev lj_cc, unsigned *err)
-{
-    const int b = blockIdx.x;
-    if (b < n_tiles) {
-        const BTile t = tiles[b];
-        const double a[3] = {c.pos.x[2 * t.r], c.pos.y[2 * t.r], c.pos.z[2 * t.r]};
-        const double bb[3] = {c.pos.x[2 * t.r + 1], c.pos.y[2 * t.r + 1], c.pos.z[2 * t.r + 1]};
-        end_tile<R, V::KE>(t, rep[t.r], v, a, bb, dt, cut_c, cut_n, prob, *d_step + (uint64_t)step_off);
-        return;
-    }
-    const int n_reset = gx * 2 * cs.R;
-    if (b < n_tiles + n_reset) {
-        const int q = b - n_tiles;
-        end_reset(q / gx, q % gx, gx, list, n, Nmax, contrib, ncontrib, max_contrib);
-        return;
-    }
-    for (int r = (b - n_tiles - n_reset) * blockDim.x + threadIdx.x; r < cs.R;
-         r += (gridDim.x - n_tiles - n_reset) * blockDim.x)
-        end_colloid(r, rep, c, cs, lj_cc, err);
-}
-
-// The arguments of the MD-step halves: the solvent view v and colloid view c
-// with the force / force_old parity of the step whose forces were computed
-// last, and what the halves read besides.
-template <typename R>
-struct StepArgs {
-    const BTile *tiles;
-    int n_tiles, gx;
-    const BRep *rep;
-    PView<R> v;
-    Vec3<R> old;  // solvent pos_old
-    PView<double> c;
-    R dt, dt_sq;
-    double cut_c, cut_n, prob;
-    const uint64_t *d_step;
-    const int *list, *n;
-    int Nmax;
-    const unsigned char *contrib;
-    int *ncontrib, *max_contrib;
-    const double *csnap;
-    LJDev lj_cc;
-    int read_species;
-    unsigned *err;
-};
-
-// block b of the end of step k (RNG step offset step_off) merged with the
-// beginning of step k + 1: [V::FIRST: one block for the colloids] n_tiles
-// particle tiles, gx * 2R counter-clearing blocks, [without V::FIRST: n_col
-// colloid velocity-half blocks].  Returns the thread's largest squared
-// displacement and sets r_tile to the tile's replica (-1 for other blocks).
-template <typename R, typename V>
-__device__ __forceinline__ double eb_vblock(int b, int n_col, const StepArgs<R> &a, const ColloidStep &cs,
-                                            int step_off, int &r_tile)
-{
-    constexpr bool kFirst = V::FIRST;
-    const int n_reset = a.gx * 2 * cs.R;
-    r_tile = -1;
-    if (kFirst && b == 0) {
-        for (int r = threadIdx.x; r < cs.R; r += blockDim.x) {
-            end_colloid(r, a.rep, a.c, cs, a.lj_cc, a.err);
-            cs.co_max[r] = colloid_begin(r, a.rep, cs.c, cs.cold, cs.c_next, cs.rat, cs.mass, cs.ms, cs.d, cs.dt,
-                                         a.err);
-        }
-        return 0;
-    }
-    b -= kFirst ? 1 : 0;
-    if (b < a.n_tiles) {
-        const BTile t = a.tiles[b];
-        const double *p = a.csnap + 6 * (size_t)t.r;
-        const double ca[3] = {p[0], p[1], p[2]}, cb[3] = {p[3], p[4], p[5]};
-        end_tile<R, V::KE>(t, a.rep[t.r], a.v, ca, cb, a.dt, a.cut_c, a.cut_n, a.prob,
-                           *a.d_step + (uint64_t)step_off);
-        // the beginning half reads what the end half wrote: velocities,
-        // flags, species, force_old entries
-        __syncthreads();
-        r_tile = t.r;
-        return begin_tile<R, V::KB>(t, a.v, a.old, a.v.force_old, a.dt, a.dt_sq, a.read_species);
-    }
-    if (b < a.n_tiles + n_reset) {
-        const int q = b - a.n_tiles;
-        end_reset(q / a.gx, q % a.gx, a.gx, a.list, a.n, a.Nmax, a.contrib, a.ncontrib, a.max_contrib);
-    } else if (!kFirst) {
-        for (int r = (b - a.n_tiles - n_reset) * blockDim.x + threadIdx.x; r < cs.R; r += n_col * blockDim.x)
-            end_colloid(r, a.rep, a.c, cs, a.lj_cc, a.err);
-    }
-    return 0;
-}
-
-// The end of MD step k and the beginning of MD step k + 1 in one launch
-// (no re-sort falls between them, and both halves see the same force /
-// force_old parity): each particle tile's block runs the end half over its
-// tile, then the beginning half; the clearing of the contribution counters
-// and the colloid velocity half run in their own blocks as in kb_step_end.
-// With V::FIRST, block 0 runs each replica's colloid velocity half and then
-// its colloid position half (one thread per replica, in that order); without
-// it the velocity halves run in the colloid blocks and the position halves in
-// the last block, after every other block has finished.  change_species reads
-// the colloid positions of step k from csnap (written by kb_pair_forces), as
-// block 0 may already be moving the colloids.
-template <typename R, typename V>
-__global__ void __launch_bounds__(kBT, V::MINB)
-    kb_step_end_begin(StepArgs<R> a, int step_off, unsigned long long *so_max, unsigned *done, int *resort,
-                      int *n_extra, ColloidStep cs, ResortLists rl, cudaGraphConditionalHandle cond, int use_cond,
-                      int *any_out)
-{
-    __shared__ int s_last;
-    __shared__ int ws[kBT / 32 + 1];
-    __shared__ double s_max[kBT / 32];
-    const int n_col = V::FIRST ? 0 : (cs.R + kBT - 1) / kBT;
-    int r_tile;
-    const double m = eb_vblock<R, V>(blockIdx.x, n_col, a, cs, step_off, r_tile);
-    if (!block_done(m, r_tile, so_max, done, s_max, &s_last)) return;
-    begin_tail<V::FIRST>(a.rep, so_max, done, resort, n_extra, cs, rl, cond, use_cond, a.err, ws, any_out);
 }
 
 // ------------------------------------------------------ re-sort / sort
@@ -843,24 +999,73 @@ __global__ void kb_zero_slots(TileSet ts, int *count, unsigned char *is_md,
     }
 }
 
-// apply_pbc (src/md.f90:202-217), then key = replica's first slot + the
-// particle's slot, histogram with one atomic per distinct key per warp
+// The pending md_pos steps of the free particles (adv - base of the replica,
+// added one by one: each step's rounding is kept), the end of their md_vel
+// steps, apply_pbc (src/md.f90:202-217), then key = replica's first slot + the
+// particle's slot, histogram with one atomic per distinct key per warp.  Ends
+// the active particles' places (aidx).
 template <typename R>
 __global__ void __launch_bounds__(kBT)
-    kb_pbc_key_count(TileSet ts, const BRep *rep, PView<R> v, int *key, int *count)
+    kb_advance_key_count(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, int *aidx, const int *adv,
+                         const int *base, R dt, int *key, int *count)
 {
     const int lane = threadIdx.x & 31;
     for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
         const BTile t = ts.tiles[ts.ids[kt]];
         const BRep &rp = rep[t.r];
         const Grid g = rp.g;
-        for (long long base = t.begin; base < t.end; base += blockDim.x) {
-            long long i = base + threadIdx.x;
-            bool ok = i < t.end;
+        const PView<R> v = pick(v0, v1, rp.cur);
+        const int steps = adv[t.r] - base[t.r];
+        for (long long b = t.begin; b < t.end; b += blockDim.x) {
+            const long long i = b + threadIdx.x;
+            const bool ok = i < t.end;
             int k = -1;
             if (ok) {
-                apply_pbc_one(v, i, g.edges[0], g.edges[1], g.edges[2]);
-                k = rp.soff + slot_of(g, (double)v.pos.x[i], (double)v.pos.y[i], (double)v.pos.z[i]);
+                R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
+                const R vx = v.vel.x[i], vy = v.vel.y[i], vz = v.vel.z[i];
+                bool moved = false;
+                if (aidx[i] < 0) {
+                    const R hx = dt * vx, hy = dt * vy, hz = dt * vz;
+#pragma unroll 4
+                    for (int j = 0; j < steps; j++) {
+                        x = x + hx;
+                        y = y + hy;
+                        z = z + hz;
+                    }
+                    // md_pos adds the zero force term too: -0 becomes +0
+                    moved = steps > 0;
+                    x = moved ? x + (R)0 : x;
+                    y = moved ? y + (R)0 : y;
+                    z = moved ? z + (R)0 : z;
+                    const R nx = md_vel_free(vx, dt), ny = md_vel_free(vy, dt), nz = md_vel_free(vz, dt);
+                    if (!same_bits(nx, vx) || !same_bits(ny, vy) || !same_bits(nz, vz)) {
+                        v.vel.x[i] = nx;
+                        v.vel.y[i] = ny;
+                        v.vel.z[i] = nz;
+                    }
+                } else {
+                    aidx[i] = -1;
+                }
+                const int jx = floor_div_edge((double)x, g.edges[0]), jy = floor_div_edge((double)y, g.edges[1]),
+                          jz = floor_div_edge((double)z, g.edges[2]);
+                if (jx) {
+                    v.ix[i] += jx;
+                    x = x - (R)(jx * g.edges[0]);
+                }
+                if (jy) {
+                    v.iy[i] += jy;
+                    y = y - (R)(jy * g.edges[1]);
+                }
+                if (jz) {
+                    v.iz[i] += jz;
+                    z = z - (R)(jz * g.edges[2]);
+                }
+                if (moved || jx || jy || jz) {
+                    v.pos.x[i] = x;
+                    v.pos.y[i] = y;
+                    v.pos.z[i] = z;
+                }
+                k = rp.soff + slot_of(g, (double)x, (double)y, (double)z);
                 key[i] = k;
             }
             unsigned peers = __match_any_sync(0xffffffffu, k);
@@ -894,25 +1099,42 @@ __global__ void __launch_bounds__(kBT) kb_scan_reduce(TileSet ts, const int *cou
     }
 }
 
-// tile offsets of every active replica (its first particle + the sums of
-// its earlier tiles); the replica's colloids get apply_pbc and pos_old = pos
-__global__ void kb_scan_reps(int R, const int *flag, const BRep *rep, const int *first, const int *ntiles,
-                             const long long *tile_sum, long long *tile_off, PView<double> c, Vec3<double> cold)
+// Per replica of the sort (one block): the tile offsets (its first particle +
+// the sums of its earlier tiles); the colloids' apply_pbc and pos_old = pos;
+// the buffers change places (the gather writes the other one); the lists of
+// active particles start anew and the pending md_pos steps are done.
+__global__ void __launch_bounds__(kBT)
+    kb_scan_reps(const int *flag, BRep *rep, const int *first, const int *ntiles, const long long *tile_sum,
+                 long long *tile_off, PView<double> c, Vec3<double> cold, int *adv, int *base, int *nl, int *nx,
+                 int *nf, int *s_free, int *fresh)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) {
-        if (flag && !flag[r]) continue;
-        long long acc = rep[r].off;
-        for (int k = 0; k < ntiles[r]; k++) {
-            tile_off[first[r] + k] = acc;
-            acc += tile_sum[first[r] + k];
-        }
+    __shared__ int ws[33];
+    const int r = blockIdx.x;
+    if (flag && !flag[r]) return;
+    long long acc = rep[r].off;
+    const int f0 = first[r], nt = ntiles[r];
+    for (int k0 = 0; k0 < nt; k0 += kBT) {
+        const int k = k0 + threadIdx.x;
+        int tot;
+        const int ex = block_excl_scan(k < nt ? (int)tile_sum[f0 + k] : 0, ws, &tot);
+        if (k < nt) tile_off[f0 + k] = acc + ex;
+        acc += tot;
+    }
+    if (threadIdx.x < 2) {
+        const int k = 2 * r + threadIdx.x;
         const double *e = rep[r].g.edges;
-        for (int k = 2 * r; k < 2 * r + 2; k++) {
-            apply_pbc_one(c, k, e[0], e[1], e[2]);
-            cold.x[k] = c.pos.x[k];
-            cold.y[k] = c.pos.y[k];
-            cold.z[k] = c.pos.z[k];
-        }
+        apply_pbc_one(c, k, e[0], e[1], e[2]);
+        cold.x[k] = c.pos.x[k];
+        cold.y[k] = c.pos.y[k];
+        cold.z[k] = c.pos.z[k];
+    }
+    if (threadIdx.x == 32) {
+        rep[r].cur ^= 1;
+        if (!flag) adv[r] = 0;  // the interval's sort
+        base[r] = adv[r];
+        nl[r] = nx[r] = nf[r] = 0;
+        s_free[r] = INT_MAX;
+        fresh[r] = 0;
     }
 }
 
@@ -999,17 +1221,22 @@ __global__ void kb_segsort(TileSet ts, const int *count, const int *start, int *
     }
 }
 
+// Every field through perm into the replica's other buffer (current since
+// kb_scan_reps).  Only particles with MD or PAST_MD set have force entries: they
+// are moved and zeroed behind, so the buffer that is not current holds none.
+// Flagged particles are listed (key is free after the placement).
 template <typename R>
-__global__ void __launch_bounds__(kBT) kb_gather(TileSet ts, PView<R> s, PView<R> d, const int *perm)
+__global__ void __launch_bounds__(kBT, 4)
+    kb_gather(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, const int *perm, int *flist, int *nf)
 {
     for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
         const BTile t = ts.tiles[ts.ids[kt]];
+        const BRep &rp = rep[t.r];
+        const PView<R> d = pick(v0, v1, rp.cur), s = pick(v1, v0, rp.cur);
         for (long long j = t.begin + threadIdx.x; j < t.end; j += blockDim.x) {
             const int i = perm[j];
             R px = s.pos.x[i], py = s.pos.y[i], pz = s.pos.z[i];
             R vx = s.vel.x[i], vy = s.vel.y[i], vz = s.vel.z[i];
-            R fx = s.force.x[i], fy = s.force.y[i], fz = s.force.z[i];
-            R gx = s.force_old.x[i], gy = s.force_old.y[i], gz = s.force_old.z[i];
             int ix = s.ix[i], iy = s.iy[i], iz = s.iz[i];
             int id = s.id[i], sp = s.species[i], fl = s.flags[i];
             d.pos.x[j] = px;
@@ -1018,47 +1245,23 @@ __global__ void __launch_bounds__(kBT) kb_gather(TileSet ts, PView<R> s, PView<R
             d.vel.x[j] = vx;
             d.vel.y[j] = vy;
             d.vel.z[j] = vz;
-            d.force.x[j] = fx;
-            d.force.y[j] = fy;
-            d.force.z[j] = fz;
-            d.force_old.x[j] = gx;
-            d.force_old.y[j] = gy;
-            d.force_old.z[j] = gz;
             d.ix[j] = ix;
             d.iy[j] = iy;
             d.iz[j] = iz;
             d.id[j] = id;
             d.species[j] = sp;
             d.flags[j] = fl;
-        }
-    }
-}
-
-// the sorted arrays back into place; the gathered positions stay as pos_old
-template <typename R>
-__global__ void __launch_bounds__(kBT) kb_copyback(TileSet ts, PView<R> d, PView<R> s)
-{
-    for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
-        const BTile t = ts.tiles[ts.ids[kt]];
-        for (long long j = t.begin + threadIdx.x; j < t.end; j += blockDim.x) {
-            d.pos.x[j] = s.pos.x[j];
-            d.pos.y[j] = s.pos.y[j];
-            d.pos.z[j] = s.pos.z[j];
-            d.vel.x[j] = s.vel.x[j];
-            d.vel.y[j] = s.vel.y[j];
-            d.vel.z[j] = s.vel.z[j];
-            d.force.x[j] = s.force.x[j];
-            d.force.y[j] = s.force.y[j];
-            d.force.z[j] = s.force.z[j];
-            d.force_old.x[j] = s.force_old.x[j];
-            d.force_old.y[j] = s.force_old.y[j];
-            d.force_old.z[j] = s.force_old.z[j];
-            d.ix[j] = s.ix[j];
-            d.iy[j] = s.iy[j];
-            d.iz[j] = s.iz[j];
-            d.id[j] = s.id[j];
-            d.species[j] = s.species[j];
-            d.flags[j] = s.flags[j];
+            if (fl & kActiveBits) {
+                flist[rp.off + atomicAdd(nf + t.r, 1)] = (int)j;
+                if (fl & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
+                    for (int k = 0; k < 3; k++) {
+                        d.force[k][j] = s.force[k][i];
+                        d.force_old[k][j] = s.force_old[k][i];
+                        s.force[k][i] = 0;
+                        s.force_old[k][i] = 0;
+                    }
+                }
+            }
         }
     }
 }
@@ -1069,7 +1272,8 @@ __global__ void __launch_bounds__(kBT) kb_copyback(TileSet ts, PView<R> d, PView
 // neighbouring replica's particles, which are read and not used)
 template <typename R>
 __global__ void __launch_bounds__(kNlBlockThreads)
-    kb_update_list(const int *flag, const BRep *rep, PView<double> c, PView<R> s, const int *count, const int *start,
+    kb_update_list(const int *flag, const BRep *rep, PView<double> c, PView<R> v0, PView<R> v1, const int *count,
+                   const int *start,
                    const int *stencil, int n_stencil, double radiussq, LJDev lj, int Nmax, int *list, int *n,
                    unsigned char *is_md, unsigned char *is_reac, unsigned *err)
 {
@@ -1078,18 +1282,21 @@ __global__ void __launch_bounds__(kNlBlockThreads)
     const int i = blockIdx.x, r = i >> 1;
     if (flag && !flag[r]) return;
     const BRep &rp = rep[r];
+    const PView<R> s = pick(v0, v1, rp.cur);
     update_list_block<R>(i, rp.g, c.pos.x, c.pos.y, c.pos.z, c.species, s.pos.x, s.pos.y, s.pos.z, s.species,
                          count + rp.soff, start + rp.soff, stencil, n_stencil, radiussq, lj, 1, Nmax, list, n,
                          is_md + rp.soff, is_reac + rp.soff, err, NlStage{nl_stage, &bar});
 }
 
-// the list kernel's dynamic shared memory above the default limit, set once
+// the kernels with dynamic shared memory above the default limit, set once
 // per precision (at batch creation, before any stream capture)
 template <typename R>
-static int allow_list_stage()
+static int allow_shared()
 {
     static bool set = false;
     if (!set) {
+        RMPCD_CUDA_TRY(cudaFuncSetAttribute(kb_md<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)sizeof(MdShared)));
         RMPCD_CUDA_TRY(cudaFuncSetAttribute(kb_update_list<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)nl_stage_bytes<R>()));
         set = true;
@@ -1105,11 +1312,13 @@ static int allow_list_stage()
 template <typename R>
 __global__ void __launch_bounds__(kBT)
     kb_srd_refuel(const BTile *stiles, int n_stiles, const BTile *ptiles, const BRep *rep, const int *count,
-                  const int *start, PView<R> v, PView<double> c, SrdParams q, const uint64_t *d_step, int step_off)
+                  const int *start, PView<R> v0, PView<R> v1, PView<double> c, SrdParams q, const uint64_t *d_step,
+                  int step_off)
 {
     if ((int)blockIdx.x < n_stiles) {
         const BTile t = stiles[blockIdx.x];
         const BRep &rp = rep[t.r];
+        const PView<R> v = pick(v0, v1, rp.cur);
         q.seed = rp.seed;
         q.step = *d_step + (uint64_t)step_off;
         for (long long s = t.begin + threadIdx.x; s < t.end; s += blockDim.x)
@@ -1118,6 +1327,7 @@ __global__ void __launch_bounds__(kBT)
     }
     const BTile t = ptiles[blockIdx.x - n_stiles];
     const BRep &rp = rep[t.r];
+    const PView<R> v = pick(v0, v1, rp.cur);
     const double a[3] = {c.pos.x[2 * t.r], c.pos.y[2 * t.r], c.pos.z[2 * t.r]};
     const double b[3] = {c.pos.x[2 * t.r + 1], c.pos.y[2 * t.r + 1], c.pos.z[2 * t.r + 1]};
     for (long long i = t.begin + threadIdx.x; i < t.end; i += blockDim.x)
@@ -1165,30 +1375,40 @@ static int resort_grid(int n_tiles)
 }
 
 // the re-sort of the flagged replicas (flag = resort flags, lists = their
-// tiles) or of every replica (flag = null, lists = all tiles)
+// tiles) or of every replica (flag = null, lists = all tiles), then the active
+// particles of what was sorted
 template <typename R>
-static void resort_launches(Batch *b, const int *flag, bool all, cudaStream_t st, int shift_step_off)
+static TileSet particle_tiles(const Batch *b, const int *flag)
 {
-    PView<R> cur = phys<R>(b->sol, 0), alt = phys<R>(b->sol, 1);
-    PView<double> cv = phys<double>(b->col, 0), ca = phys<double>(b->col, 1);
-    TileSet pts{b->ptile, all ? b->all_p : b->act_p, all ? b->n_all : b->n_act};
-    TileSet sts{b->stile, all ? b->all_s : b->act_s, (all ? b->n_all : b->n_act) + 1};
+    return TileSet{b->ptile, flag ? b->act_p : b->all_p, flag ? b->n_act : b->n_all};
+}
+
+template <typename R>
+static void resort_launches(Batch *b, const int *flag, cudaStream_t st, int shift_step_off)
+{
+    const PView<R> v0 = phys<R>(b->sol, 0), v1 = phys<R>(b->sol, 1);
+    const PView<double> cv = phys<double>(b->col, 0);
+    const TileSet pts = particle_tiles<R>(b, flag);
+    const TileSet sts{b->stile, flag ? b->act_s : b->all_s, (flag ? b->n_act : b->n_all) + 1};
     const int gp = resort_grid(b->n_ptile), gs = resort_grid(b->n_stile);
+    const R dt = (R)(b->prm.tau / b->prm.N_MD);
     kb_zero_slots<<<gs, kBT, 0, st>>>(sts, b->count, b->is_md, b->is_reac, b->n_big, b->R, b->rep, b->d_step,
                                       shift_step_off);
-    kb_pbc_key_count<R><<<gp, kBT, 0, st>>>(pts, b->rep, cur, b->sol->key, b->count);
+    kb_advance_key_count<R><<<gp, kBT, 0, st>>>(pts, b->rep, v0, v1, b->aidx, b->adv, b->base, dt, b->sol->key,
+                                                b->count);
     kb_scan_reduce<<<gs, kBT, 0, st>>>(sts, b->count, b->tile_sum);
-    kb_scan_reps<<<grid_cap(b->R, 128), 128, 0, st>>>(b->R, flag, b->rep, b->stile_first, b->stile_count, b->tile_sum,
-                                                      b->tile_off, cv, ca.pos);
+    kb_scan_reps<<<b->R, kBT, 0, st>>>(flag, b->rep, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, cv,
+                                       phys<double>(b->col, 1).pos, b->adv, b->base, b->nl, b->nx, b->nf, b->s_free,
+                                       b->fresh);
     kb_scan_apply<<<gs, kBT, 0, st>>>(sts, b->count, b->tile_off, b->start, b->cursor);
     kb_perm<<<gp, kBT, 0, st>>>(pts, b->sol->key, b->cursor, b->sol->perm);
     kb_segsort<<<gs, kBT, 0, st>>>(sts, b->count, b->start, b->sol->perm, b->big, b->n_big);
     launch_segsort_big(b->start, b->count, b->big, b->n_big, b->sol->perm, b->sol->key, st);
-    kb_gather<R><<<gp, kBT, 0, st>>>(pts, cur, alt, b->sol->perm);
-    kb_copyback<R><<<gp, kBT, 0, st>>>(pts, cur, alt);
+    kb_gather<R><<<gp, kBT, 0, st>>>(pts, b->rep, v0, v1, b->sol->perm, b->sol->key, b->nf);
     kb_update_list<R><<<2 * b->R, kNlBlockThreads, nl_stage_bytes<R>(), st>>>(
-        flag, b->rep, cv, cur, b->count, b->start, b->stencil, b->n_stencil, b->prm.list_radius * b->prm.list_radius,
-        b->lj_sc, b->Nmax, b->list, b->nn, b->is_md, b->is_reac, dev_error_word());
+        flag, b->rep, cv, v0, v1, b->count, b->start, b->stencil, b->n_stencil,
+        b->prm.list_radius * b->prm.list_radius, b->lj_sc, b->Nmax, b->list, b->nn, b->is_md, b->is_reac,
+        dev_error_word());
 }
 
 static void note(Batch *b, cudaError_t e)
@@ -1205,171 +1425,157 @@ static int list_gx(const Batch *b)
     return gx > 64 ? 64 : gx < 1 ? 1 : gx;
 }
 
-// the MD-step halves' arguments with force / force_old of the given parity
-template <typename R>
-static StepArgs<R> step_args(const Batch *b, int parity, int gx)
+// Blocks per replica of kb_md, one block per SM: as many as leave every
+// replica's cluster resident at once (a replica's 6,000 active particles then
+// take 2, 3, 6 or 12 per thread and step), 8 being the portable maximum.
+// Clusters of 8 and 4 blocks do not fill every SM of a processing cluster, so
+// their share of the device is taken as 128 of 148.
+static int md_cluster(const Batch *b)
 {
+    const int set = kClusters[shape_var(b->shape)];
+    if (set) return set;
+    const int sms = sm_count(), most = sms * 128 / 148;
+    return b->R * 8 <= most ? 8 : b->R * 4 <= most ? 4 : b->R * 2 <= sms ? 2 : 1;
+}
+
+// the active particles of the replicas in flag (every one when null), then
+// their MD steps up to the next re-sort or the interval's end
+template <typename R>
+static void md_launches(Batch *b, const int *flag, cudaStream_t st, cudaGraphConditionalHandle cond)
+{
+    const PView<R> v0 = phys<R>(b->sol, 0), v1 = phys<R>(b->sol, 1);
     const double dt = b->prm.tau / b->prm.N_MD;
-    const double dt_sq = dt * dt / 2;
-    return StepArgs<R>{b->ptile, b->n_ptile, gx, b->rep, live<R>(b->sol, parity), phys<R>(b->sol, 1).pos,
-                       live<double>(b->col, parity), (R)dt, (R)dt_sq, b->prm.cut_sq_C, b->prm.cut_sq_N, b->prm.prob,
-                       b->d_step, b->list, b->nn, b->Nmax, b->contrib, b->ncontrib, b->max_contrib, b->csnap,
-                       b->lj_cc, b->read_species ? 1 : 0, dev_error_word()};
+    const int gx = list_gx(b), gp = resort_grid(b->n_ptile);
+    kb_claim<<<dim3(gx, 2 * b->R), kBT, 0, st>>>(flag, b->rep, b->list, b->nn, b->Nmax, b->aidx, b->act, b->nl,
+                                                 b->mult);
+    kb_classify<R><<<gp + gx * 2 * b->R + b->R, kBT, 0, st>>>(
+        particle_tiles<R>(b, flag), gp, gx, b->R, flag, b->rep, v0, v1, (R)dt, b->prm.skin * 0.89, b->prm.N_MD,
+        b->read_species ? 1 : 0, b->base, b->fresh, b->s_free, b->list, b->nn, b->Nmax, b->aidx, b->act, b->nl, b->nx,
+        b->mult, b->amap, b->sol->key, b->nf);
+    MdArgs<R> a;
+    a.rep = b->rep;
+    a.v0 = v0;
+    a.v1 = v1;
+    a.c = phys<double>(b->col, 0);
+    a.cold = phys<double>(b->col, 1).pos;
+    for (int k = 0; k < 3; k++) a.rat[k] = b->rattle[k];
+    a.mass = b->vv_mass;
+    a.ms = b->ms;
+    a.bond = b->prm.bond;
+    a.dt = dt;
+    a.skin = b->prm.skin;
+    a.dt_r = (R)dt;
+    a.dt_sq_r = (R)(dt * dt / 2);
+    a.cut_c = b->prm.cut_sq_C;
+    a.cut_n = b->prm.cut_sq_N;
+    a.prob = b->prm.prob;
+    a.lj_sc = b->lj_sc;
+    a.lj_cc = b->lj_cc;
+    a.R_ = b->R;
+    a.N_MD = b->prm.N_MD;
+    a.Nmax = b->Nmax;
+    a.start = flag ? 0 : 1;
+    a.read_species = b->read_species ? 1 : 0;
+    a.d_step = b->d_step;
+    a.n = b->nn;
+    a.amap = b->amap;
+    a.act = b->act;
+    a.nl = b->nl;
+    a.nx = b->nx;
+    a.mult = b->mult;
+    a.pf = b->pf;
+    a.cf = b->cf;
+    a.s_free = b->s_free;
+    a.fresh = b->fresh;
+    a.adv = b->adv;
+    a.resort = b->resort;
+    a.n_extra = b->n_extra;
+    a.rl = ResortLists{b->ptile_first, b->ptile_count, b->stile_first, b->stile_count, b->act_p, b->act_s, b->n_act};
+    a.done = b->done;
+    a.any = b->any;
+    a.cond = cond;
+    a.use_cond = b->capturing ? 1 : 0;
+    a.err = dev_error_word();
+    const int blocks = md_cluster(b);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks * b->R);
+    cfg.blockDim = dim3(kMdThreads);
+    cfg.dynamicSmemBytes = sizeof(MdShared);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = blocks;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    note(b, cudaLaunchKernelEx(&cfg, kb_md<R>, a));
 }
 
-// the MD step's forces: the pair forces, then their three consumers (skip,
-// if given: see kb_pair_forces)
+// an interval's MD steps in the graph being captured on st: the steps up to
+// every replica's first re-sort, then a WHILE node whose body re-sorts the
+// replicas that wait for it and continues them
 template <typename R>
-static void force_launches(Batch *b, cudaStream_t st, const int *skip)
-{
-    const PView<R> s = live<R>(b->sol, b->parity);
-    const PView<double> c = live<double>(b->col, b->parity);
-    const int gx = list_gx(b);
-    kb_pair_forces<R><<<dim3(gx, 2 * b->R), 256, 0, st>>>(b->rep, c, s, b->list, b->nn, b->Nmax, b->lj_sc, b->pair_f,
-                                                          b->pair_e, b->contrib, b->ncontrib, b->max_contrib,
-                                                          b->prm.cut_sq_C, b->csnap, skip);
-    kb_apply_sum<R><<<gx * 2 * b->R + 3 * b->R, 256, 0, st>>>(
-        b->rep, b->R, gx, b->list, b->nn, b->Nmax, b->contrib, b->pair_f, b->ncontrib, b->max_contrib, s.force.x,
-        s.force.y, s.force.z, c.force.x, c.force.y, c.force.z, b->clist, b->cn, skip);
-}
-
-// the program's re-sort test, as an IF node of the graph g being captured on
-// st whose body (captured on `nested`) is the re-sort of the flagged
-// replicas, followed by the step's forces when with_forces; cond was created
-// before the kernel that sets it was captured
-template <typename R>
-static void capture_conditional_resort(Batch *b, cudaStream_t st, cudaGraph_t g, cudaGraphConditionalHandle cond,
-                                       cudaStream_t nested, bool with_forces)
+static void capture_md(Batch *b, cudaStream_t st)
 {
     cudaStreamCaptureStatus cs;
+    cudaGraph_t g = nullptr;
+    note(b, cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, nullptr, nullptr));
+    cudaGraphConditionalHandle cond = 0;
+    note(b, cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
+    md_launches<R>(b, nullptr, st, cond);
     const cudaGraphNode_t *deps = nullptr;
     size_t nd = 0;
     note(b, cudaStreamGetCaptureInfo(st, &cs, nullptr, nullptr, &deps, &nd));
     cudaGraphNodeParams cp{};
     cp.type = cudaGraphNodeTypeConditional;
     cp.conditional.handle = cond;
-    cp.conditional.type = cudaGraphCondTypeIf;
+    cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
     cudaGraphNode_t node = nullptr;
     note(b, cudaGraphAddNode(&node, g, deps, nd, &cp));
     if (b->cap_err != cudaSuccess) return;
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     note(b, cudaStreamUpdateCaptureDependencies(st, &node, 1, cudaStreamSetCaptureDependencies));
-    note(b, cudaStreamBeginCaptureToGraph(nested, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    resort_launches<R>(b, b->resort, false, nested, -1);
-    if (with_forces) force_launches<R>(b, nested, nullptr);
+    note(b, cudaStreamBeginCaptureToGraph(b->body, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    resort_launches<R>(b, b->resort, b->body, -1);
+    md_launches<R>(b, b->resort, b->body, cond);
     cudaGraph_t out = nullptr;
-    note(b, cudaStreamEndCapture(nested, &out));
-}
-
-// a fresh IF-node handle in the graph being captured on st (0 when not
-// capturing)
-static cudaGraphConditionalHandle new_cond(Batch *b, cudaStream_t st)
-{
-    cudaGraphConditionalHandle cond = 0;
-    if (b->capturing) {
-        cudaStreamCaptureStatus st_cap;
-        cudaGraph_t g = nullptr;
-        note(b, cudaStreamGetCaptureInfo(st, &st_cap, nullptr, &g, nullptr, nullptr));
-        note(b, cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
-    }
-    return cond;
-}
-
-// MD step k of the interval: its beginning (for k = 0; later steps begin in
-// the previous step's kb_step_end_begin), the re-sort test, the forces and
-// its end, merged with the beginning of step k + 1 unless k is the last
-template <typename R, typename V>
-static void md_step_launches(Batch *b, int k)
-{
-    cudaStream_t st = stream();
-    const double dt = b->prm.tau / b->prm.N_MD;
-    const double dt_sq = dt * dt / 2;
-    PView<R> s = live<R>(b->sol, b->parity);
-    PView<double> c = live<double>(b->col, b->parity);
-    PView<R> alt = phys<R>(b->sol, 1);
-    PView<double> ca = phys<double>(b->col, 1);
-    ColloidStep cs{c, ca.pos, c.force_old, {b->rattle[0], b->rattle[1], b->rattle[2]}, b->vv_mass, b->ms,
-                   b->prm.bond, dt, b->prm.skin, b->R, b->co_max};
-    const ResortLists rl{b->ptile_first, b->ptile_count, b->stile_first, b->stile_count, b->act_p, b->act_s, b->n_act};
-    const int use_cond = b->capturing ? 1 : 0, read_species = b->read_species ? 1 : 0;
-    cudaGraphConditionalHandle cond = b->cond_next;
-    if (k == 0) {
-        cond = new_cond(b, st);
-        kb_step_begin<R, V><<<b->n_ptile + (V::FIRST ? 1 : 0), kBT, 0, st>>>(
-            b->ptile, b->rep, s, alt.pos, s.force_old, (R)dt, (R)dt_sq, b->so_max, b->done, b->resort, b->n_extra,
-            cs, rl, cond, use_cond, read_species, dev_error_word(), b->any);
-    }
-    // switch_force: the cleared entries become `force` (the re-sort does not
-    // read the force buffers)
-    b->parity ^= 1;
-    s = live<R>(b->sol, b->parity);
-    c = live<double>(b->col, b->parity);
-    cs.c = c;
-    cs.c_next = c.force_old;
-    const int gx = list_gx(b);
-    if (b->capturing) {
-        // the re-sort test as an IF node whose body re-sorts and then
-        // evaluates the forces, beside a branch that evaluates them at once
-        // unless the beginning decided to re-sort: the IF node's latency then
-        // overlaps the forces of every step without a re-sort
-        note(b, cudaEventRecord(b->ev_fork, st));
-        note(b, cudaStreamWaitEvent(b->side, b->ev_fork, 0));
-        cudaStreamCaptureStatus st_cap;
-        cudaGraph_t g = nullptr;
-        note(b, cudaStreamGetCaptureInfo(st, &st_cap, nullptr, &g, nullptr, nullptr));
-        capture_conditional_resort<R>(b, st, g, cond, b->body, true);
-        force_launches<R>(b, b->side, b->any);
-        note(b, cudaEventRecord(b->ev_join, b->side));
-        note(b, cudaStreamWaitEvent(st, b->ev_join, 0));
-    } else {
-        resort_launches<R>(b, b->resort, false, st, -1);
-        force_launches<R>(b, st, nullptr);
-    }
-    const int n_col_blocks = (b->R + kBT - 1) / kBT;
-    const int n_reset = gx * 2 * b->R;
-    if (k + 1 < b->prm.N_MD) {
-        b->cond_next = new_cond(b, st);
-        kb_step_end_begin<R, V><<<(V::FIRST ? 1 : n_col_blocks) + b->n_ptile + n_reset, kBT, 0, st>>>(
-            step_args<R>(b, b->parity, gx), k, b->so_max, b->done, b->resort, b->n_extra, cs, rl, b->cond_next,
-            use_cond, b->any);
-    } else {
-        b->cond_next = 0;
-        kb_step_end<R, V><<<b->n_ptile + n_reset + n_col_blocks, kBT, 0, st>>>(
-            b->ptile, b->n_ptile, gx, b->rep, s, c, (R)dt, b->prm.cut_sq_C, b->prm.cut_sq_N, b->prm.prob, b->d_step,
-            k, b->list, b->nn, b->Nmax, b->contrib, b->ncontrib, b->max_contrib, cs, b->lj_cc, dev_error_word());
-    }
-}
-
-template <typename R, int Var>
-static void md_steps(Batch *b)
-{
-    for (int k = 0; k < b->prm.N_MD; k++) md_step_launches<R, typename BVarOf<R, Var>::T>(b, k);
+    note(b, cudaStreamEndCapture(b->body, &out));
 }
 
 template <typename R>
-static void interval_launches(Batch *b)
+static int interval_launches(Batch *b)
 {
     cudaStream_t st = stream();
     const int N_MD = b->prm.N_MD;
-    switch (shape_var(b->shape)) {
-    case 1: md_steps<R, 1>(b); break;
-    case 2: md_steps<R, 2>(b); break;
-    case 3: md_steps<R, 3>(b); break;
-    case 4: md_steps<R, 4>(b); break;
-    default: md_steps<R, 0>(b); break;
+    if (b->capturing) {
+        capture_md<R>(b, st);
+    } else {
+        md_launches<R>(b, nullptr, st, 0);
+        for (;;) {
+            int any = 0;
+            if (b->cap_err != cudaSuccess)
+                return fail(RMPCD_ERR_CUDA, "dimer batch: %s", cudaGetErrorString(b->cap_err));
+            RMPCD_CUDA_TRY(cudaMemcpyAsync(&any, b->any, sizeof(int), cudaMemcpyDeviceToHost, st));
+            RMPCD_CUDA_TRY(cudaStreamSynchronize(st));
+            if (!any) break;
+            resort_launches<R>(b, b->resort, st, -1);
+            md_launches<R>(b, b->resort, st, 0);
+        }
     }
-    resort_launches<R>(b, nullptr, true, st, N_MD);
+    resort_launches<R>(b, nullptr, st, N_MD);
     SrdParams q{};
     q.sin_a = 1;
     q.cos_a = 0;
     q.thermostat = b->prm.thermostat ? 1 : 0;
     q.hydro = b->prm.hydro ? 1 : 0;
     q.t_factor = b->prm.thermostat ? sqrt(b->prm.T) : 0.0;
-    kb_srd_refuel<R><<<b->n_stile + b->n_ptile, kBT, 0, st>>>(b->stile, b->n_stile, b->ptile, b->rep, b->count, b->start,
-                                                              live<R>(b->sol, b->parity), live<double>(b->col, b->parity),
-                                                              q, b->d_step, N_MD + 1);
+    kb_srd_refuel<R><<<b->n_stile + b->n_ptile, kBT, 0, st>>>(b->stile, b->n_stile, b->ptile, b->rep, b->count,
+                                                              b->start, phys<R>(b->sol, 0), phys<R>(b->sol, 1),
+                                                              phys<double>(b->col, 0), q, b->d_step, N_MD + 1);
     kb_advance<<<1, 1, 0, st>>>(b->d_step, (uint64_t)N_MD + 2);
+    return RMPCD_OK;
 }
 
 template <typename R>
@@ -1378,12 +1584,14 @@ static int run_t(Batch *b, int n_intervals)
     cudaStream_t st = stream();
     for (int it = 0; it < n_intervals; it++) {
         PhaseTimer t("batch_interval");
+        b->ran = true;
         if (!b->use_graph) {
-            interval_launches<R>(b);
+            b->cap_err = cudaSuccess;
+            int rc = interval_launches<R>(b);
+            if (rc) return rc;
             RMPCD_CHECK_LAUNCH();
         } else {
-            const int p0 = b->parity;
-            if (!b->exec[p0]) {
+            if (!b->exec) {
                 cudaGraph_t g = nullptr;
                 b->cap_err = cudaSuccess;
                 RMPCD_CUDA_TRY(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1392,18 +1600,15 @@ static int run_t(Batch *b, int n_intervals)
                 b->capturing = false;
                 cudaError_t e = cudaStreamEndCapture(st, &g);
                 if (e == cudaSuccess && b->cap_err != cudaSuccess) e = b->cap_err;
-                if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[p0], g, 0);
+                if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec, g, 0);
                 if (g) cudaGraphDestroy(g);
                 if (e != cudaSuccess) {
-                    b->exec[p0] = nullptr;
-                    b->parity = p0;
+                    b->exec = nullptr;
                     cudaGetLastError();
                     return fail(RMPCD_ERR_CUDA, "interval graph: %s", cudaGetErrorString(e));
                 }
-            } else {
-                b->parity ^= (b->prm.N_MD & 1);
             }
-            RMPCD_CUDA_TRY(cudaGraphLaunch(b->exec[p0], st));
+            RMPCD_CUDA_TRY(cudaGraphLaunch(b->exec, st));
         }
         b->step += (uint64_t)b->prm.N_MD + 2;
     }
@@ -1414,21 +1619,16 @@ static void free_batch(Batch *b)
 {
     if (!b) return;
     cudaStreamSynchronize(stream());
-    for (auto &e : b->exec)
-        if (e) cudaGraphExecDestroy(e);
+    if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->body) cudaStreamDestroy(b->body);
-    if (b->side) cudaStreamDestroy(b->side);
-    if (b->ev_fork) cudaEventDestroy(b->ev_fork);
-    if (b->ev_join) cudaEventDestroy(b->ev_join);
     rmpcd_particles_destroy(b->sol);
     rmpcd_particles_destroy(b->col);
     void *ptrs[] = {b->rep, b->ptile, b->stile, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, b->count,
-                    b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->pair_f, b->pair_e,
-                    b->contrib, b->ncontrib, b->max_contrib, b->clist, b->cn, b->so_max, b->co_max, b->csnap, b->resort,
-                    b->n_extra,
-                    b->big, b->n_big, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step, b->done,
-                    b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s, b->n_all,
-                    b->any};
+                    b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->act, b->nl, b->nx,
+                    b->aidx, b->amap, b->mult, b->pf, b->cf, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
+                    b->n_extra, b->big, b->n_big, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
+                    b->done, b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s,
+                    b->n_all, b->any};
     for (void *q : ptrs) cudaFree(q);
     for (int *l : b->luts) cudaFree(l);
     delete b;
@@ -1490,24 +1690,22 @@ static int build_particle_tiles(Batch *b, long long ptile)
     return RMPCD_OK;
 }
 
-// copy one particle system's current arrays (and pos_old) to/from the batch
-// system at offset off; force/force_old follow the batch's parity
-static int move_particles(Batch *b, rmpcd_particles *big, rmpcd_particles *p, long long off, bool to_batch)
+// copy one particle system's current arrays (and pos_old) to/from buffer bc of
+// the batch system at offset off; pos_old is buffer bo's positions
+static int move_particles(rmpcd_particles *big, int bc, int bo, rmpcd_particles *p, long long off, bool to_batch)
 {
     const size_t rs = (size_t)big->rsize, n = (size_t)p->N;
-    const int bc = 0, pc = p->cur;
+    const int pc = p->cur;
     for (int k = 0; k < 3; k++) {
-        char *bp = (char *)big->pos[bc][k] + off * rs, *bo = (char *)big->pos[1][k] + off * rs;
-        char *bv = (char *)big->vel[bc][k] + off * rs;
-        char *bf = (char *)(b->parity ? big->force_old : big->force)[bc][k] + off * rs;
-        char *bg = (char *)(b->parity ? big->force : big->force_old)[bc][k] + off * rs;
-        int *bi = big->image[bc][k] + off;
         struct {
             void *a, *b;
             size_t bytes;
-        } m[] = {{bp, p->pos[pc][k], n * rs},     {bo, p->pos[1 - pc][k], n * rs}, {bv, p->vel[pc][k], n * rs},
-                 {bf, p->force[pc][k], n * rs},   {bg, p->force_old[pc][k], n * rs},
-                 {bi, p->image[pc][k], n * sizeof(int)}};
+        } m[] = {{(char *)big->pos[bc][k] + off * rs, p->pos[pc][k], n * rs},
+                 {(char *)big->pos[bo][k] + off * rs, p->pos[1 - pc][k], n * rs},
+                 {(char *)big->vel[bc][k] + off * rs, p->vel[pc][k], n * rs},
+                 {(char *)big->force[bc][k] + off * rs, p->force[pc][k], n * rs},
+                 {(char *)big->force_old[bc][k] + off * rs, p->force_old[pc][k], n * rs},
+                 {big->image[bc][k] + off, p->image[pc][k], n * sizeof(int)}};
         for (auto &e : m) {
             int rc = to_batch ? d2d(e.a, e.b, e.bytes) : d2d(e.b, e.a, e.bytes);
             if (rc) return rc;
@@ -1569,11 +1767,10 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     b->ms.n = col[0]->n_species;
     for (int s = 0; s < RMPCD_MAX_SPECIES; s++) b->ms.m[s] = col[0]->mass[s];
     // replica layout and tiles
-    // default shape: variant 0 and 1024-particle tiles, smaller only for
-    // batches too small to give ~2 tiles per SM: each tile's block is one
-    // round trip to DRAM, so fewer, fuller tiles beat more blocks (one 32^3
-    // dimer: 1024-particle tiles take the MD step from 45.8 to 38.0 us against
-    // 256-particle ones); rmpcd_dimer_batch_autotune times the others
+    // default shape: the cluster by the number of replicas (md_cluster) and
+    // 1024-particle tiles, smaller only for batches too small to give ~2 tiles
+    // per SM: each tile's block is one round trip to DRAM, so fewer, fuller
+    // tiles beat more blocks; rmpcd_dimer_batch_autotune times the others
     long long n_total = 0;
     for (int r = 0; r < R; r++) n_total += sol[r]->N;
     int tile_k = 2;  // kPTiles[2] = 1024
@@ -1596,9 +1793,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
         p.soff = (int)soff;
         p.S = c->S;
         p.seed = rngs[r].seed;
-        p.serial = 0;
-        for (int k = 0; k < 3; k++)
-            if (2 * nl[r]->max_i + 1 > c->L[k]) p.serial = 1;
+        p.cur = 0;
         volatile float lf = (float)c->L[0] * 0.45f;
         volatile float ff = lf * lf;
         p.far = (double)ff;
@@ -1635,18 +1830,15 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
               !dalloc(&b->tile_off, stl.size()) && !dalloc(&b->count, soff) && !dalloc(&b->start, soff) &&
               !dalloc(&b->cursor, soff) && !dalloc(&b->is_md, soff) && !dalloc(&b->is_reac, soff) &&
               !dalloc(&b->stencil, 3 * (size_t)b->n_stencil) && !dalloc(&b->list, ne) && !dalloc(&b->nn, 2 * (size_t)R) &&
-              !dalloc(&b->pair_f, 3 * ne) && !dalloc(&b->pair_e, ne) && !dalloc(&b->contrib, ne) &&
-              !dalloc(&b->ncontrib, off) && !dalloc(&b->max_contrib, R) && !dalloc(&b->clist, ne) &&
-              !dalloc(&b->cn, 2 * (size_t)R) && !dalloc(&b->so_max, R) && !dalloc(&b->co_max, R) &&
-              !dalloc(&b->csnap, 6 * (size_t)R) && !dalloc(&b->resort, R) &&
+              !dalloc(&b->act, off) && !dalloc(&b->nl, R) && !dalloc(&b->nx, R) && !dalloc(&b->aidx, off) &&
+              !dalloc(&b->amap, ne) && !dalloc(&b->mult, ne) && !dalloc(&b->pf, 6 * ne) && !dalloc(&b->cf, ne) &&
+              !dalloc(&b->nf, R) && !dalloc(&b->s_free, R) && !dalloc(&b->adv, R) && !dalloc(&b->base, R) &&
+              !dalloc(&b->fresh, R) && !dalloc(&b->resort, R) &&
               !dalloc(&b->n_extra, R) && !dalloc(&b->big, soff) && !dalloc(&b->n_big, 1) &&
               !dalloc(&b->rattle[0], 2 * (size_t)R) && !dalloc(&b->rattle[1], 2 * (size_t)R) &&
               !dalloc(&b->rattle[2], 2 * (size_t)R) && !dalloc(&b->vv_mass, 2 * (size_t)R) && !dalloc(&b->d_step, 1) &&
               !dalloc(&b->done, 1) && cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking) == cudaSuccess &&
               !dalloc(&b->any, 1) &&
-              cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) == cudaSuccess &&
-              cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) == cudaSuccess &&
               !dalloc(&b->ptile_first, R) && !dalloc(&b->ptile_count, R) && !dalloc(&b->act_p, cap_p) &&
               !dalloc(&b->act_s, stl.size()) && !dalloc(&b->n_act, 2) && !dalloc(&b->all_p, cap_p) &&
               !dalloc(&b->all_s, stl.size()) && !dalloc(&b->n_all, 2);
@@ -1659,7 +1851,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
         free_batch(b);
         return RMPCD_ERR_CUDA;
     }
-    if ((b->precision == RMPCD_FP32 ? allow_list_stage<float>() : allow_list_stage<double>()) != RMPCD_OK) {
+    if ((b->precision == RMPCD_FP32 ? allow_shared<float>() : allow_shared<double>()) != RMPCD_OK) {
         free_batch(b);
         return RMPCD_ERR_CUDA;
     }
@@ -1688,9 +1880,12 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     RMPCD_CUDA_TRY(cudaMemcpyAsync(b->n_act, n_none, sizeof(n_none), cudaMemcpyHostToDevice, st));
     RMPCD_CUDA_TRY(cudaMemcpyAsync(b->vv_mass, vm.data(), vm.size() * sizeof(double), cudaMemcpyHostToDevice, st));
     RMPCD_CUDA_TRY(cudaMemcpyAsync(b->d_step, &b->step, sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    RMPCD_CUDA_TRY(cudaMemsetAsync(b->ncontrib, 0, (size_t)off * sizeof(int), st));
-    RMPCD_CUDA_TRY(cudaMemsetAsync(b->max_contrib, 0, (size_t)R * sizeof(int), st));
-    RMPCD_CUDA_TRY(cudaMemsetAsync(b->so_max, 0, (size_t)R * sizeof(unsigned long long), st));
+    RMPCD_CUDA_TRY(cudaMemsetAsync(b->aidx, 0xff, (size_t)off * sizeof(int), st));
+    for (int *z : {b->nl, b->nx, b->nf, b->adv, b->base})
+        RMPCD_CUDA_TRY(cudaMemsetAsync(z, 0, (size_t)R * sizeof(int), st));
+    const std::vector<int> never(R, INT_MAX), yes(R, 1);
+    RMPCD_CUDA_TRY(cudaMemcpyAsync(b->s_free, never.data(), R * sizeof(int), cudaMemcpyHostToDevice, st));
+    RMPCD_CUDA_TRY(cudaMemcpyAsync(b->fresh, yes.data(), R * sizeof(int), cudaMemcpyHostToDevice, st));
     RMPCD_CUDA_TRY(cudaMemsetAsync(b->n_extra, 0, (size_t)R * sizeof(int), st));
     RMPCD_CUDA_TRY(cudaMemsetAsync(b->resort, 0, (size_t)R * sizeof(int), st));
     RMPCD_CUDA_TRY(cudaMemsetAsync(b->done, 0, sizeof(unsigned), st));
@@ -1698,7 +1893,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     d2d(b->stencil, nl[0]->stencil, 3 * (size_t)b->n_stencil * sizeof(int));
     for (int r = 0; r < R; r++) {
         const BRep &p = b->rep_h[r];
-        if ((rc = move_particles(b, b->sol, sol[r], p.off, true)) || (rc = move_particles(b, b->col, col[r], 2 * r, true))) {
+        if ((rc = move_particles(b->sol, 0, 1, sol[r], p.off, true)) || (rc = move_particles(b->col, 0, 1, col[r], 2 * r, true))) {
             free_batch(b);
             return rc;
         }
@@ -1710,6 +1905,14 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
         k_list_offset<<<grid_cap(2 * (long long)b->Nmax, 256), 256, 0, st>>>(b->list + (size_t)2 * r * b->Nmax, nl[r]->list,
                                                                           nl[r]->n, 2, b->Nmax, p.off);
         d2d(b->nn + 2 * r, nl[r]->n, 2 * sizeof(int));
+    }
+    {
+        TileSet all{b->ptile, b->all_p, b->n_all};
+        const int gp = resort_grid(b->n_ptile);
+        if (b->precision == RMPCD_FP32)
+            kb_collect_flagged<float><<<gp, kBT, 0, st>>>(all, b->rep, phys<float>(b->sol, 0), b->sol->key, b->nf);
+        else
+            kb_collect_flagged<double><<<gp, kBT, 0, st>>>(all, b->rep, phys<double>(b->sol, 0), b->sol->key, b->nf);
     }
     {
         int *neg = nullptr, h_neg = 1;
@@ -1735,14 +1938,18 @@ static int scatter(Batch *b, int r, rmpcd_particles *sol, rmpcd_particles *col, 
     RMPCD_ARG(b && r >= 0 && r < b->R, "dimer batch: replica index out of range");
     const BRep &p = b->rep_h[r];
     cudaStream_t st = stream();
-    int rc;
+    BRep now;
+    RMPCD_CUDA_TRY(cudaMemcpyAsync(&now, b->rep + r, sizeof(BRep), cudaMemcpyDeviceToHost, st));
+    int rc = sync();
+    if (rc) return rc;
     if (sol) {
         RMPCD_ARG(sol->N == p.n && sol->precision == b->precision, "dimer batch: solvent handle does not match");
-        if ((rc = move_particles(b, b->sol, sol, p.off, false))) return rc;
+        // an interval ends with its sort, where pos_old = pos
+        if ((rc = move_particles(b->sol, now.cur, b->ran ? now.cur : 1, sol, p.off, false))) return rc;
     }
     if (col) {
         RMPCD_ARG(col->N == 2 && col->precision == RMPCD_FP64, "dimer batch: colloid handle does not match");
-        if ((rc = move_particles(b, b->col, col, 2 * r, false))) return rc;
+        if ((rc = move_particles(b->col, 0, 1, col, 2 * r, false))) return rc;
         if (!col->pos_rattle[0])
             for (int k = 0; k < 3; k++) RMPCD_CUDA_TRY(cudaMalloc(&col->pos_rattle[k], 2 * sizeof(double)));
         for (int k = 0; k < 3; k++) d2d(col->pos_rattle[k], b->rattle[k] + 2 * r, 2 * sizeof(double));
@@ -1753,9 +1960,6 @@ static int scatter(Batch *b, int r, rmpcd_particles *sol, rmpcd_particles *col, 
         k_add_offset<<<grid_cap(p.S, 256), 256, 0, st>>>(cells->start, b->start + p.soff, p.S, -p.off);
         d2d(cells->is_md, b->is_md + p.soff, (size_t)p.S);
         d2d(cells->is_reac, b->is_reac + p.soff, (size_t)p.S);
-        BRep now;
-        RMPCD_CUDA_TRY(cudaMemcpyAsync(&now, b->rep + r, sizeof(BRep), cudaMemcpyDeviceToHost, st));
-        if ((rc = sync())) return rc;
         for (int k = 0; k < 3; k++) cells->origin[k] = now.g.origin[k];
     }
     if (nl) {
@@ -1775,11 +1979,10 @@ static int set_shape(Batch *b, int s)
     RMPCD_CUDA_TRY(cudaStreamSynchronize(stream()));
     int rc = build_particle_tiles(b, kPTiles[shape_tile(s)]);
     if (rc) return rc;
-    for (auto &e : b->exec)
-        if (e) {
-            cudaGraphExecDestroy(e);
-            e = nullptr;
-        }
+    if (b->exec) {
+        cudaGraphExecDestroy(b->exec);
+        b->exec = nullptr;
+    }
     b->shape = s;
     return RMPCD_OK;
 }
@@ -1897,36 +2100,12 @@ int rmpcd_dimer_batch_shape_info(int precision, int shape, int *particles_per_ti
 {
     RMPCD_ARG(precision == RMPCD_FP32 || precision == RMPCD_FP64, "precision must be RMPCD_FP32 or RMPCD_FP64");
     RMPCD_ARG(shape >= 0 && shape < kBShapes, "no such engine shape");
-    int kb, ke, mb;
-    bool cf;
-    const int v = shape_var(shape);
-    if (precision == RMPCD_FP32) {
-        using V0 = BVarOf<float, 0>::T;
-        using V1 = BVarOf<float, 1>::T;
-        using V2 = BVarOf<float, 2>::T;
-        using V3 = BVarOf<float, 3>::T;
-        using V4 = BVarOf<float, 4>::T;
-        kb = v == 0 ? V0::KB : v == 1 ? V1::KB : v == 2 ? V2::KB : v == 3 ? V3::KB : V4::KB;
-        ke = v == 0 ? V0::KE : v == 1 ? V1::KE : v == 2 ? V2::KE : v == 3 ? V3::KE : V4::KE;
-        mb = v == 0 ? V0::MINB : v == 1 ? V1::MINB : v == 2 ? V2::MINB : v == 3 ? V3::MINB : V4::MINB;
-        cf = v == 0 ? V0::FIRST : v == 1 ? V1::FIRST : v == 2 ? V2::FIRST : v == 3 ? V3::FIRST : V4::FIRST;
-    } else {
-        using V0 = BVarOf<double, 0>::T;
-        using V1 = BVarOf<double, 1>::T;
-        using V2 = BVarOf<double, 2>::T;
-        using V3 = BVarOf<double, 3>::T;
-        using V4 = BVarOf<double, 4>::T;
-        kb = v == 0 ? V0::KB : v == 1 ? V1::KB : v == 2 ? V2::KB : v == 3 ? V3::KB : V4::KB;
-        ke = v == 0 ? V0::KE : v == 1 ? V1::KE : v == 2 ? V2::KE : v == 3 ? V3::KE : V4::KE;
-        mb = v == 0 ? V0::MINB : v == 1 ? V1::MINB : v == 2 ? V2::MINB : v == 3 ? V3::MINB : V4::MINB;
-        cf = v == 0 ? V0::FIRST : v == 1 ? V1::FIRST : v == 2 ? V2::FIRST : v == 3 ? V3::FIRST : V4::FIRST;
-    }
     if (particles_per_tile) *particles_per_tile = (int)kPTiles[shape_tile(shape)];
     if (list_entries_per_thread) *list_entries_per_thread = kListPer[shape_list(shape)];
-    if (colloid_block_first) *colloid_block_first = cf ? 1 : 0;
-    if (per_thread_begin) *per_thread_begin = kb;
-    if (per_thread_end) *per_thread_end = ke;
-    if (blocks_per_sm) *blocks_per_sm = mb;
+    if (colloid_block_first) *colloid_block_first = 1;
+    if (per_thread_begin) *per_thread_begin = kMdPer;
+    if (per_thread_end) *per_thread_end = kMdPer;
+    if (blocks_per_sm) *blocks_per_sm = kClusters[shape_var(shape)];
     return RMPCD_OK;
 }
 
@@ -1997,7 +2176,7 @@ int rmpcd_dimer_batch_info(const rmpcd_dimer_batch *b, int *n_replicas, long lon
     if (n_extra_sorting) {
         RMPCD_CUDA_TRY(cudaMemcpyAsync(n_extra_sorting, b->n_extra, (size_t)b->R * sizeof(int), cudaMemcpyDeviceToHost,
                                        stream()));
-        return sync();
+        return rmpcd::sync();
     }
     return RMPCD_OK;
 }
