@@ -494,22 +494,20 @@ int rmpcd_dimer_batch_scatter(rmpcd_dimer_batch *batch, int replica, rmpcd_parti
 int rmpcd_dimer_batch_info(const rmpcd_dimer_batch *batch, int *n_replicas, long long *n_solvent,
                            int *n_extra_sorting);
 /* Engine shapes (no counterpart in the reference): particles per tile of the
- * sort's particle kernels, the blocks that run a replica's MD steps
- * (blocks_per_sm; 0: chosen by the number of replicas, one block per SM), the
- * solvent particles of the MD steps that each of their threads keeps in
- * registers (per_thread_begin = per_thread_end), the list entries per thread
- * of the kernels that list those particles, and colloid_block_first = 1 (the
- * colloids' turn belongs to a replica's first block).  Every shape gives the
- * same results bit for bit.  A batch starts on 1024-particle tiles (smaller
- * when that gives fewer than ~2 tiles per SM), blocks by the number of
- * replicas and one list entry per thread. */
+ * sort's particle kernels, the warps that move a replica's solvent in its MD
+ * steps (per_thread_begin = per_thread_end; one block per replica,
+ * blocks_per_sm = 1), the list entries per thread of the kernels that list that
+ * solvent, and colloid_block_first = 1 (the colloids have warps of their own).
+ * Every shape gives the same results bit for bit.  A batch starts on
+ * 1024-particle tiles (smaller when that gives fewer than ~2 tiles per SM), 16
+ * warps and one list entry per thread. */
 int rmpcd_dimer_batch_shapes(int precision, int *n_shapes);
 int rmpcd_dimer_batch_shape_info(int precision, int shape, int *particles_per_tile, int *per_thread_begin,
                                  int *per_thread_end, int *blocks_per_sm, int *list_entries_per_thread,
                                  int *colloid_block_first);
 int rmpcd_dimer_batch_set_shape(rmpcd_dimer_batch *batch, int shape);
 int rmpcd_dimer_batch_get_shape(const rmpcd_dimer_batch *batch, int *shape);
-/* The engine's autotuner: every tile size and block count with one list
+/* The engine's autotuner: every tile size and number of warps with one list
  * entry per thread, then the fastest of them with each other list setting,
  * runs one interval (capture and warm-up) and n_intervals timed intervals of
  * the batch itself -- real intervals of the run, since every shape gives the

@@ -9,20 +9,21 @@
 // system apply to every replica at once.
 //
 // MD steps touch only the solvent that can interact.  A particle that is in
-// neither bead's neighbor list and carries no MD, PAST_MD, REAC or WALL flag
-// flies freely until the next re-sort: no force can reach it before the list
-// is rebuilt, so its md_pos steps depend on nothing but its own position and
+// neither bead's neighbor list and carries no MD, PAST_MD, REAC or WALL flag, or
+// whose way stays clear of the beads, flies freely until the next re-sort: no
+// force can reach it before the list is rebuilt, so its md_pos steps depend on nothing but its own position and
 // velocity.  Such particles stay where they are in memory; the re-sort (or the
 // interval's end) advances each by its pending md_pos steps in one pass, adding
 // dt * v once per step so that every rounding is that of the steps one by one.
-// The others -- the active particles, ~6,000 per dimer at sigma = 2 -- are
-// advanced by kb_md, one thread-block cluster per replica, which runs the MD
-// steps one after another without leaving the kernel: pair forces, md_vel,
-// change_species, the colloid sums, velocity-Verlet and RATTLE, the next
-// step's md_pos, until the program's re-sort test
+// The others -- the active particles, some 800 per dimer at sigma = 2: those
+// with flags and those of the lists whose straight way may take them to a bead
+// before the next re-sort -- are advanced by kb_md, one block per replica, which
+// runs the MD steps one after another without leaving the kernel: pair forces,
+// md_vel, change_species, the colloid sums, velocity-Verlet and RATTLE, the
+// next step's md_pos, until the program's re-sort test
 // (programs/single_dimer_pbc.f90:323-330) fires or the interval's MD steps are
 // done.  The test needs the largest solvent displacement: of the active
-// particles the cluster has it, of the free ones kb_classify has computed the
+// particles the block has it, of the free ones kb_classify has computed the
 // first step at which any of them reaches the threshold, by the same additions
 // and the same comparison.  Replicas re-sort at steps of their own: a launch of
 // kb_md ends when each of its replicas waits for a re-sort or is done, then one
@@ -39,7 +40,6 @@
 // Arithmetic per particle is that of the single-system kernels
 // (stepops.cuh, nlist_ops.cuh), so replica r reproduces, bit for bit, the
 // same program run alone through the C ABI with its own seed.
-#include <cooperative_groups.h>
 #include <climits>
 #include <cmath>
 #include <cstring>
@@ -64,11 +64,10 @@ constexpr int kTile = 1024;  // slots per slot tile
 constexpr int kBT = 256;     // threads per tile block
 
 // Engine shapes (rmpcd_dimer_batch_autotune): the particles per tile of the
-// sort's particle kernels, the blocks a replica's MD steps run on (the cluster
-// of kb_md; 0: chosen by the number of replicas) and the list entries per
-// thread of the kernels that make the active list.  Every shape gives the same
+// sort's particle kernels, the threads of kb_md that move a replica's solvent,
+// and the list entries per thread of the kernels that make the active list.  Every shape gives the same
 // results bit for bit: they only decide which thread handles which particle.
-constexpr int kClusters[] = {0, 8, 4, 2, 1};
+constexpr int kPartThreads[] = {512, 448, 384, 320, 256};
 constexpr int kBVars = 5;
 constexpr long long kPTiles[] = {256, 512, 1024, 2048, 4096};  // particles per tile
 constexpr int kNPTiles = 5;
@@ -77,7 +76,7 @@ constexpr int kNPTiles = 5;
 constexpr int kListPer[] = {1, 4};
 constexpr int kNListPer = 2;
 constexpr int kBShapes = kNListPer * kBVars * kNPTiles;
-// shape s: particle tile kPTiles[s % kNPTiles], cluster kClusters[(s /
+// shape s: particle tile kPTiles[s % kNPTiles], threads kPartThreads[(s /
 // kNPTiles) % kBVars], list entries per thread kListPer[s / (kNPTiles * kBVars)]
 __host__ __device__ inline int shape_tile(int s) { return s % kNPTiles; }
 __host__ __device__ inline int shape_var(int s) { return (s / kNPTiles) % kBVars; }
@@ -99,6 +98,12 @@ struct BRep {
     uint64_t seed;
     double far;     // refuel distance (single-precision expression of the program)
     Grid g;         // cells; origin rewritten on the device by the grid shift
+};
+
+// a pair force in global memory: its place in the order of addition and the force
+struct MdTerm {
+    int e, pad;
+    double f[3];
 };
 
 }  // namespace rmpcd
@@ -133,10 +138,13 @@ struct rmpcd_dimer_batch {
     // nl[r] of the neighbor lists first, then nx[r] flagged ones outside them
     int *act = nullptr, *nl = nullptr, *nx = nullptr;
     int *aidx = nullptr;       // per particle: its place in act, -1 when it flies freely
-    int *amap = nullptr;       // per list entry: the place in act of its particle
+    int *ent = nullptr;        // per listed active particle: an entry of it in list 0 and in list 1, or -1
+    int *next = nullptr;       // per list entry: another entry of the same particle in the list, or -1
     int *mult = nullptr;       // per listed active particle: entries in list 0 | entries in list 1 << 16
-    double *pf = nullptr;      // per listed active particle: pair forces from beads 0 and 1 (6 doubles)
-    unsigned char *cf = nullptr;  // ... and which of the two act on it (particles beyond kb_md's shared flags)
+    // pair forces beyond what kb_md holds in shared memory
+    rmpcd::MdTerm *over = nullptr, *terms = nullptr;
+    unsigned long long *keys[2] = {nullptr, nullptr};
+    int *n_over = nullptr;
     int *nf = nullptr;         // per replica: flagged particles, listed in sol->key from the replica's first place
     int *s_free = nullptr;     // per replica: first MD step at which a free particle forces a re-sort
     int *adv = nullptr, *base = nullptr;  // per replica: md_pos steps done this interval, and those in memory
@@ -262,39 +270,84 @@ __global__ void kb_collect_flagged(TileSet ts, const BRep *rep, PView<R> v, int 
     }
 }
 
-// The listed particles of the replicas in flag (every one when null) become
-// active, each once: its place in act goes to aidx.
-__global__ void kb_claim(const int *flag, const BRep *rep, const int *list, const int *n, int Nmax, int *aidx, int *act,
-                         int *nl, int *mult)
+// Whether a particle at p with velocity v may come within `reach` of the point c
+// in the next time T of free flight, in a periodic box of edges L (single
+// precision; reach holds the margin for it)
+__device__ __forceinline__ bool may_meet(const float p[3], const float v[3], const float c[3], const float L[3],
+                                         float reach, float T)
+{
+    float d[3], a = 0, b = 0;
+    bool one_image = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float x = p[k] - c[k], h = 0.5f * L[k];
+        d[k] = x < -h ? x + L[k] : x > h ? x - L[k] : x;
+        one_image = one_image && fabsf(d[k]) + T * fabsf(v[k]) < L[k] - reach;
+        a += v[k] * v[k];
+        b += d[k] * v[k];
+    }
+    const float t = a > 0 ? fminf(fmaxf(-b / a, 0.0f), T) : 0.0f;
+    float m = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const float x = d[k] + t * v[k];
+        m += x * x;
+    }
+    return !(one_image && m > reach * reach);
+}
+
+// The listed particles of the replicas in flag (every one when null) that may
+// come within a cut of a bead before the next re-sort become active, each
+// once: its place in act goes to aidx.  Until a re-sort a bead stays within
+// skin / 10 of its pos_old (the re-sort test, programs/single_dimer_pbc.f90:324-329),
+// and a particle without force flies straight, so that of the ~4,800 listed
+// particles of a sigma = 2 dimer some 800 are left.
+template <typename R>
+__global__ void __launch_bounds__(kBT)
+    kb_claim(const int *flag, const BRep *rep, PView<R> v0, PView<R> v1, Vec3<double> cold, R dt, float reach,
+             float margin, int N_MD, const int *base, const int *list, const int *n, int Nmax, int *aidx, int *act,
+             int *nl, int *mult, int *ent)
 {
     const int i = blockIdx.y, r = i >> 1;
     if (flag && !flag[r]) return;
-    const long long off = rep[r].off;
+    const BRep &rp = rep[r];
+    const long long off = rp.off;
+    const PView<R> v = pick(v0, v1, rp.cur);
+    const int steps = N_MD - base[r];
+    float L[3], c[2][3];
+    for (int k = 0; k < 3; k++) {
+        L[k] = (float)rp.g.edges[k];
+        for (int h = 0; h < 2; h++) c[h][k] = (float)cold[k][2 * r + h];
+    }
+    // the rounding of every addition of the flight, and of this test
+    const float far = reach + margin + (1e-5f + (sizeof(R) == 4 ? 2.4e-7f : 4.4e-16f) * (float)steps) * (L[0] + L[1] + L[2]);
+    const float T = (float)dt * (float)steps * 1.0001f;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n[i]; e += gridDim.x * blockDim.x) {
         const int idx = list[(size_t)i * Nmax + e];
+        const float p[3] = {(float)v.pos.x[idx], (float)v.pos.y[idx], (float)v.pos.z[idx]};
+        const float u[3] = {(float)v.vel.x[idx], (float)v.vel.y[idx], (float)v.vel.z[idx]};
+        if (!may_meet(p, u, c[0], L, far, T) && !may_meet(p, u, c[1], L, far, T)) continue;
         if (atomicCAS(aidx + idx, -1, -2) != -1) continue;
         const int a = atomicAdd(nl + r, 1);
         act[off + a] = idx;
         aidx[idx] = a;
-        mult[(size_t)2 * r * Nmax + a] = 0;
+        const size_t w = (size_t)2 * r * Nmax + a;
+        mult[w] = 0;
+        ent[2 * w] = ent[2 * w + 1] = -1;
     }
 }
 
-// steps[r] <- the first MD step at whose test some free particle of replica r
-// has moved sqrt(d2) >= thr from pos_old (programs/single_dimer_pbc.f90:324-329,
+// *steps <- the first MD step at whose test the free particle i has moved
+// sqrt(d2) >= thr from pos_old (programs/single_dimer_pbc.f90:324-329,
 // src/particle_system.f90:357-378).  A particle's earliest possible step
-// follows from its speed (with a margin for the rounding of each addition);
-// only the particles that could be first -- a few per replica -- go through
-// their additions one by one.
+// follows from its speed (reach bounds the distance of one addition, its
+// rounding included); only the particles that could be first -- a few per
+// replica -- go through their additions one by one.
 template <typename R>
-__device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &old, long long i, int fresh, R dt,
-                                              double thr, int base, int n_rem, double slack, int read_species,
-                                              int *steps)
+__device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &old, long long i, R vx, R vy, R vz,
+                                              float reach, int fresh, R dt, double thr, int base, int n_rem,
+                                              int read_species, const int *aidx, int best, int *steps)
 {
-    if (read_species && v.species[i] < 0) return;
-    const R vx = v.vel.x[i], vy = v.vel.y[i], vz = v.vel.z[i];
-    const float ux = (float)vx, uy = (float)vy, uz = (float)vz;
-    float reach = (float)dt * sqrtf(ux * ux + uy * uy + uz * uz) * 1.001f + (float)slack;
     float left = (float)thr;
     if (fresh) {
         // positions and pos_old are the caller's: any distance, any place
@@ -307,7 +360,9 @@ __device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &
     if (!(reach * (float)n_rem >= left)) return;
     int lo = left > 0 ? (int)fminf(left / reach, 1e9f) - 1 : 1;  // no crossing before the lo-th addition
     if (lo < 1) lo = 1;
-    if (base + lo - 1 >= *(volatile int *)steps) return;
+    if (base + lo - 1 >= best) return;
+    if ((v.flags[i] & kActiveBits) || aidx[i] >= 0) return;
+    if (read_species && v.species[i] < 0) return;
     const R hx = dt * vx, hy = dt * vy, hz = dt * vz;
     R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
     const double ox = fresh ? (double)old.x[i] : (double)x, oy = fresh ? (double)old.y[i] : (double)y,
@@ -322,20 +377,19 @@ __device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &
             atomicMin(steps, base + j - 1);
             return;
         }
-        if (base + j - 1 >= *(volatile int *)steps) return;
     }
 }
 
 // After kb_claim: the first step at which a free particle forces a re-sort
-// (particle tiles), the places of the list entries and their multiplicities
-// (gx blocks per bead), and the flagged particles outside the lists, which
+// (particle tiles), every listed particle's entries in the two lists, counted
+// and chained (gx blocks per bead), and the flagged particles outside the lists, which
 // become active behind the listed ones (one block per replica).
 template <typename R>
 __global__ void __launch_bounds__(kBT)
     kb_classify(TileSet ts, int n_tile_blocks, int gx, int R_, const int *flag, const BRep *rep, PView<R> v0,
                 PView<R> v1, R dt, double thr, int N_MD, int read_species, const int *base, const int *fresh,
                 int *s_free, const int *list, const int *n, int Nmax, int *aidx, int *act, const int *nl, int *nx,
-                int *mult, int *amap, const int *key, const int *nf)
+                int *mult, int *ent, int *next, const int *key, const int *nf)
 {
     int b = blockIdx.x;
     if (b < n_tile_blocks) {
@@ -347,10 +401,36 @@ __global__ void __launch_bounds__(kBT)
             const int b0 = base[t.r], fr = fresh[t.r];
             // three components, each rounded by at most half an ulp of a
             // position inside twice the box
-            const double slack = (sizeof(R) == 4 ? 2.4e-7 : 4.4e-16) * (rp.g.edges[0] + rp.g.edges[1] + rp.g.edges[2]);
-            for (long long i = t.begin + threadIdx.x; i < t.end; i += blockDim.x)
-                if (!(v.flags[i] & kActiveBits) && aidx[i] < 0)
-                    free_crossing<R>(v, old, i, fr, dt, thr, b0, N_MD - b0, slack, read_species, s_free + t.r);
+            const float slack =
+                (sizeof(R) == 4 ? 2.4e-7f : 4.4e-16f) * (float)(rp.g.edges[0] + rp.g.edges[1] + rp.g.edges[2]);
+            // the velocities alone rule out nearly every particle: four per
+            // thread and pass, loaded before any is used
+            constexpr int K = 4;
+            for (long long i0 = t.begin + threadIdx.x; i0 < t.end; i0 += K * kBT) {
+                R vx[K], vy[K], vz[K];
+                const int best = *(volatile int *)(s_free + t.r);  // so far; it only falls
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const long long i = i0 + k * kBT;
+                    if (i < t.end) {
+                        vx[k] = v.vel.x[i];
+                        vy[k] = v.vel.y[i];
+                        vz[k] = v.vel.z[i];
+                    }
+                }
+                const float steps = (float)(min(N_MD, best) - b0);
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    const long long i = i0 + k * kBT;
+                    if (i >= t.end) break;
+                    const float ux = (float)vx[k], uy = (float)vy[k], uz = (float)vz[k];
+                    const float reach = (float)dt * sqrtf(ux * ux + uy * uy + uz * uz) * 1.001f + slack;
+                    // (one step more: best is the step of the addition before it)
+                    if (fr || reach * (steps + 1.0f) >= (float)thr)
+                        free_crossing<R>(v, old, i, vx[k], vy[k], vz[k], reach, fr, dt, thr, b0, N_MD - b0,
+                                         read_species, aidx, best, s_free + t.r);
+                }
+            }
         }
         return;
     }
@@ -361,8 +441,10 @@ __global__ void __launch_bounds__(kBT)
         for (int e = (b % gx) * blockDim.x + threadIdx.x; e < n[i]; e += gx * blockDim.x) {
             const size_t q = (size_t)i * Nmax + e;
             const int a = aidx[list[q]];
-            amap[q] = a;
-            atomicAdd(mult + (size_t)2 * r * Nmax + a, (i & 1) ? 1 << 16 : 1);
+            if (a < 0) continue;
+            const size_t w = (size_t)2 * r * Nmax + a;
+            atomicAdd(mult + w, (i & 1) ? 1 << 16 : 1);
+            next[q] = atomicExch(ent + 2 * w + (i & 1), e);
         }
         return;
     }
@@ -378,14 +460,20 @@ __global__ void __launch_bounds__(kBT)
     }
 }
 
-// kb_md: threads per block, active particles per thread kept in registers
-// (the others go through memory in every step), list entries per bead whose
-// places are kept in shared memory, and particles whose force flags are
-constexpr int kMdThreads = 512;
-constexpr int kMdPer = 2;
-constexpr int kMdMap = 4096;
-constexpr int kMdFlags = 8192;
-constexpr int kMdList = 1024;  // contributing entries compacted at a time (FP64 colloid sums)
+// kb_md's block: the warps that add up the pair forces and move the beads
+// (half of them per bead), then those that have the particles; and what it
+// holds of a step in shared memory (a list beyond kMdBits entries or more
+// terms than fit go through md_slow_sums)
+constexpr int kMdSum = 256;
+constexpr int kMdThreads = kMdSum + 512;
+constexpr int kMdQueue = 1024;    // pairs of a particle and a bead that may reach it
+constexpr int kMdTerms = 512;     // pair forces per bead
+constexpr int kMdBits = 16384;    // list entries per bead covered by the bit map
+constexpr size_t kMdSmem = 224 * 1024;  // dynamic shared memory
+// A particle is queued for the next step's pair forces before the beads have
+// moved: within this distance more than the cuts, which is far above a bead's
+// way in a step; a bead that moves farther makes the queue anew.
+constexpr float kMdWay = 0.02f;
 
 template <typename R>
 struct MdArgs {
@@ -399,12 +487,14 @@ struct MdArgs {
     double bond, dt, skin;
     R dt_r, dt_sq_r;
     double cut_c, cut_n, prob;
+    float reach;          // the largest cut, with a margin for single precision less than 1e-5 (Lx + Ly + Lz)
     LJDev lj_sc, lj_cc;
     int R_, N_MD, Nmax, start, read_species;
     const uint64_t *d_step;
-    const int *n, *amap, *act, *nl, *nx, *mult;
-    double *pf;
-    unsigned char *cf;
+    const int *n, *next, *ent, *act, *nl, *nx, *mult;
+    MdTerm *over, *terms;         // 2 * R * Nmax each: terms beyond the shared ones, terms to be put in order
+    unsigned long long *keys[2];  // sort keys of the latter
+    int *n_over;                  // per bead, one counter per step parity
     const int *s_free, *fresh;
     int *adv, *resort, *n_extra;
     ResortLists rl;
@@ -418,64 +508,135 @@ struct MdArgs {
 // one active solvent particle
 template <typename R>
 struct Part {
-    int idx;
-    int f, sp, m;       // flags, species, multiplicity in the two lists
     R p[3], v[3], o[3]; // position, velocity, pos_old
     R g[3];             // the last evaluation's force (zero without MD and PAST_MD)
+    int f, sp;          // flags, species
 };
 
+template <typename R>
+__host__ __device__ constexpr size_t md_part_bytes()
+{
+    return 18 * sizeof(R) + 8 * sizeof(int);
+}
+
+// the fields of a block's particles in shared memory, cap of each
+template <typename R>
+struct MdParts {
+    R *r;    // p[3], v[3], o[3], g[3], then the step's forces of the two beads, cap each
+    int *i;  // idx, flags, species, multiplicities, entries in the two lists, what
+             // the step has for the particle (bit h: bead h is queued, bit 2:
+             // flags), what came of it (bit h: bead h acts, bit 2: REAC)
+    int cap;
+    __device__ R &real(int field, int s) const { return r[(size_t)field * cap + s]; }
+    __device__ int &num(int field, int s) const { return i[(size_t)field * cap + s]; }
+};
+
+// a / b rounded to nearest for a divisor used again: with y = 1 / b rounded to
+// nearest, two corrections by exact residuals give the correctly rounded
+// quotient (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34(1), 1990); operands near the ends of the
+// exponent range, zeros and non-finite ones take the division itself.
+struct MdDiv {
+    double b, y;
+    bool safe;
+    __device__ void set(double d)
+    {
+        b = d;
+        y = 1.0 / d;
+        safe = fabs(d) > 1e-100 && fabs(d) < 1e100;
+    }
+    __device__ __forceinline__ double of(double a) const
+    {
+        if (!(safe && fabs(a) > 1e-180 && fabs(a) < 1e180)) return a / b;
+        double q = a * y;
+        q = __fma_rn(__fma_rn(-b, q, a), y, q);
+        return __fma_rn(__fma_rn(-b, q, a), y, q);
+    }
+};
+
+// What the steps need of the replica and the block
+template <typename R>
+struct MdBox {
+    double L[3];
+    float lf[3], hf[3];
+    float reach_sq, queue_sq;  // squared reach of a bead, and with kMdWay more
+    int cs[2];
+    uint64_t seed;
+    long long off;
+    int r, nl, na;        // replica; listed and active particles
+    int run[2];           // entries per leaf of the tree, each bead's list
+    int cur;              // buffer of the replica's current arrays
+    MdParts<R> parts;
+};
+
+// The beads of a replica in warp 0 of its block 0: lane 3 i + k has component k of
+// bead i (the other lanes mirror lane 0), so that the divisions of a
+// velocity-Verlet half or a RATTLE correction run side by side.  The divisors
+// are kept with their reciprocals: a step is a chain of five quotients and a
+// root, each waiting for the one before.
+struct MdBead {
+    double pos, vel, force, fold;
+    MdDiv vv, m, kk;       // 2 x own mass; own RATTLE mass; bond^2 (1/m1 + 1/m2)
+    double dt_inv_mass;    // dt (1/m1 + 1/m2)
+    double L;
+    int i, k, sp0, sp1;
+};
+
+// What the turn needs of the beads' positions alone, before the step's forces
+// are there: separation, its square, the reciprocal of RATTLE's divisor and
+// the beads' own force (compute_force_n2, src/neighbor_list.f90:227-264)
+struct MdPair {
+    double s, rsq, f;
+    MdDiv g;
+    bool acts;
+};
+
+// The block's shared memory: the step's bead positions and decisions, the queue
+// of particles that need more than free flight; behind it the pair forces
+// (MdTotals) and the particles, field by field (MdParts).
+template <typename R>
 struct MdShared {
-    double pos[3][2], vel[3][2], force[3][2], fold[3][2], old[3][2], rat[3][2];  // the beads (block 0)
-    double x[6];                 // bead positions of the current step
-    double wmax[8 * (kMdThreads / 32)];  // every warp's largest squared displacement (block 0)
-    double wsum[2][3][kMdThreads / 64];
-    double val[2][3][256];
-    int lst[2][kMdList];
-    int wcnt[2][kMdThreads / 64];
-    int map[2][kMdMap];
-    unsigned char cf[kMdFlags];  // which beads act on the particle (block 0)
-    int species[2];
+    MdBox<R> box;
+    double x[2][6];         // bead positions, by step parity
+    double old[6], rat[6];  // pos_old and pos_rattle of the beads
+    double f[2][3];         // the beads' force sums
+    double wsum[2][3][kNlBlockThreads / 32];
+    int stop, over, last;   // re-sort by the beads or s_free, by an active particle's displacement
+    int anew;               // a bead went farther than kMdWay
+    int spill;              // step + 1 of the last one with a term in global memory
+    int nq[2], cnt[2][2];   // by step parity: particles queued; pair forces per bead
+    int tot[2];             // slow sums: terms gathered
     int ws[33];
-    int stop, last;
+    int q[2][kMdQueue];     // queued particles, by step parity
 };
 
-template <typename R>
-__device__ __forceinline__ void md_load(Part<R> &q, const MdArgs<R> &A, const PView<R> &v, const Vec3<R> &old,
-                                        long long off, int r, int a, int nl, bool fresh)
-{
-    const int i = A.act[off + a];
-    q.idx = i;
-    q.f = v.flags[i];
-    q.sp = v.species[i];
-    q.m = a < nl ? A.mult[(size_t)2 * r * A.Nmax + a] : 0;
-    const bool forced = q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT));
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        q.p[k] = v.pos[k][i];
-        q.v[k] = v.vel[k][i];
-        q.o[k] = fresh ? old[k][i] : q.p[k];
-        q.g[k] = forced ? v.force[k][i] : (R)0;
-    }
-}
+// the pair forces of a step, each with its list entry and the step that wrote
+// it, and what puts them in order
+struct MdTotals {
+    double f[2][3][kMdTerms], g[2][3][kMdTerms];  // as they come, and in order
+    int2 te[2][kMdTerms];                 // step + 1, place in the order of addition
+    unsigned bits[2][kMdBits / 32];       // places with a term in this step
+    unsigned short base[2][kMdBits / 32]; // terms before each word's places
+};
 
-template <typename R>
-__device__ __forceinline__ void md_store(const Part<R> &q, const PView<R> &v)
+// the block's named barriers: of the summing warps, and between them and the
+// particles' warps (arrive: without waiting)
+__device__ __forceinline__ void md_sync(int id, int threads)
 {
-    const int i = q.idx;
-    v.flags[i] = q.f;
-    v.species[i] = q.sp;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        v.pos[k][i] = q.p[k];
-        v.vel[k][i] = q.v[k];
-        v.force[k][i] = q.g[k];
-    }
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+__device__ __forceinline__ void md_arrive(int id, int threads)
+{
+    asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int kBarSum = 1, kBarPart = 2, kBarForces = 3, kBarTurn = 4;
 
 // md_pos (src/md.f90:61-77), the PAST_MD / MD roll (src/neighbor_list.f90:180-188)
-// and the squared displacement of maximum_displacement (0 for species < 0)
+// and whether the particle's displacement is sqrt(d2) >= thr
+// (src/particle_system.f90:357-378: not for species < 0); the exact test runs
+// where the one in single precision is not clear
 template <typename R>
-__device__ __forceinline__ double md_begin(Part<R> &q, R dt, R dt_sq, int read_species)
+__device__ __forceinline__ bool md_begin(Part<R> &q, R dt, R dt_sq, int read_species, double thr, float near_sq)
 {
     const bool md = (q.f >> MD_BIT) & 1;
 #pragma unroll
@@ -485,53 +646,228 @@ __device__ __forceinline__ double md_begin(Part<R> &q, R dt, R dt_sq, int read_s
     }
     q.f = md ? q.f | (1 << PAST_MD_BIT) : q.f & ~(1 << PAST_MD_BIT);
     q.f &= ~(1 << MD_BIT);
-    if (read_species && q.sp < 0) return 0;
+    const float c0 = (float)(q.p[0] - q.o[0]), c1 = (float)(q.p[1] - q.o[1]), c2 = (float)(q.p[2] - q.o[2]);
+    if (c0 * c0 + c1 * c1 + c2 * c2 < near_sq) return false;
+    if (read_species && q.sp < 0) return false;
     const double d0 = (double)q.p[0] - (double)q.o[0], d1 = (double)q.p[1] - (double)q.o[1],
                  d2 = (double)q.p[2] - (double)q.o[2];
-    return d0 * d0 + d1 * d1 + d2 * d2;
+    return sqrt(d0 * d0 + d1 * d1 + d2 * d2) >= thr;
 }
 
-// pair forces of the particle's list entries (src/neighbor_list.f90:198-219, in
-// (bead, entry) order), flag_particles_nl of the catalytic bead
-// (programs/single_dimer_pbc.f90:493-509), md_vel (src/md.f90:219-237) and
-// change_species (programs/single_dimer_pbc.f90:511-542).  Returns which beads
-// act on it; their forces go to pf[0..5].
-template <typename R>
-__device__ __forceinline__ int md_forces_end(Part<R> &q, const MdArgs<R> &A, const double X[6], const int cs[2],
-                                             const double L[3], double *pf, uint64_t seed, uint64_t step,
-                                             long long off)
+__device__ __forceinline__ float md_image_f(float d, float L, float h)
 {
-    int acts = 0;
-    R nf[3] = {0, 0, 0};
-    double r_sq[2];
-    const double px = (double)q.p[0], py = (double)q.p[1], pz = (double)q.p[2];
-    const int sp0 = q.sp;
-    if (q.m && sp0 > 0) {
+    return d < -h ? d + L : d > h ? d - L : d;
+}
+
+template <typename R>
+__device__ __forceinline__ const PView<R> &md_view(const MdArgs<R> &A, const MdBox<R> &B)
+{
+    return B.cur ? A.v1 : A.v0;
+}
+template <typename R>
+__device__ __forceinline__ const Vec3<R> &md_old(const MdArgs<R> &A, const MdBox<R> &B)
+{
+    return B.cur ? A.v0.pos : A.v1.pos;
+}
+
+// What a particle at p with flags f has to do besides flying freely: bit h, bead h
+// may be within reach (squared; a distance in single precision decides), bit 2,
+// it has flags.  Three quarters of the active particles have nothing.
+template <typename R>
+__device__ __forceinline__ int md_busy(const double *X, const MdBox<R> &B, const R p[3], int f, float reach_sq)
+{
+    float d[2] = {0, 0};
+#pragma unroll
+    for (int k = 0; k < 3; k++)
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const int times = i ? q.m >> 16 : q.m & 0xffff;
-            if (!times) continue;
-            const double d0 = min_image_d(X[3 * i] - px, L[0]), d1 = min_image_d(X[3 * i + 1] - py, L[1]),
-                         d2 = min_image_d(X[3 * i + 2] - pz, L[2]);
-            r_sq[i] = d0 * d0 + d1 * d1 + d2 * d2;
-            const int tt = (sp0 - 1) + A.lj_sc.n1 * (cs[i] - 1);
-            if (r_sq[i] <= A.lj_sc.cut_sq[tt]) {
-                const double fr = lj_force_over_r(r_sq[i], A.lj_sc.epsilon[tt], A.lj_sc.sigma[tt]);
-                const double f0 = fr * d0, f1 = fr * d1, f2 = fr * d2;
-                pf[3 * i] = f0;
-                pf[3 * i + 1] = f1;
-                pf[3 * i + 2] = f2;
-                for (int t = 0; t < times; t++) {
-                    nf[0] = nf[0] - (R)f0;
-                    nf[1] = nf[1] - (R)f1;
-                    nf[2] = nf[2] - (R)f2;
-                }
-                acts |= 1 << i;
-                q.f |= (1 << MD_BIT) | (cs[i] == 1 ? (1 << CATALYZED_BIT) : 0);
-            }
-            if (i == 0 && sp0 == 1 && r_sq[0] < A.cut_c) q.f |= 1 << REAC_BIT;
+            const float c = md_image_f((float)X[3 * i + k] - (float)p[k], B.lf[k], B.hf[k]);
+            d[i] += c * c;
         }
+    return (d[0] > reach_sq ? 0 : 1) | (d[1] > reach_sq ? 0 : 2) | ((f & kActiveBits) ? 4 : 0);
+}
+
+template <typename R>
+__device__ __forceinline__ Part<R> md_read(const MdBox<R> &B, const MdArgs<R> &A, int i, int &idx, bool from_old)
+{
+    Part<R> q;
+    if (i < B.parts.cap && !from_old) {
+        idx = B.parts.num(0, i);
+        q.f = B.parts.num(1, i);
+        q.sp = B.parts.num(2, i);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            q.p[k] = B.parts.real(k, i);
+            q.v[k] = B.parts.real(3 + k, i);
+            q.o[k] = B.parts.real(6 + k, i);
+            q.g[k] = B.parts.real(9 + k, i);
+        }
+        return q;
     }
+    idx = A.act[B.off + i];
+    q.f = md_view(A, B).flags[idx];
+    q.sp = md_view(A, B).species[idx];
+    const bool forced = q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT));
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        q.p[k] = md_view(A, B).pos[k][idx];
+        q.v[k] = md_view(A, B).vel[k][idx];
+        q.o[k] = md_old(A, B)[k][idx];
+        q.g[k] = forced ? md_view(A, B).force[k][idx] : (R)0;
+    }
+    return q;
+}
+
+// in_place: to the particle arrays (those beyond the shared memory, and every
+// one at the end)
+template <typename R>
+__device__ __forceinline__ void md_write(const MdBox<R> &B, const MdArgs<R> &A, int i, int idx, const Part<R> &q, bool in_place)
+{
+    if (i < B.parts.cap && !in_place) {
+        B.parts.num(1, i) = q.f;
+        B.parts.num(2, i) = q.sp;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            B.parts.real(k, i) = q.p[k];
+            B.parts.real(3 + k, i) = q.v[k];
+            B.parts.real(9 + k, i) = q.g[k];
+        }
+        return;
+    }
+    md_view(A, B).flags[idx] = q.f;
+    md_view(A, B).species[idx] = q.sp;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        md_view(A, B).pos[k][idx] = q.p[k];
+        md_view(A, B).vel[k][idx] = q.v[k];
+        md_view(A, B).force[k][idx] = q.g[k];
+    }
+}
+
+// multiplicities and entries of particle i in the two lists
+template <typename R>
+__device__ __forceinline__ int md_entries(const MdBox<R> &B, const MdArgs<R> &A, int i, int e[2])
+{
+    if (i < B.parts.cap) {
+        e[0] = B.parts.num(4, i);
+        e[1] = B.parts.num(5, i);
+        return B.parts.num(3, i);
+    }
+    if (i >= B.nl) return 0;
+    const size_t w = (size_t)2 * B.r * A.Nmax + i;
+    e[0] = A.ent[2 * w];
+    e[1] = A.ent[2 * w + 1];
+    return A.mult[w];
+}
+
+// The place of entry e in the order in which a bead's pair forces are added: list
+// order in the FP64 form; in the FP32 form leaf by leaf of colloid_tree_block's
+// tree (entries t, t + 256, ... of leaf t in that order), run entries per leaf.
+template <typename R>
+__device__ __forceinline__ int md_order(int e, int run)
+{
+    return sizeof(R) == 8 ? e : (e & (kNlBlockThreads - 1)) * run + (e >> 8);
+}
+
+// The pair force f of bead i, once for each of the particle's entries in its
+// list: the term, and the entry's bit in the bead's map (terms without room to
+// global memory)
+template <typename R>
+__device__ __forceinline__ void md_push(MdShared<R> &sh, const MdBox<R> &B, const MdArgs<R> &A, MdTotals &tot, int i,
+                                        int k, int e, int times, double f0, double f1, double f2)
+{
+    const int par = k & 1;
+    for (int t = 0; t < times; t++) {
+        const int s = atomicAdd(&sh.cnt[par][i], 1), o = md_order<R>(e, B.run[i]);
+        if (s < kMdTerms && o < kMdBits) {
+            atomicOr(&tot.bits[i][o >> 5], 1u << (o & 31));
+            tot.te[i][s] = make_int2(k + 1, o);
+            tot.f[i][0][s] = f0;
+            tot.f[i][1][s] = f1;
+            tot.f[i][2][s] = f2;
+        } else {
+            const int b = 2 * B.r + i;
+            MdTerm *g = A.over + (size_t)b * A.Nmax + atomicAdd(A.n_over + 2 * b + par, 1);
+            g->e = o;
+            g->f[0] = f0;
+            g->f[1] = f1;
+            g->f[2] = f2;
+            sh.spill = k + 1;
+        }
+        if (t + 1 < times) e = A.next[(size_t)(2 * B.r + i) * A.Nmax + e];
+    }
+}
+
+// pair forces of a queued particle's list entries (src/neighbor_list.f90:198-219,
+// in (bead, entry) order) and flag_particles_nl of the catalytic bead
+// (programs/single_dimer_pbc.f90:493-509): the step's force and the flags
+template <typename R>
+__device__ __forceinline__ int md_forces(MdShared<R> &sh, const MdBox<R> &B, const MdArgs<R> &A, MdTotals &tot, int i,
+                                         int k, const R p[3], int sp, int f, R nf[3])
+{
+    int e[2];
+    const int m = md_entries(B, A, i, e);
+    const double *X = sh.x[k & 1];
+    nf[0] = nf[1] = nf[2] = 0;
+    if (!m || sp <= 0) return f;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int times = h ? m >> 16 : m & 0xffff;
+        if (!times) continue;
+        const double d0 = min_image_d(X[3 * h] - (double)p[0], B.L[0]),
+                     d1 = min_image_d(X[3 * h + 1] - (double)p[1], B.L[1]),
+                     d2 = min_image_d(X[3 * h + 2] - (double)p[2], B.L[2]);
+        const double r_sq = d0 * d0 + d1 * d1 + d2 * d2;
+        const int tt = (sp - 1) + A.lj_sc.n1 * (B.cs[h] - 1);
+        if (r_sq <= A.lj_sc.cut_sq[tt]) {
+            const double fr = lj_force_over_r(r_sq, A.lj_sc.epsilon[tt], A.lj_sc.sigma[tt]);
+            const double f0 = fr * d0, f1 = fr * d1, f2 = fr * d2;
+            for (int t = 0; t < times; t++) {
+                nf[0] = nf[0] - (R)f0;
+                nf[1] = nf[1] - (R)f1;
+                nf[2] = nf[2] - (R)f2;
+            }
+            md_push(sh, B, A, tot, h, k, e[h], times, f0, f1, f2);
+            f |= (1 << MD_BIT) | (B.cs[h] == 1 ? (1 << CATALYZED_BIT) : 0);
+        }
+        if (h == 0 && sp == 1 && r_sq < A.cut_c) f |= 1 << REAC_BIT;
+    }
+    return f;
+}
+
+// the pair force of bead h on particle i of the shared memory: to the
+// particle's pf, with what came of it, and to the bead's terms
+template <typename R>
+__device__ __forceinline__ void md_pair_force(MdShared<R> &sh, const MdBox<R> &B, const MdArgs<R> &A, MdTotals &tot,
+                                              int i, int h, int k)
+{
+    const double *X = sh.x[k & 1] + 3 * h;
+    const int sp = B.parts.num(2, i), m = B.parts.num(3, i), times = h ? m >> 16 : m & 0xffff;
+    if (!times || sp <= 0) return;
+    const double d0 = min_image_d(X[0] - (double)B.parts.real(0, i), B.L[0]),
+                 d1 = min_image_d(X[1] - (double)B.parts.real(1, i), B.L[1]),
+                 d2 = min_image_d(X[2] - (double)B.parts.real(2, i), B.L[2]);
+    const double r_sq = d0 * d0 + d1 * d1 + d2 * d2;
+    const int tt = (sp - 1) + A.lj_sc.n1 * (B.cs[h] - 1);
+    if (r_sq <= A.lj_sc.cut_sq[tt]) {
+        const double fr = lj_force_over_r(r_sq, A.lj_sc.epsilon[tt], A.lj_sc.sigma[tt]);
+        const double f0 = fr * d0, f1 = fr * d1, f2 = fr * d2;
+        md_push(sh, B, A, tot, h, k, B.parts.num(4 + h, i), times, f0, f1, f2);
+        B.parts.real(12 + 3 * h, i) = (R)f0;
+        B.parts.real(13 + 3 * h, i) = (R)f1;
+        B.parts.real(14 + 3 * h, i) = (R)f2;
+        atomicOr(&B.parts.num(7, i), 1 << h);
+    }
+    if (h == 0 && sp == 1 && r_sq < A.cut_c) atomicOr(&B.parts.num(7, i), 4);
+}
+
+// md_vel (src/md.f90:219-237) and change_species
+// (programs/single_dimer_pbc.f90:511-542) of a queued particle, given the step's
+// force nf
+template <typename R>
+__device__ __forceinline__ void md_end(Part<R> &q, const double *X, const MdBox<R> &B, const MdArgs<R> &A,
+                                       const R nf[3], int idx, uint64_t step)
+{
     const R dt = A.dt_r;
     if (!((q.f >> WALL_BIT) & 1)) {
         if (q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
@@ -548,91 +884,209 @@ __device__ __forceinline__ int md_forces_end(Part<R> &q, const MdArgs<R> &A, con
         double d[2];
 #pragma unroll
         for (int i = 0; i < 2; i++) {
-            const double d0 = min_image_d(X[3 * i] - px, L[0]), d1 = min_image_d(X[3 * i + 1] - py, L[1]),
-                         d2 = min_image_d(X[3 * i + 2] - pz, L[2]);
+            const double d0 = min_image_d(X[3 * i] - (double)q.p[0], B.L[0]),
+                         d1 = min_image_d(X[3 * i + 1] - (double)q.p[1], B.L[1]),
+                         d2 = min_image_d(X[3 * i + 2] - (double)q.p[2], B.L[2]);
             d[i] = d0 * d0 + d1 * d1 + d2 * d2;
         }
         if ((d[0] > A.cut_c) && (d[1] > A.cut_n)) {
             double u0, u1;
-            rng::uniform2(seed, step, (uint32_t)(q.idx - off), rng::REACT, 0, u0, u1);
+            rng::uniform2(B.seed, step, (uint32_t)(idx - B.off), rng::REACT, 0, u0, u1);
             if (u0 <= A.prob) q.sp = 2;
             q.f &= ~(1 << REAC_BIT);
         }
     }
 #pragma unroll
     for (int k = 0; k < 3; k++) q.g[k] = nf[k];
-    return acts;
 }
 
-// the place in act of entry e of bead h's list, and whether the bead acts on it
-__device__ __forceinline__ int md_place(const MdShared &sh, const int *amap, int h, int e)
-{
-    return e < kMdMap ? sh.map[h][e] : amap[e];
-}
-__device__ __forceinline__ bool md_acts(const MdShared &sh, const unsigned char *cf, int h, int a)
-{
-    const int c = a < kMdFlags ? sh.cf[a] : __ldcg(cf + a);
-    return (c >> h) & 1;
-}
-
-// Bead h's force += the sum of its pair forces, one half of the block per bead
-// (src/neighbor_list.f90:214-218): in list order in the FP64 form -- the
-// contributing entries are compacted in order and three threads add them one
-// by one -- and in the FP32 form by colloid_tree_block's fixed tree.
+// a warp's level of the tree of colloid_tree_block: its leaves' sums to wsum
 template <typename R>
-__device__ __forceinline__ void md_colloid_sums(MdShared &sh, const MdArgs<R> &A, int r)
+__device__ __forceinline__ void md_tree_warp(MdShared<R> &sh, double3 leaf, int h, int l)
 {
-    constexpr int H = kMdThreads / 2, NW = H / 32;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        leaf.x = leaf.x + __shfl_xor_sync(0xffffffffu, leaf.x, o);
+        leaf.y = leaf.y + __shfl_xor_sync(0xffffffffu, leaf.y, o);
+        leaf.z = leaf.z + __shfl_xor_sync(0xffffffffu, leaf.z, o);
+    }
+    if ((l & 31) == 0) {
+        sh.wsum[h][0][l >> 5] = leaf.x;
+        sh.wsum[h][1][l >> 5] = leaf.y;
+        sh.wsum[h][2][l >> 5] = leaf.z;
+    }
+}
+
+// Pair forces that do not all fit in shared memory (beads larger than sigma = 4
+// at density 10): both beads' terms are put in order in global memory and added
+// from there, half of the summing warps per bead (FP32: up to the tree's warp
+// level).
+template <typename R>
+__device__ __noinline__ void md_slow_sums(MdShared<R> &sh, const MdArgs<R> &A, const MdTotals &tt, int r, int k)
+{
+    constexpr int H = kMdSum / 2;
+    const int h = threadIdx.x / H, t = threadIdx.x % H, b = 2 * r + h;
+    MdTerm *terms = A.terms + (size_t)b * A.Nmax;
+    const MdTerm *over = A.over + (size_t)b * A.Nmax;
+    unsigned long long *ka = A.keys[0] + (size_t)b * A.Nmax, *kb = A.keys[1] + (size_t)b * A.Nmax;
+    if (threadIdx.x < 2) sh.tot[threadIdx.x] = 0;
+    md_sync(kBarSum, kMdSum);
+    const int m = *(volatile int *)(A.n_over + 2 * b + (k & 1));
+    for (int j = t; j < kMdTerms + m; j += H) {
+        MdTerm x;
+        if (j < kMdTerms) {
+            if (tt.te[h][j].x != k + 1) continue;
+            x.e = tt.te[h][j].y;
+            for (int c = 0; c < 3; c++) x.f[c] = tt.f[h][c][j];
+        } else {
+            x.e = __ldcg(&over[j - kMdTerms].e);
+            for (int c = 0; c < 3; c++) x.f[c] = __ldcg(&over[j - kMdTerms].f[c]);
+        }
+        const int at = atomicAdd(&sh.tot[h], 1);
+        terms[at] = x;
+        ka[at] = ((unsigned long long)x.e << 32) | (unsigned)at;
+    }
+    md_sync(kBarSum, kMdSum);
+    const int n = sh.tot[h], most = max(sh.tot[0], sh.tot[1]);
+    for (int w = 1; w < most; w <<= 1) {
+        for (int i = t; i < n; i += H) {
+            const int run = i / w, r0 = run * w;
+            const unsigned long long v = ka[i];
+            const int p0 = (run & 1) ? r0 - w : r0 + w, pn = (run & 1) ? w : min(w, max(0, n - p0));
+            int lo = 0, hi = pn;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (ka[p0 + mid] < v) lo = mid + 1;
+                else hi = mid;
+            }
+            kb[((run & 1) ? p0 : r0) + (i - r0) + lo] = v;
+        }
+        md_sync(kBarSum, kMdSum);
+        unsigned long long *x = ka;
+        ka = kb;
+        kb = x;
+    }
+    if constexpr (sizeof(R) == 8) {
+        if (t < 3) {
+            double acc = 0;
+#pragma unroll 8
+            for (int j = 0; j < n; j++) acc = acc + terms[(unsigned)ka[j]].f[t];
+            sh.f[h][t] = acc;
+        }
+    } else {
+        // every leaf's run of the sorted keys, then the tree
+        const int run = sh.box.run[h];
+        for (int q = 0; q < 2; q++) {
+            const int l = t + q * H;
+            int lo = 0, hi = n;
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if ((int)(ka[mid] >> 32) < l * run) lo = mid + 1;
+                else hi = mid;
+            }
+            double3 leaf = make_double3(0, 0, 0);
+            for (int j = lo; j < n && (int)(ka[j] >> 32) < (l + 1) * run; j++) {
+                const MdTerm &x = terms[(unsigned)ka[j]];
+                leaf.x = leaf.x + x.f[0];
+                leaf.y = leaf.y + x.f[1];
+                leaf.z = leaf.z + x.f[2];
+            }
+            md_tree_warp(sh, leaf, h, l);
+        }
+    }
+}
+
+// sh.f[h] = the sum of bead h's pair forces (src/neighbor_list.f90:214-218), half
+// of the summing warps per bead.  The bit map gives every term its place among
+// the step's terms; the FP64 form adds them one after another in list order,
+// one thread per component, as the reference does; the FP32 form adds each
+// leaf's terms and then up colloid_tree_block's tree.
+template <typename R>
+__device__ __forceinline__ void md_colloid_sums(MdShared<R> &sh, MdTotals &tt, const MdArgs<R> &A, int r, int n0,
+                                                int n1, int k)
+{
+    constexpr int H = kMdSum / 2;
     const int h = threadIdx.x / H, t = threadIdx.x % H, lane = t & 31, w = t >> 5;
-    const int ni = A.n[2 * r + h];
-    const int *amap = A.amap + (size_t)(2 * r + h) * A.Nmax;
-    const double *pf = A.pf + (size_t)2 * r * A.Nmax * 6 + 3 * h;
-    const unsigned char *cf = A.cf + (size_t)2 * r * A.Nmax;
-    if constexpr (sizeof(R) == 4) {
-        static_assert(H == kNlBlockThreads, "colloid_tree_block's order");
-        double a0 = 0, a1 = 0, a2 = 0;
-        for (int e0 = t; e0 < ni; e0 += 32 * H) {
-            unsigned mask = 0;
-            for (int u = 0; u < 32; u++) {
-                const int e = e0 + u * H;
-                if (e >= ni) break;
-                if (md_acts(sh, cf, h, md_place(sh, amap, h, e))) mask |= 1u << u;
-            }
-            while (mask) {
-                double f[4][3];
-                unsigned got = 0;
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (mask) {
-                        const double *q = pf + 6 * (size_t)md_place(sh, amap, h, e0 + (__ffs(mask) - 1) * H);
-                        mask &= mask - 1;
-                        f[k][0] = __ldcg(q);
-                        f[k][1] = __ldcg(q + 1);
-                        f[k][2] = __ldcg(q + 2);
-                        got |= 1u << k;
-                    }
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if ((got >> k) & 1) {
-                        a0 = a0 + f[k][0];
-                        a1 = a1 + f[k][1];
-                        a2 = a2 + f[k][2];
-                    }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            a0 = a0 + __shfl_xor_sync(0xffffffffu, a0, o);
-            a1 = a1 + __shfl_xor_sync(0xffffffffu, a1, o);
-            a2 = a2 + __shfl_xor_sync(0xffffffffu, a2, o);
-        }
-        if (lane == 0) {
-            sh.wsum[h][0][w] = a0;
-            sh.wsum[h][1][w] = a1;
-            sh.wsum[h][2][w] = a2;
-        }
-        __syncthreads();
+    const int n = h ? n1 : n0;
+    if (sh.spill == k + 1) {
+        md_slow_sums<R>(sh, A, tt, r, k);
+    } else {
+        // terms before each word: a warp per bead, runs of words per lane
+        const int places = sizeof(R) == 8 ? n : kNlBlockThreads * sh.box.run[h];
+        const int words = min((places + 31) / 32, kMdBits / 32), m = sh.cnt[k & 1][h];
         if (w == 0) {
+            const int per = (words + 31) / 32, q0 = min(words, lane * per), q1 = min(words, q0 + per);
+            int c = 0;
+            for (int q = q0; q < q1; q++) c += __popc(tt.bits[h][q]);
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            int run = inc - c;
+            for (int q = q0; q < q1; q++) {
+                tt.base[h][q] = (unsigned short)run;
+                run += __popc(tt.bits[h][q]);
+            }
+        }
+        md_sync(kBarSum, kMdSum);
+        // the terms before place o (none is beyond the map, or it would have
+        // gone to global memory)
+        auto before = [&](int o) {
+            return o >= kMdBits ? m : tt.base[h][o >> 5] + __popc(tt.bits[h][o >> 5] & ((1u << (o & 31)) - 1u));
+        };
+        // into order
+        for (int j = t; j < m; j += H) {
+            const int at = before(tt.te[h][j].y);
+            tt.g[h][0][at] = tt.f[h][0][j];
+            tt.g[h][1][at] = tt.f[h][1][j];
+            tt.g[h][2][at] = tt.f[h][2][j];
+        }
+        md_sync(kBarSum, kMdSum);
+        if constexpr (sizeof(R) == 8) {
+            if (t < 3) {
+                const double *g = tt.g[h][t];
+                double acc = 0;
+                int j = 0;
+                if (m >= 8) {
+                    double v[8], u[8];
+#pragma unroll
+                    for (int c = 0; c < 8; c++) v[c] = g[c];
+                    for (; j + 16 <= m; j += 8) {
+#pragma unroll
+                        for (int c = 0; c < 8; c++) u[c] = g[j + 8 + c];
+#pragma unroll
+                        for (int c = 0; c < 8; c++) acc = acc + v[c];
+#pragma unroll
+                        for (int c = 0; c < 8; c++) v[c] = u[c];
+                    }
+#pragma unroll
+                    for (int c = 0; c < 8; c++) acc = acc + v[c];
+                    j += 8;
+                }
+                for (; j < m; j++) acc = acc + g[j];
+                sh.f[h][t] = acc;
+            }
+        } else {
+            const int run = sh.box.run[h];
+            for (int q = 0; q < 2; q++) {
+                const int l = t + q * H;
+                const int lo = run ? before(l * run) : 0, hi = run && l < kNlBlockThreads - 1 ? before((l + 1) * run) : m;
+                double3 leaf = make_double3(0, 0, 0);
+                for (int j = lo; j < hi; j++) {
+                    leaf.x = leaf.x + tt.g[h][0][j];
+                    leaf.y = leaf.y + tt.g[h][1][j];
+                    leaf.z = leaf.z + tt.g[h][2][j];
+                }
+                md_tree_warp(sh, leaf, h, l);
+            }
+        }
+    }
+    if constexpr (sizeof(R) == 4) {
+        md_sync(kBarSum, kMdSum);
+        if (w == 0) {
+            constexpr int NW = kNlBlockThreads / 32;
             double b0 = lane < NW ? sh.wsum[h][0][lane] : 0.0, b1 = lane < NW ? sh.wsum[h][1][lane] : 0.0,
                    b2 = lane < NW ? sh.wsum[h][2][lane] : 0.0;
 #pragma unroll
@@ -642,296 +1096,370 @@ __device__ __forceinline__ void md_colloid_sums(MdShared &sh, const MdArgs<R> &A
                 b2 = b2 + __shfl_xor_sync(0xffffffffu, b2, o);
             }
             if (lane == 0) {
-                sh.force[0][h] = sh.force[0][h] + b0;
-                sh.force[1][h] = sh.force[1][h] + b1;
-                sh.force[2][h] = sh.force[2][h] + b2;
+                sh.f[h][0] = b0;
+                sh.f[h][1] = b1;
+                sh.f[h][2] = b2;
             }
         }
-        __syncthreads();
-    } else {
-        // each warp takes a contiguous run of the list
-        const int per = (ni + 32 * NW - 1) / (32 * NW) * 32;
-        const int e_lo = w * per, e_hi = min(ni, e_lo + per);
-        int cnt = 0;
-        for (int e = e_lo + lane; e - lane < e_hi; e += 32) {
-            const bool on = e < e_hi && md_acts(sh, cf, h, md_place(sh, amap, h, e));
-            cnt += __popc(__ballot_sync(0xffffffffu, on));
-        }
-        if (lane == 0) sh.wcnt[h][w] = cnt;
-        __syncthreads();
-        int before = 0, tot[2] = {0, 0};
-        for (int k = 0; k < NW; k++) {
-            if (k < w) before += sh.wcnt[h][k];
-            tot[0] += sh.wcnt[0][k];
-            tot[1] += sh.wcnt[1][k];
-        }
-        const int most = max(tot[0], tot[1]), mine = tot[h];
-        double acc = 0;  // thread c < 3 of the half adds component c
-        for (int c0 = 0; c0 < most; c0 += kMdList) {
-            int at = before;
-            for (int e = e_lo + lane; e - lane < e_hi; e += 32) {
-                const int a = e < e_hi ? md_place(sh, amap, h, e) : 0;
-                const bool on = e < e_hi && md_acts(sh, cf, h, a);
-                const unsigned bal = __ballot_sync(0xffffffffu, on);
-                const int k = at + __popc(bal & ((1u << lane) - 1u));
-                if (on && k >= c0 && k < c0 + kMdList) sh.lst[h][k - c0] = a;
-                at += __popc(bal);
-            }
-            __syncthreads();
-            for (int v0 = 0; v0 < kMdList && c0 + v0 < most; v0 += H) {
-                const int m = min(H, mine - c0 - v0);
-                if (t < m) {
-                    const double *q = pf + 6 * (size_t)sh.lst[h][v0 + t];
-                    sh.val[h][0][t] = __ldcg(q);
-                    sh.val[h][1][t] = __ldcg(q + 1);
-                    sh.val[h][2][t] = __ldcg(q + 2);
-                }
-                __syncthreads();
-                if (t < 3) {
-#pragma unroll 8
-                    for (int k = 0; k < m; k++) acc = acc + sh.val[h][t][k];
-                }
-                __syncthreads();
-            }
-        }
-        if (t < 3) sh.force[t][h] = sh.force[t][h] + acc;
-        __syncthreads();
     }
+    md_sync(kBarSum, kMdSum);
 }
 
-__device__ inline PView<double> md_beads(MdShared &sh)
+__device__ __forceinline__ double md_lane(double x, int l) { return __shfl_sync(0xffffffffu, x, l); }
+// x . y of values whose components lanes l0, l0 + 1, l0 + 2 hold
+__device__ __forceinline__ double md_dot(double x, double y, int l0)
 {
-    PView<double> c{};
-    c.N = 2;
-    c.pos = {sh.pos[0], sh.pos[1], sh.pos[2]};
-    c.vel = {sh.vel[0], sh.vel[1], sh.vel[2]};
-    c.force = {sh.force[0], sh.force[1], sh.force[2]};
-    c.force_old = {sh.fold[0], sh.fold[1], sh.fold[2]};
-    c.species = sh.species;
-    return c;
+    const double p = x * y;
+    return md_lane(p, l0) + md_lane(p, l0 + 1) + md_lane(p, l0 + 2);
+}
+
+template <typename R>
+__device__ __forceinline__ MdPair md_pair(const MdBead &b, const MdArgs<R> &A)
+{
+    MdPair p;
+    p.s = min_image_d(md_lane(b.pos, b.k) - md_lane(b.pos, b.k + 3), b.L);
+    p.rsq = md_dot(p.s, p.s, 0);
+    p.g.set(b.dt_inv_mass * p.rsq);
+    p.acts = p.rsq <= A.lj_cc.cut_sq[(b.sp0 - 1) + A.lj_cc.n1 * (b.sp1 - 1)];
+    p.f = 0;
+    if (p.acts) {
+        const int tt = (b.sp1 - 1) + A.lj_cc.n1 * (b.sp0 - 1);
+        p.f = lj_force_over_r(p.rsq, A.lj_cc.epsilon[tt], A.lj_cc.sigma[tt]) * p.s;
+    }
+    return p;
 }
 
 // compute_force_n2, the colloid velocity half and RATTLE's velocity correction
 // (src/neighbor_list.f90:227-264, programs/single_dimer_pbc.f90:356-359,
-// src/md.f90:298-319)
+// src/md.f90:298-319), the arithmetic of force_n2_one, colloid_vv_vel_one and
+// rattle_vel_dimer
 template <typename R>
-__device__ __forceinline__ void md_colloid_end(MdShared &sh, const MdArgs<R> &A, int r, const double e[3])
+__device__ __forceinline__ void md_colloid_end(MdBead &b, const MdPair &p, const MdArgs<R> &A)
 {
-    PView<double> c = md_beads(sh);
-    for (int m = 0; m < 2; m++)
-        force_n2_one(m, c.pos.x, c.pos.y, c.pos.z, c.species, 2, e[0], e[1], e[2], A.lj_cc, c.force.x, c.force.y,
-                     c.force.z);
-    colloid_vv_vel_one(c, 0, A.mass[2 * r], A.dt);
-    colloid_vv_vel_one(c, 1, A.mass[2 * r + 1], A.dt);
-    rattle_vel_dimer(c, A.ms, A.bond, E3{{e[0], e[1], e[2]}}, A.err);
+    if (p.acts) b.force = b.i == 0 ? b.force + p.f : b.force - p.f;
+    b.vel = b.vel + b.vv.of(A.dt * (b.force + b.fold));
+    const double dv = md_lane(b.vel, b.k) - md_lane(b.vel, b.k + 3);
+    const double kk = b.kk.of(md_dot(dv, p.s, 0));
+    const double c = b.m.of(kk * p.s);
+    b.vel = b.i == 0 ? b.vel - c : b.vel + c;
 }
 
-// the colloid position half, RATTLE and switch_force
-// (programs/single_dimer_pbc.f90:311-322); returns the beads' displacement
+// the colloid position half, RATTLE (colloid_vv_pos_one, rattle_pos_dimer) and
+// switch_force (programs/single_dimer_pbc.f90:311-322); returns the beads' largest
+// displacement
 template <typename R>
-__device__ __forceinline__ double md_colloid_begin(MdShared &sh, const MdArgs<R> &A, int r, const double e[3])
+__device__ __forceinline__ double md_colloid_begin(MdShared<R> &sh, MdBead &b, const MdPair &p, const MdArgs<R> &A)
 {
-    PView<double> c = md_beads(sh);
-    for (int k = 0; k < 3; k++)
-        for (int i = 0; i < 2; i++) sh.rat[k][i] = sh.pos[k][i];
-    colloid_vv_pos_one(c, 0, A.mass[2 * r], A.dt);
-    colloid_vv_pos_one(c, 1, A.mass[2 * r + 1], A.dt);
-    rattle_pos_dimer(c, sh.rat[0], sh.rat[1], sh.rat[2], A.ms, A.bond, A.dt, E3{{e[0], e[1], e[2]}}, A.err);
-    Vec3<double> o = {sh.old[0], sh.old[1], sh.old[2]};
-    const double m0 = disp_sq_one(c.pos, o, c.species, 0), m1 = disp_sq_one(c.pos, o, c.species, 1);
-    for (int k = 0; k < 3; k++)
-        for (int i = 0; i < 2; i++) {
-            sh.fold[k][i] = sh.force[k][i];
-            sh.force[k][i] = 0;
-        }
+    if (threadIdx.x < 6) sh.rat[threadIdx.x] = b.pos;
+    b.pos = b.pos + A.dt * b.vel + b.vv.of(A.dt * A.dt * b.force);
+    const double s = min_image_d(md_lane(b.pos, b.k) - md_lane(b.pos, b.k + 3), b.L);
+    const double ssq = md_dot(s, s, 0), rs = md_dot(p.s, s, 0);
+    const double disc = rs * rs - p.rsq * (ssq - A.bond * A.bond);
+    if (disc < 0 && threadIdx.x == 0) atomicOr(A.err, DEV_ERR_RATTLE);
+    const double g = p.g.of(rs - sqrt(disc));
+    const double dp = b.m.of(g * A.dt * p.s), dv = b.m.of(g * p.s);
+    b.pos = b.i == 0 ? b.pos - dp : b.pos + dp;
+    b.vel = b.i == 0 ? b.vel - dv : b.vel + dv;
+    const double d = b.pos - sh.old[3 * b.i + b.k];
+    const double q0 = md_dot(d, d, 0), q1 = md_dot(d, d, 3);
+    const double m0 = b.sp0 < 0 ? 0 : q0, m1 = b.sp1 < 0 ? 0 : q1;
+    b.fold = b.force;
+    b.force = 0;
     return sqrt(m0 > m1 ? m0 : m1);
 }
 
-// warp 0 of block 0: with the displacements of MD step k's beginning complete,
-// the colloid position half and the re-sort test of step k
-// (programs/single_dimer_pbc.f90:311-330), then the bead positions and the
-// decision to every block of the cluster
+// warp 0: the end of MD step k - 1 (end), the colloid position half and the beads'
+// part of the re-sort test of step k (begin; programs/single_dimer_pbc.f90:311-330),
+// then the bead positions and the decision for all warps
 template <typename R>
-__device__ __forceinline__ void md_turn(MdShared &sh, const MdArgs<R> &A, int r, const double e[3], int k, int blocks,
-                                        bool end, bool begin)
+__device__ __forceinline__ void md_turn(MdShared<R> &sh, MdBead &b, const MdPair &p, const MdArgs<R> &A, int k,
+                                        int s_free, bool end, bool begin)
 {
-    namespace cg = cooperative_groups;
     const int lane = threadIdx.x;
-    if (end && lane == 0) md_colloid_end<R>(sh, A, r, e);
+    if (end) {
+        b.force = b.force + sh.f[b.i][b.k];
+        md_colloid_end<R>(b, p, A);
+    }
     if (begin) {
-        double m = 0;
-        for (int w = lane; w < blocks * (kMdThreads / 32); w += 32) m = m > sh.wmax[w] ? m : sh.wmax[w];
-        m = warp_max(m);
-        if (lane == 0) {
-            const double co = md_colloid_begin<R>(sh, A, r, e);
-            const double so = sqrt(m);
-            sh.stop = (co >= A.skin * 0.1) || (so >= A.skin * 0.89) || k >= A.s_free[r];
-        }
-        __syncwarp();
-        if (lane < blocks) {
-            MdShared *to = cg::this_cluster().map_shared_rank(&sh, lane);
-            for (int q = 0; q < 6; q++) to->x[q] = sh.pos[q % 3][q / 3];
-            if (lane > 0) to->stop = sh.stop;
-        }
+        const double from = b.pos;
+        const double co = md_colloid_begin<R>(sh, b, p, A);
+        // (not "less than": a NaN makes the queue anew as well)
+        const bool far = __any_sync(0xffffffffu, !((float)fabs(b.pos - from) < 0.5f * kMdWay));
+        if (lane < 6) sh.x[k & 1][lane] = b.pos;
+        if (lane == 6) sh.stop = (co >= A.skin * 0.1) || k >= s_free;
+        if (lane == 7) sh.anew = far;
     }
 }
 
 // The MD steps of every replica (start) or of those that were re-sorted
-// (resort[r]), one cluster per replica, each until its next re-sort or the
-// interval's end.  Per step two cluster barriers: after every particle's
-// forces, velocity and next position (the bead sums and the re-sort test need
-// them), and after the beads' turn (the particles need their positions).
-// Latency bound: a step is this chain of barriers, L2 round trips of the pair
-// forces to block 0 and one thread's bead arithmetic.
+// (resort[r]), one block per replica, each until its next re-sort or the
+// interval's end.  A step: the queued particles -- those a bead may reach, by a
+// distance in single precision, and those with flags -- get their pair forces;
+// while the first eight warps add these in order and move the beads, the
+// others move the particles and queue those of the next step.  Latency bound:
+// one pair force, the ordered sum and the beads' chain of quotients, one after
+// the other, at an instruction every ~6 cycles of a code that no warp runs
+// twice in a row; FP64 throughput and memory play no part.  (A cluster of eight
+// blocks per replica spent two cluster barriers of ~2,000 cycles per step.)
 template <typename R>
-__global__ void __launch_bounds__(kMdThreads, 1) kb_md(MdArgs<R> A)
+__global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ MdArgs<R> A)
 {
-    namespace cg = cooperative_groups;
     extern __shared__ __align__(16) unsigned char md_smem[];
-    MdShared &sh = *reinterpret_cast<MdShared *>(md_smem);
-    cg::cluster_group cl = cg::this_cluster();
-    const int blocks = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-    const int r = blockIdx.x / blocks;
+    MdShared<R> &sh = *reinterpret_cast<MdShared<R> *>(md_smem);
+    constexpr size_t kHead = (sizeof(MdShared<R>) + 15) & ~(size_t)15;
+    constexpr size_t kParts = (kHead + sizeof(MdTotals) + 15) & ~(size_t)15;
+    static_assert(kParts + 64 * 1024 <= kMdSmem, "room for particles");
+    MdTotals &totals = *reinterpret_cast<MdTotals *>(md_smem + kHead);
+    const int r = blockIdx.x;
     const int t = threadIdx.x;
-    int need = 0;
+    const int all = blockDim.x;
     if (A.start || A.resort[r]) {
         const BRep &rp = A.rep[r];
-        const long long off = rp.off;
-        const uint64_t seed = rp.seed, step0 = *A.d_step;
-        const double L[3] = {rp.g.edges[0], rp.g.edges[1], rp.g.edges[2]};
-        const PView<R> v = pick(A.v0, A.v1, rp.cur);
-        const Vec3<R> old = rp.cur ? A.v0.pos : A.v1.pos;
-        const bool fresh = A.fresh[r] != 0;
-        const int nl = A.nl[r], na = nl + A.nx[r];
-        const int nthr = blocks * kMdThreads, tid = rank * kMdThreads + t;
-        double *pf = A.pf + (size_t)2 * r * A.Nmax * 6;
-        unsigned char *cf = A.cf + (size_t)2 * r * A.Nmax;
-        MdShared *sh0 = cl.map_shared_rank(&sh, 0);
-        cl.sync();  // every block runs before its shared memory is written from another
+        MdBox<R> &W = sh.box;
+        if (t == 0) {
+            W.off = rp.off;
+            W.seed = rp.seed;
+            W.r = r;
+            for (int k = 0; k < 3; k++) {
+                W.L[k] = rp.g.edges[k];
+                W.lf[k] = (float)rp.g.edges[k];
+                W.hf[k] = 0.5f * (float)rp.g.edges[k];
+            }
+            for (int i = 0; i < 2; i++) W.cs[i] = A.c.species[2 * r + i];
+            // single precision of positions inside twice the box: 1e-5 of the
+            // edges is far above the rounding of a distance
+            const float reach = A.reach + 1e-5f * (float)(rp.g.edges[0] + rp.g.edges[1] + rp.g.edges[2]);
+            W.reach_sq = reach * reach;
+            W.queue_sq = (reach + kMdWay) * (reach + kMdWay);
+            W.cur = rp.cur;
+            W.nl = A.nl[r];
+            W.na = W.nl + A.nx[r];
+            for (int h = 0; h < 2; h++) W.run[h] = (A.n[2 * r + h] + kNlBlockThreads - 1) / kNlBlockThreads;
+            W.parts.cap = (int)((kMdSmem - kParts) / md_part_bytes<R>());
+            W.parts.r = reinterpret_cast<R *>(md_smem + kParts);
+            W.parts.i = reinterpret_cast<int *>(W.parts.r + 18 * (size_t)W.parts.cap);
+            sh.stop = sh.over = sh.spill = 0;
+            sh.anew = 1;
+            for (int p = 0; p < 2; p++) {
+                sh.nq[p] = sh.cnt[p][0] = sh.cnt[p][1] = 0;
+                A.n_over[4 * r + 2 * p] = A.n_over[4 * r + 2 * p + 1] = 0;
+            }
+        }
+        for (int q = t; q < 2 * (kMdBits / 32); q += all) (&totals.bits[0][0])[q] = 0;
+        for (int q = t; q < 2 * kMdTerms; q += all) (&totals.te[0][0])[q] = make_int2(0, 0);
+        __syncthreads();
+        const MdBox<R> &B = sh.box;
+        const int s_free = A.s_free[r];
         int k = A.start ? 0 : A.adv[r] - 1;
-        const int cs[2] = {A.c.species[2 * r], A.c.species[2 * r + 1]};
-        // this thread's particles: kMdPer in registers, the rest in place
-        Part<R> q[kMdPer];
-#pragma unroll
-        for (int u = 0; u < kMdPer; u++)
-            if (tid + u * nthr < na) md_load(q[u], A, v, old, off, r, tid + u * nthr, nl, fresh);
-        double m = 0;
-        if (A.start) {
-            // force_old of the last interval's end is no longer current
-            auto clear_old = [&](const Part<R> &p) {
-                if ((p.f >> PAST_MD_BIT) & 1) v.force_old.x[p.idx] = v.force_old.y[p.idx] = v.force_old.z[p.idx] = 0;
-            };
-#pragma unroll
-            for (int u = 0; u < kMdPer; u++)
-                if (tid + u * nthr < na) {
-                    clear_old(q[u]);
-                    const double d = md_begin(q[u], A.dt_r, A.dt_sq_r, A.read_species);
-                    m = m > d ? m : d;
+        if (t < kMdSum) {
+            // ---- the beads ----
+            const int n0 = A.n[2 * r], n1 = A.n[2 * r + 1];
+            MdBead b{};
+            MdPair pair{};
+            if (t < 32) {
+                b.i = t < 6 ? t / 3 : 0;
+                b.k = t < 6 ? t % 3 : 0;
+                const int c = 2 * r + b.i;
+                b.pos = A.c.pos[b.k][c];
+                b.vel = A.c.vel[b.k][c];
+                b.force = A.c.force[b.k][c];
+                b.fold = A.c.force_old[b.k][c];
+                if (t < 6) {
+                    sh.old[t] = A.cold[b.k][c];
+                    sh.rat[t] = A.rat[b.k][c];
                 }
-        }
-        for (int a = tid + kMdPer * nthr; a < na; a += nthr) {
-            Part<R> p;
-            md_load(p, A, v, old, off, r, a, nl, fresh);
-            if (!fresh)
-                for (int c = 0; c < 3; c++) old[c][p.idx] = p.o[c];
-            if (A.start) {
-                if ((p.f >> PAST_MD_BIT) & 1) v.force_old.x[p.idx] = v.force_old.y[p.idx] = v.force_old.z[p.idx] = 0;
-                const double d = md_begin(p, A.dt_r, A.dt_sq_r, A.read_species);
-                m = m > d ? m : d;
-                md_store(p, v);
+                __syncwarp();
+                b.sp0 = B.cs[0];
+                b.sp1 = B.cs[1];
+                const double m1 = bead_mass(A.ms, B.cs, 0, A.err), m2 = bead_mass(A.ms, B.cs, 1, A.err);
+                const double inv_mass = 1 / m1 + 1 / m2;
+                b.vv.set(2 * A.mass[c]);
+                b.m.set(b.i == 0 ? m1 : m2);
+                b.kk.set(A.bond * A.bond * inv_mass);
+                b.dt_inv_mass = A.dt * inv_mass;
+                b.L = B.L[b.k];
+                pair = md_pair<R>(b, A);
+                if (A.start) {
+                    md_turn<R>(sh, b, pair, A, k, s_free, false, true);
+                    pair = md_pair<R>(b, A);
+                } else if (t < 6) {
+                    // resumed after a re-sort: the step's forces come next
+                    sh.x[k & 1][t] = b.pos;
+                }
+                __syncwarp();
+                if (t == 0) sh.anew = 1;  // there is no queue yet
             }
-        }
-        if (rank == 0) {
-            for (int h = 0; h < 2; h++)
-                for (int e = t; e < min(A.n[2 * r + h], kMdMap); e += kMdThreads)
-                    sh.map[h][e] = A.amap[(size_t)(2 * r + h) * A.Nmax + e];
+            __syncthreads();
+            while (!(sh.stop | sh.over)) {
+                const bool last = k + 1 == A.N_MD;
+                md_sync(kBarForces, all);
+                md_colloid_sums<R>(sh, totals, A, r, n0, n1, k);
+                if (t < 32) {
+                    md_turn<R>(sh, b, pair, A, k + 1, s_free, true, !last);
+                } else {
+                    // ready for the step after the next forces
+                    // (256 places more: the FP32 form's leaves are of whole runs)
+                    for (int q = t - 32; q < (max(n0, n1) + 287) / 32 && q < kMdBits / 32; q += kMdSum - 32)
+                        totals.bits[0][q] = totals.bits[1][q] = 0;
+                    if (t < 34) {
+                        sh.cnt[k & 1][t - 32] = 0;
+                        A.n_over[2 * (2 * r + t - 32) + (k & 1)] = 0;
+                    }
+                    if (t == 34) sh.nq[k & 1] = 0;
+                }
+                md_sync(kBarTurn, all);
+                // in the shadow of the forces: what the next turn needs of the
+                // positions
+                if (t < 32) pair = md_pair<R>(b, A);
+                k++;
+                if (last) break;
+            }
             if (t < 6) {
-                const int c = t % 3, i = t / 3;
-                sh.pos[c][i] = A.c.pos[c][2 * r + i];
-                sh.vel[c][i] = A.c.vel[c][2 * r + i];
-                sh.force[c][i] = A.c.force[c][2 * r + i];
-                sh.fold[c][i] = A.c.force_old[c][2 * r + i];
-                sh.old[c][i] = A.cold[c][2 * r + i];
-                sh.rat[c][i] = A.rat[c][2 * r + i];
-                if (c == 0) sh.species[i] = cs[i];
-            }
-        }
-        m = warp_max(m);
-        if ((t & 31) == 0) sh0->wmax[rank * (kMdThreads / 32) + (t >> 5)] = m;
-        cl.sync();
-        if (rank == 0 && t < 32) {
-            if (A.start) {
-                md_turn<R>(sh, A, r, L, k, blocks, false, true);
-            } else if (t < blocks) {
-                // resumed after a re-sort: the step's forces come next
-                MdShared *to = cl.map_shared_rank(&sh, t);
-                for (int c = 0; c < 6; c++) to->x[c] = sh.pos[c % 3][c / 3];
-                to->stop = 0;
-            }
-        }
-        cl.sync();
-        while (!sh.stop) {
-            const bool last = k + 1 == A.N_MD;
-            const double X[6] = {sh.x[0], sh.x[1], sh.x[2], sh.x[3], sh.x[4], sh.x[5]};
-            m = 0;
-            // one particle's forces and end of step k, then its beginning of step k + 1
-            auto one = [&](Part<R> &p, int a) {
-                if (last) {
-                    // the interval's last step leaves force_old behind
-                    const bool past = (p.f >> PAST_MD_BIT) & 1;
-                    for (int c = 0; c < 3; c++) v.force_old[c][p.idx] = past ? p.g[c] : (R)0;
-                }
-                const int acts = md_forces_end(p, A, X, cs, L, pf + 6 * (size_t)a, seed, step0 + (uint64_t)k, off);
-                if (a < nl) {
-                    if (a < kMdFlags) sh0->cf[a] = (unsigned char)acts;
-                    else cf[a] = (unsigned char)acts;
-                }
-                if (!last) {
-                    const double d = md_begin(p, A.dt_r, A.dt_sq_r, A.read_species);
-                    m = m > d ? m : d;
-                }
-            };
-#pragma unroll
-            for (int u = 0; u < kMdPer; u++)
-                if (tid + u * nthr < na) one(q[u], tid + u * nthr);
-            for (int a = tid + kMdPer * nthr; a < na; a += nthr) {
-                Part<R> p;
-                md_load(p, A, v, old, off, r, a, nl, true);
-                one(p, a);
-                md_store(p, v);
-            }
-            m = warp_max(m);
-            if ((t & 31) == 0) sh0->wmax[rank * (kMdThreads / 32) + (t >> 5)] = m;
-            cl.sync();
-            if (rank == 0) {
-                md_colloid_sums<R>(sh, A, r);
-                if (t < 32) md_turn<R>(sh, A, r, L, k + 1, blocks, true, !last);
-            }
-            cl.sync();
-            k++;
-            if (last) break;
-        }
-        need = k < A.N_MD;  // stopped in front of step k's forces
-#pragma unroll
-        for (int u = 0; u < kMdPer; u++)
-            if (tid + u * nthr < na) md_store(q[u], v);
-        if (rank == 0) {
-            if (t < 6) {
-                const int c = t % 3, i = t / 3;
-                A.c.pos[c][2 * r + i] = sh.pos[c][i];
-                A.c.vel[c][2 * r + i] = sh.vel[c][i];
-                A.c.force[c][2 * r + i] = sh.force[c][i];
-                A.c.force_old[c][2 * r + i] = sh.fold[c][i];
-                A.rat[c][2 * r + i] = sh.rat[c][i];
+                const int c = 2 * r + b.i;
+                A.c.pos[b.k][c] = b.pos;
+                A.c.vel[b.k][c] = b.vel;
+                A.c.force[b.k][c] = b.force;
+                A.c.force_old[b.k][c] = b.fold;
+                A.rat[b.k][c] = sh.rat[t];
             }
             if (t == 0) {
+                const int need = k < A.N_MD;  // stopped in front of step k's forces
                 A.adv[r] = need ? k + 1 : A.N_MD;
                 A.resort[r] = need;
                 if (need) A.n_extra[r] += 1;
             }
+        } else {
+            // ---- the particles ----
+            const int me = t - kMdSum, threads = all - kMdSum;
+            const bool fresh = A.fresh[r] != 0;
+            const double thr = A.skin * 0.89;
+            const float near_sq = 0.99f * (float)thr * (float)thr;
+            const uint64_t step0 = *A.d_step;
+            for (int i = me; i < B.na; i += threads) {
+                int idx;
+                Part<R> q = md_read(B, A, i, idx, true);
+                if (!fresh)
+                    for (int c = 0; c < 3; c++) {
+                        q.o[c] = q.p[c];
+                        if (i >= B.parts.cap) md_old(A, B)[c][idx] = q.p[c];
+                    }
+                if (A.start) {
+                    // force_old of the last interval's end is no longer current
+                    if ((q.f >> PAST_MD_BIT) & 1)
+                        for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = 0;
+                    if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over = 1;
+                }
+                if (i < B.parts.cap) {
+                    B.parts.num(0, i) = idx;
+                    int m = 0, e[2] = {0, 0};
+                    if (i < B.nl) {
+                        const size_t w = (size_t)2 * r * A.Nmax + i;
+                        m = A.mult[w];
+                        e[0] = A.ent[2 * w];
+                        e[1] = A.ent[2 * w + 1];
+                    }
+                    B.parts.num(3, i) = m;
+                    B.parts.num(4, i) = e[0];
+                    B.parts.num(5, i) = e[1];
+                    for (int c = 0; c < 3; c++) B.parts.real(6 + c, i) = q.o[c];
+                }
+                md_write(B, A, i, idx, q, false);
+            }
+            __syncthreads();
+            while (!(sh.stop | sh.over)) {
+                const bool last = k + 1 == A.N_MD;
+                const int par = k & 1;
+                const double *X = sh.x[par];
+                const int shared = min(B.na, B.parts.cap);
+                if (sh.anew || sh.nq[par] > kMdQueue) {
+                    // no queue (the first step, a bead that leapt) or one too long
+                    for (int i = me; i < shared; i += threads) {
+                        const R p[3] = {B.parts.real(0, i), B.parts.real(1, i), B.parts.real(2, i)};
+                        const int m = md_busy(X, B, p, B.parts.num(1, i), B.queue_sq);
+                        B.parts.num(6, i) = m;
+                        B.parts.num(7, i) = 0;
+                        if (m & 1) md_pair_force(sh, B, A, totals, i, 0, k);
+                        if (m & 2) md_pair_force(sh, B, A, totals, i, 1, k);
+                    }
+                } else {
+                    const int nq = sh.nq[par];
+                    for (int s = me; s < nq; s += threads) {
+                        const int e = sh.q[par][s];
+                        md_pair_force(sh, B, A, totals, e >> 1, e & 1, k);
+                    }
+                }
+                // the particles that the shared memory does not hold: their
+                // forces wait in force_old, whose entry is written again below
+                for (int i = B.parts.cap + me; i < B.na; i += threads) {
+                    int idx;
+                    const Part<R> q = md_read(B, A, i, idx, false);
+                    if (!md_busy(X, B, q.p, q.f, B.reach_sq)) continue;
+                    R nf[3];
+                    md_view(A, B).flags[idx] = md_forces(sh, B, A, totals, i, k, q.p, q.sp, q.f, nf);
+                    for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = nf[c];
+                }
+                md_arrive(kBarForces, all);
+                md_sync(kBarPart, threads);  // the forces are written
+                // every particle's end of step k and beginning of step k + 1
+                for (int i = me; i < B.na; i += threads) {
+                    const bool in = i < B.parts.cap;
+                    int idx;
+                    Part<R> q = md_read(B, A, i, idx, false);
+                    const bool past = (q.f >> PAST_MD_BIT) & 1;
+                    const R gl[3] = {past ? q.g[0] : (R)0, past ? q.g[1] : (R)0, past ? q.g[2] : (R)0};
+                    // (forces only add flags, so the test gives what it gave)
+                    if (in ? B.parts.num(6, i) : md_busy(X, B, q.p, q.f, B.reach_sq)) {
+                        R nf[3] = {0, 0, 0};
+                        if (in) {
+                            const int came = B.parts.num(7, i), m = B.parts.num(3, i);
+#pragma unroll
+                            for (int h = 0; h < 2; h++)
+                                if ((came >> h) & 1) {
+                                    q.f |= (1 << MD_BIT) | (B.cs[h] == 1 ? (1 << CATALYZED_BIT) : 0);
+                                    for (int u = 0; u < (h ? m >> 16 : m & 0xffff); u++)
+                                        for (int c = 0; c < 3; c++) nf[c] = nf[c] - B.parts.real(12 + 3 * h + c, i);
+                                }
+                            if (came & 4) q.f |= 1 << REAC_BIT;
+                        } else {
+                            for (int c = 0; c < 3; c++) nf[c] = md_view(A, B).force_old[c][idx];
+                        }
+                        md_end(q, X, B, A, nf, idx, step0 + (uint64_t)k);
+                        if (!in && !last)
+                            for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = 0;
+                    } else {
+                        for (int c = 0; c < 3; c++) q.v[c] = md_vel_free(q.v[c], A.dt_r);
+                    }
+                    if (last) {
+                        // the interval's last step leaves force_old behind
+                        for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = gl[c];
+                    } else {
+                        if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over = 1;
+                        if (in) {
+                            const int m = md_busy(X, B, q.p, q.f, B.queue_sq);
+                            B.parts.num(6, i) = m;
+                            B.parts.num(7, i) = 0;
+                            if (m & 3) {
+                                const int s = atomicAdd(&sh.nq[1 - par], (m & 1) + (m >> 1 & 1));
+                                const int e = 2 * i + (m & 1 ? 0 : 1);
+                                if (s < kMdQueue) sh.q[1 - par][s] = e;
+                                if ((m & 3) == 3 && s + 1 < kMdQueue) sh.q[1 - par][s + 1] = 2 * i + 1;
+                            }
+                        }
+                    }
+                    md_write(B, A, i, idx, q, false);
+                }
+                md_sync(kBarTurn, all);
+                k++;
+                if (last) break;
+            }
+            for (int i = me; i < min(B.na, B.parts.cap); i += threads) {
+                int idx;
+                const Part<R> q = md_read(B, A, i, idx, false);
+                md_write(B, A, i, idx, q, true);
+            }
         }
+        __syncthreads();
     }
-    if (rank != 0) return;
     // the last replica to finish lists the tiles of those to re-sort and sets
     // the graph's loop condition
     if (t == 0) {
@@ -942,7 +1470,7 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(MdArgs<R> A)
     if (!sh.last) return;
     __threadfence();
     int any = 0, base_p = 0, base_s = 0;
-    for (int r0 = 0; r0 < A.R_; r0 += kMdThreads) {
+    for (int r0 = 0; r0 < A.R_; r0 += all) {
         const int q = r0 + t;
         const int nd = q < A.R_ ? __ldcg(A.resort + q) : 0;
         any |= nd;
@@ -1016,60 +1544,77 @@ __global__ void __launch_bounds__(kBT)
         const Grid g = rp.g;
         const PView<R> v = pick(v0, v1, rp.cur);
         const int steps = adv[t.r] - base[t.r];
-        for (long long b = t.begin; b < t.end; b += blockDim.x) {
-            const long long i = b + threadIdx.x;
-            const bool ok = i < t.end;
-            int k = -1;
-            if (ok) {
-                R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
-                const R vx = v.vel.x[i], vy = v.vel.y[i], vz = v.vel.z[i];
-                bool moved = false;
-                if (aidx[i] < 0) {
-                    const R hx = dt * vx, hy = dt * vy, hz = dt * vz;
-#pragma unroll 4
-                    for (int j = 0; j < steps; j++) {
-                        x = x + hx;
-                        y = y + hy;
-                        z = z + hz;
-                    }
-                    // md_pos adds the zero force term too: -0 becomes +0
-                    moved = steps > 0;
-                    x = moved ? x + (R)0 : x;
-                    y = moved ? y + (R)0 : y;
-                    z = moved ? z + (R)0 : z;
-                    const R nx = md_vel_free(vx, dt), ny = md_vel_free(vy, dt), nz = md_vel_free(vz, dt);
-                    if (!same_bits(nx, vx) || !same_bits(ny, vy) || !same_bits(nz, vz)) {
-                        v.vel.x[i] = nx;
-                        v.vel.y[i] = ny;
-                        v.vel.z[i] = nz;
-                    }
-                } else {
-                    aidx[i] = -1;
+        constexpr int K = 2;  // particles per thread and pass, loaded before any is moved
+        for (long long b = t.begin; b < t.end; b += K * kBT) {
+            R x[K], y[K], z[K], vx[K], vy[K], vz[K];
+            int act[K];
+#pragma unroll
+            for (int c = 0; c < K; c++) {
+                const long long i = b + c * kBT + threadIdx.x;
+                if (i < t.end) {
+                    x[c] = v.pos.x[i];
+                    y[c] = v.pos.y[i];
+                    z[c] = v.pos.z[i];
+                    vx[c] = v.vel.x[i];
+                    vy[c] = v.vel.y[i];
+                    vz[c] = v.vel.z[i];
+                    act[c] = aidx[i];
                 }
-                const int jx = floor_div_edge((double)x, g.edges[0]), jy = floor_div_edge((double)y, g.edges[1]),
-                          jz = floor_div_edge((double)z, g.edges[2]);
-                if (jx) {
-                    v.ix[i] += jx;
-                    x = x - (R)(jx * g.edges[0]);
-                }
-                if (jy) {
-                    v.iy[i] += jy;
-                    y = y - (R)(jy * g.edges[1]);
-                }
-                if (jz) {
-                    v.iz[i] += jz;
-                    z = z - (R)(jz * g.edges[2]);
-                }
-                if (moved || jx || jy || jz) {
-                    v.pos.x[i] = x;
-                    v.pos.y[i] = y;
-                    v.pos.z[i] = z;
-                }
-                k = rp.soff + slot_of(g, (double)x, (double)y, (double)z);
-                key[i] = k;
             }
-            unsigned peers = __match_any_sync(0xffffffffu, k);
-            if (ok && lane == __ffs(peers) - 1) atomicAdd(count + k, __popc(peers));
+#pragma unroll
+            for (int c = 0; c < K; c++) {
+                const long long i = b + c * kBT + threadIdx.x;
+                const bool ok = i < t.end;
+                int k = -1;
+                if (ok) {
+                    bool moved = false;
+                    if (act[c] < 0) {
+                        const R hx = dt * vx[c], hy = dt * vy[c], hz = dt * vz[c];
+#pragma unroll 4
+                        for (int j = 0; j < steps; j++) {
+                            x[c] = x[c] + hx;
+                            y[c] = y[c] + hy;
+                            z[c] = z[c] + hz;
+                        }
+                        // md_pos adds the zero force term too: -0 becomes +0
+                        moved = steps > 0;
+                        x[c] = moved ? x[c] + (R)0 : x[c];
+                        y[c] = moved ? y[c] + (R)0 : y[c];
+                        z[c] = moved ? z[c] + (R)0 : z[c];
+                        const R nx = md_vel_free(vx[c], dt), ny = md_vel_free(vy[c], dt), nz = md_vel_free(vz[c], dt);
+                        if (!same_bits(nx, vx[c]) || !same_bits(ny, vy[c]) || !same_bits(nz, vz[c])) {
+                            v.vel.x[i] = nx;
+                            v.vel.y[i] = ny;
+                            v.vel.z[i] = nz;
+                        }
+                    } else {
+                        aidx[i] = -1;
+                    }
+                    const int jx = floor_div_edge((double)x[c], g.edges[0]), jy = floor_div_edge((double)y[c], g.edges[1]),
+                              jz = floor_div_edge((double)z[c], g.edges[2]);
+                    if (jx) {
+                        v.ix[i] += jx;
+                        x[c] = x[c] - (R)(jx * g.edges[0]);
+                    }
+                    if (jy) {
+                        v.iy[i] += jy;
+                        y[c] = y[c] - (R)(jy * g.edges[1]);
+                    }
+                    if (jz) {
+                        v.iz[i] += jz;
+                        z[c] = z[c] - (R)(jz * g.edges[2]);
+                    }
+                    if (moved || jx || jy || jz) {
+                        v.pos.x[i] = x[c];
+                        v.pos.y[i] = y[c];
+                        v.pos.z[i] = z[c];
+                    }
+                    k = rp.soff + slot_of(g, (double)x[c], (double)y[c], (double)z[c]);
+                    key[i] = k;
+                }
+                unsigned peers = __match_any_sync(0xffffffffu, k);
+                if (ok && lane == __ffs(peers) - 1) atomicAdd(count + k, __popc(peers));
+            }
         }
     }
 }
@@ -1296,7 +1841,7 @@ static int allow_shared()
     static bool set = false;
     if (!set) {
         RMPCD_CUDA_TRY(cudaFuncSetAttribute(kb_md<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)sizeof(MdShared)));
+                                            (int)kMdSmem));
         RMPCD_CUDA_TRY(cudaFuncSetAttribute(kb_update_list<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)nl_stage_bytes<R>()));
         set = true;
@@ -1425,19 +1970,6 @@ static int list_gx(const Batch *b)
     return gx > 64 ? 64 : gx < 1 ? 1 : gx;
 }
 
-// Blocks per replica of kb_md, one block per SM: as many as leave every
-// replica's cluster resident at once (a replica's 6,000 active particles then
-// take 2, 3, 6 or 12 per thread and step), 8 being the portable maximum.
-// Clusters of 8 and 4 blocks do not fill every SM of a processing cluster, so
-// their share of the device is taken as 128 of 148.
-static int md_cluster(const Batch *b)
-{
-    const int set = kClusters[shape_var(b->shape)];
-    if (set) return set;
-    const int sms = sm_count(), most = sms * 128 / 148;
-    return b->R * 8 <= most ? 8 : b->R * 4 <= most ? 4 : b->R * 2 <= sms ? 2 : 1;
-}
-
 // the active particles of the replicas in flag (every one when null), then
 // their MD steps up to the next re-sort or the interval's end
 template <typename R>
@@ -1446,12 +1978,16 @@ static void md_launches(Batch *b, const int *flag, cudaStream_t st, cudaGraphCon
     const PView<R> v0 = phys<R>(b->sol, 0), v1 = phys<R>(b->sol, 1);
     const double dt = b->prm.tau / b->prm.N_MD;
     const int gx = list_gx(b), gp = resort_grid(b->n_ptile);
-    kb_claim<<<dim3(gx, 2 * b->R), kBT, 0, st>>>(flag, b->rep, b->list, b->nn, b->Nmax, b->aidx, b->act, b->nl,
-                                                 b->mult);
+    double cut_sq = b->prm.cut_sq_C;
+    for (double c : b->lj_sc.cut_sq) cut_sq = c > cut_sq ? c : cut_sq;
+    const float reach = (float)sqrt(cut_sq) * 1.0001f + 1e-3f;
+    kb_claim<R><<<dim3(gx, 2 * b->R), kBT, 0, st>>>(flag, b->rep, v0, v1, phys<double>(b->col, 1).pos, (R)dt, reach,
+                                                    (float)(b->prm.skin * 0.1) * 1.0001f, b->prm.N_MD, b->base, b->list,
+                                                    b->nn, b->Nmax, b->aidx, b->act, b->nl, b->mult, b->ent);
     kb_classify<R><<<gp + gx * 2 * b->R + b->R, kBT, 0, st>>>(
         particle_tiles<R>(b, flag), gp, gx, b->R, flag, b->rep, v0, v1, (R)dt, b->prm.skin * 0.89, b->prm.N_MD,
         b->read_species ? 1 : 0, b->base, b->fresh, b->s_free, b->list, b->nn, b->Nmax, b->aidx, b->act, b->nl, b->nx,
-        b->mult, b->amap, b->sol->key, b->nf);
+        b->mult, b->ent, b->next, b->sol->key, b->nf);
     MdArgs<R> a;
     a.rep = b->rep;
     a.v0 = v0;
@@ -1478,13 +2014,18 @@ static void md_launches(Batch *b, const int *flag, cudaStream_t st, cudaGraphCon
     a.read_species = b->read_species ? 1 : 0;
     a.d_step = b->d_step;
     a.n = b->nn;
-    a.amap = b->amap;
+    a.next = b->next;
+    a.ent = b->ent;
     a.act = b->act;
     a.nl = b->nl;
     a.nx = b->nx;
     a.mult = b->mult;
-    a.pf = b->pf;
-    a.cf = b->cf;
+    a.over = b->over;
+    a.terms = b->terms;
+    a.keys[0] = b->keys[0];
+    a.keys[1] = b->keys[1];
+    a.n_over = b->n_over;
+    a.reach = reach;
     a.s_free = b->s_free;
     a.fresh = b->fresh;
     a.adv = b->adv;
@@ -1496,20 +2037,8 @@ static void md_launches(Batch *b, const int *flag, cudaStream_t st, cudaGraphCon
     a.cond = cond;
     a.use_cond = b->capturing ? 1 : 0;
     a.err = dev_error_word();
-    const int blocks = md_cluster(b);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(blocks * b->R);
-    cfg.blockDim = dim3(kMdThreads);
-    cfg.dynamicSmemBytes = sizeof(MdShared);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = blocks;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    note(b, cudaLaunchKernelEx(&cfg, kb_md<R>, a));
+    kb_md<R><<<b->R, kMdSum + kPartThreads[shape_var(b->shape)], kMdSmem, st>>>(a);
+    note(b, cudaGetLastError());
 }
 
 // an interval's MD steps in the graph being captured on st: the steps up to
@@ -1625,7 +2154,7 @@ static void free_batch(Batch *b)
     rmpcd_particles_destroy(b->col);
     void *ptrs[] = {b->rep, b->ptile, b->stile, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, b->count,
                     b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->act, b->nl, b->nx,
-                    b->aidx, b->amap, b->mult, b->pf, b->cf, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
+                    b->aidx, b->next, b->mult, b->ent, b->over, b->terms, b->keys[0], b->keys[1], b->n_over, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
                     b->n_extra, b->big, b->n_big, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
                     b->done, b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s,
                     b->n_all, b->any};
@@ -1767,8 +2296,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     b->ms.n = col[0]->n_species;
     for (int s = 0; s < RMPCD_MAX_SPECIES; s++) b->ms.m[s] = col[0]->mass[s];
     // replica layout and tiles
-    // default shape: the cluster by the number of replicas (md_cluster) and
-    // 1024-particle tiles, smaller only for batches too small to give ~2 tiles
+    // default shape: 512 threads for a replica's MD steps and 1024-particle tiles, smaller only for batches too small to give ~2 tiles
     // per SM: each tile's block is one round trip to DRAM, so fewer, fuller
     // tiles beat more blocks; rmpcd_dimer_batch_autotune times the others
     long long n_total = 0;
@@ -1831,7 +2359,9 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
               !dalloc(&b->cursor, soff) && !dalloc(&b->is_md, soff) && !dalloc(&b->is_reac, soff) &&
               !dalloc(&b->stencil, 3 * (size_t)b->n_stencil) && !dalloc(&b->list, ne) && !dalloc(&b->nn, 2 * (size_t)R) &&
               !dalloc(&b->act, off) && !dalloc(&b->nl, R) && !dalloc(&b->nx, R) && !dalloc(&b->aidx, off) &&
-              !dalloc(&b->amap, ne) && !dalloc(&b->mult, ne) && !dalloc(&b->pf, 6 * ne) && !dalloc(&b->cf, ne) &&
+              !dalloc(&b->next, ne) && !dalloc(&b->mult, ne) && !dalloc(&b->ent, 2 * ne) && !dalloc(&b->over, ne) &&
+              !dalloc(&b->terms, ne) && !dalloc(&b->keys[0], ne) && !dalloc(&b->keys[1], ne) &&
+              !dalloc(&b->n_over, 4 * (size_t)R) &&
               !dalloc(&b->nf, R) && !dalloc(&b->s_free, R) && !dalloc(&b->adv, R) && !dalloc(&b->base, R) &&
               !dalloc(&b->fresh, R) && !dalloc(&b->resort, R) &&
               !dalloc(&b->n_extra, R) && !dalloc(&b->big, soff) && !dalloc(&b->n_big, 1) &&
@@ -2103,9 +2633,10 @@ int rmpcd_dimer_batch_shape_info(int precision, int shape, int *particles_per_ti
     if (particles_per_tile) *particles_per_tile = (int)kPTiles[shape_tile(shape)];
     if (list_entries_per_thread) *list_entries_per_thread = kListPer[shape_list(shape)];
     if (colloid_block_first) *colloid_block_first = 1;
-    if (per_thread_begin) *per_thread_begin = kMdPer;
-    if (per_thread_end) *per_thread_end = kMdPer;
-    if (blocks_per_sm) *blocks_per_sm = kClusters[shape_var(shape)];
+    const int warps = kPartThreads[shape_var(shape)] / 32;
+    if (per_thread_begin) *per_thread_begin = warps;
+    if (per_thread_end) *per_thread_end = warps;
+    if (blocks_per_sm) *blocks_per_sm = 1;
     return RMPCD_OK;
 }
 
