@@ -53,7 +53,7 @@
 #include "rmpcd_common.cuh"
 #include "rng.cuh"
 #include "sortcore.cuh"
-#include "sortnet.cuh"
+#include "sorttile.cuh"
 #include "state.cuh"
 #include "stepops.cuh"
 #include "timers.cuh"
@@ -154,7 +154,8 @@ struct rmpcd_dimer_batch {
     // only to 1 or 2 inside the batch, so otherwise every particle passes
     // maximum_displacement's species >= 0 test and species need not be read
     bool read_species = true;
-    int *resort = nullptr, *n_extra = nullptr, *big = nullptr, *n_big = nullptr;
+    int *resort = nullptr, *n_extra = nullptr;
+    int *tmp = nullptr;  // order_tile's scratch
     double *rattle[3] = {nullptr, nullptr, nullptr};
     double *vv_mass = nullptr;
     uint64_t *d_step = nullptr;
@@ -1496,25 +1497,21 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
 
 // ------------------------------------------------------ re-sort / sort
 
-// count = 0, is_md = 0, is_reac = 1 over the active replicas' slots; block 0
-// also clears the big-cell queue and, for the interval's sort, draws every
-// replica's grid shift (random_shift, src/cell_system.f90:153-163)
+// count = 0, is_md = 0, is_reac = 1 over the active replicas' slots; for the
+// interval's sort, block 0 also draws every replica's grid shift (random_shift, src/cell_system.f90:153-163)
 __global__ void kb_zero_slots(TileSet ts, int *count, unsigned char *is_md,
-                              unsigned char *is_reac, int *n_big, int R, BRep *rep, const uint64_t *d_step,
+                              unsigned char *is_reac, int R, BRep *rep, const uint64_t *d_step,
                               int shift_step_off)
 {
-    if (blockIdx.x == 0) {
-        if (threadIdx.x == 0) *n_big = 0;
-        if (shift_step_off >= 0) {
-            const uint64_t step = *d_step + (uint64_t)shift_step_off;
-            for (int r = threadIdx.x; r < R; r += blockDim.x) {
-                double u0, u1, u2, u3;
-                rng::uniform2(rep[r].seed, step, 0, rng::SHIFT, 0, u0, u1);
-                rng::uniform2(rep[r].seed, step, 1, rng::SHIFT, 0, u2, u3);
-                rep[r].g.origin[0] = u0 - 1;
-                rep[r].g.origin[1] = u1 - 1;
-                rep[r].g.origin[2] = u2 - 1;
-            }
+    if (blockIdx.x == 0 && shift_step_off >= 0) {
+        const uint64_t step = *d_step + (uint64_t)shift_step_off;
+        for (int r = threadIdx.x; r < R; r += blockDim.x) {
+            double u0, u1, u2, u3;
+            rng::uniform2(rep[r].seed, step, 0, rng::SHIFT, 0, u0, u1);
+            rng::uniform2(rep[r].seed, step, 1, rng::SHIFT, 0, u2, u3);
+            rep[r].g.origin[0] = u0 - 1;
+            rep[r].g.origin[1] = u1 - 1;
+            rep[r].g.origin[2] = u2 - 1;
         }
     }
     for (int k = blockIdx.x; k < *ts.n; k += gridDim.x) {
@@ -1730,7 +1727,7 @@ __global__ void __launch_bounds__(kBT) kb_scan_apply(TileSet ts, const int *coun
     }
 }
 
-// place every particle inside its cell (in-cell order fixed by kb_segsort)
+// place every particle inside its cell (in-cell order fixed by kb_order_gather)
 __global__ void __launch_bounds__(kBT) kb_perm(TileSet ts, const int *key, int *cursor, int *perm)
 {
     const int lane = threadIdx.x & 31;
@@ -1749,37 +1746,30 @@ __global__ void __launch_bounds__(kBT) kb_perm(TileSet ts, const int *key, int *
     }
 }
 
-__global__ void kb_segsort(TileSet ts, const int *count, const int *start, int *perm, int *big, int *n_big)
-{
-    for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
-        const BTile t = ts.tiles[ts.ids[kt]];
-        for (long long s = t.begin + threadIdx.x; s < t.end; s += blockDim.x) {
-            int n = count[s];
-            if (n <= 1) continue;
-            if (n > kSmallSegmentMax) {
-                int q = atomicAdd(n_big, 1);
-                big[q] = (int)s;
-                continue;
-            }
-            sort_segment(perm + start[s], n);
-        }
-    }
-}
-
 // Every field through perm into the replica's other buffer (current since
-// kb_scan_reps).  Only particles with MD or PAST_MD set have force entries: they
-// are moved and zeroed behind, so the buffer that is not current holds none.
-// Flagged particles are listed (key is free after the placement).
+// kb_scan_reps), each cell's indices put in order on the way (order_tile).
+// Only particles with MD or PAST_MD set have force entries: they are moved and
+// zeroed behind, so the buffer that is not current holds none.  Flagged
+// particles are listed in flist; tmp is order_tile's scratch.
+constexpr int kOrderPerTile = kTile / kOrderSlots;
+
 template <typename R>
-__global__ void __launch_bounds__(kBT, 4)
-    kb_gather(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, const int *perm, int *flist, int *nf)
+__global__ void __launch_bounds__(kOrderThreads, 4)
+    kb_order_gather(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, const int *count, const int *start, int *perm,
+                    int *tmp, int *flist, int *nf)
 {
-    for (int kt = blockIdx.x; kt < *ts.n; kt += gridDim.x) {
-        const BTile t = ts.tiles[ts.ids[kt]];
+    __shared__ OrderTile sh;
+    for (int kt = blockIdx.x; kt < *ts.n * kOrderPerTile; kt += gridDim.x) {
+        const BTile t = ts.tiles[ts.ids[kt / kOrderPerTile]];
+        const long long s0 = t.begin + (long long)(kt % kOrderPerTile) * kOrderSlots;
+        if (s0 >= t.end) continue;
         const BRep &rp = rep[t.r];
         const PView<R> d = pick(v0, v1, rp.cur), s = pick(v1, v0, rp.cur);
-        for (long long j = t.begin + threadIdx.x; j < t.end; j += blockDim.x) {
-            const int i = perm[j];
+        int a0, np;
+        __syncthreads();  // the last tile's indices are read
+        const int *src = order_tile(sh, (int)s0, (int)min(s0 + kOrderSlots, t.end), count, start, perm, tmp, a0, np);
+        for (int q = threadIdx.x; q < np; q += kOrderThreads) {
+            const int i = src[q], j = a0 + q;
             R px = s.pos.x[i], py = s.pos.y[i], pz = s.pos.z[i];
             R vx = s.vel.x[i], vy = s.vel.y[i], vz = s.vel.z[i];
             int ix = s.ix[i], iy = s.iy[i], iz = s.iz[i];
@@ -1797,7 +1787,7 @@ __global__ void __launch_bounds__(kBT, 4)
             d.species[j] = sp;
             d.flags[j] = fl;
             if (fl & kActiveBits) {
-                flist[rp.off + atomicAdd(nf + t.r, 1)] = (int)j;
+                flist[rp.off + atomicAdd(nf + t.r, 1)] = j;
                 if (fl & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
                     for (int k = 0; k < 3; k++) {
                         d.force[k][j] = s.force[k][i];
@@ -1937,7 +1927,7 @@ static void resort_launches(Batch *b, const int *flag, cudaStream_t st, int shif
     const TileSet sts{b->stile, flag ? b->act_s : b->all_s, (flag ? b->n_act : b->n_all) + 1};
     const int gp = resort_grid(b->n_ptile), gs = resort_grid(b->n_stile);
     const R dt = (R)(b->prm.tau / b->prm.N_MD);
-    kb_zero_slots<<<gs, kBT, 0, st>>>(sts, b->count, b->is_md, b->is_reac, b->n_big, b->R, b->rep, b->d_step,
+    kb_zero_slots<<<gs, kBT, 0, st>>>(sts, b->count, b->is_md, b->is_reac, b->R, b->rep, b->d_step,
                                       shift_step_off);
     kb_advance_key_count<R><<<gp, kBT, 0, st>>>(pts, b->rep, v0, v1, b->aidx, b->adv, b->base, dt, b->sol->key,
                                                 b->count);
@@ -1947,9 +1937,8 @@ static void resort_launches(Batch *b, const int *flag, cudaStream_t st, int shif
                                        b->fresh);
     kb_scan_apply<<<gs, kBT, 0, st>>>(sts, b->count, b->tile_off, b->start, b->cursor);
     kb_perm<<<gp, kBT, 0, st>>>(pts, b->sol->key, b->cursor, b->sol->perm);
-    kb_segsort<<<gs, kBT, 0, st>>>(sts, b->count, b->start, b->sol->perm, b->big, b->n_big);
-    launch_segsort_big(b->start, b->count, b->big, b->n_big, b->sol->perm, b->sol->key, st);
-    kb_gather<R><<<gp, kBT, 0, st>>>(pts, b->rep, v0, v1, b->sol->perm, b->sol->key, b->nf);
+    kb_order_gather<R><<<resort_grid(b->n_stile * kOrderPerTile), kOrderThreads, 0, st>>>(
+        sts, b->rep, v0, v1, b->count, b->start, b->sol->perm, b->tmp, b->sol->key, b->nf);
     kb_update_list<R><<<2 * b->R, kNlBlockThreads, nl_stage_bytes<R>(), st>>>(
         flag, b->rep, cv, v0, v1, b->count, b->start, b->stencil, b->n_stencil,
         b->prm.list_radius * b->prm.list_radius, b->lj_sc, b->Nmax, b->list, b->nn, b->is_md, b->is_reac,
@@ -2155,7 +2144,7 @@ static void free_batch(Batch *b)
     void *ptrs[] = {b->rep, b->ptile, b->stile, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, b->count,
                     b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->act, b->nl, b->nx,
                     b->aidx, b->next, b->mult, b->ent, b->over, b->terms, b->keys[0], b->keys[1], b->n_over, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
-                    b->n_extra, b->big, b->n_big, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
+                    b->n_extra, b->tmp, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
                     b->done, b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s,
                     b->n_all, b->any};
     for (void *q : ptrs) cudaFree(q);
@@ -2364,7 +2353,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
               !dalloc(&b->n_over, 4 * (size_t)R) &&
               !dalloc(&b->nf, R) && !dalloc(&b->s_free, R) && !dalloc(&b->adv, R) && !dalloc(&b->base, R) &&
               !dalloc(&b->fresh, R) && !dalloc(&b->resort, R) &&
-              !dalloc(&b->n_extra, R) && !dalloc(&b->big, soff) && !dalloc(&b->n_big, 1) &&
+              !dalloc(&b->n_extra, R) && !dalloc(&b->tmp, off) &&
               !dalloc(&b->rattle[0], 2 * (size_t)R) && !dalloc(&b->rattle[1], 2 * (size_t)R) &&
               !dalloc(&b->rattle[2], 2 * (size_t)R) && !dalloc(&b->vv_mass, 2 * (size_t)R) && !dalloc(&b->d_step, 1) &&
               !dalloc(&b->done, 1) && cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking) == cudaSuccess &&

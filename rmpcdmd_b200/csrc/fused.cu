@@ -856,6 +856,7 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
     k_rec_gather_to_soa<R><<<grid_for(p->N, 256), 256, 0, st>>>(p->rec[rb], p->perm, side, alt<R>(p), p->N);
     RMPCD_CHECK_LAUNCH();
     p->cur = 1 - p->cur;
+    p->alt_force_clean = p->cur_force_gated = false;
     return RMPCD_OK;
 }
 

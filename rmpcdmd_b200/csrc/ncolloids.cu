@@ -113,7 +113,7 @@ __device__ inline void stream_vel_gated(const PView<R> &v, long long i, int f, R
 // (src/md.f90:79-102, :239-263) for every particle outside the MD cells
 // (cellmap: each particle's slot, from the last sort), fused with the key
 // pass of the sort that follows (apply_pbc, the slot in the cells' grid and
-// its count, as k_pbc_key_count): one linear pass, the streamed position kept
+// its count): one linear pass, the streamed position kept
 // in registers and written once with its wrap.  Per particle the arithmetic
 // is the catch-up's (the position step reading the velocity before its
 // update) followed by the key pass's.
@@ -692,6 +692,9 @@ static int catch_up_and_sort(NcLoop &L, bool full_pos_old)
     int rc = L.s->precision == RMPCD_FP32 ? catch_up_key_t<float>(L, dtl) : catch_up_key_t<double>(L, dtl);
     if (!rc) rc = rmpcd_apply_pbc(L.c, L.cells->edges);
     if (!rc) rc = sort_keyed_flagged(L.cells, L.s, L.cellmap);  // the solvent's wrap and keys are done
+    // before the run's first two flag rolls an entry with PAST_MD may hold a
+    // force of the caller's, which stays when the flag goes
+    if (L.seq < 3) L.s->cur_force_gated = false;
     L.st->last_sort = L.st->t;
     if (!rc && cudaMemsetAsync(L.ctl, 0, sizeof(int), stream()) != cudaSuccess)
         rc = fail(RMPCD_ERR_CUDA, "n_colloids sort: step counter reset failed");
@@ -926,6 +929,8 @@ extern "C" int rmpcd_ncolloids_run(rmpcd_particles *solvent, rmpcd_particles *co
     L.dt = params->tau / params->N_MD;
     L.full_rolls = 2;
     L.graphs = false;
+    // the caller may have changed forces or flags since the last call
+    solvent->cur_force_gated = false;
     PhaseTimer timer("ncolloids_run");
     // the solvent is sorted on entry: its slots from the cell ranges
     k_fill_cellmap<<<grid_full((long long)cells->S * kLanesPerCell, 256), 256, 0, stream()>>>(

@@ -1,12 +1,12 @@
 #include "keys.cuh"
 #include "scan.cuh"
 #include "sortcore.cuh"
-#include "sortnet.cuh"
+#include "sorttile.cuh"
 #include "timers.cuh"
 
 namespace rmpcd {
 
-constexpr int kSmallSegment = kSmallSegmentMax;
+constexpr int kSmallSegment = kOrderSmall;
 
 // key[i] = slot of particle i; histogram with one atomic per distinct key
 // per warp (consecutive particles usually share a cell).
@@ -23,46 +23,6 @@ __global__ void k_key_count(Grid g, const R *__restrict__ x, const R *__restrict
         int s = -1;
         if (ok) {
             s = slot_of(g, (double)x[i], (double)y[i], (double)z[i]);
-            key[i] = s;
-        }
-        unsigned peers = __match_any_sync(0xffffffffu, s);
-        if (ok && lane == __ffs(peers) - 1) atomicAdd(count + s, __popc(peers));
-    }
-}
-
-// the same with apply_pbc (src/md.f90:202-217) done on each particle first:
-// the wrapped position is the one keyed, and pos / image are written only
-// for particles that wrap
-template <typename R>
-__global__ void k_pbc_key_count(Grid g, PView<R> v, double e0, double e1, double e2, int N,
-                                int *__restrict__ key, int *__restrict__ count)
-{
-    const int lane = threadIdx.x & 31;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < N; base += stride) {
-        long long i = base + threadIdx.x;
-        bool ok = i < N;
-        int s = -1;
-        if (ok) {
-            R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
-            const int jx = floor_div_edge((double)x, e0), jy = floor_div_edge((double)y, e1),
-                      jz = floor_div_edge((double)z, e2);
-            if (jx) {
-                v.ix[i] += jx;
-                x = x - (R)(jx * e0);
-                v.pos.x[i] = x;
-            }
-            if (jy) {
-                v.iy[i] += jy;
-                y = y - (R)(jy * e1);
-                v.pos.y[i] = y;
-            }
-            if (jz) {
-                v.iz[i] += jz;
-                z = z - (R)(jz * e2);
-                v.pos.z[i] = z;
-            }
-            s = slot_of(g, (double)x, (double)y, (double)z);
             key[i] = s;
         }
         unsigned peers = __match_any_sync(0xffffffffu, s);
@@ -128,67 +88,37 @@ __global__ void k_segsort_small(const int *__restrict__ start, const int *__rest
     }
 }
 
-__device__ inline int lower_bound_int(const int *a, int n, int v)
-{
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        int mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-
-// one block per long segment: bottom-up merge sort of distinct values, every
-// element placed by its rank in the partner run; tmp is scratch of the same
-// extent as the segment
+// one block per long segment (tmp: scratch of the extent of perm)
 __global__ void k_segsort_big(const int *__restrict__ start, const int *__restrict__ count,
                               const int *__restrict__ big, const int *__restrict__ n_big,
                               int *__restrict__ perm, int *__restrict__ tmp)
 {
     for (int q = blockIdx.x; q < *n_big; q += gridDim.x) {
-        int s = big[q];
-        int n = count[s];
-        int *a = perm + start[s];
-        int *b = tmp + start[s];
-        int *src = a, *dst = b;
-        for (int w = 1; w < n; w <<= 1) {
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                int run = i / w;
-                int r0 = run * w;
-                int v = src[i];
-                int pos;
-                if ((run & 1) == 0) {
-                    int p0 = r0 + w;
-                    int pn = min(w, max(0, n - p0));
-                    pos = r0 + (i - r0) + lower_bound_int(src + p0, pn, v);
-                } else {
-                    int p0 = r0 - w;
-                    pos = p0 + (i - r0) + lower_bound_int(src + p0, w, v);
-                }
-                dst[pos] = v;
-            }
-            __syncthreads();
-            int *t = src;
-            src = dst;
-            dst = t;
-        }
-        if (src != a)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = src[i];
-        __syncthreads();
+        const int s = big[q];
+        block_merge_sort(perm + start[s], tmp + start[s], count[s]);
     }
 }
 
-// gated != 0: a particle with neither MD nor PAST_MD set is known to have
-// zero force and force_old, so those are written as zeros without a read
+// Every field through perm, each cell's indices put in order on the way
+// (order_tile), one block per tile of slots.  gated != 0: a particle with
+// neither MD nor PAST_MD set has zero force and force_old in both the source
+// and -- the caller's guarantee -- the target arrays; the others' entries are
+// moved and zeroed behind, so that after the buffers change places the same
+// holds for the next gated sort and the 24 / 48 B per particle of zeros are
+// not written (128^3 FP32 colloid run: 165 -> 160 ms
+// with the order taken into the gather).
 template <typename R>
-__global__ void k_gather(PView<R> s, PView<R> d, const int *__restrict__ perm, int N,
-                         int with_force, int with_force_old, int gated)
+__global__ void __launch_bounds__(kOrderThreads, 4)
+    k_order_gather(PView<R> s, PView<R> d, const int *__restrict__ count, const int *__restrict__ start, int S,
+                   int *perm, int *tmp, int with_force, int with_force_old, int gated)
 {
+    __shared__ OrderTile sh;
     const int fmask = (1 << MD_BIT) | (1 << PAST_MD_BIT);
-    for (long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x; j < N;
-         j += (long long)gridDim.x * blockDim.x) {
-        const int i = perm[j];
+    const int s0 = blockIdx.x * kOrderSlots;
+    int a0, np;
+    const int *src = order_tile(sh, s0, min(s0 + kOrderSlots, S), count, start, perm, tmp, a0, np);
+    for (int q = threadIdx.x; q < np; q += kOrderThreads) {
+        const int i = src[q], j = a0 + q;
         // all loads first: twelve independent gathers in flight per thread
         R px = s.pos.x[i], py = s.pos.y[i], pz = s.pos.z[i];
         R vx = s.vel.x[i], vy = s.vel.y[i], vz = s.vel.z[i];
@@ -206,16 +136,20 @@ __global__ void k_gather(PView<R> s, PView<R> d, const int *__restrict__ perm, i
         d.id[j] = id;
         d.species[j] = sp;
         d.flags[j] = fl;
-        const bool live = !gated || (fl & fmask);
+        if (gated && !(fl & fmask)) continue;
         if (with_force) {
-            d.force.x[j] = live ? s.force.x[i] : (R)0;
-            d.force.y[j] = live ? s.force.y[i] : (R)0;
-            d.force.z[j] = live ? s.force.z[i] : (R)0;
+            d.force.x[j] = s.force.x[i];
+            d.force.y[j] = s.force.y[i];
+            d.force.z[j] = s.force.z[i];
         }
         if (with_force_old) {
-            d.force_old.x[j] = live ? s.force_old.x[i] : (R)0;
-            d.force_old.y[j] = live ? s.force_old.y[i] : (R)0;
-            d.force_old.z[j] = live ? s.force_old.z[i] : (R)0;
+            d.force_old.x[j] = s.force_old.x[i];
+            d.force_old.y[j] = s.force_old.y[i];
+            d.force_old.z[j] = s.force_old.z[i];
+        }
+        if (gated) {
+            s.force.x[i] = s.force.y[i] = s.force.z[i] = 0;
+            s.force_old.x[i] = s.force_old.y[i] = s.force_old.z[i] = 0;
         }
     }
 }
@@ -247,9 +181,9 @@ int build_perm_unsorted(rmpcd_cells *c, rmpcd_particles *p, int *cellmap)
     return RMPCD_OK;
 }
 
-int build_perm(rmpcd_cells *c, rmpcd_particles *p, int *cellmap)
+int build_perm(rmpcd_cells *c, rmpcd_particles *p)
 {
-    int rc = build_perm_unsorted(c, p, cellmap);
+    int rc = build_perm_unsorted(c, p, nullptr);
     if (rc) return rc;
     return sort_perm_segments(c, p);
 }
@@ -269,14 +203,27 @@ int sort_perm_segments(rmpcd_cells *c, rmpcd_particles *p)
 }
 
 template <typename R>
-static int gather_t(rmpcd_particles *p, bool gated = false)
+static int gather_t(rmpcd_cells *c, rmpcd_particles *p, bool gated = false)
 {
+    cudaStream_t st = stream();
+    const int to = 1 - p->cur;
     if (p->N > 0) {
-        k_gather<R><<<grid_for(p->N, 256), 256, 0, stream()>>>(
-            cur<R>(p), alt<R>(p), p->perm, p->N, p->force_zero ? 0 : 1, p->force_old_zero ? 0 : 1, gated ? 1 : 0);
+        if (gated) {
+            // the target's force arrays have to be zero: they are from the
+            // third gated sort in a row on
+            for (int k = 0; k < 3 && !p->alt_force_clean; k++) {
+                RMPCD_CUDA_TRY(cudaMemsetAsync(p->force[to][k], 0, (size_t)p->N * p->rsize, st));
+                RMPCD_CUDA_TRY(cudaMemsetAsync(p->force_old[to][k], 0, (size_t)p->N * p->rsize, st));
+            }
+        }
+        k_order_gather<R><<<grid_full(c->S, kOrderSlots), kOrderThreads, 0, st>>>(
+            cur<R>(p), alt<R>(p), c->count, c->start, c->S, p->perm, p->key, p->force_zero ? 0 : 1,
+            p->force_old_zero ? 0 : 1, gated ? 1 : 0);
         RMPCD_CHECK_LAUNCH();
     }
-    p->cur = 1 - p->cur;
+    p->alt_force_clean = gated && p->cur_force_gated;
+    p->cur_force_gated = gated;
+    p->cur = to;
     // fields that were not gathered are all zero: keep the live pointer on the
     // (zero) previous arrays
     for (int k = 0; k < 3; k++) {
@@ -294,16 +241,10 @@ static int gather_t(rmpcd_particles *p, bool gated = false)
     return RMPCD_OK;
 }
 
-void launch_segsort_big(const int *start, const int *count, const int *big, const int *n_big, int *perm,
-                        int *tmp, cudaStream_t st)
+int gather_all(rmpcd_cells *c, rmpcd_particles *p)
 {
-    k_segsort_big<<<64, 512, 0, st>>>(start, count, big, n_big, perm, tmp);
-}
-
-int gather_all(rmpcd_particles *p)
-{
-    if (p->precision == RMPCD_FP32) return gather_t<float>(p);
-    return gather_t<double>(p);
+    if (p->precision == RMPCD_FP32) return gather_t<float>(c, p);
+    return gather_t<double>(c, p);
 }
 
 template <typename R>
@@ -315,36 +256,15 @@ static int sort_keyed_flagged_t(rmpcd_cells *c, rmpcd_particles *p, int *cellmap
         if (rc) return rc;
     }
     PhaseTimer t("sort");
-    int rc = build_perm(c, p, cellmap);
+    int rc = build_perm_unsorted(c, p, cellmap);
     if (rc) return rc;
-    return gather_t<R>(p, true);
+    return gather_t<R>(c, p, true);
 }
 
 int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap)
 {
     if (p->precision == RMPCD_FP32) return sort_keyed_flagged_t<float>(c, p, cellmap);
     return sort_keyed_flagged_t<double>(c, p, cellmap);
-}
-
-template <typename R>
-static int sort_particles_flagged_t(rmpcd_cells *c, rmpcd_particles *p, const double edges[3])
-{
-    {
-        PhaseTimer t("count");
-        cudaStream_t st = stream();
-        RMPCD_CUDA_TRY(cudaMemsetAsync(c->count, 0, (size_t)c->S * sizeof(int), st));
-        if (p->N > 0)
-            k_pbc_key_count<R><<<grid_for(p->N, 256), 256, 0, st>>>(grid_of(c), cur<R>(p), edges[0], edges[1],
-                                                                   edges[2], p->N, p->key, c->count);
-        RMPCD_CHECK_LAUNCH();
-    }
-    return sort_keyed_flagged_t<R>(c, p, nullptr);
-}
-
-int sort_particles_flagged(rmpcd_cells *c, rmpcd_particles *p, const double edges[3])
-{
-    if (p->precision == RMPCD_FP32) return sort_particles_flagged_t<float>(c, p, edges);
-    return sort_particles_flagged_t<double>(c, p, edges);
 }
 
 // cell_system_t%sort_particles (src/cell_system.f90:131-151): the positions
@@ -448,9 +368,9 @@ int sort_particles(rmpcd_cells *c, rmpcd_particles *p)
         if (rc) return rc;
     }
     PhaseTimer t("sort");
-    rc = build_perm(c, p);
+    rc = build_perm_unsorted(c, p, nullptr);
     if (rc) return rc;
-    return gather_all(p);
+    return gather_all(c, p);
 }
 
 }  // namespace rmpcd

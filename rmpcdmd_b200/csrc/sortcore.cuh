@@ -8,10 +8,11 @@
 //   scan       exclusive scan count -> start, cursor
 //   perm       one pass over keys: warp-aggregated cursor atomics give every
 //              particle a place inside its cell: perm[place] = i
-//   segsort    each cell's perm segment is sorted ascending, which restores
-//              the reference's single-thread order (stable in i)
-//   gather     dst[j] = src[perm[j]] for every field: coalesced writes,
-//              reads local in the Hilbert order
+//   gather     tile by tile, each cell's perm segment is put in ascending
+//              order in shared memory, which restores the reference's
+//              single-thread order (stable in i), then dst[j] = src[perm[j]]
+//              for every field: coalesced writes, reads local in the Hilbert
+//              order
 #pragma once
 #include "state.cuh"
 
@@ -24,26 +25,21 @@ int build_perm_unsorted(rmpcd_cells *c, rmpcd_particles *p, int *cellmap = nullp
 // ascending sort of every cell's perm segment (uses cursor[] and key[] as scratch)
 int sort_perm_segments(rmpcd_cells *c, rmpcd_particles *p);
 // both of the above
-int build_perm(rmpcd_cells *c, rmpcd_particles *p, int *cellmap = nullptr);
-// gather every field through perm into the other buffer and flip buffers
-int gather_all(rmpcd_particles *p);
+int build_perm(rmpcd_cells *c, rmpcd_particles *p);
+// gather every field through perm (unsorted inside the cells) into the other
+// buffer and flip buffers
+int gather_all(rmpcd_cells *c, rmpcd_particles *p);
 // full sort
 int sort_particles(rmpcd_cells *c, rmpcd_particles *p);
 // positions of `from` into `to` in cell order (cell_system_t%sort_particles)
 int sort_positions(rmpcd_cells *c, const rmpcd_particles *from, rmpcd_particles *to);
-// apply_pbc with the given edges, then the full sort, for a system in which a
-// particle with neither MD nor PAST_MD set has zero force and force_old (the
-// state compute_force and its flag roll maintain): those entries are written
-// as zeros instead of being gathered
-int sort_particles_flagged(rmpcd_cells *c, rmpcd_particles *p, const double edges[3]);
-// the same sort after its key pass (p->key holds every particle's slot in the
-// cells' grid, c->count their counts): scan, placement and gated gather;
+// the sort of a wrapped system after its key pass (p->key holds every
+// particle's slot in the cells' grid, c->count their counts), for a system in
+// which a particle with neither MD nor PAST_MD set has zero force and
+// force_old (the state compute_force and its flag roll maintain): scan,
+// placement and a gather that moves force entries only where there are any;
 // cellmap (if given) receives the slot of every particle of the sorted arrays
 int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap);
-// ascending merge sort of the *n_big queued cells big[] of more than 64
-// particles (tmp: scratch of the extent of perm)
-void launch_segsort_big(const int *start, const int *count, const int *big, const int *n_big, int *perm,
-                        int *tmp, cudaStream_t st);
 // maximum-displacement reductions into p->d_max (r^2 as ordered bits), no
 // synchronisation: maximum_displacement over all particles, and over the
 // particles of is_md cells (src/particle_system.f90:357-410)
@@ -67,7 +63,4 @@ int compute_force_impl(rmpcd_particles *ps1, rmpcd_particles *ps2, rmpcd_nlist *
 // drops the n_colloids loop kept between calls if it refers to `handle` (a
 // particle system, cell system or neighbor list being destroyed)
 void ncolloids_forget(const void *handle);
-// largest cell handled by sort_segment; larger ones go to launch_segsort_big
-constexpr int kSmallSegmentMax = 64;
-
 }  // namespace rmpcd

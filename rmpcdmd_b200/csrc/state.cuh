@@ -76,6 +76,11 @@ struct rmpcd_particles {
     // permuting them (a permutation of zeros is zeros)
     bool force_zero = true;
     bool force_old_zero = true;
+    // set by a gated sort: force entries of the current buffer are zero except
+    // for MD / PAST_MD particles; force and force_old of the other buffer are
+    // all zero (a gated sort of such a current buffer leaves them so)
+    bool cur_force_gated = false;
+    bool alt_force_clean = true;
     double *n2_terms = nullptr;  // pair energies of compute_force_n2, C (C - 1) / 2
     long long n2_cap = 0;
 };
