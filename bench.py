@@ -38,11 +38,10 @@ T_INIT = 1.0 / 3.0
 TAU = 1.0
 SEED = 20241203
 # HBM bytes the fused interval kernel must move per particle and per slot:
-# read + write of the full particle record (32 B FP32, 56 B FP64), the
-# permutation index (4 B) and the next key (4 B); per slot the count and start
-# read and the next count written
-BYTES_PER_PARTICLE = {32: 72, 64: 120}
-BYTES_PER_SLOT = 12
+# read + write of the full particle record (32 B FP32, 64 B FP64); per slot the
+# count read, the next count written, a count and a list head cleared
+BYTES_PER_PARTICLE = {32: 64, 64: 128}
+BYTES_PER_SLOT = 16
 # Minimum bytes of one whole interval (stream + sort + collide) over the
 # reference's particle state kept as separate arrays (FP32: pos 12, vel 12,
 # image 12, species/flags 4, id 4 = 44 B; FP64: 72 B): key pass reads pos+vel
@@ -62,7 +61,7 @@ def peaks():
 
 def profile_traffic(precision):
     """dram bytes per particle of the fused kernel from the committed ncu summary, or None."""
-    f = ROOT / "profiles" / "k_bulk_interval.md"
+    f = ROOT / "profiles" / "k_bucket_interval.md"
     if not f.exists():
         return None
     key = f"dram_bytes_per_particle_fp{precision}:"
@@ -201,7 +200,7 @@ def roofline(N, S, precision, phase, peak, peak_kind):
     alg = N * BYTES_PER_PARTICLE[precision] + S * BYTES_PER_SLOT
     achieved = alg / avg / 1e9
     t = profile_traffic(precision)
-    return {"kernel": "k_bulk_interval", "bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
+    return {"kernel": "k_bucket_interval", "bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
             "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
             "traffic": None if t is None else int(t * N), "algorithmic_bytes": int(alg),
             "avg_launch_ms": round(avg * 1e3, 4), "launches": calls}
@@ -565,11 +564,10 @@ def run_ours(args):
                          "fp32_over_fp64_call_by_call": value / cbc_value}
     out["phases_ms"] = {k: round(v[0] * 1e3 / max(1, args.steps), 4)
                         for k, v in r32["phases"].items()}
-    # kernels launched per step: fused interval, 2 scan kernels, placement;
-    # plus, once per timed call, the record packing (1) and the FP32 end of
-    # the run: entry positions of the records (1), segment sort (2), records
-    # back from entry positions (1), gather into the API arrays (1)
-    out["gpu_launches"] = 4 * args.steps + 6
+    # kernels launched per step: the fused interval; plus, once per timed call,
+    # the bucket packing (1), the slot scan (2) and the API arrays from the
+    # buckets (1)
+    out["gpu_launches"] = args.steps + 4
     if not args.no_e2e:
         e2e_steps = max(1, min(args.e2e_steps, args.steps))
         path = ("rmpcd_particles_upload x6 (pinned host, reference (3,N) layout) -> rmpcd_bulk_run(1) "

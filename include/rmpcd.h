@@ -386,7 +386,7 @@ int rmpcd_velocity_sums(rmpcd_particles *p, double out[4]);
  * particles are in ascending order of their position on entry. */
 int rmpcd_bulk_run(rmpcd_particles *p, rmpcd_cells *cells, rmpcd_rng *rng,
                    double tau, int has_alpha, double alpha, int n_intervals);
-/* Tile shapes of the fused interval kernel (slots per block, resident
+/* Tile shapes of the fused interval kernel (cells per block, resident
  * blocks per SM).  All shapes give the same results bit for bit; one is in
  * use per precision once set; until then the size of the box chooses (and
  * rmpcd_bulk_get_shape reports 0, the choice for large boxes).  No counterpart

@@ -36,6 +36,7 @@ static void free_cells(rmpcd_cells *c)
     cudaFree(c->is_md);
     cudaFree(c->is_reac);
     cudaFree(c->lut);
+    cudaFree(c->bucket_map);
     cudaFree(c->scan_tmp);
     cudaFree(c->axes);
     cudaFree(c->d_red);

@@ -1,10 +1,15 @@
-// The bulk-fluid interval as one fused pass per interval (plus a slot scan
-// and a key scatter), replacing the loop of test/setup_bulk_decay.f90:112-121:
+// The bulk-fluid interval as one fused pass per interval, replacing the loop of
+// test/setup_bulk_decay.f90:112-121:
 //
 //     simple_mpcd_step -> mpcd_stream_periodic(tau) -> random_shift -> sort
 //
-// Layout: inside the schedule each particle is one packed record holding what
-// changes or is needed every interval,
+// Two schedules give the same arrays: buckets (buckets.cuh: fixed room per
+// cell, one kernel per interval) and, where their memory or the density speaks
+// against them (bulk_run_t), the gather described here: one pass plus a slot
+// scan and a key scatter.
+//
+// Layout: inside a schedule each particle is one packed record holding what
+// changes or is needed every interval, for the gather
 //   FP32 (32 B, two 16-byte chunks):  [vx vy vz species] [px py pz idx]
 //   FP64 (56 B, seven 8-byte words):  vx vy vz (species,idx) px py pz
 // where idx is the particle's position when the schedule started.  image,
@@ -14,7 +19,7 @@
 // part (16 / 32 B) is what the collision needs for a whole cell at once; the
 // rest is needed particle by particle.
 //
-// Data flow of interval i (grid G_i, next grid G_{i+1}):
+// Data flow of interval i of the gather (grid G_i, next grid G_{i+1}):
 //   P1  k_bulk_interval  one block per tile of consecutive Hilbert slots of
 //       G_i.  The tile's particles are a contiguous range in G_i order; the
 //       block loads the range's source indices (perm), sorts each cell's
@@ -36,6 +41,8 @@
 // image update for each particle that wraps.
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
+#include <utility>
 
 #include "async_copy.cuh"
 #include "cellops.cuh"
@@ -43,7 +50,7 @@
 #include "rng.cuh"
 #include "scan.cuh"
 #include "sortcore.cuh"
-#include "sortnet.cuh"
+#include "sorttile.cuh"
 #include "timers.cuh"
 
 namespace rmpcd {
@@ -73,18 +80,19 @@ struct Rec<double> {
     __device__ static double *pos(unsigned char *r) { return (double *)r + 4; }
 };
 
-// Tile shape of k_bulk_interval: slots (cells) per block, staged-particle
+// Tile shape of the interval kernels: slots (cells) per block, staged-particle
 // capacity and resident blocks per SM (launch bound).  The capacity is more
-// than 7 standard deviations above the mean tile occupancy at density 10; an
+// than 6 standard deviations above the mean tile occupancy at density 10; an
 // over-full tile takes the global-memory path.  Every shape gives the same
 // results bit for bit (the tile size changes only which block handles a
 // cell); the shape in use is chosen per precision by rmpcd_bulk_set_shape or
-// rmpcd_bulk_autotune, or else by the size of the box (pick_shape).
-template <int SL_, int CAP_, int MINB_>
+// rmpcd_bulk_autotune, or else by the box and its density (pick_shape).
+template <int SL_, int CAP_, int MINB_, int T_ = 256>
 struct Shape {
     static constexpr int kSlots = SL_;
     static constexpr int kCap = CAP_;
     static constexpr int kMinBlocks = MINB_;
+    static constexpr int kThreads = T_;
 };
 
 template <typename R>
@@ -117,8 +125,8 @@ struct CellRot {
     R m[3][3];
 };
 
-template <typename R>
-__device__ inline CellRot<R> cell_rotation(int slot, const FusedArgs<R> &A)
+template <typename R, typename Args>
+__device__ inline CellRot<R> cell_rotation(int slot, const Args &A)
 {
     double n0, n1, n2;
     if (A.axes) {
@@ -236,10 +244,10 @@ __device__ inline int wrap_jump(R x, double L)
     else return floor_div_edge(x, L);
 }
 
-// mpcd_stream_periodic of one particle (src/mpcd.f90:450-455); returns its
-// slot in G_{i+1}; a wrap updates the particle's image at its idx
-template <typename R>
-__device__ inline int stream_values(const FusedArgs<R> &A, R &x, R &y, R &z, R vx, R vy, R vz, int idx)
+// mpcd_stream_periodic of one particle (src/mpcd.f90:450-455); a wrap updates
+// the particle's image at its idx
+template <typename R, typename Args>
+__device__ inline void stream_position(const Args &A, R &x, R &y, R &z, R vx, R vy, R vz, int idx)
 {
     x = x + vx * A.dt;
     y = y + vy * A.dt;
@@ -257,6 +265,13 @@ __device__ inline int stream_values(const FusedArgs<R> &A, R &x, R &y, R &z, R v
         z = z - (R)(jz * A.e2);
         A.iz[idx] += jz;
     }
+}
+
+// the same; returns the particle's slot in G_{i+1}
+template <typename R>
+__device__ inline int stream_values(const FusedArgs<R> &A, R &x, R &y, R &z, R vx, R vy, R vz, int idx)
+{
+    stream_position<R>(A, x, y, z, vx, vy, vz, idx);
     return slot_of(A.g_next, (double)x, (double)y, (double)z);
 }
 
@@ -649,70 +664,93 @@ __global__ void k_rec_gather_to_soa(const unsigned char *rec, const int *perm, P
     }
 }
 
+}  // namespace rmpcd
+
+#include "buckets.cuh"
+
+namespace rmpcd {
+
 // the shapes a precision can run with, and the one in use
 template <typename R>
 struct ShapeEntry {
-    void (*kernel)(FusedArgs<R>);
-    int slots;
+    void (*interval)(BucketArgs<R>);
+    void (*to_soa)(BucketGrid, BucketMap, int, const int *, const int *, PView<R>, PView<R>, int *, int *, unsigned *);
+    int slots, cap;
     size_t smem;
-    int min_blocks;
+    int min_blocks, threads;
 };
 
 template <typename R, typename S>
 constexpr ShapeEntry<R> entry()
 {
-    return {k_bulk_interval<R, S>, S::kSlots, fused_smem<R, S>(), S::kMinBlocks};
+    return {k_bucket_interval<R, S>, k_buckets_to_soa<R, S>, S::kSlots, S::kCap, sizeof(BucketTile<R, S>), S::kMinBlocks, S::kThreads};
 }
 
 template <typename R>
 struct Shapes;
 template <>
 struct Shapes<float> {
-    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<128, 1792, 4>>(), entry<float, Shape<32, 512, 4>>(),
-                                                  entry<float, Shape<96, 1408, 5>>(), entry<float, Shape<64, 1024, 6>>(),
-                                                  entry<float, Shape<160, 2176, 4>>(), entry<float, Shape<16, 288, 4>>()};
-    static constexpr int by_size[] = {0, 3, 1, 5};  // widest first (pick_shape)
+    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<32, 480, 12, 128>>(),
+                                                  entry<float, Shape<16, 256, 6, 256>>(),
+                                                  entry<float, Shape<72, 912, 6, 256>>()};
+    static constexpr int by_wave[] = {1, 0, 2};  // by the cells that one wave of blocks holds
 };
 template <>
 struct Shapes<double> {
-    static constexpr ShapeEntry<double> list[] = {entry<double, Shape<64, 1024, 4>>(), entry<double, Shape<112, 1600, 3>>(),
-                                                   entry<double, Shape<32, 512, 4>>(), entry<double, Shape<16, 288, 4>>(),
-                                                   entry<double, Shape<160, 2176, 2>>(), entry<double, Shape<96, 1408, 3>>()};
-    static constexpr int by_size[] = {0, 2, 3};
+    static constexpr ShapeEntry<double> list[] = {entry<double, Shape<24, 352, 8, 128>>(),
+                                                   entry<double, Shape<16, 256, 5, 256>>()};
+    static constexpr int by_wave[] = {1, 0};
 };
+constexpr int kLargeBox = 0;  // the shape for boxes of several waves
+// the interval on gathered records (where buckets would take too much memory)
+template <typename R>
+using GatherShape = std::conditional_t<sizeof(R) == 4, Shape<128, 1792, 4>, Shape<64, 1024, 4>>;
+
 template <typename R>
 constexpr int n_shapes()
 {
     return (int)(sizeof(Shapes<R>::list) / sizeof(Shapes<R>::list[0]));
 }
 
-static int g_shape[2] = {-1, -1};  // shape set: [0] FP32, [1] FP64; -1 = by the size of the box
+static int g_shape[2] = {-1, -1};  // shape set: [0] FP32, [1] FP64; -1 = by box and density
 
-// The shape of a run: the one set, or the widest of by_size whose tiles, over
-// the cells of the box, number at least kMinTiles (about two per SM); a box
-// with fewer takes the narrowest.  A tile's block is a chain of latencies
-// (index copy, gather, collision, streaming) about as long as its passes over
-// the particles, so a small box wants every SM busy with short blocks and a
-// large one wants tiles wide enough to hide the chain.  us per interval
-// (slots per tile x blocks per SM): 16^3 FP32 20.7 (16 x 4), 24.7 (64 x 6),
-// 28.6 (128 x 4), FP64 22.3 (16 x 4), 25.7 (64 x 4), 28.6 (96 x 3); 24^3 FP64
-// 30.8 (32 x 4), 37.6 (64 x 4); 32^3 FP32 31.9 (64 x 6), 33.3 (128 x 4); 128^3
-// FP32 682 (128 x 4), 713 (64 x 6), FP64 1153 (64 x 4), 1177 (96 x 3), 1431
-// (96 x 4).
-constexpr int kMinTiles = 260;
+static int num_sms()
+{
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+}
 
+static long long box_cells(const rmpcd_cells *c) { return (long long)c->L[0] * c->L[1] * c->L[2]; }
+
+static double mean_occupancy(const rmpcd_particles *p, const rmpcd_cells *c)
+{
+    return (double)p->N / (double)box_cells(c);
+}
+
+// The shape of a run: the one set, or the first of by_wave whose blocks hold all
+// cells of the box at once, or else the one for boxes of several waves.  A tile's block
+// is a chain of latencies (record copy, collision, counting atomics), so a
+// small box takes the shape with the most threads per particle, as long as its
+// tiles all run at once; many small blocks, with few warps waiting at each
+// barrier, are best for a large box; and a box just above one wave of those
+// takes a wider tile that fits.  us per interval (slots x blocks per SM x
+// threads): 16^3 FP32 9.3 (16 x 6 x 256), 13.9 (32 x 12 x 128), FP64 9.4 (16 x 5
+// x 256), 13.4 (24 x 8 x 128); 24^3 FP32 12.1, 14.6, FP64 16.4, 15.1; 32^3 FP32
+// 21.0, 16.3, FP64 25.2, 25.7; 61,500 cells FP32 27.2 (32 x 12 x 128), 23.1 (72 x
+// 6 x 256); 128^3 FP32 531 (32 x 12 x 128), 545 (72 x 6 x 256), 552 (96 x 5 x
+// 256), FP64 931 (24 x 8 x 128), 963 (40 x 5 x 256), 989 (48 x 4 x 256).
 template <typename R>
 static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c)
 {
     const int set = g_shape[sizeof(R) == 8];
     if (set >= 0) return Shapes<R>::list[set];
-    const long long cells = (long long)c->L[0] * c->L[1] * c->L[2];
-    int pick = 0;
-    for (int k : Shapes<R>::by_size) {
-        pick = k;
-        if (cells / Shapes<R>::list[k].slots >= kMinTiles) break;
+    for (int k : Shapes<R>::by_wave) {
+        const ShapeEntry<R> &e = Shapes<R>::list[k];
+        if (box_cells(c) <= (long long)e.slots * e.min_blocks * num_sms()) return e;
     }
-    return Shapes<R>::list[pick];
+    return Shapes<R>::list[kLargeBox];
 }
 
 template <typename R>
@@ -720,10 +758,86 @@ static int prepare_shapes()
 {
     static bool done[2] = {false, false};
     if (done[sizeof(R) == 8]) return RMPCD_OK;
-    for (int k = 0; k < n_shapes<R>(); k++)
-        RMPCD_CUDA_TRY(cudaFuncSetAttribute(Shapes<R>::list[k].kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)Shapes<R>::list[k].smem));
+    for (int k = 0; k < n_shapes<R>(); k++) {
+        const ShapeEntry<R> &e = Shapes<R>::list[k];
+        RMPCD_CUDA_TRY(cudaFuncSetAttribute(e.interval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem));
+        RMPCD_CUDA_TRY(cudaFuncSetAttribute(e.to_soa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem));
+    }
+    RMPCD_CUDA_TRY(cudaFuncSetAttribute(k_bulk_interval<R, GatherShape<R>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)fused_smem<R, GatherShape<R>>()));
     done[sizeof(R) == 8] = true;
+    return RMPCD_OK;
+}
+
+// Records per bucket: about 4.4 standard deviations above the mean occupancy
+// of the cells (24 at density 10: one cell of a uniform fluid in 20,000
+// overflows into its list).
+static int bucket_cap(double mean) { return ((int)ceil(mean + 4.3 * sqrt(mean)) + 7) & ~7; }
+
+// The numbering of the buckets of a box with more slots than cells, laid out
+// once per cell system: the slots of the box's cells by rank, then the others.
+__global__ void k_mark_cells(const int *lut, int n_lut, int *mark)
+{
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_lut; c += gridDim.x * blockDim.x) mark[lut[c]] = 1;
+}
+// rank (exclusive) holds the marked slots before each slot
+__global__ void k_number_buckets(const int *mark, const int *rank, int S, int n_cells, int *of_slot, int *slot_of)
+{
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
+        const int b = mark[s] ? rank[s] : n_cells + (s - rank[s]);
+        of_slot[s] = b;
+        slot_of[b] = s;
+    }
+}
+__global__ void k_bucket_lut(const int *lut, int n_lut, const int *of_slot, int *out)
+{
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_lut; c += gridDim.x * blockDim.x) out[c] = of_slot[lut[c]];
+}
+
+// uses c->count_next (zero between runs) and c->cursor as scratch
+static int ensure_bucket_map(rmpcd_cells *c)
+{
+    if (c->n_lut == c->S || c->bucket_map) return RMPCD_OK;
+    cudaStream_t st = stream();
+    int *map = nullptr;
+    RMPCD_CUDA_TRY(cudaMalloc(&map, (2 * (size_t)c->S + c->n_lut) * sizeof(int)));
+    c->bucket_map = map;
+    k_mark_cells<<<grid_for(c->n_lut, 256), 256, 0, st>>>(c->lut, c->n_lut, c->count_next);
+    const int rc = exclusive_scan(c->count_next, c->cursor, nullptr, c->S, c->scan_tmp, nullptr, st);
+    if (rc) return rc;
+    k_number_buckets<<<grid_for(c->S, 256), 256, 0, st>>>(c->count_next, c->cursor, c->S, c->n_lut, map, map + c->S);
+    k_bucket_lut<<<grid_for(c->n_lut, 256), 256, 0, st>>>(c->lut, c->n_lut, map, map + 2 * (size_t)c->S);
+    RMPCD_CHECK_LAUNCH();
+    RMPCD_CUDA_TRY(cudaMemsetAsync(c->count_next, 0, (size_t)c->S * sizeof(int), st));
+    return RMPCD_OK;
+}
+
+// The bucket arrays (one allocation): two grids of n_rec * cap records, pools
+// of N records and their links, list heads of three grids and the counters.
+// *ok = false when they would take more than a quarter of the free memory (the
+// records of the gather take a third of their bytes), or there is none.
+template <typename R>
+static int ensure_buckets(rmpcd_particles *p, int S, int n_rec, int cap, bool *ok)
+{
+    const size_t B = Bucket<R>::kBytes;
+    const size_t bytes = 2 * ((size_t)n_rec * cap + p->N) * B + 2 * (size_t)p->N * 4 + (3 * (size_t)S + 6) * 4;
+    *ok = true;
+    if (p->bkt_bytes >= bytes) return RMPCD_OK;
+    size_t free_bytes = 0, total = 0;
+    RMPCD_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total));
+    *ok = bytes <= (free_bytes + p->bkt_bytes) / 4;
+    if (!*ok) return RMPCD_OK;
+    if (p->buckets) RMPCD_CUDA_TRY(cudaStreamSynchronize(stream()));
+    cudaFree(p->buckets);
+    p->buckets = nullptr;
+    p->bkt_bytes = 0;
+    if (cudaMalloc(&p->buckets, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        p->buckets = nullptr;
+        *ok = false;
+        return RMPCD_OK;
+    }
+    p->bkt_bytes = bytes;
     return RMPCD_OK;
 }
 
@@ -743,15 +857,109 @@ static int ensure_records(rmpcd_particles *p)
     return RMPCD_OK;
 }
 
+// the next interval's grid shift (rng step r->step + 1) as an origin
+static void next_origin(const rmpcd_rng *r, double origin[3])
+{
+    double u0, u1, u2, u3;
+    rng::uniform2(r->seed, r->step + 1, 0, rng::SHIFT, 0, u0, u1);
+    rng::uniform2(r->seed, r->step + 1, 1, rng::SHIFT, 0, u2, u3);
+    origin[0] = u0 - 1;
+    origin[1] = u1 - 1;
+    origin[2] = u2 - 1;
+}
+
+template <typename R>
+static int bulk_run_buckets(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double tau, int has_alpha, double alpha,
+                            int n_intervals, int cap)
+{
+    cudaStream_t st = stream();
+    const ShapeEntry<R> &shape = pick_shape<R>(c);
+    int rc = ensure_bucket_map(c);
+    if (rc) return rc;
+    BucketMap map{nullptr, nullptr};
+    if (c->bucket_map) map = {c->bucket_map, c->bucket_map + c->S};
+    // image, flags and id stay in the current API arrays, addressed by idx
+    const PView<R> side = cur<R>(p);
+    // counts of grid i in cnt[i % 3]; the slots' counts are consumed by the
+    // pack before grid 2 takes their array
+    int *cnt[3] = {c->cursor, c->count_next, c->count};
+    const size_t rec = (size_t)c->n_lut * cap * Bucket<R>::kBytes, pool = (size_t)p->N * Bucket<R>::kBytes;
+    int *link = (int *)(p->buckets + 2 * (rec + pool)), *head = link + 2 * (size_t)p->N, *n_pool = head + 3 * (size_t)c->S;
+    auto grid = [&](int i) {
+        return BucketGrid{p->buckets + (i & 1) * (rec + pool), p->buckets + (i & 1) * (rec + pool) + rec,
+                          link + (size_t)(i & 1) * p->N, cnt[i % 3], head + (size_t)(i % 3) * c->S, n_pool + i % 3,
+                          cap, c->n_lut};
+    };
+    {
+        PhaseTimer t("pack");
+        RMPCD_CUDA_TRY(cudaMemsetAsync(n_pool, 0, 6 * sizeof(int), st));
+        k_soa_to_buckets<R><<<grid_for((long long)c->S * 32, kFusedThreads), kFusedThreads, 0, st>>>(
+            side, grid(0), map, c->S, c->count, c->start, grid(1).count, grid(1).head, grid(1).n_pool);
+        RMPCD_CHECK_LAUNCH();
+    }
+    BucketArgs<R> A;
+    A.S = c->S;
+    A.map = map;
+    A.ix = side.ix;
+    A.iy = side.iy;
+    A.iz = side.iz;
+    A.e0 = c->edges[0];
+    A.e1 = c->edges[1];
+    A.e2 = c->edges[2];
+    A.dt = (R)tau;
+    A.sin_a = has_alpha ? sin(alpha) : 1;
+    A.cos_a = has_alpha ? cos(alpha) : 0;
+    A.seed = r->seed;
+    A.axes = c->axes;
+    A.err = dev_error_word();
+    A.ids = p->perm;
+    A.ids_tmp = p->key;
+    A.g_next = grid_of(c);
+    if (c->bucket_map) A.g_next.lut = c->bucket_map + 2 * (size_t)c->S;
+    const int nblocks = (c->S + shape.slots - 1) / shape.slots;
+    for (int it = 0; it < n_intervals; it++) {
+        const BucketGrid clear = grid(it + 2);
+        A.in = grid(it);
+        A.out = grid(it + 1);
+        A.count_clear = clear.count;
+        A.head_clear = clear.head;
+        A.n_pool_clear = clear.n_pool;
+        A.step = r->step;
+        next_origin(r, A.g_next.origin);
+        PhaseTimer t("interval_fused");
+        shape.interval<<<nblocks, shape.threads, shape.smem, st>>>(A);
+        RMPCD_CHECK_LAUNCH();
+        r->step += 2;
+    }
+    for (int k = 0; k < 3; k++) c->origin[k] = A.g_next.origin[k];
+    // the last grid's counts by slot, in the array of the grid before it; the
+    // third array was cleared by the last interval
+    c->count = cnt[n_intervals % 3];
+    c->count_next = cnt[(n_intervals + 1) % 3];
+    c->cursor = cnt[(n_intervals + 2) % 3];
+    PhaseTimer t("sort");
+    if (c->bucket_map) {
+        std::swap(c->count, c->cursor);
+        k_bucket_counts_to_slots<<<grid_for(c->S, 256), 256, 0, st>>>(c->cursor, map.slot_of, c->S, c->count);
+        RMPCD_CHECK_LAUNCH();
+    }
+    rc = exclusive_scan(c->count, c->start, c->cursor, c->S, c->scan_tmp, nullptr, st);
+    if (rc) return rc;
+    shape.to_soa<<<nblocks, shape.threads, shape.smem, st>>>(grid(n_intervals), map, c->S, c->count, c->start, side,
+                                                             alt<R>(p), p->perm, p->key, dev_error_word());
+    RMPCD_CHECK_LAUNCH();
+    p->cur = 1 - p->cur;
+    p->alt_force_clean = p->cur_force_gated = false;
+    return RMPCD_OK;
+}
+
 template <typename R>
 static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double tau, int has_alpha,
                           double alpha, int n_intervals)
 {
     cudaStream_t st = stream();
-    int rc = prepare_shapes<R>();
-    if (rc) return rc;
-    const ShapeEntry<R> &shape = pick_shape<R>(c);
-    rc = ensure_records<R>(p);
+    using S = GatherShape<R>;
+    int rc = ensure_records<R>(p);
     if (rc) return rc;
     double sin_a = 1, cos_a = 0;
     if (has_alpha) {
@@ -766,7 +974,7 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
     // image, flags and id stay in the current API arrays, addressed by idx
     const PView<R> side = cur<R>(p);
     int rb = 0;  // record buffer holding the current arrays
-    const int nblocks = (c->S + shape.slots - 1) / shape.slots;
+    const int nblocks = (c->S + S::kSlots - 1) / S::kSlots;
     const int ntiles = nblocks;
     // slots fit the packed key for every box up to 2^22 slots (128^3 is 2^21);
     // larger boxes keep plain keys and regroup them in k_perm
@@ -774,11 +982,6 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
     int *perm = nullptr;  // identity for the first interval (data sorted on entry)
     for (int it = 0; it < n_intervals; it++) {
         uint64_t step_c = r->step;
-        uint64_t step_s = r->step + 1;
-        r->step += 2;
-        double u0, u1, u2, u3;
-        rng::uniform2(r->seed, step_s, 0, rng::SHIFT, 0, u0, u1);
-        rng::uniform2(r->seed, step_s, 1, rng::SHIFT, 0, u2, u3);
         FusedArgs<R> A;
         A.in = p->rec[rb];
         A.out = p->rec[1 - rb];
@@ -795,9 +998,8 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
         A.iy = side.iy;
         A.iz = side.iz;
         A.g_next = grid_of(c);
-        A.g_next.origin[0] = u0 - 1;
-        A.g_next.origin[1] = u1 - 1;
-        A.g_next.origin[2] = u2 - 1;
+        next_origin(r, A.g_next.origin);
+        r->step += 2;
         A.e0 = c->edges[0];
         A.e1 = c->edges[1];
         A.e2 = c->edges[2];
@@ -810,7 +1012,7 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
         A.err = dev_error_word();
         {
             PhaseTimer t("interval_fused");
-            shape.kernel<<<nblocks, kFusedThreads, shape.smem, st>>>(A);
+            k_bulk_interval<R, S><<<nblocks, kFusedThreads, fused_smem<R, S>(), st>>>(A);
             RMPCD_CHECK_LAUNCH();
         }
         rb = 1 - rb;
@@ -860,6 +1062,28 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
     return RMPCD_OK;
 }
 
+// The schedule of a run: buckets, unless the tiles of the shape in use would
+// not hold the mean occupancy with 5 standard deviations to spare (from density
+// 11 on; over-full tiles are slow) or there is too little memory: the gather.
+// us per interval (buckets, gather): 16^3 FP32 9.3, 20.7, FP64 9.4, 22.3; 32^3
+// FP32 16.3, 31.9, FP64 25.7, 44; 64^3 FP32 77.7, 107, FP64 129, 173; 128^3 FP32
+// 531, 682, FP64 931, 1153.
+template <typename R>
+static int bulk_run_t(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double tau, int has_alpha, double alpha,
+                      int n_intervals)
+{
+    int rc = prepare_shapes<R>();
+    if (rc) return rc;
+    const ShapeEntry<R> &shape = pick_shape<R>(c);
+    const double mean = mean_occupancy(p, c), tile = mean * shape.slots;
+    bool buckets = tile + 5 * sqrt(tile) <= shape.cap;
+    const int cap = bucket_cap(mean);
+    if (buckets) rc = ensure_buckets<R>(p, c->S, c->n_lut, cap, &buckets);
+    if (rc) return rc;
+    if (buckets) return bulk_run_buckets<R>(p, c, r, tau, has_alpha, alpha, n_intervals, cap);
+    return bulk_run_fused<R>(p, c, r, tau, has_alpha, alpha, n_intervals);
+}
+
 }  // namespace rmpcd
 
 using namespace rmpcd;
@@ -899,10 +1123,10 @@ static int autotune_t(const int L[3], double tau, int n_intervals, int *best, fl
         int best_k = 0;
         for (int k = 0; !rc && k < n_shapes<R>(); k++) {
             g_shape[sizeof(R) == 8] = k;
-            rc = bulk_run_fused<R>(p, c, &r, tau, 0, 0.0, 1);
+            rc = bulk_run_t<R>(p, c, &r, tau, 0, 0.0, 1);
             if (rc) break;
             cudaEventRecord(e0, stream());
-            rc = bulk_run_fused<R>(p, c, &r, tau, 0, 0.0, n_intervals);
+            rc = bulk_run_t<R>(p, c, &r, tau, 0, 0.0, n_intervals);
             cudaEventRecord(e1, stream());
             if (!rc) rc = sync();
             float ms = 0;
@@ -985,6 +1209,6 @@ extern "C" int rmpcd_bulk_run(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, 
         }
         return RMPCD_OK;
     }
-    if (p->precision == RMPCD_FP32) return bulk_run_fused<float>(p, c, r, tau, has_alpha, alpha, n_intervals);
-    return bulk_run_fused<double>(p, c, r, tau, has_alpha, alpha, n_intervals);
+    if (p->precision == RMPCD_FP32) return bulk_run_t<float>(p, c, r, tau, has_alpha, alpha, n_intervals);
+    return bulk_run_t<double>(p, c, r, tau, has_alpha, alpha, n_intervals);
 }

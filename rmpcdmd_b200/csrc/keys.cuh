@@ -25,11 +25,20 @@ __host__ __device__ inline void cell_coords(const Grid &g, double x, double y, d
     if ((!g.has_walls) && (p[2] == g.L[2])) p[2] = 0;
 }
 
+__device__ inline bool in_grid(const Grid &g, const int p[3])
+{
+    return (unsigned)p[0] < (unsigned)g.L[0] && (unsigned)p[1] < (unsigned)g.L[1] && (unsigned)p[2] < (unsigned)g.L[2];
+}
+
+// the table's entry of a cell in the grid
+__device__ inline int cell_entry(const Grid &g, const int p[3])
+{
+    return __ldg(g.lut + (p[0] + g.L[0] * (p[1] + g.L[1] * p[2])));
+}
+
 __device__ inline int slot_of_cell(const Grid &g, const int p[3])
 {
-    if ((unsigned)p[0] < (unsigned)g.L[0] && (unsigned)p[1] < (unsigned)g.L[1] &&
-        (unsigned)p[2] < (unsigned)g.L[2])
-        return __ldg(g.lut + (p[0] + g.L[0] * (p[1] + g.L[1] * p[2])));
+    if (in_grid(g, p)) return cell_entry(g, p);
     return hilbert::compact_index(p, g.M);
 }
 

@@ -253,6 +253,7 @@ static void free_particles(rmpcd_particles *p)
     cudaFree(p->rec[0]);
     cudaFree(p->rec[1]);
     cudaFree(p->n2_terms);
+    cudaFree(p->buckets);
     delete p;
 }
 

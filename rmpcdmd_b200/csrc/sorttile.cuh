@@ -27,21 +27,24 @@ struct OrderTile {
     unsigned char cell[kOrderCap];
 };
 
-__device__ inline int lower_bound_int(const int *a, int n, int v)
+// entries of a[0, n), ascending by key, whose key is below v
+template <typename Key, typename V>
+__device__ inline int lower_bound_by(const int *a, int n, V v, Key key)
 {
     int lo = 0, hi = n;
     while (lo < hi) {
         int mid = (lo + hi) >> 1;
-        if (a[mid] < v) lo = mid + 1;
+        if (key(a[mid]) < v) lo = mid + 1;
         else hi = mid;
     }
     return lo;
 }
 
-// ascending order of the n distinct values a[0, n) by the whole block:
-// bottom-up merge sort, every element placed by its rank in the partner run;
-// b is scratch of the same extent
-__device__ inline void block_merge_sort(int *a, int *b, int n)
+// the n values a[0, n), with distinct keys, into ascending order of their keys
+// by the whole block: bottom-up merge sort, every element placed by its rank in
+// the partner run; b is scratch of the same extent
+template <typename Key>
+__device__ inline void block_merge_sort(int *a, int *b, int n, Key key)
 {
     int *src = a, *dst = b;
     for (int w = 1; w < n; w <<= 1) {
@@ -53,10 +56,10 @@ __device__ inline void block_merge_sort(int *a, int *b, int n)
             if ((run & 1) == 0) {
                 int p0 = r0 + w;
                 int pn = min(w, max(0, n - p0));
-                pos = r0 + (i - r0) + lower_bound_int(src + p0, pn, v);
+                pos = r0 + (i - r0) + lower_bound_by(src + p0, pn, key(v), key);
             } else {
                 int p0 = r0 - w;
-                pos = p0 + (i - r0) + lower_bound_int(src + p0, w, v);
+                pos = p0 + (i - r0) + lower_bound_by(src + p0, w, key(v), key);
             }
             dst[pos] = v;
         }
@@ -68,6 +71,10 @@ __device__ inline void block_merge_sort(int *a, int *b, int n)
     if (src != a)
         for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = src[i];
     __syncthreads();
+}
+__device__ inline void block_merge_sort(int *a, int *b, int n)
+{
+    block_merge_sort(a, b, n, [](int v) { return v; });
 }
 
 // Orders slots [s0, s1), s1 - s0 <= kOrderSlots, by a block of kOrderThreads;

@@ -31,6 +31,9 @@ struct rmpcd_cells {
     unsigned char *is_md = nullptr;
     unsigned char *is_reac = nullptr;
     int *lut = nullptr;        // n_lut: slot of cell (p0 + L0*(p1 + L1*p2))
+    // bulk schedule, boxes with S > n_lut: bucket of every slot (S), slot of
+    // every bucket (S), bucket of every cell (n_lut)
+    int *bucket_map = nullptr;
     int *scan_tmp = nullptr;   // tile totals of the slot scan
     int scan_blocks = 0;
     double *axes = nullptr;    // injected SRD axes (3*S) or null
@@ -72,6 +75,8 @@ struct rmpcd_particles {
     // 6 reals (pos, vel) + 6 ints (image, id, species, flags) per particle
     unsigned char *rec[2] = {nullptr, nullptr};
     size_t rec_bytes = 0;
+    unsigned char *buckets = nullptr;  // bucket arrays of the bulk schedule
+    size_t bkt_bytes = 0;
     // force / force_old entries known to be exactly zero: the sort skips
     // permuting them (a permutation of zeros is zeros)
     bool force_zero = true;
