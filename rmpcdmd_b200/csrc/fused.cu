@@ -714,14 +714,6 @@ constexpr int n_shapes()
 
 static int g_shape[2] = {-1, -1};  // shape set: [0] FP32, [1] FP64; -1 = by box and density
 
-static int num_sms()
-{
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-}
-
 static long long box_cells(const rmpcd_cells *c) { return (long long)c->L[0] * c->L[1] * c->L[2]; }
 
 static double mean_occupancy(const rmpcd_particles *p, const rmpcd_cells *c)
@@ -748,7 +740,7 @@ static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c)
     if (set >= 0) return Shapes<R>::list[set];
     for (int k : Shapes<R>::by_wave) {
         const ShapeEntry<R> &e = Shapes<R>::list[k];
-        if (box_cells(c) <= (long long)e.slots * e.min_blocks * num_sms()) return e;
+        if (box_cells(c) <= (long long)e.slots * e.min_blocks * sm_count()) return e;
     }
     return Shapes<R>::list[kLargeBox];
 }

@@ -81,7 +81,7 @@ __global__ void k_pair_forces(const double *cx, const double *cy, const double *
 // are collected for k_apply_multi
 template <typename R>
 __global__ void k_apply_single(const int *list, const int *n, int Nmax, const unsigned char *contrib,
-                               const double *pf, const int *ncontrib, R *fx, R *fy, R *fz,
+                               const double *pf, int *ncontrib, R *fx, R *fy, R *fz,
                                unsigned long long *mkeys, int *m_count, const int *gate)
 {
     if (gate && *gate) return;
@@ -93,7 +93,7 @@ __global__ void k_apply_single(const int *list, const int *n, int Nmax, const un
 
 template <typename R>
 __global__ void k_apply_multi(const int *list, const int *n, int C, int Nmax, const unsigned char *contrib,
-                              const double *pf, const int *ncontrib, int *max_contrib, int serial,
+                              const double *pf, int *ncontrib, int *max_contrib, int serial,
                               R *fx, R *fy, R *fz, const unsigned long long *mkeys, int *m_count,
                               const int *gate)
 {
@@ -105,7 +105,7 @@ __global__ void k_apply_multi(const int *list, const int *n, int C, int Nmax, co
     if (threadIdx.x == 0) *max_contrib = 0;
     if (mc < 2) return;
     const int m = *m_count;
-    if (!apply_multi_sorted_block(mkeys, m, pf, fx, fy, fz))
+    if (!apply_multi_sorted_block(mkeys, m, pf, ncontrib, fx, fy, fz))
         apply_multi_block(list, n, C, Nmax, contrib, pf, ncontrib, serial, fx, fy, fz);
     __syncthreads();
     if (threadIdx.x == 0) *m_count = 0;
@@ -215,17 +215,6 @@ __global__ void __launch_bounds__(1024) k_energy(const int *cn, const int *clist
             return pe[q + clist[q + (f - pre[lo])]];
         },
         total, out);
-}
-
-__global__ void k_reset_contrib(const int *list, const int *n, int Nmax, const unsigned char *contrib,
-                                int *ncontrib, const int *gate)
-{
-    if (gate && *gate) return;
-    const int i = blockIdx.y;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n[i]; e += gridDim.x * blockDim.x) {
-        size_t q = (size_t)i * Nmax + e;
-        if (contrib[q]) ncontrib[list[q]] = 0;
-    }
 }
 
 // compute_force_n2, src/neighbor_list.f90:227-264: a thread per colloid for
@@ -506,9 +495,8 @@ int compute_force_impl(rmpcd_particles *ps1, rmpcd_particles *ps2, rmpcd_nlist *
     int *cn = nl->d_status + 16;
     int *clist = nl->d_status + 16 + 2 * nl->Npoints;
     double *e_out = (double *)ps1->d_sums;
-    // k_apply_multi leaves max_contrib at zero and the scratch starts at zero,
-    // so the n_colloids loop (n2 given) skips this clear; other callers keep it
-    if (!n2) RMPCD_CUDA_TRY(cudaMemsetAsync(max_contrib, 0, sizeof(int), s));
+    // the scratch starts at zero; k_apply_single and k_apply_multi leave the
+    // contribution counts, and k_apply_multi max_contrib and m_count, at zero
     ps2->force_zero = false;
     ps1->force_zero = false;
     if (C > 0) {
@@ -577,7 +565,6 @@ int compute_force_impl(rmpcd_particles *ps1, rmpcd_particles *ps2, rmpcd_nlist *
                                                     nl->ncontrib, max_contrib, serial, v.force.x, v.force.y, v.force.z, nl->mkeys,
                                                    m_count, gate);
         }
-        k_reset_contrib<<<grid, 256, 0, s>>>(nl->list, nl->n, nl->Nmax, nl->contrib, nl->ncontrib, gate);
         if (energy) k_energy<<<1, 1024, 0, s>>>(cn, clist, C, nl->Nmax, nl->pair_e, nl->e_pre, e_out);
         if (fork) RMPCD_CUDA_TRY(cudaStreamWaitEvent(s, n2->ev_join, 0));
         RMPCD_CHECK_LAUNCH();

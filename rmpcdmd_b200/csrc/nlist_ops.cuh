@@ -311,19 +311,6 @@ __device__ inline void pair_force_entry(size_t q, const double x[3], int s1, con
     contrib[q] = c;
 }
 
-// solvent force - f of entry q when its particle has exactly one contribution
-template <typename R>
-__device__ inline void apply_single_entry(size_t q, const int *list, const unsigned char *contrib, const double *pf,
-                                          const int *ncontrib, R *fx, R *fy, R *fz)
-{
-    if (!contrib[q]) return;
-    int idx = list[q];
-    if (ncontrib[idx] != 1) return;
-    fx[idx] = fx[idx] - (R)pf[3 * q];
-    fy[idx] = fy[idx] - (R)pf[3 * q + 1];
-    fz[idx] = fz[idx] - (R)pf[3 * q + 2];
-}
-
 // Particles with several contributions must receive their subtractions in
 // the reference's (colloid, entry) order.  The single-contribution pass
 // collects them as 64-bit keys (particle << 32 | entry index q, with
@@ -334,7 +321,7 @@ constexpr int kMultiSortMax = 4096;
 
 template <typename R>
 __device__ inline void apply_single_or_collect(size_t q, const int *list, const unsigned char *contrib,
-                                               const double *pf, const int *ncontrib, R *fx, R *fy, R *fz,
+                                               const double *pf, int *ncontrib, R *fx, R *fy, R *fz,
                                                unsigned long long *mkeys, int *m_count)
 {
     if (!contrib[q]) return;
@@ -344,6 +331,7 @@ __device__ inline void apply_single_or_collect(size_t q, const int *list, const 
         fx[idx] = fx[idx] - (R)pf[3 * q];
         fy[idx] = fy[idx] - (R)pf[3 * q + 1];
         fz[idx] = fz[idx] - (R)pf[3 * q + 2];
+        ncontrib[idx] = 0;  // for the next evaluation; no other entry has this particle
     } else if (nc > 1) {
         const int k = atomicAdd(m_count, 1);
         if (k < kMultiSortMax) mkeys[k] = ((unsigned long long)(unsigned)idx << 32) | (unsigned long long)q;
@@ -354,8 +342,8 @@ __device__ inline void apply_single_or_collect(size_t q, const int *list, const 
 // in (colloid, entry) order; returns false (nothing applied) when more keys
 // were collected than the block sorts
 template <typename R>
-__device__ inline bool apply_multi_sorted_block(const unsigned long long *mkeys, int m, const double *pf, R *fx,
-                                                R *fy, R *fz)
+__device__ inline bool apply_multi_sorted_block(const unsigned long long *mkeys, int m, const double *pf,
+                                                int *ncontrib, R *fx, R *fy, R *fz)
 {
     __shared__ unsigned long long sk[kMultiSortMax];
     if (m > kMultiSortMax) return false;
@@ -388,6 +376,7 @@ __device__ inline bool apply_multi_sorted_block(const unsigned long long *mkeys,
             fy[idx] = fy[idx] - (R)pf[3 * q + 1];
             fz[idx] = fz[idx] - (R)pf[3 * q + 2];
         }
+        ncontrib[idx] = 0;  // for the next evaluation
     }
     __syncthreads();
     return true;
@@ -398,7 +387,7 @@ __device__ inline bool apply_multi_sorted_block(const unsigned long long *mkeys,
 // in which case a single thread applies everything in order (one block)
 template <typename R>
 __device__ inline void apply_multi_block(const int *list, const int *n, int C, int Nmax, const unsigned char *contrib,
-                                         const double *pf, const int *ncontrib, int serial, R *fx, R *fy, R *fz)
+                                         const double *pf, int *ncontrib, int serial, R *fx, R *fy, R *fz)
 {
     for (int i = 0; i < C; i++) {
         const int ni = n[i];
@@ -427,6 +416,11 @@ __device__ inline void apply_multi_block(const int *list, const int *n, int C, i
         }
         __syncthreads();
     }
+    for (int i = 0; i < C; i++)
+        for (int e = threadIdx.x; e < n[i]; e += blockDim.x) {
+            const size_t q = (size_t)i * Nmax + e;
+            if (contrib[q]) ncontrib[list[q]] = 0;  // for the next evaluation
+        }
 }
 
 // f1 = sum of colloid i's pair forces in list order; force(:,i) += f1; the

@@ -1,6 +1,7 @@
 // particle_system_t on the GPU (src/particle_system.f90): allocation, host
 // transfers in the reference (3,N) layout, sort, displacement bounds, random
 // placement and Maxwell initial velocities.
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -68,10 +69,47 @@ __global__ void k_count_nonfinite(Vec3<R> pos, Vec3<R> vel, long long N, unsigne
     }
 }
 
+// The maximum over the grid of every thread's m into *host (mapped host memory)
+// by the block that finishes last, which leaves acc[0] (the maximum) and acc[1]
+// (finished blocks) at zero for the next reduction.
+__device__ inline void grid_max_to_host(double m, unsigned long long *acc, unsigned long long *host)
+{
+    warp_max_into(acc, m);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(acc + 1, 1ull) == gridDim.x - 1) {
+        __threadfence();
+        *(volatile unsigned long long *)host = atomicExch(acc, 0ull);
+        acc[1] = 0;
+        __threadfence_system();
+    }
+}
+
+// the three components of a vector field set to zero, or copied, in one launch
+template <typename R>
+__global__ void k_zero3(Vec3<R> a, long long N)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+        a.x[i] = 0;
+        a.y[i] = 0;
+        a.z[i] = 0;
+    }
+}
+template <typename R>
+__global__ void k_copy3(Vec3<R> a, Vec3<R> b, long long N)
+{
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
+        const R x = a.x[i], y = a.y[i], z = a.z[i];
+        b.x[i] = x;
+        b.y[i] = y;
+        b.z[i] = z;
+    }
+}
+
 // maximum_displacement, src/particle_system.f90:357-378
 template <typename R>
-__global__ void k_max_disp(Vec3<R> pos, Vec3<R> old, const int *species, int N,
-                           unsigned long long *out)
+__global__ void k_max_disp(Vec3<R> pos, Vec3<R> old, const int *species, int N, unsigned long long *acc,
+                           unsigned long long *host)
 {
     double m = 0;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N;
@@ -79,14 +117,14 @@ __global__ void k_max_disp(Vec3<R> pos, Vec3<R> old, const int *species, int N,
         double r = disp_sq_one(pos, old, species, i);
         m = m > r ? m : r;
     }
-    warp_max_into(out, m);
+    grid_max_to_host(m, acc, host);
 }
 
 // cell_maximum_displacement, src/particle_system.f90:380-410
 template <typename R>
 __global__ void k_cell_max_disp(const int *count, const int *start, const unsigned char *is_md,
-                                int S, Vec3<R> pos, Vec3<R> old, const int *species,
-                                unsigned long long *out)
+                                int S, Vec3<R> pos, Vec3<R> old, const int *species, unsigned long long *acc,
+                                unsigned long long *host)
 {
     double m = 0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < S; s += gridDim.x * blockDim.x) {
@@ -102,7 +140,7 @@ __global__ void k_cell_max_disp(const int *count, const int *start, const unsign
             }
         }
     }
-    warp_max_into(out, m);
+    grid_max_to_host(m, acc, host);
 }
 
 // random_placement, src/particle_system.f90:250-302: uniform positions,
@@ -188,38 +226,68 @@ int fixed_order_sum(const double *a, int N, double *d_out)
     return RMPCD_OK;
 }
 
-int launch_max_disp(rmpcd_particles *p)
+// the mapped host word of the displacement maxima
+static int ensure_h_max(rmpcd_particles *p)
 {
-    cudaStream_t s = stream();
-    RMPCD_CUDA_TRY(cudaMemsetAsync(p->d_max, 0, 8, s));
-    if (p->N > 0) {
-        if (p->precision == RMPCD_FP32) {
-            PView<float> a = cur<float>(p), b = alt<float>(p);
-            k_max_disp<float><<<grid_for(p->N, 256), 256, 0, s>>>(a.pos, b.pos, a.species, p->N, p->d_max);
-        } else {
-            PView<double> a = cur<double>(p), b = alt<double>(p);
-            k_max_disp<double><<<grid_for(p->N, 256), 256, 0, s>>>(a.pos, b.pos, a.species, p->N, p->d_max);
-        }
-        RMPCD_CHECK_LAUNCH();
-    }
+    if (p->h_max) return RMPCD_OK;
+    RMPCD_CUDA_TRY(cudaHostAlloc((void **)&p->h_max, 64, cudaHostAllocMapped));
+    RMPCD_CUDA_TRY(cudaHostGetDevicePointer((void **)&p->h_max_dev, p->h_max, 0));
     return RMPCD_OK;
 }
 
-int launch_cell_max_disp(rmpcd_cells *c, rmpcd_particles *p)
+// waits for the reduction just launched: the maximum r
+static int read_h_max(const rmpcd_particles *p, double *r)
 {
-    cudaStream_t s = stream();
-    RMPCD_CUDA_TRY(cudaMemsetAsync(p->d_max, 0, 8, s));
-    if (p->precision == RMPCD_FP32) {
-        PView<float> a = cur<float>(p), b = alt<float>(p);
-        k_cell_max_disp<float><<<grid_full(c->S, 256), 256, 0, s>>>(c->count, c->start, c->is_md, c->S, a.pos,
-                                                                   b.pos, a.species, p->d_max);
-    } else {
-        PView<double> a = cur<double>(p), b = alt<double>(p);
-        k_cell_max_disp<double><<<grid_full(c->S, 256), 256, 0, s>>>(c->count, c->start, c->is_md, c->S, a.pos,
-                                                                    b.pos, a.species, p->d_max);
-    }
+    RMPCD_CHECK_LAUNCH();
+    const int rc = sync();
+    if (rc) return rc;
+    const unsigned long long bits = *(volatile unsigned long long *)p->h_max;
+    double m;
+    memcpy(&m, &bits, 8);
+    *r = sqrt(m);
+    return RMPCD_OK;
+}
+
+template <typename R>
+static int max_disp_t(rmpcd_particles *p, double *r)
+{
+    const PView<R> a = cur<R>(p), b = alt<R>(p);
+    // eight blocks per SM: each block ends with an atomic on one counter
+    const int blocks = std::min(grid_for(p->N, 256), 8 * sm_count());
+    k_max_disp<R><<<blocks, 256, 0, stream()>>>(a.pos, b.pos, a.species, p->N, p->d_max + 1, p->h_max_dev);
+    return read_h_max(p, r);
+}
+
+template <typename R>
+static int cell_max_disp_t(rmpcd_cells *c, rmpcd_particles *p, double *r)
+{
+    const PView<R> a = cur<R>(p), b = alt<R>(p);
+    k_cell_max_disp<R><<<grid_full(c->S, 256), 256, 0, stream()>>>(c->count, c->start, c->is_md, c->S, a.pos, b.pos,
+                                                                  a.species, p->d_max + 1, p->h_max_dev);
+    return read_h_max(p, r);
+}
+
+template <typename R>
+static int zero3_t(rmpcd_particles *p, void *const a[3])
+{
+    k_zero3<R><<<grid_for(p->N, 256), 256, 0, stream()>>>(Vec3<R>{(R *)a[0], (R *)a[1], (R *)a[2]}, p->N);
     RMPCD_CHECK_LAUNCH();
     return RMPCD_OK;
+}
+
+template <typename R>
+static int copy3_t(rmpcd_particles *p, void *const a[3], void *const b[3])
+{
+    k_copy3<R><<<grid_for(p->N, 256), 256, 0, stream()>>>(Vec3<R>{(R *)a[0], (R *)a[1], (R *)a[2]},
+                                                          Vec3<R>{(R *)b[0], (R *)b[1], (R *)b[2]}, p->N);
+    RMPCD_CHECK_LAUNCH();
+    return RMPCD_OK;
+}
+
+static int copy3(rmpcd_particles *p, void *const a[3], void *const b[3])
+{
+    if (p->N == 0) return RMPCD_OK;
+    return p->precision == RMPCD_FP32 ? copy3_t<float>(p, a, b) : copy3_t<double>(p, a, b);
 }
 
 }  // namespace rmpcd
@@ -247,6 +315,7 @@ static void free_particles(rmpcd_particles *p)
     cudaFree(p->id_to_idx);
     cudaFree(p->gauss);
     cudaFree(p->d_max);
+    cudaFreeHost(p->h_max);
     cudaFree(p->d_sums);
     cudaFree(p->d_ints);
     cudaFree(p->stage);
@@ -374,6 +443,7 @@ int rmpcd_particles_init(rmpcd_particles **out, int Nmax, int n_species, const d
         free_particles(p);
         return fail(RMPCD_ERR_CUDA, "particle_system_t%%init: device allocation failed (N=%d)", Nmax);
     }
+    cudaMemsetAsync(p->d_max, 0, 64, st);
     for (int b = 0; b < 2; b++) {
         for (int k = 0; k < 3; k++) {
             cudaMemsetAsync(p->pos[b][k], 0, rb, st);
@@ -498,32 +568,21 @@ int rmpcd_particles_maximum_displacement(rmpcd_particles *p, double *r)
 {
     RMPCD_ARG(p && r, "null argument");
     PhaseTimer t("maximum disp");
-    cudaStream_t s = stream();
-    int rc0 = launch_max_disp(p);
-    if (rc0) return rc0;
-    unsigned long long bits = 0;
-    RMPCD_CUDA_TRY(cudaMemcpyAsync(&bits, p->d_max, 8, cudaMemcpyDeviceToHost, s));
-    int rc = sync();
+    *r = 0;
+    if (p->N == 0) return sync();
+    const int rc = ensure_h_max(p);
     if (rc) return rc;
-    double m;
-    memcpy(&m, &bits, 8);
-    *r = sqrt(m);
-    return RMPCD_OK;
+    return p->precision == RMPCD_FP32 ? max_disp_t<float>(p, r) : max_disp_t<double>(p, r);
 }
 
 int rmpcd_cell_maximum_displacement(rmpcd_cells *c, rmpcd_particles *p, double delta_t, double *r)
 {
     RMPCD_ARG(c && p && r, "null argument");
-    cudaStream_t s = stream();
-    int rc0 = launch_cell_max_disp(c, p);
-    if (rc0) return rc0;
-    unsigned long long bits = 0;
-    RMPCD_CUDA_TRY(cudaMemcpyAsync(&bits, p->d_max, 8, cudaMemcpyDeviceToHost, s));
-    int rc = sync();
+    int rc = ensure_h_max(p);
+    double a = 0;
+    if (!rc) rc = p->precision == RMPCD_FP32 ? cell_max_disp_t<float>(c, p, &a) : cell_max_disp_t<double>(c, p, &a);
     if (rc) return rc;
-    double m;
-    memcpy(&m, &bits, 8);
-    double a = sqrt(m), b = c->max_v * delta_t;
+    const double b = c->max_v * delta_t;
     *r = a > b ? a : b;
     return RMPCD_OK;
 }
@@ -618,9 +677,11 @@ int rmpcd_particles_switch_force(rmpcd_particles *p)
 int rmpcd_particles_zero_force(rmpcd_particles *p)
 {
     RMPCD_ARG(p, "null argument");
-    if (p->N > 0)
-        for (int k = 0; k < 3; k++)
-            RMPCD_CUDA_TRY(cudaMemsetAsync(p->force[p->cur][k], 0, (size_t)p->N * p->rsize, stream()));
+    if (p->N > 0) {
+        void *const *f = p->force[p->cur];
+        const int rc = p->precision == RMPCD_FP32 ? zero3_t<float>(p, f) : zero3_t<double>(p, f);
+        if (rc) return rc;
+    }
     p->force_zero = true;
     return RMPCD_OK;
 }
@@ -651,21 +712,15 @@ int rmpcd_particles_count_nonfinite(const rmpcd_particles *p, long long *n_bad)
 int rmpcd_particles_copy_pos_old(rmpcd_particles *p)
 {
     RMPCD_ARG(p, "null argument");
-    if (p->N > 0)
-        for (int k = 0; k < 3; k++)
-            RMPCD_CUDA_TRY(cudaMemcpyAsync(p->pos[1 - p->cur][k], p->pos[p->cur][k], (size_t)p->N * p->rsize,
-                                           cudaMemcpyDeviceToDevice, stream()));
-    return RMPCD_OK;
+    return copy3(p, p->pos[p->cur], p->pos[1 - p->cur]);
 }
 
 // force_old = force (programs/single_dimer_pbc.f90:295)
 int rmpcd_particles_copy_force_old(rmpcd_particles *p)
 {
     RMPCD_ARG(p, "null argument");
-    if (p->N > 0)
-        for (int k = 0; k < 3; k++)
-            RMPCD_CUDA_TRY(cudaMemcpyAsync(p->force_old[p->cur][k], p->force[p->cur][k], (size_t)p->N * p->rsize,
-                                           cudaMemcpyDeviceToDevice, stream()));
+    const int rc = copy3(p, p->force[p->cur], p->force_old[p->cur]);
+    if (rc) return rc;
     p->force_old_zero = p->force_zero;
     return RMPCD_OK;
 }
@@ -676,10 +731,7 @@ int rmpcd_particles_copy_pos_rattle(rmpcd_particles *p)
     if (p->N == 0) return RMPCD_OK;
     if (!p->pos_rattle[0])
         for (int k = 0; k < 3; k++) RMPCD_CUDA_TRY(cudaMalloc(&p->pos_rattle[k], (size_t)p->N * p->rsize));
-    for (int k = 0; k < 3; k++)
-        RMPCD_CUDA_TRY(cudaMemcpyAsync(p->pos_rattle[k], p->pos[p->cur][k], (size_t)p->N * p->rsize,
-                                       cudaMemcpyDeviceToDevice, stream()));
-    return RMPCD_OK;
+    return copy3(p, p->pos[p->cur], p->pos_rattle);
 }
 
 int rmpcd_particles_set_gauss(rmpcd_particles *p, const double *gauss)

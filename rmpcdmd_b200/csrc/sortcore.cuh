@@ -40,11 +40,6 @@ int sort_positions(rmpcd_cells *c, const rmpcd_particles *from, rmpcd_particles 
 // placement and a gather that moves force entries only where there are any;
 // cellmap (if given) receives the slot of every particle of the sorted arrays
 int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap);
-// maximum-displacement reductions into p->d_max (r^2 as ordered bits), no
-// synchronisation: maximum_displacement over all particles, and over the
-// particles of is_md cells (src/particle_system.f90:357-410)
-int launch_max_disp(rmpcd_particles *p);
-int launch_cell_max_disp(rmpcd_cells *c, rmpcd_particles *p);
 // compute_force_n2 of the colloids run right after compute_force, with the
 // colloid sums, on a second stream beside the solvent force application
 // (the two branches write disjoint arrays; each array sees the arithmetic

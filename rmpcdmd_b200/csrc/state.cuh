@@ -65,7 +65,11 @@ struct rmpcd_particles {
     int *perm = nullptr;             // N, source index of each sorted slot
     int *id_to_idx = nullptr;        // N, built on demand
     double *gauss = nullptr;         // injected normals (3*N) or null
-    unsigned long long *d_max = nullptr;  // max-reduction word
+    // reduction words: [0] a call's own, [1] [2] the displacement maximum and its
+    // block counter, zero between calls; h_max: where that maximum is written,
+    // mapped host memory
+    unsigned long long *d_max = nullptr;
+    unsigned long long *h_max = nullptr, *h_max_dev = nullptr;
     double *d_sums = nullptr;        // reduction scratch
     int sums_cap = 0;
     int *d_ints = nullptr;           // small integer scratch (64 ints)
