@@ -155,7 +155,6 @@ struct rmpcd_dimer_batch {
     // maximum_displacement's species >= 0 test and species need not be read
     bool read_species = true;
     int *resort = nullptr, *n_extra = nullptr;
-    int *tmp = nullptr;  // order_tile's scratch
     double *rattle[3] = {nullptr, nullptr, nullptr};
     double *vv_mass = nullptr;
     uint64_t *d_step = nullptr;
@@ -1750,13 +1749,13 @@ __global__ void __launch_bounds__(kBT) kb_perm(TileSet ts, const int *key, int *
 // kb_scan_reps), each cell's indices put in order on the way (order_tile).
 // Only particles with MD or PAST_MD set have force entries: they are moved and
 // zeroed behind, so the buffer that is not current holds none.  Flagged
-// particles are listed in flist; tmp is order_tile's scratch.
+// particles are listed in flist.
 constexpr int kOrderPerTile = kTile / kOrderSlots;
 
 template <typename R>
 __global__ void __launch_bounds__(kOrderThreads, 4)
     kb_order_gather(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, const int *count, const int *start, int *perm,
-                    int *tmp, int *flist, int *nf)
+                    int *flist, int *nf)
 {
     __shared__ OrderTile sh;
     for (int kt = blockIdx.x; kt < *ts.n * kOrderPerTile; kt += gridDim.x) {
@@ -1767,7 +1766,7 @@ __global__ void __launch_bounds__(kOrderThreads, 4)
         const PView<R> d = pick(v0, v1, rp.cur), s = pick(v1, v0, rp.cur);
         int a0, np;
         __syncthreads();  // the last tile's indices are read
-        const int *src = order_tile(sh, (int)s0, (int)min(s0 + kOrderSlots, t.end), count, start, perm, tmp, a0, np);
+        const int *src = order_tile(sh, (int)s0, (int)min(s0 + kOrderSlots, t.end), count, start, perm, d.id, a0, np);
         for (int q = threadIdx.x; q < np; q += kOrderThreads) {
             const int i = src[q], j = a0 + q;
             R px = s.pos.x[i], py = s.pos.y[i], pz = s.pos.z[i];
@@ -1938,7 +1937,7 @@ static void resort_launches(Batch *b, const int *flag, cudaStream_t st, int shif
     kb_scan_apply<<<gs, kBT, 0, st>>>(sts, b->count, b->tile_off, b->start, b->cursor);
     kb_perm<<<gp, kBT, 0, st>>>(pts, b->sol->key, b->cursor, b->sol->perm);
     kb_order_gather<R><<<resort_grid(b->n_stile * kOrderPerTile), kOrderThreads, 0, st>>>(
-        sts, b->rep, v0, v1, b->count, b->start, b->sol->perm, b->tmp, b->sol->key, b->nf);
+        sts, b->rep, v0, v1, b->count, b->start, b->sol->perm, b->sol->key, b->nf);
     kb_update_list<R><<<2 * b->R, kNlBlockThreads, nl_stage_bytes<R>(), st>>>(
         flag, b->rep, cv, v0, v1, b->count, b->start, b->stencil, b->n_stencil,
         b->prm.list_radius * b->prm.list_radius, b->lj_sc, b->Nmax, b->list, b->nn, b->is_md, b->is_reac,
@@ -2144,7 +2143,7 @@ static void free_batch(Batch *b)
     void *ptrs[] = {b->rep, b->ptile, b->stile, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, b->count,
                     b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->act, b->nl, b->nx,
                     b->aidx, b->next, b->mult, b->ent, b->over, b->terms, b->keys[0], b->keys[1], b->n_over, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
-                    b->n_extra, b->tmp, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
+                    b->n_extra, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
                     b->done, b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s,
                     b->n_all, b->any};
     for (void *q : ptrs) cudaFree(q);
@@ -2416,7 +2415,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
               !dalloc(&b->n_over, 4 * (size_t)R) &&
               !dalloc(&b->nf, R) && !dalloc(&b->s_free, R) && !dalloc(&b->adv, R) && !dalloc(&b->base, R) &&
               !dalloc(&b->fresh, R) && !dalloc(&b->resort, R) &&
-              !dalloc(&b->n_extra, R) && !dalloc(&b->tmp, off) &&
+              !dalloc(&b->n_extra, R) &&
               !dalloc(&b->rattle[0], 2 * (size_t)R) && !dalloc(&b->rattle[1], 2 * (size_t)R) &&
               !dalloc(&b->rattle[2], 2 * (size_t)R) && !dalloc(&b->vv_mass, 2 * (size_t)R) && !dalloc(&b->d_step, 1) &&
               !dalloc(&b->done, 1) && cudaStreamCreateWithFlags(&b->body, cudaStreamNonBlocking) == cudaSuccess &&

@@ -22,6 +22,7 @@
 //     The host reads the decision as soon as the kernel writes it, while the
 //     forces run; on a step that re-sorts the gated kernels return at once
 //     and the host issues the sort, then the forces.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -109,6 +110,10 @@ __device__ inline void stream_vel_gated(const PView<R> &v, long long i, int f, R
     }
 }
 
+// particles of a thread in flight in the catch-up (21 M particles FP32: 307 us
+// with one, 256 us with two, 279 us with four)
+constexpr int kCatchRounds = 2;
+
 // The catch-up of cell_md_pos then cell_md_vel with md_flag = .false.
 // (src/md.f90:79-102, :239-263) for every particle outside the MD cells
 // (cellmap: each particle's slot, from the last sort), fused with the key
@@ -122,46 +127,73 @@ __global__ void k_catch_up_key_count(const int *__restrict__ cellmap, const unsi
                                      PView<R> v, R dt, R dt_sq, Grid g, double e0, double e1, double e2,
                                      int *__restrict__ key, int *__restrict__ count)
 {
+    constexpr int U = kCatchRounds;
     const int lane = threadIdx.x & 31;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < N; base += stride) {
-        const long long i = base + threadIdx.x;
-        const bool ok = i < N;
-        int slot = -1;
-        if (ok) {
-            R x, y, z;
-            const bool catch_up = !is_md[cellmap[i]];
-            if (catch_up) {
-                const int f = v.flags[i];
-                moved_pos(v, i, f, dt, dt_sq, x, y, z);
-                stream_vel_gated(v, i, f, dt);
-            } else {
-                x = v.pos.x[i];
-                y = v.pos.y[i];
-                z = v.pos.z[i];
+    const long long stride = (long long)gridDim.x * blockDim.x * U;
+    for (long long base = ((long long)blockIdx.x * blockDim.x) * U + threadIdx.x; base - threadIdx.x < N; base += stride) {
+        R x[U], y[U], z[U], vx[U], vy[U], vz[U];
+        int f[U], slot[U];
+        bool catch_up[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long i = base + (long long)u * blockDim.x;
+            f[u] = 0;
+            slot[u] = -1;
+            if (i < N) {
+                slot[u] = cellmap[i];
+                f[u] = v.flags[i];
+                x[u] = v.pos.x[i];
+                y[u] = v.pos.y[i];
+                z[u] = v.pos.z[i];
+                vx[u] = v.vel.x[i];
+                vy[u] = v.vel.y[i];
+                vz[u] = v.vel.z[i];
             }
-            const int jx = floor_div_edge((double)x, e0), jy = floor_div_edge((double)y, e1),
-                      jz = floor_div_edge((double)z, e2);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) catch_up[u] = slot[u] >= 0 && !is_md[slot[u]];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const long long i = base + (long long)u * blockDim.x;
+            slot[u] = -1;
+            if (i >= N) continue;
+            if (catch_up[u]) {
+                R fx = 0, fy = 0, fz = 0;
+                if (f[u] & kForceFlags) {
+                    fx = v.force.x[i];
+                    fy = v.force.y[i];
+                    fz = v.force.z[i];
+                }
+                x[u] = x[u] + dt * vx[u] + dt_sq * fx;
+                y[u] = y[u] + dt * vy[u] + dt_sq * fy;
+                z[u] = z[u] + dt * vz[u] + dt_sq * fz;
+                stream_vel_gated(v, i, f[u], dt);
+            }
+            const int jx = floor_div_edge((double)x[u], e0), jy = floor_div_edge((double)y[u], e1),
+                      jz = floor_div_edge((double)z[u], e2);
             if (jx) {
                 v.ix[i] += jx;
-                x = x - (R)(jx * e0);
+                x[u] = x[u] - (R)(jx * e0);
             }
             if (jy) {
                 v.iy[i] += jy;
-                y = y - (R)(jy * e1);
+                y[u] = y[u] - (R)(jy * e1);
             }
             if (jz) {
                 v.iz[i] += jz;
-                z = z - (R)(jz * e2);
+                z[u] = z[u] - (R)(jz * e2);
             }
-            if (catch_up || jx) v.pos.x[i] = x;
-            if (catch_up || jy) v.pos.y[i] = y;
-            if (catch_up || jz) v.pos.z[i] = z;
-            slot = slot_of(g, (double)x, (double)y, (double)z);
-            key[i] = slot;
+            if (catch_up[u] || jx) v.pos.x[i] = x[u];
+            if (catch_up[u] || jy) v.pos.y[i] = y[u];
+            if (catch_up[u] || jz) v.pos.z[i] = z[u];
+            slot[u] = slot_of(g, (double)x[u], (double)y[u], (double)z[u]);
+            key[i] = slot[u];
         }
-        const unsigned peers = __match_any_sync(0xffffffffu, slot);
-        if (ok && lane == __ffs(peers) - 1) atomicAdd(count + slot, __popc(peers));
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const unsigned peers = __match_any_sync(0xffffffffu, slot[u]);
+            if (slot[u] >= 0 && lane == __ffs(peers) - 1) atomicAdd(count + slot[u], __popc(peers));
+        }
     }
 }
 
@@ -173,42 +205,6 @@ __global__ void k_fill_cellmap(const int *count, const int *start, int S, int *c
         const int s = (int)(q / kLanesPerCell), g = (int)(q % kLanesPerCell);
         for (int i = start[s] + g; i < start[s] + count[s]; i += kLanesPerCell) cellmap[i] = s;
     }
-}
-
-// cell_md_pos with md_flag = .true. (src/md.f90:79-102) over the listed MD
-// cells, eight lanes per cell, fused with cell_maximum_displacement over the
-// same cells (src/particle_system.f90:380-410): each new position is measured
-// against pos_old as it is written (the value that is stored); the squared
-// maximum goes to *out.  kVel: the previous MD step's cell_md_vel
-// (src/md.f90:239-263) runs first, particle by particle (nothing changes the
-// flags or forces between the two)
-template <typename R, bool kVel>
-__global__ void k_md_cells_pos_disp(const int *list, const int *n_list, const int *count, const int *start,
-                                    PView<R> v, Vec3<R> old, R dt, R dt_sq, unsigned long long *out)
-{
-    const long long n = (long long)*n_list * kLanesPerCell;
-    double m = 0;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int s = list[q / kLanesPerCell], g = (int)(q % kLanesPerCell);
-        const int a = start[s], c = count[s];
-        for (int i = a + g; i < a + c; i += kLanesPerCell) {
-            const int f = v.flags[i];
-            if (kVel) stream_vel_gated(v, i, f, dt);
-            R x, y, z;
-            moved_pos(v, i, f, dt, dt_sq, x, y, z);
-            v.pos.x[i] = x;
-            v.pos.y[i] = y;
-            v.pos.z[i] = z;
-            if (v.species[i] >= 0) {
-                const double d0 = (double)x - (double)old.x[i];
-                const double d1 = (double)y - (double)old.y[i];
-                const double d2 = (double)z - (double)old.z[i];
-                const double r = d0 * d0 + d1 * d1 + d2 * d2;
-                m = m > r ? m : r;
-            }
-        }
-    }
-    warp_max_into(out, m);
 }
 
 // cell_md_vel with md_flag = .true. (src/md.f90:239-263) over the listed MD
@@ -257,50 +253,61 @@ __device__ inline void zero_colloid_force(const Vec3<double> &cf, int nc)
     }
 }
 
-// the roll + clear below restricted to the listed MD cells.  Between two
-// sorts the list is fixed and compute_force flags only list entries, which
-// lie in MD cells; so once two rolls have run over every particle after a
-// sort (the first turns flags carried through the sort into PAST_MD, the
-// second clears them), no particle outside the MD cells has MD or PAST_MD
-// set or a non-zero force entry, and rolling the MD cells alone gives the
-// same flags and forces as rolling all N.
-template <typename R>
-__global__ void k_md_cells_roll_clear(const int *list, const int *n_list, const int *count, const int *start,
-                                      int *flags, Vec3<R> force, Vec3<double> cf, int nc, const int *gate)
-{
-    if (gate && *gate) return;
-    zero_colloid_force(cf, nc);
-    const long long n = (long long)*n_list * kLanesPerCell;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int s = list[q / kLanesPerCell], g = (int)(q % kLanesPerCell);
-        const int a = start[s], c = count[s];
-        for (int i = a + g; i < a + c; i += kLanesPerCell) {
-            const int f = flags[i];
-            if (f & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
-                force.x[i] = 0;
-                force.y[i] = 0;
-                force.z[i] = 0;
-                flag_roll_one(flags, i);
-            }
-        }
-    }
-}
-
 // zero_force of the solvent fused with the PAST_MD/MD roll: only entries of
 // particles with MD or PAST_MD set can be non-zero
 template <typename R>
-__global__ void k_roll_clear(int *flags, Vec3<R> force, long long N, Vec3<double> cf, int nc, const int *gate)
+__device__ inline void roll_clear_one(int *flags, const Vec3<R> &force, int i)
+{
+    const int f = flags[i];
+    if (f & kForceFlags) {
+        force.x[i] = 0;
+        force.y[i] = 0;
+        force.z[i] = 0;
+        flag_roll_one(flags, i);
+    }
+}
+
+// the roll over the listed MD cells and, for two rolls after a sort, over the
+// particles of `flagged` in other cells.  Between two sorts the list is fixed
+// and compute_force flags only list entries, which lie in MD cells, so these
+// are all flagged particles: those that the sort (or the start of the run)
+// found, until both their bits have gone, and those of the MD cells.  (Two rolls
+// over all 21 M particles of a 128^3 box took 43 us each, 5 times per 100 MD
+// steps; the MD cells alone take 5.)
+template <typename R>
+__global__ void k_md_cells_roll_clear(const int *list, const int *n_list, const int *count, const int *start,
+                                      const int *flagged, const int *n_flagged, const int *cellmap,
+                                      const unsigned char *is_md, int *flags, Vec3<R> force, Vec3<double> cf, int nc,
+                                      const int *gate)
 {
     if (gate && *gate) return;
     zero_colloid_force(cf, nc);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-        const int f = flags[i];
-        if (f & ((1 << MD_BIT) | (1 << PAST_MD_BIT))) {
-            force.x[i] = 0;
-            force.y[i] = 0;
-            force.z[i] = 0;
-            flag_roll_one(flags, i);
+    const long long step = (long long)gridDim.x * blockDim.x, q0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (flagged)
+        for (long long q = q0; q < *n_flagged; q += step) {
+            const int i = flagged[q];
+            if (!is_md[cellmap[i]]) roll_clear_one(flags, force, i);
         }
+    const long long n = (long long)*n_list * kLanesPerCell;
+    for (long long q = q0; q < n; q += step) {
+        const int s = list[q / kLanesPerCell], g = (int)(q % kLanesPerCell);
+        const int a = start[s], c = count[s];
+        for (int i = a + g; i < a + c; i += kLanesPerCell) roll_clear_one(flags, force, i);
+    }
+}
+
+// the flagged particles, in any order
+__global__ void k_list_flagged(const int *flags, int N, int *flagged, int *n_flagged)
+{
+    const int lane = threadIdx.x & 31;
+    for (long long base = (long long)blockIdx.x * blockDim.x; base < N; base += (long long)gridDim.x * blockDim.x) {
+        const long long i = base + threadIdx.x;
+        const bool on = i < N && (flags[i] & kForceFlags);
+        const unsigned b = __ballot_sync(0xffffffffu, on);
+        int k = 0;
+        if (lane == 0 && b) k = atomicAdd(n_flagged, __popc(b));
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (on) flagged[k + __popc(b & ((1u << lane) - 1u))] = (int)i;
     }
 }
 
@@ -317,7 +324,7 @@ __device__ inline void nc_resort_test(unsigned long long *so_bits, double co_sq,
     const int n = ctl[0] + 1;
     ctl[0] = n;
     const double delta_t = __dmul_rn(dt, (double)n);
-    const double a = sqrt(__longlong_as_double((long long)*so_bits));
+    const double a = sqrt(__longlong_as_double((long long)__ldcg(so_bits)));
     const double b = __dmul_rn(max_v, delta_t);
     const double so_max = a > b ? a : b;
     const double co_max = sqrt(co_sq);
@@ -329,34 +336,77 @@ __device__ inline void nc_resort_test(unsigned long long *so_bits, double co_sq,
     *so_bits = 0;  // cleared for the next MD step's position pass
 }
 
-// The colloid part of an MD step up to the re-sort test, one block: the
-// previous MD step's velocity half when due, the position half (the colloid
-// velocity Verlet of programs/n_colloids_pbc.f90:222-224, :248-249), the
-// colloids' largest displacement since the last sort (maximum_displacement,
-// src/particle_system.f90:357-378; a maximum, so the same in any order), then
-// the re-sort test.  Each colloid's updates are those of rmpcd_colloid_vv_vel
-// and rmpcd_colloid_vv_pos, which touch no other colloid.
-constexpr int kNcColloidThreads = 256;
+// An MD step up to the re-sort test, in one launch.
+// Solvent: cell_md_pos with md_flag = .true. (src/md.f90:79-102) over the listed
+// MD cells, eight lanes per cell, fused with cell_maximum_displacement over the
+// same cells (src/particle_system.f90:380-410): each new position is measured
+// against pos_old as it is written (the value that is stored); the squared
+// maximum goes to acc[0].  kVel: the previous MD step's cell_md_vel
+// (src/md.f90:239-263) runs first, particle by particle (nothing changes the
+// flags or forces between the two).
+// Colloids, by block 0 (the first to start, while the others are at the
+// solvent): the previous MD step's velocity half when due, the position half
+// (the colloid velocity Verlet of programs/n_colloids_pbc.f90:222-224, :248-249)
+// and their largest displacement since the last sort (maximum_displacement,
+// src/particle_system.f90:357-378).  Each colloid's updates are those of
+// rmpcd_colloid_vv_vel and rmpcd_colloid_vv_pos, which touch no other colloid.
+// The block that finishes last makes the re-sort test (acc[3]: blocks finished,
+// acc[4]: the colloids' maximum).  128^3 with 200 colloids, FP32: 19.9 us for
+// 17.4 and, in a kernel of their own after it, 4.0 us for the colloids.
+constexpr int kNcStepThreads = 256;
 
-template <bool kVel>
-__global__ void __launch_bounds__(kNcColloidThreads)
-    k_nc_colloid_begin(PView<double> c, Vec3<double> c_old, double mass, double dt,
-                       unsigned long long *so_bits, int *ctl, int *h_ctl, double max_v, double skin)
+template <typename R, bool kVel>
+__global__ void __launch_bounds__(kNcStepThreads)
+    k_nc_step_begin(const int *list, const int *n_list, const int *count, const int *start, PView<R> v, Vec3<R> old,
+                    R dt, R dt_sq, PView<double> c, Vec3<double> c_old, double mass, double c_dt,
+                    unsigned long long *acc, int *ctl, int *h_ctl, double max_v, double skin)
 {
-    __shared__ double s_m[kNcColloidThreads / 32];
-    double m = 0;
-    for (int i = threadIdx.x; i < c.N; i += blockDim.x) {
-        if (kVel) colloid_vv_vel_one(c, i, mass, dt);
-        colloid_vv_pos_one(c, i, mass, dt);
-        const double r = disp_sq_one(c.pos, c_old, c.species, i);
-        m = m > r ? m : r;
+    if (blockIdx.x == 0) {
+        __shared__ double s_m[kNcStepThreads / 32];
+        double m = 0;
+        for (int i = threadIdx.x; i < c.N; i += blockDim.x) {
+            if (kVel) colloid_vv_vel_one(c, i, mass, c_dt);
+            colloid_vv_pos_one(c, i, mass, c_dt);
+            const double r = disp_sq_one(c.pos, c_old, c.species, i);
+            m = m > r ? m : r;
+        }
+        m = warp_max(m);
+        if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < kNcStepThreads / 32; w++) m = m > s_m[w] ? m : s_m[w];
+            acc[4] = (unsigned long long)__double_as_longlong(m);
+        }
     }
-    m = warp_max(m);
-    if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = m;
+    const long long n = (long long)*n_list * kLanesPerCell;
+    double m = 0;
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
+        const int s = list[q / kLanesPerCell], g = (int)(q % kLanesPerCell);
+        const int a = start[s], cn = count[s];
+        for (int i = a + g; i < a + cn; i += kLanesPerCell) {
+            const int f = v.flags[i];
+            if (kVel) stream_vel_gated(v, i, f, dt);
+            R x, y, z;
+            moved_pos(v, i, f, dt, dt_sq, x, y, z);
+            v.pos.x[i] = x;
+            v.pos.y[i] = y;
+            v.pos.z[i] = z;
+            if (v.species[i] >= 0) {
+                const double d0 = (double)x - (double)old.x[i];
+                const double d1 = (double)y - (double)old.y[i];
+                const double d2 = (double)z - (double)old.z[i];
+                const double r = d0 * d0 + d1 * d1 + d2 * d2;
+                m = m > r ? m : r;
+            }
+        }
+    }
+    warp_max_into(acc, m);
+    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kNcColloidThreads / 32; w++) m = m > s_m[w] ? m : s_m[w];
-        nc_resort_test(so_bits, m, ctl, h_ctl, dt, max_v, skin);
+    if (threadIdx.x == 0 && atomicAdd(acc + 3, 1ull) == gridDim.x - 1) {
+        __threadfence();
+        acc[3] = 0;
+        nc_resort_test(acc, __longlong_as_double((long long)__ldcg(acc + 4)), ctl, h_ctl, c_dt, max_v, skin);
     }
 }
 
@@ -387,7 +437,11 @@ struct NcLoop {
     // forces beside the solvent force application)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    int full_rolls = 2;  // rolls over all N still due since the last sort
+    int full_rolls = 2;  // rolls that include `flagged` still due since the last sort
+    // the particles with MD or PAST_MD set at the last sort (or at the start) are
+    // listed in the solvent's key array, free from a sort's placement to the next
+    // sort's key pass
+    int *n_flagged = nullptr;  // their number (device)
     // replayed parts of an MD step, keyed by the buffers they use: part_a up
     // to the re-sort test, part_b the forces, and step = part_a then part_b
     // gated by the test's decision (the key's last entry: vel_due + 2 full)
@@ -407,6 +461,7 @@ struct NcLoop {
         cudaFree(md_list);
         cudaFree(n_md);
         cudaFree(cellmap);
+        cudaFree(n_flagged);
         cudaFree(ctl);
         if (h_ctl) cudaFreeHost(h_ctl);
         if (ev_step) cudaEventDestroy(ev_step);
@@ -460,6 +515,7 @@ static std::vector<unsigned long long> nc_signature(const rmpcd_particles *s, co
             add(p->flags[b]);
         }
         add(p->d_max);
+        add(p->key);
     }
     add(cells);
     v.push_back((unsigned long long)cells->S);
@@ -499,6 +555,7 @@ static int nc_alloc(NcLoop &L, int S, int N)
     if (cudaMalloc(&L.md_list, (size_t)(S > 0 ? S : 1) * sizeof(int)) != cudaSuccess ||
         cudaMalloc(&L.n_md, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&L.cellmap, (size_t)(N > 0 ? N : 1) * sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&L.n_flagged, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&L.ctl, 3 * sizeof(int)) != cudaSuccess ||
         cudaHostAlloc(&L.h_ctl, 2 * sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer(&L.h_ctl_dev, L.h_ctl, 0) != cudaSuccess ||
@@ -553,22 +610,22 @@ static int list_md_cells(NcLoop &L)
     return RMPCD_OK;
 }
 
-// cell_md_pos over the MD cells, after the previous MD step's cell_md_vel
-// when that is due, and their maximum displacement (into the solvent's d_max,
-// zero on entry: cleared when the loop starts and by each re-sort test)
+// the MD step up to the re-sort test, whose last block also writes the
+// decision to the host (the solvent's d_max is zero on entry: cleared when the
+// loop starts and by each test); vel_due: with the previous step's velocity halves
 template <typename R>
-static int md_cells_pos_disp_t(NcLoop &L, bool vel_due)
+static int step_begin_t(NcLoop &L, bool vel_due)
 {
-    cudaStream_t st = stream();
     const R dt = (R)L.dt, dt_sq = (R)(L.dt * L.dt / 2);
     const PView<R> v = cur<R>(L.s);
     const Vec3<R> old = alt<R>(L.s).pos;
-    if (vel_due)
-        k_md_cells_pos_disp<R, true><<<md_cells_grid(), 256, 0, st>>>(L.md_list, L.n_md, L.cells->count,
-                                                                     L.cells->start, v, old, dt, dt_sq, L.s->d_max);
-    else
-        k_md_cells_pos_disp<R, false><<<md_cells_grid(), 256, 0, st>>>(L.md_list, L.n_md, L.cells->count,
-                                                                      L.cells->start, v, old, dt, dt_sq, L.s->d_max);
+    const PView<double> c = cur<double>(L.c);
+    const Vec3<double> c_old = alt<double>(L.c).pos;
+    auto *kernel = vel_due ? k_nc_step_begin<R, true> : k_nc_step_begin<R, false>;
+    // one wave of blocks (46 registers): each ends with an atomic on one counter
+    kernel<<<sm_count() * 5, kNcStepThreads, 0, stream()>>>(
+        L.md_list, L.n_md, L.cells->count, L.cells->start, v, old, dt, dt_sq, c, c_old, L.prm->mass, L.dt, L.s->d_max,
+        L.ctl, L.h_ctl_dev, L.cells->max_v, L.prm->skin);
     RMPCD_CHECK_LAUNCH();
     return RMPCD_OK;
 }
@@ -588,15 +645,11 @@ static int roll_clear_t(NcLoop &L, const int *gate)
     PView<R> v = cur<R>(L.s);
     const Vec3<double> cf = cur<double>(L.c).force;
     const int nc = L.c->N;
-    if (L.full_rolls > 0) {
-        const long long n = L.s->N > nc ? L.s->N : nc;
-        k_roll_clear<R><<<grid_for(n > 0 ? n : 1, 256), 256, 0, stream()>>>(v.flags, v.force, L.s->N, cf, nc, gate);
-        L.full_rolls--;
-    } else {
-        k_md_cells_roll_clear<R><<<md_cells_grid(), 256, 0, stream()>>>(L.md_list, L.n_md, L.cells->count,
-                                                                        L.cells->start, v.flags, v.force, cf, nc,
-                                                                        gate);
-    }
+    const bool full = L.full_rolls > 0;
+    k_md_cells_roll_clear<R><<<md_cells_grid(), 256, 0, stream()>>>(
+        L.md_list, L.n_md, L.cells->count, L.cells->start, full ? L.s->key : nullptr, L.n_flagged, L.cellmap,
+        L.cells->is_md, v.flags, v.force, cf, nc, gate);
+    if (full) L.full_rolls--;
     RMPCD_CHECK_LAUNCH();
     L.c->force_zero = true;
     return RMPCD_OK;
@@ -612,7 +665,7 @@ static int catch_up_key_t(NcLoop &L, double dtl)
     cudaStream_t st = stream();
     RMPCD_CUDA_TRY(cudaMemsetAsync(c->count, 0, (size_t)c->S * sizeof(int), st));
     if (L.s->N > 0)
-        k_catch_up_key_count<R><<<grid_for(L.s->N, 256), 256, 0, st>>>(
+        k_catch_up_key_count<R><<<grid_for((L.s->N + kCatchRounds - 1) / kCatchRounds, 256), 256, 0, st>>>(
             L.cellmap, c->is_md, L.s->N, cur<R>(L.s), (R)dtl, (R)dt_sq, grid_of(c), c->edges[0], c->edges[1],
             c->edges[2], L.s->key, c->count);
     RMPCD_CHECK_LAUNCH();
@@ -630,24 +683,6 @@ static int md_cells_copy_pos_t(NcLoop &L)
 }
 
 #define NC_DISPATCH(L, fn) ((L).s->precision == RMPCD_FP32 ? fn<float>(L) : fn<double>(L))
-
-// the colloid part of the MD step and the re-sort test (the solvent's
-// maximum displacement over the MD cells was taken with its positions), whose
-// kernel also writes the decision to the host
-static int colloid_begin(NcLoop &L, bool vel_due)
-{
-    cudaStream_t st = stream();
-    const PView<double> c = cur<double>(L.c);
-    const Vec3<double> c_old = alt<double>(L.c).pos;
-    if (vel_due)
-        k_nc_colloid_begin<true><<<1, kNcColloidThreads, 0, st>>>(c, c_old, L.prm->mass, L.dt, L.s->d_max, L.ctl,
-                                                                  L.h_ctl_dev, L.cells->max_v, L.prm->skin);
-    else
-        k_nc_colloid_begin<false><<<1, kNcColloidThreads, 0, st>>>(c, c_old, L.prm->mass, L.dt, L.s->d_max, L.ctl,
-                                                                   L.h_ctl_dev, L.cells->max_v, L.prm->skin);
-    RMPCD_CHECK_LAUNCH();
-    return RMPCD_OK;
-}
 
 // the re-sort decision of the MD step, after a synchronisation of the stream
 static int read_resort(NcLoop &L, bool *resort)
@@ -691,7 +726,10 @@ static int catch_up_and_sort(NcLoop &L, bool full_pos_old)
     const double dtl = (L.st->t - L.st->last_sort) * L.dt;
     int rc = L.s->precision == RMPCD_FP32 ? catch_up_key_t<float>(L, dtl) : catch_up_key_t<double>(L, dtl);
     if (!rc) rc = rmpcd_apply_pbc(L.c, L.cells->edges);
-    if (!rc) rc = sort_keyed_flagged(L.cells, L.s, L.cellmap);  // the solvent's wrap and keys are done
+    if (!rc && cudaMemsetAsync(L.n_flagged, 0, sizeof(int), stream()) != cudaSuccess)
+        rc = fail(RMPCD_ERR_CUDA, "n_colloids sort: counter reset failed");
+    // the solvent's wrap and keys are done
+    if (!rc) rc = sort_keyed_flagged(L.cells, L.s, L.cellmap, L.s->key, L.n_flagged);
     // before the run's first two flag rolls an entry with PAST_MD may hold a
     // force of the caller's, which stays when the flag goes
     if (L.seq < 3) L.s->cur_force_gated = false;
@@ -711,10 +749,7 @@ static int catch_up_and_sort(NcLoop &L, bool full_pos_old)
 // and of the colloids, run first)
 static int issue_part_a(NcLoop &L, bool vel_due)
 {
-    int rc = L.s->precision == RMPCD_FP32 ? md_cells_pos_disp_t<float>(L, vel_due)
-                                          : md_cells_pos_disp_t<double>(L, vel_due);
-    if (!rc) rc = colloid_begin(L, vel_due);
-    return rc;
+    return L.s->precision == RMPCD_FP32 ? step_begin_t<float>(L, vel_due) : step_begin_t<double>(L, vel_due);
 }
 
 // md_loop after the re-sort test (programs/n_colloids_pbc.f90:243-254) up to
@@ -854,22 +889,35 @@ static int md_step(NcLoop &L, bool want_energy, bool vel_due)
 using namespace rmpcd;
 
 static bool g_nc_graphs = true;
-// the loop kept from the last call (scratch and captured graphs), and the
-// lock that one thread at a time holds while it runs on it
+// the loops kept from the last calls (scratch and captured graphs), latest
+// last, and the lock that one thread at a time holds while it runs on one.  A
+// program that runs several systems in turn finds each one's graphs again (three
+// systems of 128^3 FP32: 135 ms per ten intervals for 152 with one loop kept);
+// a kept loop holds 4 B per particle and per slot.
+constexpr size_t kNcKept = 4;
 static std::mutex g_nc_mutex;
-static NcLoop *g_nc_loop = nullptr;
+// (never destroyed: at exit the device is gone before it would be)
+static std::vector<std::unique_ptr<NcLoop>> &g_nc_loops = *new std::vector<std::unique_ptr<NcLoop>>;
+
+// drops the kept loops that `which` selects
+template <typename F>
+static void drop_loops(F which)
+{
+    bool synced = false;
+    for (size_t k = g_nc_loops.size(); k-- > 0;) {
+        if (!which(*g_nc_loops[k])) continue;
+        if (!synced) cudaStreamSynchronize(stream());
+        synced = true;
+        g_nc_loops.erase(g_nc_loops.begin() + (long)k);
+    }
+}
 
 namespace rmpcd {
 
 void ncolloids_forget(const void *handle)
 {
     std::lock_guard<std::mutex> lk(g_nc_mutex);
-    NcLoop *L = g_nc_loop;
-    if (L && (handle == L->s || handle == L->c || handle == L->cells || handle == L->nl)) {
-        cudaStreamSynchronize(stream());
-        delete L;
-        g_nc_loop = nullptr;
-    }
+    drop_loops([&](const NcLoop &L) { return handle == L.s || handle == L.c || handle == L.cells || handle == L.nl; });
 }
 
 }  // namespace rmpcd
@@ -891,9 +939,9 @@ extern "C" int rmpcd_ncolloids_run(rmpcd_particles *solvent, rmpcd_particles *co
     RMPCD_ARG(n_intervals >= 0 && params->N_MD >= 1 && params->tau > 0, "n_intervals >= 0, N_MD >= 1, tau > 0");
     RMPCD_ARG(!thermostat || T, "a thermostatted run needs the temperatures T");
     RMPCD_ARG(colloids->precision == RMPCD_FP64, "colloids must be FP64");
-    // the loop of the previous call is reused (scratch and graphs) when its
-    // signature matches; a call that finds it in use by another thread runs
-    // on a loop of its own
+    // a kept loop is used again (scratch and graphs) when its signature
+    // matches; a call that finds the loops in use by another thread runs on a
+    // loop of its own
     std::unique_lock<std::mutex> lk(g_nc_mutex, std::try_to_lock);
     std::unique_ptr<NcLoop> own;
     NcLoop *Lp = nullptr;
@@ -901,12 +949,14 @@ extern "C" int rmpcd_ncolloids_run(rmpcd_particles *solvent, rmpcd_particles *co
     const bool keep = lk.owns_lock() && g_nc_graphs;
     if (keep) {
         sig = nc_signature(solvent, colloids, cells, nl, solvent_colloid, colloid_colloid, params);
-        if (g_nc_loop && g_nc_loop->sig == sig) {
-            Lp = g_nc_loop;
-        } else if (g_nc_loop) {
-            cudaStreamSynchronize(stream());
-            delete g_nc_loop;
-            g_nc_loop = nullptr;
+        for (size_t k = 0; k < g_nc_loops.size() && !Lp; k++)
+            if (g_nc_loops[k]->sig == sig) {
+                std::rotate(g_nc_loops.begin() + (long)k, g_nc_loops.begin() + (long)k + 1, g_nc_loops.end());
+                Lp = g_nc_loops.back().get();
+            }
+        if (!Lp && g_nc_loops.size() == kNcKept) {
+            const NcLoop *oldest = g_nc_loops.front().get();
+            drop_loops([&](const NcLoop &L) { return &L == oldest; });
         }
     }
     if (!Lp) {
@@ -939,6 +989,11 @@ extern "C" int rmpcd_ncolloids_run(rmpcd_particles *solvent, rmpcd_particles *co
     ((volatile int *)L.h_ctl)[0] = 0;
     k_nc_set_since<<<1, 1, 0, stream()>>>(L.ctl, state->t - state->last_sort);
     RMPCD_CUDA_TRY(cudaMemsetAsync(solvent->d_max, 0, 8, stream()));
+    RMPCD_CUDA_TRY(cudaMemsetAsync(L.n_flagged, 0, sizeof(int), stream()));
+    if (solvent->N > 0)
+        k_list_flagged<<<grid_for(solvent->N, 256), 256, 0, stream()>>>(solvent->flags[solvent->cur], solvent->N,
+                                                                       solvent->key, L.n_flagged);
+    RMPCD_CHECK_LAUNCH();
     int rc0 = list_md_cells(L);
     for (int k = 0; !rc0 && k < n_intervals; k++) {
         const int i = first_interval + k;
@@ -961,15 +1016,12 @@ extern "C" int rmpcd_ncolloids_run(rmpcd_particles *solvent, rmpcd_particles *co
     if (keep) {
         if (rc0) {
             // an error drops the kept loop
-            if (Lp == g_nc_loop) {
-                delete g_nc_loop;
-                g_nc_loop = nullptr;
-            }
+            drop_loops([&](const NcLoop &L) { return &L == Lp; });
         } else if (own) {
             // the force scratch may have been allocated by this call: the
             // signature is taken again before the loop is kept
             L.sig = nc_signature(solvent, colloids, cells, nl, solvent_colloid, colloid_colloid, params);
-            g_nc_loop = own.release();
+            g_nc_loops.push_back(std::move(own));
         }
     }
     if (rc0) return rc0;

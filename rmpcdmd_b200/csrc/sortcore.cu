@@ -108,15 +108,15 @@ __global__ void k_segsort_big(const int *__restrict__ start, const int *__restri
 // not written (128^3 FP32 colloid run: 165 -> 160 ms
 // with the order taken into the gather).
 template <typename R>
-__global__ void __launch_bounds__(kOrderThreads, 4)
+__global__ void __launch_bounds__(kOrderThreads, 6)
     k_order_gather(PView<R> s, PView<R> d, const int *__restrict__ count, const int *__restrict__ start, int S,
-                   int *perm, int *tmp, int with_force, int with_force_old, int gated)
+                   int *perm, int with_force, int with_force_old, int gated, int *flagged, int *n_flagged)
 {
     __shared__ OrderTile sh;
     const int fmask = (1 << MD_BIT) | (1 << PAST_MD_BIT);
     const int s0 = blockIdx.x * kOrderSlots;
     int a0, np;
-    const int *src = order_tile(sh, s0, min(s0 + kOrderSlots, S), count, start, perm, tmp, a0, np);
+    const int *src = order_tile(sh, s0, min(s0 + kOrderSlots, S), count, start, perm, d.id, a0, np);
     for (int q = threadIdx.x; q < np; q += kOrderThreads) {
         const int i = src[q], j = a0 + q;
         // all loads first: twelve independent gathers in flight per thread
@@ -136,7 +136,16 @@ __global__ void __launch_bounds__(kOrderThreads, 4)
         d.id[j] = id;
         d.species[j] = sp;
         d.flags[j] = fl;
-        if (gated && !(fl & fmask)) continue;
+        if (gated) {
+            const unsigned act = __activemask(), b = __ballot_sync(act, (fl & fmask) != 0);
+            if (!(fl & fmask)) continue;
+            if (flagged) {
+                const int lane = threadIdx.x & 31, lead = __ffs(b) - 1;
+                int k = 0;
+                if (lane == lead) k = atomicAdd(n_flagged, __popc(b));
+                flagged[__shfl_sync(b, k, lead) + __popc(b & lanemask_lt())] = j;
+            }
+        }
         if (with_force) {
             d.force.x[j] = s.force.x[i];
             d.force.y[j] = s.force.y[i];
@@ -203,7 +212,8 @@ int sort_perm_segments(rmpcd_cells *c, rmpcd_particles *p)
 }
 
 template <typename R>
-static int gather_t(rmpcd_cells *c, rmpcd_particles *p, bool gated = false)
+static int gather_t(rmpcd_cells *c, rmpcd_particles *p, bool gated = false, int *flagged = nullptr,
+                    int *n_flagged = nullptr)
 {
     cudaStream_t st = stream();
     const int to = 1 - p->cur;
@@ -217,8 +227,8 @@ static int gather_t(rmpcd_cells *c, rmpcd_particles *p, bool gated = false)
             }
         }
         k_order_gather<R><<<grid_full(c->S, kOrderSlots), kOrderThreads, 0, st>>>(
-            cur<R>(p), alt<R>(p), c->count, c->start, c->S, p->perm, p->key, p->force_zero ? 0 : 1,
-            p->force_old_zero ? 0 : 1, gated ? 1 : 0);
+            cur<R>(p), alt<R>(p), c->count, c->start, c->S, p->perm, p->force_zero ? 0 : 1,
+            p->force_old_zero ? 0 : 1, gated ? 1 : 0, flagged, n_flagged);
         RMPCD_CHECK_LAUNCH();
     }
     p->alt_force_clean = gated && p->cur_force_gated;
@@ -248,7 +258,7 @@ int gather_all(rmpcd_cells *c, rmpcd_particles *p)
 }
 
 template <typename R>
-static int sort_keyed_flagged_t(rmpcd_cells *c, rmpcd_particles *p, int *cellmap)
+static int sort_keyed_flagged_t(rmpcd_cells *c, rmpcd_particles *p, int *cellmap, int *flagged, int *n_flagged)
 {
     {
         PhaseTimer t("count");
@@ -258,13 +268,13 @@ static int sort_keyed_flagged_t(rmpcd_cells *c, rmpcd_particles *p, int *cellmap
     PhaseTimer t("sort");
     int rc = build_perm_unsorted(c, p, cellmap);
     if (rc) return rc;
-    return gather_t<R>(c, p, true);
+    return gather_t<R>(c, p, true, flagged, n_flagged);
 }
 
-int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap)
+int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap, int *flagged, int *n_flagged)
 {
-    if (p->precision == RMPCD_FP32) return sort_keyed_flagged_t<float>(c, p, cellmap);
-    return sort_keyed_flagged_t<double>(c, p, cellmap);
+    if (p->precision == RMPCD_FP32) return sort_keyed_flagged_t<float>(c, p, cellmap, flagged, n_flagged);
+    return sort_keyed_flagged_t<double>(c, p, cellmap, flagged, n_flagged);
 }
 
 // cell_system_t%sort_particles (src/cell_system.f90:131-151): the positions

@@ -38,8 +38,10 @@ int sort_positions(rmpcd_cells *c, const rmpcd_particles *from, rmpcd_particles 
 // which a particle with neither MD nor PAST_MD set has zero force and
 // force_old (the state compute_force and its flag roll maintain): scan,
 // placement and a gather that moves force entries only where there are any;
-// cellmap (if given) receives the slot of every particle of the sorted arrays
-int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap);
+// cellmap receives the slot of every particle of the sorted arrays, flagged (N
+// entries) their indices that have MD or PAST_MD set, counted in *n_flagged
+// (zero on entry)
+int sort_keyed_flagged(rmpcd_cells *c, rmpcd_particles *p, int *cellmap, int *flagged, int *n_flagged);
 // compute_force_n2 of the colloids run right after compute_force, with the
 // colloid sums, on a second stream beside the solvent force application
 // (the two branches write disjoint arrays; each array sees the arithmetic

@@ -80,7 +80,8 @@ __device__ inline void block_merge_sort(int *a, int *b, int n)
 // Orders slots [s0, s1), s1 - s0 <= kOrderSlots, by a block of kOrderThreads;
 // returns the tile's np ordered source indices, whose places start at a0.  A
 // tile of more than kOrderCap particles is ordered in perm itself (tmp: scratch
-// of the extent of perm).  Ends with a barrier; the caller puts one between
+// of the extent of perm, used at the tile's own places only; a gather passes
+// its target's ids, which it writes afterwards).  Ends with a barrier; the caller puts one between
 // its last use of the result and the next tile.
 __device__ inline const int *order_tile(OrderTile &sh, int s0, int s1, const int *__restrict__ count,
                                         const int *__restrict__ start, int *perm, int *tmp, int &a0, int &np)

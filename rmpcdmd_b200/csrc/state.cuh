@@ -66,7 +66,8 @@ struct rmpcd_particles {
     int *id_to_idx = nullptr;        // N, built on demand
     double *gauss = nullptr;         // injected normals (3*N) or null
     // reduction words: [0] a call's own, [1] [2] the displacement maximum and its
-    // block counter, zero between calls; h_max: where that maximum is written,
+    // block counter, zero between calls, [3] [4] the n_colloids step's block
+    // counter, zero between steps, and colloid maximum; h_max: where that maximum is written,
     // mapped host memory
     unsigned long long *d_max = nullptr;
     unsigned long long *h_max = nullptr, *h_max_dev = nullptr;
