@@ -198,12 +198,16 @@ __device__ __forceinline__ void bucket_means(BucketTile<float, S> &sh)
         sz += __shfl_xor_sync(0xffffffffu, sz, o);
         n_eff += __shfl_xor_sync(0xffffffffu, n_eff, o);
     }
-    if (c < S::kSlots && g == 0) {
-        sh.spin[c] = n_eff > 1;
+    if (c < S::kSlots && g < 3) {
+        if (g == 0) sh.spin[c] = n_eff > 1;
         if (n_eff > 1) {
-            sh.mat[c][3] = fixed_mean(sx, n_eff);
-            sh.mat[c][7] = fixed_mean(sy, n_eff);
-            sh.mat[c][11] = fixed_mean(sz, n_eff);
+            if constexpr (G >= 3) {  // a lane per component divides
+                sh.mat[c][4 * g + 3] = fixed_mean(g == 0 ? sx : (g == 1 ? sy : sz), n_eff);
+            } else if (g == 0) {
+                sh.mat[c][3] = fixed_mean(sx, n_eff);
+                sh.mat[c][7] = fixed_mean(sy, n_eff);
+                sh.mat[c][11] = fixed_mean(sz, n_eff);
+            }
         }
     }
 }
@@ -479,8 +483,8 @@ __device__ __forceinline__ void bucket_rank(BucketTile<double, S> &sh, int np)
 }
 
 // Bound by the round trips of each particle (cell table, counting atomic), the
-// load/store pipe (half of its cycles at 64^3 FP32) and issue (43 %), not by HBM
-// (2.6 TB/s at 128^3), so occupancy decides: one particle per thread in flight,
+// load/store pipe (69 % of its cycles at 96^3 FP32) and issue (66 %), not by HBM
+// (3.3 TB/s at 128^3), so occupancy decides: one particle per thread in flight,
 // 40 registers, 48 warps per SM (two per thread with 32 warps: 128^3 FP32 566 us
 // for 531).  With the cell's collision on one thread per cell, copies by cp.async
 // and the moved records put back in shared memory, 64^3 FP32 took 94 us for 78,

@@ -690,7 +690,7 @@ template <typename R>
 struct Shapes;
 template <>
 struct Shapes<float> {
-    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<32, 480, 12, 128>>(),
+    static constexpr ShapeEntry<float> list[] = {entry<float, Shape<24, 352, 16, 96>>(),
                                                   entry<float, Shape<16, 256, 6, 256>>(),
                                                   entry<float, Shape<72, 912, 6, 256>>()};
     static constexpr int by_wave[] = {1, 0, 2};  // by the cells that one wave of blocks holds
@@ -728,11 +728,11 @@ static double mean_occupancy(const rmpcd_particles *p, const rmpcd_cells *c)
 // tiles all run at once; many small blocks, with few warps waiting at each
 // barrier, are best for a large box; and a box just above one wave of those
 // takes a wider tile that fits.  us per interval (slots x blocks per SM x
-// threads): 16^3 FP32 9.3 (16 x 6 x 256), 13.9 (32 x 12 x 128), FP64 9.4 (16 x 5
-// x 256), 13.4 (24 x 8 x 128); 24^3 FP32 12.1, 14.6, FP64 16.4, 15.1; 32^3 FP32
-// 21.0, 16.3, FP64 25.2, 25.7; 61,500 cells FP32 27.2 (32 x 12 x 128), 23.1 (72 x
-// 6 x 256); 128^3 FP32 531 (32 x 12 x 128), 545 (72 x 6 x 256), 552 (96 x 5 x
-// 256), FP64 931 (24 x 8 x 128), 963 (40 x 5 x 256), 989 (48 x 4 x 256).
+// threads): 16^3 FP32 9.3 (16 x 6 x 256), 12.7 (24 x 16 x 96), FP64 9.4 (16 x 5 x
+// 256), 13.4 (24 x 8 x 128); 24^3 FP32 12.2, 14.3, FP64 16.4, 15.1; 32^3 FP32
+// 20.6, 15.8, FP64 25.2, 25.7; 61,500 cells FP32 25.5 (24 x 16 x 96), 23.1 (72 x 6
+// x 256); 128^3 FP32 521 (24 x 16 x 96), 531 (32 x 12 x 128), 546 (72 x 6 x 256),
+// FP64 931 (24 x 8 x 128), 963 (40 x 5 x 256), 989 (48 x 4 x 256).
 template <typename R>
 static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c)
 {
@@ -804,6 +804,10 @@ static int ensure_bucket_map(rmpcd_cells *c)
     return RMPCD_OK;
 }
 
+// allocations up to this size do not ask how much memory is free, which takes
+// as long as the allocation itself
+constexpr size_t kAskBytes = 256u << 20;
+
 // The bucket arrays (one allocation): two grids of n_rec * cap records, pools
 // of N records and their links, list heads of three grids and the counters.
 // *ok = false when they would take more than a quarter of the free memory (the
@@ -815,10 +819,12 @@ static int ensure_buckets(rmpcd_particles *p, int S, int n_rec, int cap, bool *o
     const size_t bytes = 2 * ((size_t)n_rec * cap + p->N) * B + 2 * (size_t)p->N * 4 + (3 * (size_t)S + 6) * 4;
     *ok = true;
     if (p->bkt_bytes >= bytes) return RMPCD_OK;
-    size_t free_bytes = 0, total = 0;
-    RMPCD_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total));
-    *ok = bytes <= (free_bytes + p->bkt_bytes) / 4;
-    if (!*ok) return RMPCD_OK;
+    if (bytes > kAskBytes) {
+        size_t free_bytes = 0, total = 0;
+        RMPCD_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total));
+        *ok = bytes <= (free_bytes + p->bkt_bytes) / 4;
+        if (!*ok) return RMPCD_OK;
+    }
     if (p->buckets) RMPCD_CUDA_TRY(cudaStreamSynchronize(stream()));
     cudaFree(p->buckets);
     p->buckets = nullptr;
@@ -1058,8 +1064,8 @@ static int bulk_run_fused(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, doub
 // not hold the mean occupancy with 5 standard deviations to spare (from density
 // 11 on; over-full tiles are slow) or there is too little memory: the gather.
 // us per interval (buckets, gather): 16^3 FP32 9.3, 20.7, FP64 9.4, 22.3; 32^3
-// FP32 16.3, 31.9, FP64 25.7, 44; 64^3 FP32 77.7, 107, FP64 129, 173; 128^3 FP32
-// 531, 682, FP64 931, 1153.
+// FP32 15.8, 31.9, FP64 25.7, 44; 64^3 FP32 75.7, 107, FP64 129, 173; 128^3 FP32
+// 521, 682, FP64 931, 1153.
 template <typename R>
 static int bulk_run_t(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double tau, int has_alpha, double alpha,
                       int n_intervals)
