@@ -77,6 +77,19 @@ __device__ inline void block_merge_sort(int *a, int *b, int n)
     block_merge_sort(a, b, n, [](int v) { return v; });
 }
 
+// The cells of a tile of more than kOrderCap particles, in place (tmp: scratch
+// of the same extent); n: this thread's cell.  A function of its own, so that
+// the gathers keep their registers for the tiles that there are.
+static __device__ __noinline__ void order_dense(const OrderTile &sh, int cells, int n, int *perm, int *tmp)
+{
+    __syncthreads();
+    if (n > 1 && n <= kOrderSmall) sort_segment(perm + sh.cstart[threadIdx.x], n);
+    __syncthreads();
+    for (int c = 0; c < cells; c++)
+        if (sh.ccount[c] > kOrderSmall) block_merge_sort(perm + sh.cstart[c], tmp + sh.cstart[c], sh.ccount[c]);
+    __syncthreads();
+}
+
 // Orders slots [s0, s1), s1 - s0 <= kOrderSlots, by a block of kOrderThreads;
 // returns the tile's np ordered source indices, whose places start at a0.  A
 // tile of more than kOrderCap particles is ordered in perm itself (tmp: scratch
@@ -113,12 +126,7 @@ __device__ inline const int *order_tile(OrderTile &sh, int s0, int s1, const int
         __syncthreads();
         return sh.idx;
     }
-    if (n > 1 && n <= kOrderSmall) sort_segment(perm + a, n);
-    __syncthreads();
-    for (int c = 0; c < s1 - s0; c++)
-        if (sh.ccount[c] > kOrderSmall)
-            block_merge_sort(perm + a0 + sh.cstart[c], tmp + a0 + sh.cstart[c], sh.ccount[c]);
-    __syncthreads();
+    order_dense(sh, s1 - s0, n, perm + a0, tmp + a0);
     return perm + a0;
 }
 
