@@ -412,10 +412,9 @@ int rmpcd_bulk_autotune(const int L[3], int precision, double tau, int n_interva
  * one; the loop state (MD step counters, re-sort count, the energies e1, e2
  * of each interval's last MD step) is carried in *state.  The call keeps its
  * scratch (about 4 B per slot and 4 B per solvent particle) and its captured
- * MD-step graphs for the next call, and reuses them while the handles, their
- * device arrays, the box, the LJ tables and tau, N_MD, skin and mass are the
- * same;
- * other arguments make it rebuild them.  A call made while another thread is
+ * MD-step graphs, those of the last four systems, and reuses them while the
+ * handles, their device arrays, the box, the LJ tables and tau, N_MD, skin and
+ * mass are the same; other arguments make it build others.  A call made while another thread is
  * inside this function works with scratch of its own.  No module counterpart
  * in the reference. */
 typedef struct rmpcd_ncolloids_params {
@@ -499,7 +498,7 @@ int rmpcd_dimer_batch_info(const rmpcd_dimer_batch *batch, int *n_replicas, long
  * blocks_per_sm = 1), the list entries per thread of the kernels that list that
  * solvent, and colloid_block_first = 1 (the colloids have warps of their own).
  * Every shape gives the same results bit for bit.  A batch starts on
- * 1024-particle tiles (smaller when that gives fewer than ~2 tiles per SM), 16
+ * 4096-particle tiles (smaller when that gives fewer than ~2 tiles per SM), 16
  * warps and one list entry per thread. */
 int rmpcd_dimer_batch_shapes(int precision, int *n_shapes);
 int rmpcd_dimer_batch_shape_info(int precision, int shape, int *particles_per_tile, int *per_thread_begin,

@@ -2347,12 +2347,15 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     b->ms.n = col[0]->n_species;
     for (int s = 0; s < RMPCD_MAX_SPECIES; s++) b->ms.m[s] = col[0]->mass[s];
     // replica layout and tiles
-    // default shape: 512 threads for a replica's MD steps and 1024-particle tiles, smaller only for batches too small to give ~2 tiles
-    // per SM: each tile's block is one round trip to DRAM, so fewer, fuller
-    // tiles beat more blocks; rmpcd_dimer_batch_autotune times the others
+    // default shape: 512 threads for a replica's MD steps and the largest particle
+    // tiles that give ~2 per SM: each tile's block is a chain of round trips, so
+    // fewer, fuller tiles beat more blocks (ms per interval with tiles of 256,
+    // 512, 1024, 2048, 4096: one 96^3 dimer FP32 3.3, 2.6, 2.3, 2.1, 2.1; 512
+    // replicas FP32 43.8, 36.0, 32.2, 30.7, 30.1; one 32^3 dimer FP64 0.88, 0.88,
+    // 0.87, 0.90, 0.92); rmpcd_dimer_batch_autotune times the others
     long long n_total = 0;
     for (int r = 0; r < R; r++) n_total += sol[r]->N;
-    int tile_k = 2;  // kPTiles[2] = 1024
+    int tile_k = kNPTiles - 1;
     while (tile_k > 0 && n_total / kPTiles[tile_k] < 2LL * sm_count()) tile_k--;
     b->shape = tile_k;
     long long cap_p = 0;
