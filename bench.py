@@ -209,12 +209,12 @@ def roofline(N, S, precision, phase, peak, peak_kind):
 # single_dimer_pbc configurations (MD step = tau / N_MD = 0.01)
 DIMER_N_MD = 100
 DIMER_LIST_CAPACITY = 4000
-# HBM bytes per solvent particle and MD step of the two streaming kernels of
-# the dimer engine (step begin: flags, pos r/w, vel, pos_old -- species only
-# for a batch created with a negative species; step end: flags, plus in the
-# FP64 form every velocity, in the FP32 form only those of particles with a
-# force; force entries are touched only for flagged particles)
-DIMER_BYTES_PER_MD_STEP = {32: 56, 64: 128}
+# HBM bytes per solvent particle and interval that the dimer engine cannot do
+# without (only particles near the beads take part in the MD steps): one sort
+# (advance: pos r/w, vel, key; placement: key, index; gather: index, every field
+# r/w), the classification's velocities, the collision's (r/w) with species, and
+# refuel's positions and species
+DIMER_BYTES_PER_INTERVAL = {32: 40 + 8 + 100 + 12 + 28 + 16, 64: 76 + 8 + 148 + 24 + 52 + 28}
 
 
 def dimer_boxes_batched(n=512, seed=2024):
@@ -260,14 +260,15 @@ def dimer_time(rm, dimers, n_intervals, use_graph=True, tuned=None):
 def dimer_entry(N, ms, n_intervals, precision, peak, peak_kind, extra=None):
     md_steps = n_intervals * DIMER_N_MD
     secs = ms * 1e-3
-    alg = DIMER_BYTES_PER_MD_STEP[precision] * N * md_steps
+    alg = DIMER_BYTES_PER_INTERVAL[precision] * N * n_intervals
     achieved = alg / secs / 1e9
     out = {"value": N * md_steps / secs, "us_per_md_step": round(ms * 1e3 / md_steps, 2), "intervals": n_intervals,
            "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind,
                         "unit": "GB/s", "frac": round(achieved / peak, 4),
-                        "algorithmic_bytes_per_particle_md_step": DIMER_BYTES_PER_MD_STEP[precision],
-                        "note": "streaming bytes of the MD step over the whole interval time (sort, list and "
-                                "collision included in the time only)"}}
+                        "algorithmic_bytes_per_particle_interval": DIMER_BYTES_PER_INTERVAL[precision],
+                        "note": "bytes of one sort, the collision and refuel over the whole interval time (the MD "
+                                "steps of the particles near the beads, early sorts and list included in the time "
+                                "only)"}}
     if extra is not None:
         out["n_extra_sorting"] = extra
     return out
