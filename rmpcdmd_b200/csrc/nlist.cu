@@ -502,7 +502,10 @@ int compute_force_impl(rmpcd_particles *ps1, rmpcd_particles *ps2, rmpcd_nlist *
     if (C > 0) {
         PView<double> cv = cur<double>(ps1);
         LJDev ld = lj_dev(lj);
-        int gx = (nl->Nmax + 255) / 256;
+        // room for two entries per thread: a list fills part of its capacity, and
+        // blocks without entries take their time too (200 colloids at 128^3, pair
+        // forces + solvent forces: 17.2 us with one entry, 15.4 with two, 16.8 with four)
+        int gx = (nl->Nmax + 511) / 512;
         if (gx > 64) gx = 64;
         dim3 grid(gx, C);
         // duplicates inside one list exist only when the stencil wraps the box
