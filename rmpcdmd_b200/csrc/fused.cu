@@ -670,7 +670,10 @@ __global__ void k_rec_gather_to_soa(const unsigned char *rec, const int *perm, P
 
 namespace rmpcd {
 
-// the shapes a precision can run with, and the one in use
+// the shapes a precision can run with, and the one in use.  pick_shape takes those
+// of by_wave; the others are there for rmpcd_bulk_set_shape and rmpcd_bulk_autotune
+// (us per interval at 96^3 FP32: 229.8 by shape 0, 227.6, 233.5, 233.1 by shapes 3,
+// 4, 5; 128^3 FP64: 871, 928, 966, 927, 1002 by shapes 0, 2, 3, 4, 5)
 template <typename R>
 struct ShapeEntry {
     void (*interval)(BucketArgs<R>);
@@ -692,13 +695,20 @@ template <>
 struct Shapes<float> {
     static constexpr ShapeEntry<float> list[] = {entry<float, Shape<24, 352, 16, 96>>(),
                                                   entry<float, Shape<16, 256, 6, 256>>(),
-                                                  entry<float, Shape<72, 912, 6, 256>>()};
+                                                  entry<float, Shape<72, 912, 6, 256>>(),
+                                                  entry<float, Shape<32, 480, 12, 128>>(),
+                                                  entry<float, Shape<48, 640, 8, 192>>(),
+                                                  entry<float, Shape<64, 832, 6, 256>>()};
     static constexpr int by_wave[] = {1, 0, 2};  // by the cells that one wave of blocks holds
 };
 template <>
 struct Shapes<double> {
     static constexpr ShapeEntry<double> list[] = {entry<double, Shape<24, 352, 8, 128>>(),
-                                                   entry<double, Shape<16, 256, 5, 256>>()};
+                                                   entry<double, Shape<16, 256, 5, 256>>(),
+                                                   entry<double, Shape<40, 560, 5, 256>>(),
+                                                   entry<double, Shape<32, 480, 6, 128>>(),
+                                                   entry<double, Shape<48, 640, 4, 256>>(),
+                                                   entry<double, Shape<64, 832, 3, 256>>()};
     static constexpr int by_wave[] = {1, 0};
 };
 constexpr int kLargeBox = 0;  // the shape for boxes of several waves

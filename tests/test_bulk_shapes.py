@@ -1,0 +1,16 @@
+"""The tile shapes of the bulk interval that a program may choose (no GPU is touched)."""
+import pytest
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+def test_six_shapes_can_be_chosen(rm, precision):
+    keep = rm.bulk_shape(precision)
+    try:
+        assert len(rm.bulk_shapes(precision)) >= 6
+        for k in range(6):
+            rm.set_bulk_shape(precision, k)
+            assert rm.bulk_shape(precision) == k
+        with pytest.raises(rm.RmpcdError):
+            rm.set_bulk_shape(precision, len(rm.bulk_shapes(precision)))
+    finally:
+        rm.set_bulk_shape(precision, keep)
