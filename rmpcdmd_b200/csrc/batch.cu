@@ -594,6 +594,14 @@ struct MdPair {
 // The block's shared memory: the step's bead positions and decisions, the queue
 // of particles that need more than free flight; behind it the pair forces
 // (MdTotals) and the particles, field by field (MdParts).
+//
+// What orders the words that both groups of warps use.  A step k has two points
+// between the groups: kBarForces, at which the particles' warps arrive without
+// waiting when the step's pair forces are pushed, and kBarTurn, at which all wait.
+// A bead warp may thus still be in front of kBarForces(k), its loop test
+// included, while the particles are at the second half of step k: a word that they
+// write there and a bead warp reads before kBarForces has two places, used in
+// turn.
 template <typename R>
 struct MdShared {
     MdBox<R> box;
@@ -601,10 +609,21 @@ struct MdShared {
     double old[6], rat[6];  // pos_old and pos_rattle of the beads
     double f[2][3];         // the beads' force sums
     double wsum[2][3][kNlBlockThreads / 32];
-    int stop, over, last;   // re-sort by the beads or s_free, by an active particle's displacement
-    int anew;               // a bead went farther than kMdWay
-    int spill;              // step + 1 of the last one with a term in global memory
-    int nq[2], cnt[2][2];   // by step parity: particles queued; pair forces per bead
+    // re-sort in front of step k's forces: by the beads or s_free (written by warp 0
+    // between kBarForces(k - 1) and kBarTurn(k - 1), read by all between kBarTurn(k -
+    // 1) and kBarForces(k)); by an active particle's displacement, by step parity
+    // (written for step k by the particles between their arrival at kBarForces(k - 1)
+    // and kBarTurn(k - 1), read like stop: a slow bead warp reads its step's
+    // place, which is not written again before kBarTurn(k))
+    int stop, over[2];
+    int last;               // this block is the launch's last
+    int anew;               // a bead went farther than kMdWay (written like stop, read by the particles before kBarForces)
+    int spill;              // step + 1 of the last one with a term in global memory (written before kBarForces, read after it)
+    // by step parity: particles queued for step k (counted by the particles after
+    // kBarForces(k - 1), read by them before kBarForces(k), cleared by the beads
+    // between that and kBarTurn(k)); pair forces per bead (counted before
+    // kBarForces(k), read and cleared by the beads after it)
+    int nq[2], cnt[2][2];
     int tot[2];             // slow sums: terms gathered
     int ws[33];
     int q[2][kMdQueue];     // queued particles, by step parity
@@ -629,7 +648,7 @@ __device__ __forceinline__ void md_arrive(int id, int threads)
 {
     asm volatile("barrier.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
-constexpr int kBarSum = 1, kBarPart = 2, kBarForces = 3, kBarTurn = 4;
+constexpr int kBarSum = 1, kBarPart = 2, kBarForces = 3, kBarTurn = 4, kBarReady = 5;
 
 // md_pos (src/md.f90:61-77), the PAST_MD / MD roll (src/neighbor_list.f90:180-188)
 // and whether the particle's displacement is sqrt(d2) >= thr
@@ -1238,7 +1257,7 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
             W.parts.cap = (int)((kMdSmem - kParts) / md_part_bytes<R>());
             W.parts.r = reinterpret_cast<R *>(md_smem + kParts);
             W.parts.i = reinterpret_cast<int *>(W.parts.r + 18 * (size_t)W.parts.cap);
-            sh.stop = sh.over = sh.spill = 0;
+            sh.stop = sh.over[0] = sh.over[1] = sh.spill = 0;
             sh.anew = 1;
             for (int p = 0; p < 2; p++) {
                 sh.nq[p] = sh.cnt[p][0] = sh.cnt[p][1] = 0;
@@ -1289,8 +1308,8 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                 __syncwarp();
                 if (t == 0) sh.anew = 1;  // there is no queue yet
             }
-            __syncthreads();
-            while (!(sh.stop | sh.over)) {
+            md_sync(kBarReady, all);
+            while (!(sh.stop | sh.over[k & 1])) {
                 const bool last = k + 1 == A.N_MD;
                 md_sync(kBarForces, all);
                 md_colloid_sums<R>(sh, totals, A, r, n0, n1, k);
@@ -1347,7 +1366,7 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                     // force_old of the last interval's end is no longer current
                     if ((q.f >> PAST_MD_BIT) & 1)
                         for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = 0;
-                    if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over = 1;
+                    if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over[k & 1] = 1;
                 }
                 if (i < B.parts.cap) {
                     B.parts.num(0, i) = idx;
@@ -1365,8 +1384,8 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                 }
                 md_write(B, A, i, idx, q, false);
             }
-            __syncthreads();
-            while (!(sh.stop | sh.over)) {
+            md_sync(kBarReady, all);
+            while (!(sh.stop | sh.over[k & 1])) {
                 const bool last = k + 1 == A.N_MD;
                 const int par = k & 1;
                 const double *X = sh.x[par];
@@ -1433,7 +1452,7 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                         // the interval's last step leaves force_old behind
                         for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = gl[c];
                     } else {
-                        if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over = 1;
+                        if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over[1 - par] = 1;
                         if (in) {
                             const int m = md_busy(X, B, q.p, q.f, B.queue_sq);
                             B.parts.num(6, i) = m;
