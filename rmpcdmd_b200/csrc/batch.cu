@@ -440,8 +440,10 @@ __global__ void __launch_bounds__(kBT)
         if (flag && !flag[r]) return;
         for (int e = (b % gx) * blockDim.x + threadIdx.x; e < n[i]; e += gx * blockDim.x) {
             const size_t q = (size_t)i * Nmax + e;
+            // (the flagged blocks give places from nl on at the same time: those
+            // particles' way is clear of the beads, and mult and ent hold the listed)
             const int a = aidx[list[q]];
-            if (a < 0) continue;
+            if (a < 0 || a >= nl[r]) continue;
             const size_t w = (size_t)2 * r * Nmax + a;
             atomicAdd(mult + w, (i & 1) ? 1 << 16 : 1);
             next[q] = atomicExch(ent + 2 * w + (i & 1), e);
