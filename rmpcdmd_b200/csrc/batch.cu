@@ -301,7 +301,9 @@ __device__ __forceinline__ bool may_meet(const float p[3], const float v[3], con
 // once: its place in act goes to aidx.  Until a re-sort a bead stays within
 // skin / 10 of its pos_old (the re-sort test, programs/single_dimer_pbc.f90:324-329),
 // and a particle without force flies straight, so that of the ~4,800 listed
-// particles of a sigma = 2 dimer some 800 are left.
+// particles of a sigma = 2 dimer some 800 are left.  One with MD or PAST_MD set
+// does not: half of its last force is still to change its velocity (and, with MD,
+// that force its position), wherever it has gone since, so it is always claimed.
 template <typename R>
 __global__ void __launch_bounds__(kBT)
     kb_claim(const int *flag, const BRep *rep, PView<R> v0, PView<R> v1, Vec3<double> cold, R dt, float reach,
@@ -326,7 +328,8 @@ __global__ void __launch_bounds__(kBT)
         const int idx = list[(size_t)i * Nmax + e];
         const float p[3] = {(float)v.pos.x[idx], (float)v.pos.y[idx], (float)v.pos.z[idx]};
         const float u[3] = {(float)v.vel.x[idx], (float)v.vel.y[idx], (float)v.vel.z[idx]};
-        if (!may_meet(p, u, c[0], L, far, T) && !may_meet(p, u, c[1], L, far, T)) continue;
+        const bool forced = v.flags[idx] & ((1 << MD_BIT) | (1 << PAST_MD_BIT));
+        if (!forced && !may_meet(p, u, c[0], L, far, T) && !may_meet(p, u, c[1], L, far, T)) continue;
         if (atomicCAS(aidx + idx, -1, -2) != -1) continue;
         const int a = atomicAdd(nl + r, 1);
         act[off + a] = idx;
