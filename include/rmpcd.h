@@ -388,9 +388,10 @@ int rmpcd_bulk_run(rmpcd_particles *p, rmpcd_cells *cells, rmpcd_rng *rng,
                    double tau, int has_alpha, double alpha, int n_intervals);
 /* Tile shapes of the fused interval kernel (cells per block, resident
  * blocks per SM).  All shapes give the same results bit for bit; one is in
- * use per precision once set; until then the size of the box chooses (and
- * rmpcd_bulk_get_shape reports 0, the choice for large boxes).  No counterpart
- * in the reference. */
+ * use per precision once set; until then, and after rmpcd_bulk_set_shape with
+ * -1, which rmpcd_bulk_get_shape reports in this state, the box of each run
+ * chooses.  What get_shape reports can so be put back by set_shape.  No
+ * counterpart in the reference. */
 int rmpcd_bulk_shapes(int precision, int *n_shapes, int *slots, int *min_blocks);
 int rmpcd_bulk_set_shape(int precision, int shape);
 int rmpcd_bulk_get_shape(int precision, int *shape);

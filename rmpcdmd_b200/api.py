@@ -707,12 +707,14 @@ def bulk_shapes(precision: int = FP32) -> list[tuple[int, int]]:
 
 
 def bulk_shape(precision: int = FP32) -> int:
+    """The shape set for a precision, -1 when the box of each run chooses."""
     s = C.c_int()
     call("rmpcd_bulk_get_shape", int(precision), C.byref(s))
     return s.value
 
 
 def set_bulk_shape(precision: int, shape: int) -> None:
+    """Put a shape of `bulk_shapes` in use; -1: the box of each run chooses."""
     call("rmpcd_bulk_set_shape", int(precision), int(shape))
 
 

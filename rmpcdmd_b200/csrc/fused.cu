@@ -1172,7 +1172,7 @@ extern "C" int rmpcd_bulk_set_shape(int precision, int shape)
 {
     RMPCD_ARG(precision == RMPCD_FP32 || precision == RMPCD_FP64, "precision must be 32 or 64");
     const int n = precision == RMPCD_FP32 ? n_shapes<float>() : n_shapes<double>();
-    RMPCD_ARG(shape >= 0 && shape < n, "rmpcd_bulk_set_shape: no such shape");
+    RMPCD_ARG(shape >= -1 && shape < n, "rmpcd_bulk_set_shape: no such shape");
     g_shape[precision == RMPCD_FP64] = shape;
     return RMPCD_OK;
 }
@@ -1181,7 +1181,7 @@ extern "C" int rmpcd_bulk_get_shape(int precision, int *shape)
 {
     RMPCD_ARG(shape, "null argument");
     RMPCD_ARG(precision == RMPCD_FP32 || precision == RMPCD_FP64, "precision must be 32 or 64");
-    *shape = g_shape[precision == RMPCD_FP64] < 0 ? 0 : g_shape[precision == RMPCD_FP64];
+    *shape = g_shape[precision == RMPCD_FP64];
     return RMPCD_OK;
 }
 
