@@ -14,7 +14,7 @@
 
 namespace rmpcd {
 
-// The collision kernels below work on tiles of kCellTile consecutive slots,
+// The collision kernels below work on tiles of up to kCellTile consecutive slots,
 // whose particles are one contiguous range: the block brings the range's
 // velocities and species into shared memory with coalesced loads, one thread
 // per slot runs the cell's sequential sums and updates there, and the block
@@ -22,23 +22,32 @@ namespace rmpcd {
 // touches 32 cells' ranges per warp load (64^3 at density 10: 79 us FP64 for
 // the SRD step against 30 us of HBM traffic); the cell's own chain of adds
 // then sets its pace.  64 slots per 128-thread block leave 8 (FP64) or 16
-// (FP32) blocks per SM, so that one block's loads overlap another's sums.  A
-// tile of more than kCellCap particles (7 standard deviations above the mean
-// at density 10) takes the same cell bodies on global memory.
+// (FP32) blocks per SM, so that one block's loads overlap another's sums; a
+// denser fluid's tiles have the slots that kCellCap holds (cell_tile).
+//
+// A tile of an uneven fluid with more than kCellCap particles takes the same cell
+// bodies on global memory.  Two FP64 kernels with long cell bodies, whose staging
+// leaves too few threads per SM for that, go run by run instead, each the next cells
+// that fit, when no cell has more than kRunCell particles (48^3 fluid in one octant,
+// MPC-AT step: 153 us, 278 on global memory; in the SRD kernel the second copy of
+// the body costs registers, 27 us for 23 at density 10).
 constexpr int kCellTile = 64;
 constexpr int kCellThreads = 128;
 constexpr int kCellCap = 832;
+constexpr int kRunCell = kCellCap / 5;
 
 struct CellRange {
     int n, a;          // this thread's cell: particles, first particle (n = 0: no cell)
     int a0, np;        // the tile's particles
-    __device__ CellRange(const int *__restrict__ count, const int *__restrict__ start, int S)
+    int s0, cells;     // the tile's slots
+    __device__ CellRange(const int *__restrict__ count, const int *__restrict__ start, int S, int per)
     {
-        const int s0 = blockIdx.x * kCellTile, last = min(s0 + kCellTile, S) - 1;
-        const int s = s0 + (int)threadIdx.x;
+        s0 = blockIdx.x * per;
+        cells = min(per, S - s0);
+        const int s = s0 + (int)threadIdx.x, last = s0 + cells - 1;
         n = 0;
         a = 0;
-        if (threadIdx.x < kCellTile && s < S) {
+        if ((int)threadIdx.x < cells) {
             n = count[s];
             a = start[s];
         }
@@ -47,7 +56,31 @@ struct CellRange {
     }
 };
 
-inline int cell_blocks(int S) { return (S + kCellTile - 1) / kCellTile; }
+// The cells of a tile: run(n, a, a0, np) for the particles [a0, a0 + np) in shared
+// memory, called by every thread, with the thread's cell, n = 0 when that is not
+// of the run; direct() by the threads of a tile that takes its cells on global
+// memory.  Returns the sum of the thread's results.
+template <bool kRuns, typename Run, typename Direct>
+__device__ __forceinline__ double cell_bodies(const CellRange &c, const int *__restrict__ count,
+                                              const int *__restrict__ start, Run run, Direct direct)
+{
+    if (c.np <= kCellCap) return run(c.n, c.a - c.a0, c.a0, c.np);
+    if constexpr (kRuns) {
+        if (!__syncthreads_or(c.n > kRunCell)) {
+            const int t = threadIdx.x;
+            double r = 0;
+            for (int c0 = 0, k; c0 < c.cells; c0 += k) {
+                const int a0 = start[c.s0 + c0];
+                // (its barrier also ends the run before)
+                k = __syncthreads_count(t >= c0 && t < c.cells && c.a + c.n - a0 <= kCellCap);
+                const int last = c.s0 + c0 + k - 1;
+                r += run(t >= c0 && t < c0 + k ? c.n : 0, c.a - a0, a0, start[last] + count[last] - a0);
+            }
+            return r;
+        }
+    }
+    return c.n > 0 ? direct() : 0;
+}
 
 // K arrays src[k][a0 .. a0 + np) to or from rows of kCellCap of shared memory
 template <typename T, int K>
@@ -70,25 +103,33 @@ __device__ __forceinline__ void tile_out(T *const (&dst)[K], T (*src)[kCellCap],
 }
 
 // simple_mpcd_step, src/mpcd.f90:71-183
-template <typename R>
+template <typename R, bool kStaged>
 __global__ void __launch_bounds__(kCellThreads)
-    k_simple_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+    k_simple_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, int per, R *vx, R *vy, R *vz,
                   const int *__restrict__ species, SrdParams q)
 {
-    __shared__ R sv[3][kCellCap];
-    __shared__ int ss[1][kCellCap];
-    const CellRange c(count, start, S);
-    const long long slot = (long long)blockIdx.x * kCellTile + threadIdx.x;
-    if (c.np > kCellCap) {
-        srd_slot<R>(c.n, c.a, slot, 0, vx, vy, vz, species, q);
-        return;
+    const long long slot = (long long)blockIdx.x * (kStaged ? per : kCellThreads) + threadIdx.x;
+    if constexpr (!kStaged) {
+        if (slot < S) srd_slot<R>(count[slot], start[slot], slot, 0, vx, vy, vz, species, q);
+    } else {
+        __shared__ R sv[3][kCellCap];
+        __shared__ int ss[1][kCellCap];
+        const CellRange c(count, start, S, per);
+        auto run = [=](int n, int a, int a0, int np) {
+            tile_in<R, 3>(sv, {vx, vy, vz}, a0, np);
+            tile_in<int, 1>(ss, {species}, a0, np);
+            __syncthreads();
+            srd_slot<R>(n, a, slot, -(long long)a0, sv[0], sv[1], sv[2], ss[0], q);
+            __syncthreads();
+            tile_out<R, 3>({vx, vy, vz}, sv, a0, np);
+            return 0.0;
+        };
+        auto direct = [=] {
+            srd_slot<R>(c.n, c.a, slot, 0, vx, vy, vz, species, q);
+            return 0.0;
+        };
+        cell_bodies<false>(c, count, start, run, direct);
     }
-    tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
-    tile_in<int, 1>(ss, {species}, c.a0, c.np);
-    __syncthreads();
-    srd_slot<R>(c.n, c.a - c.a0, slot, -(long long)c.a0, sv[0], sv[1], sv[2], ss[0], q);
-    __syncthreads();
-    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
 
 // The MPC-AT normals of simple_mpcd_step (src/mpcd.f90:144-160) and
@@ -198,25 +239,34 @@ __device__ __forceinline__ void at_cell(int n, int a, R *vx, R *vy, R *vz, const
 
 // simple_mpcd_step with the MPC-AT thermostat given the normals of
 // k_at_normals
-template <typename R>
+template <typename R, bool kStaged>
 __global__ void __launch_bounds__(kCellThreads)
-    k_at_cells(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+    k_at_cells(const int *__restrict__ count, const int *__restrict__ start, int S, int per, R *vx, R *vy, R *vz,
                const int *__restrict__ species, int hydro, const R *__restrict__ nx, const R *__restrict__ ny,
                const R *__restrict__ nz)
 {
-    __shared__ R sv[6][kCellCap];
-    __shared__ int ss[1][kCellCap];
-    const CellRange c(count, start, S);
-    if (c.np > kCellCap) {
-        at_cell<R>(c.n, c.a, vx, vy, vz, species, hydro, nx, ny, nz);
-        return;
+    if constexpr (!kStaged) {
+        const long long slot = (long long)blockIdx.x * kCellThreads + threadIdx.x;
+        if (slot < S) at_cell<R>(count[slot], start[slot], vx, vy, vz, species, hydro, nx, ny, nz);
+    } else {
+        __shared__ R sv[6][kCellCap];
+        __shared__ int ss[1][kCellCap];
+        const CellRange c(count, start, S, per);
+        auto run = [=](int n, int a, int a0, int np) {
+            tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, a0, np);
+            tile_in<int, 1>(ss, {species}, a0, np);
+            __syncthreads();
+            at_cell<R>(n, a, sv[0], sv[1], sv[2], ss[0], hydro, sv[3], sv[4], sv[5]);
+            __syncthreads();
+            tile_out<R, 3>({vx, vy, vz}, sv, a0, np);
+            return 0.0;
+        };
+        auto direct = [=] {
+            at_cell<R>(c.n, c.a, vx, vy, vz, species, hydro, nx, ny, nz);
+            return 0.0;
+        };
+        cell_bodies<sizeof(R) == 8>(c, count, start, run, direct);
     }
-    tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, c.a0, c.np);
-    tile_in<int, 1>(ss, {species}, c.a0, c.np);
-    __syncthreads();
-    at_cell<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0], hydro, sv[3], sv[4], sv[5]);
-    __syncthreads();
-    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
 
 struct WallArgs {
@@ -301,27 +351,33 @@ __device__ __forceinline__ void wall_cell(int n, int a, int s, R *vx, R *vy, R *
 // from k_at_normals, which deals the rejection attempts of a whole warp to its
 // lanes; drawn inside the cell loop they took a 1.2 M particle channel (FP64)
 // 148 us, one thread per cell.
-template <typename R, bool kAT>
+template <typename R, bool kAT, bool kStaged>
 __global__ void __launch_bounds__(kCellThreads)
-    k_wall_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+    k_wall_mpcd(const int *__restrict__ count, const int *__restrict__ start, int S, int per, R *vx, R *vy, R *vz,
                 const R *__restrict__ nx, const R *__restrict__ ny, const R *__restrict__ nz, SrdParams q, WallArgs w)
 {
-    __shared__ R sv[kAT ? 6 : 3][kCellCap];
-    const CellRange c(count, start, S);
-    const int slot = blockIdx.x * kCellTile + (int)threadIdx.x;
-    if (c.np > kCellCap) {
-        wall_cell<R>(c.n, c.a, slot, vx, vy, vz, nx, ny, nz, q, w);
-        return;
+    const int slot = blockIdx.x * (kStaged ? per : kCellThreads) + (int)threadIdx.x;
+    if constexpr (!kStaged) {
+        if (slot < S) wall_cell<R>(count[slot], start[slot], slot, vx, vy, vz, nx, ny, nz, q, w);
+    } else {
+        __shared__ R sv[kAT ? 6 : 3][kCellCap];
+        const CellRange c(count, start, S, per);
+        auto run = [=](int n, int a, int a0, int np) {
+            if constexpr (kAT) tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, a0, np);
+            else tile_in<R, 3>(sv, {vx, vy, vz}, a0, np);
+            __syncthreads();
+            wall_cell<R>(n, a, slot, sv[0], sv[1], sv[2], sv[kAT ? 3 : 0], sv[kAT ? 4 : 1], sv[kAT ? 5 : 2], q, w);
+            __syncthreads();
+            tile_out<R, 3>({vx, vy, vz}, sv, a0, np);
+            return 0.0;
+        };
+        auto direct = [=] {
+            wall_cell<R>(c.n, c.a, slot, vx, vy, vz, nx, ny, nz, q, w);
+            return 0.0;
+        };
+        cell_bodies<false>(c, count, start, run, direct);
     }
-    if constexpr (kAT) tile_in<R, 6>(sv, {vx, vy, vz, nx, ny, nz}, c.a0, c.np);
-    else tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
-    __syncthreads();
-    wall_cell<R>(c.n, c.a - c.a0, slot, sv[0], sv[1], sv[2], sv[kAT ? 3 : 0], sv[kAT ? 4 : 1], sv[kAT ? 5 : 2], q, w);
-    __syncthreads();
-    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
-
-constexpr int kRedBlocks = 1024;
 
 // compute_temperature, src/mpcd.f90:342-407, of the n particles from a: the
 // cell's contribution to the sum of temperatures (0 for cells that add none)
@@ -353,41 +409,53 @@ __device__ __forceinline__ double cell_temperature(int n, int a, const R *vx, co
     return kin / (double)(3 * (n_eff - 1));
 }
 
-// per-block partial sums (te, count) over the cells of one tile, for the
-// fixed-order sum of k_temperature_final
-template <typename R>
+// per-block partial sums (te, count) over the block's cells, for the fixed-order
+// sum of k_temperature_final
+template <typename R, bool kStaged>
 __global__ void __launch_bounds__(kCellThreads)
-    k_temperature(const int *__restrict__ count, const int *__restrict__ start, int S, const R *vx, const R *vy,
-                  const R *vz, const int *__restrict__ species, double *part)
+    k_temperature(const int *__restrict__ count, const int *__restrict__ start, int S, int per, const R *vx,
+                  const R *vy, const R *vz, const int *__restrict__ species, double *part)
 {
-    __shared__ R sv[3][kCellCap];
-    __shared__ int ss[1][kCellCap];
-    const CellRange c(count, start, S);
-    double te;
-    if (c.np > kCellCap) {
-        te = cell_temperature<R>(c.n, c.a, vx, vy, vz, species);
+    double te = 0, cnt = 0;
+    if constexpr (!kStaged) {
+        const long long slot = (long long)blockIdx.x * kCellThreads + threadIdx.x;
+        if (slot < S) {
+            te = cell_temperature<R>(count[slot], start[slot], vx, vy, vz, species);
+            cnt = count[slot] > 1 ? 1 : 0;
+        }
     } else {
-        tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
-        tile_in<int, 1>(ss, {species}, c.a0, c.np);
-        __syncthreads();
-        te = cell_temperature<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0]);
+        __shared__ R sv[3][kCellCap];
+        __shared__ int ss[1][kCellCap];
+        const CellRange c(count, start, S, per);
+        auto run = [=](int n, int a, int a0, int np) {
+            tile_in<R, 3>(sv, {vx, vy, vz}, a0, np);
+            tile_in<int, 1>(ss, {species}, a0, np);
+            __syncthreads();
+            return cell_temperature<R>(n, a, sv[0], sv[1], sv[2], ss[0]);
+        };
+        auto direct = [=] { return cell_temperature<R>(c.n, c.a, vx, vy, vz, species); };
+        te = cell_bodies<false>(c, count, start, run, direct);
+        cnt = c.n > 1 ? 1 : 0;
     }
-    // kCellTile = 64 slots: two warps hold values
-    __shared__ double s_te[2];
-    double cnt = c.n > 1 ? 1 : 0;
+    constexpr int W = kCellThreads / 32;
+    __shared__ double s_te[W], s_cnt[W];
     for (int o = 16; o > 0; o >>= 1) {
         te += __shfl_xor_sync(0xffffffffu, te, o);
         cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     }
-    __shared__ double s_cnt[2];
-    if ((threadIdx.x & 31) == 0 && threadIdx.x < kCellTile) {
+    if ((threadIdx.x & 31) == 0) {
         s_te[threadIdx.x >> 5] = te;
         s_cnt[threadIdx.x >> 5] = cnt;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        part[2 * (size_t)blockIdx.x] = s_te[0] + s_te[1];
-        part[2 * (size_t)blockIdx.x + 1] = s_cnt[0] + s_cnt[1];
+        // (a tile's 64 slots are the first two warps')
+        for (int w = 1; w < W; w++) {
+            te += s_te[w];
+            cnt += s_cnt[w];
+        }
+        part[2 * (size_t)blockIdx.x] = te;
+        part[2 * (size_t)blockIdx.x + 1] = cnt;
     }
 }
 
@@ -454,24 +522,33 @@ __device__ __forceinline__ void rescale_cell(int n, int a, R *vx, R *vy, R *vz, 
     }
 }
 
-template <typename R>
+template <typename R, bool kStaged>
 __global__ void __launch_bounds__(kCellThreads)
-    k_rescale(const int *__restrict__ count, const int *__restrict__ start, int S, R *vx, R *vy, R *vz,
+    k_rescale(const int *__restrict__ count, const int *__restrict__ start, int S, int per, R *vx, R *vy, R *vz,
               const int *__restrict__ species, double T)
 {
-    __shared__ R sv[3][kCellCap];
-    __shared__ int ss[1][kCellCap];
-    const CellRange c(count, start, S);
-    if (c.np > kCellCap) {
-        rescale_cell<R>(c.n, c.a, vx, vy, vz, species, T);
-        return;
+    if constexpr (!kStaged) {
+        const long long slot = (long long)blockIdx.x * kCellThreads + threadIdx.x;
+        if (slot < S) rescale_cell<R>(count[slot], start[slot], vx, vy, vz, species, T);
+    } else {
+        __shared__ R sv[3][kCellCap];
+        __shared__ int ss[1][kCellCap];
+        const CellRange c(count, start, S, per);
+        auto run = [=](int n, int a, int a0, int np) {
+            tile_in<R, 3>(sv, {vx, vy, vz}, a0, np);
+            tile_in<int, 1>(ss, {species}, a0, np);
+            __syncthreads();
+            rescale_cell<R>(n, a, sv[0], sv[1], sv[2], ss[0], T);
+            __syncthreads();
+            tile_out<R, 3>({vx, vy, vz}, sv, a0, np);
+            return 0.0;
+        };
+        auto direct = [=] {
+            rescale_cell<R>(c.n, c.a, vx, vy, vz, species, T);
+            return 0.0;
+        };
+        cell_bodies<sizeof(R) == 8>(c, count, start, run, direct);
     }
-    tile_in<R, 3>(sv, {vx, vy, vz}, c.a0, c.np);
-    tile_in<int, 1>(ss, {species}, c.a0, c.np);
-    __syncthreads();
-    rescale_cell<R>(c.n, c.a - c.a0, sv[0], sv[1], sv[2], ss[0], T);
-    __syncthreads();
-    tile_out<R, 3>({vx, vy, vz}, sv, c.a0, c.np);
 }
 
 // mpcd_stream_periodic, src/mpcd.f90:440-457
@@ -711,22 +788,82 @@ static SrdParams srd_params(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, in
 
 static int at_blocks(long long N) { return grid_full((N + 32 * kAtChunks - 1) / (32 * kAtChunks) * 32, kAtThreads); }
 
+// Slots per tile of the collision kernels: what kCellCap holds of a uniform fluid
+// of this density with four standard deviations to spare, at most kCellTile.  0: no
+// staging, a thread per slot on global memory, kCellThreads slots per block, where
+// a tile would have fewer than four slots (kMinTile: also what k_temperature's
+// partial sums have room for), from 178 particles per cell on.  us at 48^3 FP64 (SRD
+// step, MPC-AT step, rescaling) with 64 slots whatever the density, with these, and
+// with a thread per slot on global memory: density 15: 77 190 179, 38 108 37, 81 154
+// 96; 30: 174 519 437, 81 213 78, 180 360 237; 100: - , 288 785 346, 648 1287 881; 150: - ,
+// 555 1403 702, 966 1933 1364.
+constexpr int kMinTile = 4;
+static int cell_tile(const rmpcd_particles *p, const rmpcd_cells *c)
+{
+    const double mean = (double)p->N / ((double)c->L[0] * c->L[1] * c->L[2]);
+    int per = kCellTile;
+    while (per >= kMinTile && per * mean + 4 * sqrt(per * mean) > kCellCap) per--;
+    return per >= kMinTile ? per : 0;
+}
+static int cell_blocks(int S, int per)
+{
+    if (per == 0) per = kCellThreads;
+    return (S + per - 1) / per;
+}
+
 // with the thermostat, the normals go into the sort target's velocity arrays
 // (free between sorts) first
+template <typename R>
+static void simple_launches(rmpcd_particles *p, rmpcd_cells *c, const SrdParams &q)
+{
+    cudaStream_t s = stream();
+    const int per = cell_tile(p, c);
+    const int g = cell_blocks(c->S, per);
+    PView<R> v = cur<R>(p), t = alt<R>(p);
+    if (q.thermostat && !q.gauss && p->N > 0) {
+        k_at_normals<R><<<at_blocks(p->N), kAtThreads, 0, s>>>(v.species, p->N, q, t.vel.x, t.vel.y, t.vel.z);
+        auto *k = per ? k_at_cells<R, true> : k_at_cells<R, false>;
+        k<<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, per, v.vel.x, v.vel.y, v.vel.z, v.species, q.hydro, t.vel.x,
+                                     t.vel.y, t.vel.z);
+    } else {
+        auto *k = per ? k_simple_mpcd<R, true> : k_simple_mpcd<R, false>;
+        k<<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, per, v.vel.x, v.vel.y, v.vel.z, v.species, q);
+    }
+}
+
 template <typename R>
 static void wall_launches(rmpcd_particles *p, rmpcd_cells *c, const SrdParams &q, const WallArgs &w)
 {
     cudaStream_t s = stream();
-    const int g = cell_blocks(c->S);
+    const int per = cell_tile(p, c);
+    const bool at = q.thermostat && p->N > 0;
     PView<R> v = cur<R>(p), t = alt<R>(p);
-    if (q.thermostat && p->N > 0) {
-        k_at_normals<R><<<at_blocks(p->N), kAtThreads, 0, s>>>(nullptr, p->N, q, t.vel.x, t.vel.y, t.vel.z);
-        k_wall_mpcd<R, true><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, t.vel.x,
-                                                       t.vel.y, t.vel.z, q, w);
-    } else {
-        k_wall_mpcd<R, false><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, nullptr,
-                                                        nullptr, nullptr, q, w);
-    }
+    if (at) k_at_normals<R><<<at_blocks(p->N), kAtThreads, 0, s>>>(nullptr, p->N, q, t.vel.x, t.vel.y, t.vel.z);
+    auto *k = at ? (per ? k_wall_mpcd<R, true, true> : k_wall_mpcd<R, true, false>)
+                 : (per ? k_wall_mpcd<R, false, true> : k_wall_mpcd<R, false, false>);
+    k<<<cell_blocks(c->S, per), kCellThreads, 0, s>>>(c->count, c->start, c->S, per, v.vel.x, v.vel.y, v.vel.z, t.vel.x,
+                                                    t.vel.y, t.vel.z, q, w);
+}
+
+template <typename R>
+static void temperature_launches(rmpcd_particles *p, rmpcd_cells *c, double *part, double *out)
+{
+    const int per = cell_tile(p, c);
+    const int nb = cell_blocks(c->S, per);
+    PView<R> v = cur<R>(p);
+    auto *k = per ? k_temperature<R, true> : k_temperature<R, false>;
+    k<<<nb, kCellThreads, 0, stream()>>>(c->count, c->start, c->S, per, v.vel.x, v.vel.y, v.vel.z, v.species, part);
+    k_temperature_final<<<1, 1024, 0, stream()>>>(part, nb, out);
+}
+
+template <typename R>
+static void rescale_launch(rmpcd_particles *p, rmpcd_cells *c, double T)
+{
+    const int per = cell_tile(p, c);
+    PView<R> v = cur<R>(p);
+    auto *k = per ? k_rescale<R, true> : k_rescale<R, false>;
+    k<<<cell_blocks(c->S, per), kCellThreads, 0, stream()>>>(c->count, c->start, c->S, per, v.vel.x, v.vel.y, v.vel.z,
+                                                           v.species, T);
 }
 
 }  // namespace rmpcd
@@ -752,28 +889,7 @@ int rmpcd_simple_mpcd_step(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, int
         return fail(RMPCD_ERR_STOP, "requiring .not.do_hydro without thermostat in simple_mpcd_step");
     PhaseTimer t("step");
     SrdParams q = srd_params(p, c, r, has_alpha, alpha, thermostat, T, hydro);
-    cudaStream_t s = stream();
-    const int g = cell_blocks(c->S);
-    if (thermostat && !q.gauss && p->N > 0) {
-        // the normals first, into the sort target's velocity arrays (free
-        // between sorts), then the cells
-        const int gn = at_blocks(p->N);
-        DISPATCH_R(p,
-                   ({ PView<float> v = cur<float>(p), t = alt<float>(p);
-                      k_at_normals<float><<<gn, kAtThreads, 0, s>>>(v.species, p->N, q, t.vel.x, t.vel.y, t.vel.z);
-                      k_at_cells<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
-                                                          v.species, q.hydro, t.vel.x, t.vel.y, t.vel.z); }),
-                   ({ PView<double> v = cur<double>(p), t = alt<double>(p);
-                      k_at_normals<double><<<gn, kAtThreads, 0, s>>>(v.species, p->N, q, t.vel.x, t.vel.y, t.vel.z);
-                      k_at_cells<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z,
-                                                           v.species, q.hydro, t.vel.x, t.vel.y, t.vel.z); }));
-    } else {
-        DISPATCH_R(p,
-                   ({ PView<float> v = cur<float>(p);
-                      k_simple_mpcd<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }),
-                   ({ PView<double> v = cur<double>(p);
-                      k_simple_mpcd<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, q); }));
-    }
+    DISPATCH_R(p, simple_launches<float>(p, c, q), simple_launches<double>(p, c, q));
     RMPCD_CHECK_LAUNCH();
     r->step++;
     return RMPCD_OK;
@@ -810,13 +926,7 @@ int rmpcd_compute_temperature(rmpcd_particles *p, rmpcd_cells *c, double *te)
     // two doubles per tile of slots, in the slots' scatter cursors (rewritten by
     // the next count_particles or sort before they are read)
     double *part = (double *)c->cursor, *out = c->d_red;
-    const int nb = cell_blocks(c->S);
-    DISPATCH_R(p,
-               ({ PView<float> v = cur<float>(p);
-                  k_temperature<float><<<nb, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }),
-               ({ PView<double> v = cur<double>(p);
-                  k_temperature<double><<<nb, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, part); }));
-    k_temperature_final<<<1, 1024, 0, s>>>(part, nb, out);
+    DISPATCH_R(p, temperature_launches<float>(p, c, part, out), temperature_launches<double>(p, c, part, out));
     RMPCD_CHECK_LAUNCH();
     RMPCD_CUDA_TRY(cudaMemcpyAsync(te, out, sizeof(double), cudaMemcpyDeviceToHost, s));
     return sync();
@@ -826,13 +936,7 @@ int rmpcd_rescale_cells(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *, double 
 {
     RMPCD_ARG(p && c, "null argument");
     PhaseTimer t("step");
-    cudaStream_t s = stream();
-    const int g = cell_blocks(c->S);
-    DISPATCH_R(p,
-               ({ PView<float> v = cur<float>(p);
-                  k_rescale<float><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }),
-               ({ PView<double> v = cur<double>(p);
-                  k_rescale<double><<<g, kCellThreads, 0, s>>>(c->count, c->start, c->S, v.vel.x, v.vel.y, v.vel.z, v.species, T); }));
+    DISPATCH_R(p, rescale_launch<float>(p, c, T), rescale_launch<double>(p, c, T));
     RMPCD_CHECK_LAUNCH();
     return RMPCD_OK;
 }
