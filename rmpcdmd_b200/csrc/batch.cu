@@ -120,6 +120,7 @@ struct rmpcd_dimer_batch {
     rmpcd::BRep *rep = nullptr;
     rmpcd::BTile *ptile = nullptr, *stile = nullptr;
     int n_ptile = 0, n_stile = 0;
+    int order_slots = 0;  // slots per tile of the re-sort's gather, by the densest replica
     int cap_ptile = 0;  // particle tiles allocated (enough for the smallest tile size)
     int shape = 0;      // engine shape in use (kernel variant, particles per tile)
     int *stile_first = nullptr, *stile_count = nullptr;  // per replica
@@ -1774,23 +1775,22 @@ __global__ void __launch_bounds__(kBT) kb_perm(TileSet ts, const int *key, int *
 // Only particles with MD or PAST_MD set have force entries: they are moved and
 // zeroed behind, so the buffer that is not current holds none.  Flagged
 // particles are listed in flist.
-constexpr int kOrderPerTile = kTile / kOrderSlots;
-
 template <typename R>
 __global__ void __launch_bounds__(kOrderThreads, 4)
-    kb_order_gather(TileSet ts, const BRep *rep, PView<R> v0, PView<R> v1, const int *count, const int *start, int *perm,
-                    int *flist, int *nf)
+    kb_order_gather(TileSet ts, int slots, const BRep *rep, PView<R> v0, PView<R> v1, const int *count,
+                    const int *start, int *perm, int *flist, int *nf)
 {
     __shared__ OrderTile sh;
-    for (int kt = blockIdx.x; kt < *ts.n * kOrderPerTile; kt += gridDim.x) {
-        const BTile t = ts.tiles[ts.ids[kt / kOrderPerTile]];
-        const long long s0 = t.begin + (long long)(kt % kOrderPerTile) * kOrderSlots;
+    const int per = (kTile + slots - 1) / slots;
+    for (long long kt = blockIdx.x; kt < (long long)*ts.n * per; kt += gridDim.x) {
+        const BTile t = ts.tiles[ts.ids[kt / per]];
+        const long long s0 = t.begin + kt % per * slots;
         if (s0 >= t.end) continue;
         const BRep &rp = rep[t.r];
         const PView<R> d = pick(v0, v1, rp.cur), s = pick(v1, v0, rp.cur);
         int a0, np;
         __syncthreads();  // the last tile's indices are read
-        const int *src = order_tile(sh, (int)s0, (int)min(s0 + kOrderSlots, t.end), count, start, perm, d.id, a0, np);
+        const int *src = order_tile(sh, (int)s0, (int)min(s0 + slots, t.end), count, start, perm, d.id, a0, np);
         for (int q = threadIdx.x; q < np; q += kOrderThreads) {
             const int i = src[q], j = a0 + q;
             R px = s.pos.x[i], py = s.pos.y[i], pz = s.pos.z[i];
@@ -1960,8 +1960,9 @@ static void resort_launches(Batch *b, const int *flag, cudaStream_t st, int shif
                                        b->fresh);
     kb_scan_apply<<<gs, kBT, 0, st>>>(sts, b->count, b->tile_off, b->start, b->cursor);
     kb_perm<<<gp, kBT, 0, st>>>(pts, b->sol->key, b->cursor, b->sol->perm);
-    kb_order_gather<R><<<resort_grid(b->n_stile * kOrderPerTile), kOrderThreads, 0, st>>>(
-        sts, b->rep, v0, v1, b->count, b->start, b->sol->perm, b->sol->key, b->nf);
+    const long long n_order = (long long)b->n_stile * ((kTile + b->order_slots - 1) / b->order_slots);
+    kb_order_gather<R><<<resort_grid((int)(n_order < INT_MAX ? n_order : INT_MAX)), kOrderThreads, 0, st>>>(
+        sts, b->order_slots, b->rep, v0, v1, b->count, b->start, b->sol->perm, b->sol->key, b->nf);
     kb_update_list<R><<<2 * b->R, kNlBlockThreads, nl_stage_bytes<R>(), st>>>(
         flag, b->rep, cv, v0, v1, b->count, b->start, b->stencil, b->n_stencil,
         b->prm.list_radius * b->prm.list_radius, b->lj_sc, b->Nmax, b->list, b->nn, b->is_md, b->is_reac,
@@ -2430,6 +2431,12 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     b->Stot = (int)soff;
     b->cap_ptile = (int)cap_p;
     b->n_stile = (int)stl.size();
+    double densest = 0;
+    for (const BRep &p : b->rep_h) {
+        const double mean = (double)p.n / ((double)p.g.L[0] * p.g.L[1] * p.g.L[2]);
+        densest = mean > densest ? mean : densest;
+    }
+    b->order_slots = order_slots(densest);
     size_t ne = (size_t)2 * R * b->Nmax;
     bool ok = !dalloc(&b->rep, R) && !dalloc(&b->ptile, cap_p) && !dalloc(&b->stile, stl.size()) &&
               !dalloc(&b->stile_first, R) && !dalloc(&b->stile_count, R) && !dalloc(&b->tile_sum, stl.size()) &&

@@ -50,6 +50,7 @@
 #include "rng.cuh"
 #include "scan.cuh"
 #include "sortcore.cuh"
+#include "sortnet.cuh"
 #include "sorttile.cuh"
 #include "timers.cuh"
 

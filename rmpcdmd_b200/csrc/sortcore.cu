@@ -1,12 +1,13 @@
 #include "keys.cuh"
 #include "scan.cuh"
 #include "sortcore.cuh"
+#include "sortnet.cuh"
 #include "sorttile.cuh"
 #include "timers.cuh"
 
 namespace rmpcd {
 
-constexpr int kSmallSegment = kOrderSmall;
+constexpr int kSmallSegment = 64;
 
 // key[i] = slot of particle i; histogram with one atomic per distinct key
 // per warp (consecutive particles usually share a cell).
@@ -31,7 +32,7 @@ __global__ void k_key_count(Grid g, const R *__restrict__ x, const R *__restrict
 }
 
 // place every particle inside its cell; the order inside a cell is fixed
-// afterwards by k_segsort.  Each warp handles kPermRounds groups of 32
+// afterwards, by k_order_gather or sort_perm_segments.  Each warp handles kPermRounds groups of 32
 // consecutive particles and issues all their cursor atomics before using any
 // result, so the atomic round trips overlap.  cellmap (if given) receives the
 // slot of every place: the slot of each particle of the sorted arrays.
@@ -110,13 +111,13 @@ __global__ void k_segsort_big(const int *__restrict__ start, const int *__restri
 template <typename R>
 __global__ void __launch_bounds__(kOrderThreads, 6)
     k_order_gather(PView<R> s, PView<R> d, const int *__restrict__ count, const int *__restrict__ start, int S,
-                   int *perm, int with_force, int with_force_old, int gated, int *flagged, int *n_flagged)
+                   int slots, int *perm, int with_force, int with_force_old, int gated, int *flagged, int *n_flagged)
 {
     __shared__ OrderTile sh;
     const int fmask = (1 << MD_BIT) | (1 << PAST_MD_BIT);
-    const int s0 = blockIdx.x * kOrderSlots;
+    const int s0 = blockIdx.x * slots;
     int a0, np;
-    const int *src = order_tile(sh, s0, min(s0 + kOrderSlots, S), count, start, perm, d.id, a0, np);
+    const int *src = order_tile(sh, s0, min(s0 + slots, S), count, start, perm, d.id, a0, np);
     for (int q = threadIdx.x; q < np; q += kOrderThreads) {
         const int i = src[q], j = a0 + q;
         // all loads first: twelve independent gathers in flight per thread
@@ -226,8 +227,9 @@ static int gather_t(rmpcd_cells *c, rmpcd_particles *p, bool gated = false, int 
                 RMPCD_CUDA_TRY(cudaMemsetAsync(p->force_old[to][k], 0, (size_t)p->N * p->rsize, st));
             }
         }
-        k_order_gather<R><<<grid_full(c->S, kOrderSlots), kOrderThreads, 0, st>>>(
-            cur<R>(p), alt<R>(p), c->count, c->start, c->S, p->perm, p->force_zero ? 0 : 1,
+        const int slots = order_slots((double)p->N / ((double)c->L[0] * c->L[1] * c->L[2]));
+        k_order_gather<R><<<grid_full(c->S, slots), kOrderThreads, 0, st>>>(
+            cur<R>(p), alt<R>(p), c->count, c->start, c->S, slots, p->perm, p->force_zero ? 0 : 1,
             p->force_old_zero ? 0 : 1, gated ? 1 : 0, flagged, n_flagged);
         RMPCD_CHECK_LAUNCH();
     }
