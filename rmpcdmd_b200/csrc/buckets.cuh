@@ -296,15 +296,75 @@ __device__ __forceinline__ int bucket_move(const BucketTile<double, S> &sh, cons
     return key;
 }
 
+// A node of the pool.  kMany (over-full tiles): one atomic for the threads of the
+// warp that are here, since every overflow of the grid counts on this one address
+// (resting 48^3 fluid in one octant, FP32: 721 us per interval with an atomic each, 386
+// so); in the other tiles, where one cell in
+// 20,000 overflows, the shuffle's convergence costs 0.7 %.
+template <bool kMany>
+__device__ __forceinline__ int pool_node(const BucketGrid &g)
+{
+    if constexpr (!kMany) return atomicAdd(g.n_pool, 1);
+    const unsigned here = __activemask();
+    const int lead = __ffs(here) - 1;
+    int base = 0;
+    if ((int)(threadIdx.x & 31) == lead) base = atomicAdd(g.n_pool, __popc(here));
+    return __shfl_sync(here, base, lead) + __popc(here & lanemask_lt());
+}
+
 // where record number `place` of bucket key goes: its bucket, or a new node of
 // its list
-template <typename R>
+template <typename R, bool kMany>
 __device__ __forceinline__ unsigned char *bucket_place(const BucketGrid &g, int key, int place)
 {
     if (place < g.cap_of(key)) return g.rec + ((size_t)key * g.cap + place) * Bucket<R>::kBytes;
-    const int node = atomicAdd(g.n_pool, 1);
+    const int node = pool_node<kMany>(g);
     g.link[node] = atomicExch(g.head + key, node);
     return g.pool + (size_t)node * Bucket<R>::kBytes;
+}
+
+// FP64: rank and order of the tile's particles by their order words
+template <typename S>
+__device__ __forceinline__ void bucket_rank(BucketTile<double, S> &sh, int np)
+{
+    for (int j = threadIdx.x; j < np; j += S::kThreads) {
+        const int c = sh.cell[j], a = sh.cstart[c], n = sh.ccount[c];
+        const int lo = sh.rec[j][3].z, hi = sh.rec[j][3].w;
+        int r = 0;
+#pragma unroll 4
+        for (int k = a; k < a + n; k++) {
+            const int2 o = *(const int2 *)&sh.rec[k][3].z;
+            r += o.y < hi || (o.y == hi && o.x < lo);
+        }
+        sh.rank[j] = (unsigned short)r;
+        sh.ord[a + r] = (unsigned short)j;
+    }
+}
+
+// Rotates, streams, keys and counts the np particles in shared memory; a record
+// goes out when its place is back (one particle at a time: more warps per SM
+// hide the round trip better than two particles per thread).
+template <typename R, typename S, bool kMany>
+__device__ __forceinline__ void bucket_move_all(const BucketTile<R, S> &sh, const BucketArgs<R> &A, int np)
+{
+    constexpr int Q = Bucket<R>::kChunks;
+    const int t = threadIdx.x, lane = t & 31;
+    const unsigned below = lanemask_lt();
+    for (int jb = 0; jb < np; jb += S::kThreads) {
+        const int j = jb + t;
+        int4 rec[Q];
+        int key = -1, base = 0;
+        if (j < np) key = bucket_move<S>(sh, A, j, rec);
+        const unsigned peers = __match_any_sync(0xffffffffu, key);
+        const int lead = __ffs(peers) - 1;
+        if (j < np && lane == lead) base = atomicAdd(A.out.count + key, __popc(peers));
+        const int place = __shfl_sync(0xffffffffu, base, lead) + __popc(peers & below);
+        if (j < np) {
+            unsigned char *p = bucket_place<R, kMany>(A.out, key, place);
+            store_record(p, rec[0], rec[1]);
+            if constexpr (Q == 4) store_record(p + 32, rec[2], rec[3]);
+        }
+    }
 }
 
 // The particles of an over-full tile (more than fit in shared memory) as
@@ -333,27 +393,77 @@ __device__ inline unsigned long long bucket_order(const unsigned char *p)
     else return ((const unsigned long long *)p)[7];
 }
 
-// An over-full tile: the block takes one cell after the other, reading the
-// records where they are
-template <typename R, typename S>
-__device__ __noinline__ void bucket_dense_tile(BucketTile<R, S> &sh, const BucketArgs<R> &A, int b0, int n, int a, int np)
+// FP64: a run of cells of an over-full tile whose m particles ids[0, m) fit in shared
+// memory; n: the particles of this thread's cell in the run, a: its first one.  In
+// turn, cell by cell as below, a resting 48^3 fluid in one octant took 1074 us per
+// interval for 347; the FP32 form, which has no ranks to make, gains nothing from it
+// and its kernel would spill.
+template <typename S>
+__device__ __noinline__ void bucket_dense_run(BucketTile<double, S> &sh, const BucketArgs<double> &A, int b0, int n,
+                                                 int a, int m, const int *ids)
 {
-    constexpr int W = Bucket<R>::kBytes / 4;
     const int t = threadIdx.x;
-    __shared__ int s_base, s_eff;
-    __shared__ unsigned long long s_sum[3];
-    if (t == 0) s_base = atomicAdd(A.in.n_pool + 3, np);
+    if (m == 0) return;
     if (t < S::kSlots) {
         sh.cstart[t] = a;
         sh.ccount[t] = n;
+        if (n > 0) {
+            const int slot = A.map.slot_of ? A.map.slot_of[b0 + t] : b0 + t;
+            sh.slot[t] = slot;
+            if (n > 1) {
+                const CellRot<double> o = cell_rotation<double>(slot, A);
+                for (int i = 0; i < 9; i++) sh.mat[t][4 * (i / 3) + i % 3] = o.m[i / 3][i % 3];
+            }
+            for (int k = 0; k < n; k++) sh.cell[a + k] = (unsigned char)t;
+        }
     }
     __syncthreads();
+    for (int j = t; j < m; j += S::kThreads) {
+        const int4 *p = (const int4 *)bucket_record<double>(A.in, b0 + sh.cell[j], ids[j]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) sh.rec[j][q] = p[q];
+    }
+    __syncthreads();
+    bucket_rank<S>(sh, m);
+    __syncthreads();
+    bucket_means<S>(sh);
+    __syncthreads();
+    bucket_move_all<double, S, true>(sh, A, m);
+}
+
+// An over-full tile: cell by cell, the records read where they are; FP64 in runs
+// of the next cells that fit in shared memory as long as there are any
+template <typename R, typename S>
+__device__ __noinline__ void bucket_dense_tile(BucketTile<R, S> &sh, const BucketArgs<R> &A, int b0, int n, int a, int np)
+{
+    constexpr int W = Bucket<R>::kBytes / 4, SL = S::kSlots, CAP = S::kCap;
+    const int t = threadIdx.x;
+    __shared__ int s_base, s_eff;
+    __shared__ int s_first[SL + 1];  // each cell's first particle in the tile
+    __shared__ unsigned long long s_sum[3];
+    if (t == 0) {
+        s_base = atomicAdd(A.in.n_pool + 3, np);
+        s_first[SL] = np;
+    }
+    if (t < SL) s_first[t] = a;
+    __syncthreads();
     int *ids = A.ids + s_base, *tmp = A.ids_tmp + s_base;
-    if (t < S::kSlots) bucket_list(A.in, b0 + t, n, ids + a);
-    for (int c = 0; c < S::kSlots; c++) {
-        const int m = sh.ccount[c], b = b0 + c;
+    if (t < SL) bucket_list(A.in, b0 + t, n, ids + a);
+    int run = 1;
+    for (int c = 0; c < SL; c += run) {
+        const int f = s_first[c];
+        if constexpr (sizeof(R) == 8) {
+            // (its barrier also ends the run before)
+            run = __syncthreads_count(t >= c && t < SL && a + n - f <= CAP);
+            if (run > 0) {
+                bucket_dense_run<S>(sh, A, b0, t >= c && t < c + run ? n : 0, a - f, s_first[c + run] - f, ids + f);
+                continue;
+            }
+        }
+        run = 1;
+        const int m = s_first[c + 1] - f, b = b0 + c;
         if (m == 0) continue;
-        int *id = ids + sh.cstart[c];
+        int *id = ids + f;
         const int slot = A.map.slot_of ? A.map.slot_of[b] : b;
         if (t < 3) s_sum[t] = 0;
         if (t == 0) s_eff = 0;
@@ -376,7 +486,7 @@ __device__ __noinline__ void bucket_dense_tile(BucketTile<R, S> &sh, const Bucke
             if (n_eff > 1)
                 for (int i = 0; i < 3; i++) lv[i] = fixed_mean((long long)s_sum[i], n_eff);
         } else {
-            block_merge_sort(id, tmp + sh.cstart[c], m,
+            block_merge_sort(id, tmp + f, m,
                              [&](int q) { return bucket_order<R>(bucket_record<R>(A.in, b, q)); });
             if (t < 3) {
                 double s = 0;
@@ -407,7 +517,7 @@ __device__ __noinline__ void bucket_dense_tile(BucketTile<R, S> &sh, const Bucke
                 w[14] = k;
                 w[15] = slot;
             }
-            int *o = (int *)bucket_place<R>(A.out, key, atomicAdd(A.out.count + key, 1));
+            int *o = (int *)bucket_place<R, true>(A.out, key, atomicAdd(A.out.count + key, 1));
             for (int i = 0; i < W; i++) o[i] = w[i];
         }
         __syncthreads();
@@ -464,24 +574,6 @@ __device__ __forceinline__ void bucket_drained(BucketTile<R, S> &sh, bool arrive
     if (!arrived && !mbar_wait_bounded(&sh.bar, 0, kBulkPolls)) atomicOr(err, DEV_ERR_BULK_UNDRAINED);
 }
 
-// FP64: rank and order of the tile's particles by their order words
-template <typename S>
-__device__ __forceinline__ void bucket_rank(BucketTile<double, S> &sh, int np)
-{
-    for (int j = threadIdx.x; j < np; j += S::kThreads) {
-        const int c = sh.cell[j], a = sh.cstart[c], n = sh.ccount[c];
-        const int lo = sh.rec[j][3].z, hi = sh.rec[j][3].w;
-        int r = 0;
-#pragma unroll 4
-        for (int k = a; k < a + n; k++) {
-            const int2 o = *(const int2 *)&sh.rec[k][3].z;
-            r += o.y < hi || (o.y == hi && o.x < lo);
-        }
-        sh.rank[j] = (unsigned short)r;
-        sh.ord[a + r] = (unsigned short)j;
-    }
-}
-
 // Bound by the round trips of each particle (cell table, counting atomic), the
 // load/store pipe (69 % of its cycles at 96^3 FP32) and issue (66 %), not by HBM
 // (3.3 TB/s at 128^3), so occupancy decides: one particle per thread in flight,
@@ -534,26 +626,7 @@ __global__ void __launch_bounds__(S::kThreads, S::kMinBlocks) k_bucket_interval(
     }
     bucket_means<S>(sh);
     __syncthreads();
-    // rotate, stream, key and count; the record goes out when its place is back
-    // (one particle at a time: more warps per SM hide the round trip better than
-    // two particles per thread)
-    constexpr int Q = Bucket<R>::kChunks;
-    const unsigned below = lanemask_lt();
-    for (int jb = 0; jb < np; jb += S::kThreads) {
-        const int j = jb + t;
-        int4 rec[Q];
-        int key = -1, base = 0;
-        if (j < np) key = bucket_move<S>(sh, A, j, rec);
-        const unsigned peers = __match_any_sync(0xffffffffu, key);
-        const int lead = __ffs(peers) - 1;
-        if (j < np && lane == lead) base = atomicAdd(A.out.count + key, __popc(peers));
-        const int place = __shfl_sync(0xffffffffu, base, lead) + __popc(peers & below);
-        if (j < np) {
-            unsigned char *p = bucket_place<R>(A.out, key, place);
-            store_record(p, rec[0], rec[1]);
-            if constexpr (Q == 4) store_record(p + 32, rec[2], rec[3]);
-        }
-    }
+    bucket_move_all<R, S, false>(sh, A, np);
     bucket_drained<R, S>(sh, arrived, A.err);
 }
 

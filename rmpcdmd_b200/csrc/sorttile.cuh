@@ -42,7 +42,7 @@ struct OrderTile {
 
 // The n values a[0, n), with distinct keys, into ascending order of their keys
 // by the whole block; b is scratch of the same extent.  Pieces of 32 by rank, then
-// runs merged two by two, a thread taking 32 places of the result at a time:
+// runs merged two by two, a thread taking up to 32 places of the result at a time:
 // where they begin in the two runs takes one search, the rest is a walk along
 // both.  (A search per element made a sort of the system with 276,000 particles in one
 // cell take 18.4 ms; now 6.4, of which this is a part.)
@@ -59,9 +59,11 @@ __device__ inline void block_merge_sort(int *a, int *b, int n, Key key)
         b[q + r] = v;
     }
     __syncthreads();
+    int per = 1;
+    while (per < P && per * T < n) per <<= 1;
     int *src = b, *dst = a;
     for (long long w = P; w < n; w <<= 1) {
-        for (long long o = (long long)P * threadIdx.x; o < n; o += (long long)P * T) {
+        for (long long o = (long long)per * threadIdx.x; o < n; o += (long long)per * T) {
             const long long p = o / (2 * w) * (2 * w);
             const int na = (int)min(w, n - p), nb = (int)max(0LL, min(w, n - p - w)), d = (int)(o - p);
             const int *A = src + p, *B = A + na;
@@ -73,7 +75,7 @@ __device__ inline void block_merge_sort(int *a, int *b, int n, Key key)
                 else hi = mid;
             }
             int i = lo, j = d - lo;
-            const int e = min(P, na + nb - d);
+            const int e = min(per, na + nb - d);
             int va = i < na ? A[i] : 0, vb = j < nb ? B[j] : 0;
             decltype(key(0)) ka = 0, kb = 0;
             if (i < na) ka = key(va);
