@@ -732,26 +732,40 @@ static double mean_occupancy(const rmpcd_particles *p, const rmpcd_cells *c)
     return (double)p->N / (double)box_cells(c);
 }
 
-// The shape of a run: the one set, or the first of by_wave whose blocks hold all
-// cells of the box at once, or else the one for boxes of several waves.  A tile's block
-// is a chain of latencies (record copy, collision, counting atomics), so a
-// small box takes the shape with the most threads per particle, as long as its
-// tiles all run at once; many small blocks, with few warps waiting at each
-// barrier, are best for a large box; and a box just above one wave of those
-// takes a wider tile that fits.  us per interval (slots x blocks per SM x
-// threads): 16^3 FP32 9.3 (16 x 6 x 256), 12.7 (24 x 16 x 96), FP64 9.4 (16 x 5 x
-// 256), 13.4 (24 x 8 x 128); 24^3 FP32 12.2, 14.3, FP64 16.4, 15.1; 32^3 FP32
-// 20.6, 15.8, FP64 25.2, 25.7; 61,500 cells FP32 25.5 (24 x 16 x 96), 23.1 (72 x 6
-// x 256); 128^3 FP32 521 (24 x 16 x 96), 531 (32 x 12 x 128), 546 (72 x 6 x 256),
-// FP64 931 (24 x 8 x 128), 963 (40 x 5 x 256), 989 (48 x 4 x 256).
+// whether a shape's tiles hold a mean occupancy with 5 standard deviations to
+// spare (up to density 11, 10.7 for the 72-cell shape)
 template <typename R>
-static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c)
+static bool holds(const ShapeEntry<R> &e, double mean)
+{
+    const double tile = mean * e.slots;
+    return tile + 5 * sqrt(tile) <= e.cap;
+}
+
+// The shape of a run: the one set, or the first of by_wave whose tiles hold the
+// mean occupancy and whose blocks hold all cells of the box at once, or else the one
+// for boxes of several waves.  A tile's block is a chain of latencies (record copy,
+// collision, counting atomics), so a small box takes the shape with the most threads
+// per particle, as long as its tiles all run at once; many small blocks, with few
+// warps waiting at each barrier, are best for a large box; and a box just above one
+// wave of those (56,832 cells on 148 SMs) takes the 72-cell tiles if it is one wave
+// of them (63,936).  Between one and two waves the small blocks are best again, since
+// blocks of a second wave start as the first ones end.  us per interval by cells,
+// FP32 with 16 x 6 x 256 (cells x blocks per SM x threads), 24 x 16 x 96, 72 x 6 x 256:
+//   4,096  8.8 11.2 13.1    13,824 11.2 13.0 13.6    15,000 13.3 13.3 13.8    32,768 19.2 14.6 15.8
+//   54,872 37.5 20.8 20.7   59,280 39.5 23.2 20.9    61,500 32.1 23.0 20.7    62,400 40.5 24.4 21.6
+//   64,000 41.7 24.7 24.9   74,088 44.1 25.6 27.9    112,896 59.2 33.3 34.8   120,000 61.4 36.9 36.6
+//   127,500 65.4 39.1 38.4  140,608 70.1 41.7 44.0   262,144 112 69.1 74.1    2,097,152 846 467 493
+// FP64 with 16 x 5 x 256, 24 x 8 x 128, 40 x 5 x 256 (the 48-cell tiles are within 1 %):
+//   4,096  8.8 12.8 11.7    8,000 11.1 13.2 13.2     13,824 15.3 14.3 14.8    32,768 24.0 24.1 25.0
+//   54,872 51.9 33.5 35.4   112,896 84.3 59.7 62.6   262,144 160 120 128      2,097,152 1218 871 928
+template <typename R>
+static const ShapeEntry<R> &pick_shape(const rmpcd_cells *c, double mean)
 {
     const int set = g_shape[sizeof(R) == 8];
     if (set >= 0) return Shapes<R>::list[set];
     for (int k : Shapes<R>::by_wave) {
         const ShapeEntry<R> &e = Shapes<R>::list[k];
-        if (box_cells(c) <= (long long)e.slots * e.min_blocks * sm_count()) return e;
+        if (holds(e, mean) && box_cells(c) <= (long long)e.slots * e.min_blocks * sm_count()) return e;
     }
     return Shapes<R>::list[kLargeBox];
 }
@@ -879,10 +893,9 @@ static void next_origin(const rmpcd_rng *r, double origin[3])
 
 template <typename R>
 static int bulk_run_buckets(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double tau, int has_alpha, double alpha,
-                            int n_intervals, int cap)
+                            int n_intervals, int cap, const ShapeEntry<R> &shape)
 {
     cudaStream_t st = stream();
-    const ShapeEntry<R> &shape = pick_shape<R>(c);
     int rc = ensure_bucket_map(c);
     if (rc) return rc;
     BucketMap map{nullptr, nullptr};
@@ -1083,13 +1096,13 @@ static int bulk_run_t(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double t
 {
     int rc = prepare_shapes<R>();
     if (rc) return rc;
-    const ShapeEntry<R> &shape = pick_shape<R>(c);
-    const double mean = mean_occupancy(p, c), tile = mean * shape.slots;
-    bool buckets = tile + 5 * sqrt(tile) <= shape.cap;
+    const double mean = mean_occupancy(p, c);
+    const ShapeEntry<R> &shape = pick_shape<R>(c, mean);
+    bool buckets = holds(shape, mean);
     const int cap = bucket_cap(mean);
     if (buckets) rc = ensure_buckets<R>(p, c->S, c->n_lut, cap, &buckets);
     if (rc) return rc;
-    if (buckets) return bulk_run_buckets<R>(p, c, r, tau, has_alpha, alpha, n_intervals, cap);
+    if (buckets) return bulk_run_buckets<R>(p, c, r, tau, has_alpha, alpha, n_intervals, cap, shape);
     return bulk_run_fused<R>(p, c, r, tau, has_alpha, alpha, n_intervals);
 }
 
