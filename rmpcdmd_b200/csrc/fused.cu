@@ -811,14 +811,11 @@ __global__ void k_bucket_lut(const int *lut, int n_lut, const int *of_slot, int 
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_lut; c += gridDim.x * blockDim.x) out[c] = of_slot[lut[c]];
 }
 
-// uses c->count_next (zero between runs) and c->cursor as scratch
-static int ensure_bucket_map(rmpcd_cells *c)
+// the numbering into map (of_slot, slot_of, the cells' buckets); uses
+// c->count_next, zero before and after, and c->cursor as scratch
+static int number_buckets(rmpcd_cells *c, int *map)
 {
-    if (c->n_lut == c->S || c->bucket_map) return RMPCD_OK;
     cudaStream_t st = stream();
-    int *map = nullptr;
-    RMPCD_CUDA_TRY(cudaMalloc(&map, (2 * (size_t)c->S + c->n_lut) * sizeof(int)));
-    c->bucket_map = map;
     k_mark_cells<<<grid_for(c->n_lut, 256), 256, 0, st>>>(c->lut, c->n_lut, c->count_next);
     const int rc = exclusive_scan(c->count_next, c->cursor, nullptr, c->S, c->scan_tmp, nullptr, st);
     if (rc) return rc;
@@ -826,6 +823,29 @@ static int ensure_bucket_map(rmpcd_cells *c)
     k_bucket_lut<<<grid_for(c->n_lut, 256), 256, 0, st>>>(c->lut, c->n_lut, map, map + 2 * (size_t)c->S);
     RMPCD_CHECK_LAUNCH();
     RMPCD_CUDA_TRY(cudaMemsetAsync(c->count_next, 0, (size_t)c->S * sizeof(int), st));
+    return RMPCD_OK;
+}
+
+// The map of a box with more slots than cells, kept with the cell system once it
+// is complete.  *ok = false when there is no memory for it.
+static int ensure_bucket_map(rmpcd_cells *c, bool *ok)
+{
+    if (c->n_lut == c->S || c->bucket_map) return RMPCD_OK;
+    int *map = nullptr;
+    if (cudaMalloc(&map, (2 * (size_t)c->S + c->n_lut) * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        *ok = false;
+        return RMPCD_OK;
+    }
+    const int rc = number_buckets(c, map);
+    if (rc) {
+        // no marks stay behind in the array that every run expects to be zero
+        cudaMemsetAsync(c->count_next, 0, (size_t)c->S * sizeof(int), stream());
+        cudaStreamSynchronize(stream());
+        cudaFree(map);
+        return rc;
+    }
+    c->bucket_map = map;
     return RMPCD_OK;
 }
 
@@ -896,8 +916,6 @@ static int bulk_run_buckets(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, do
                             int n_intervals, int cap, const ShapeEntry<R> &shape)
 {
     cudaStream_t st = stream();
-    int rc = ensure_bucket_map(c);
-    if (rc) return rc;
     BucketMap map{nullptr, nullptr};
     if (c->bucket_map) map = {c->bucket_map, c->bucket_map + c->S};
     // image, flags and id stay in the current API arrays, addressed by idx
@@ -965,7 +983,7 @@ static int bulk_run_buckets(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, do
         k_bucket_counts_to_slots<<<grid_for(c->S, 256), 256, 0, st>>>(c->cursor, map.slot_of, c->S, c->count);
         RMPCD_CHECK_LAUNCH();
     }
-    rc = exclusive_scan(c->count, c->start, c->cursor, c->S, c->scan_tmp, nullptr, st);
+    int rc = exclusive_scan(c->count, c->start, c->cursor, c->S, c->scan_tmp, nullptr, st);
     if (rc) return rc;
     shape.to_soa<<<nblocks, shape.threads, shape.smem, st>>>(grid(n_intervals), map, c->S, c->count, c->start, side,
                                                              alt<R>(p), p->perm, p->key, dev_error_word());
@@ -1101,6 +1119,7 @@ static int bulk_run_t(rmpcd_particles *p, rmpcd_cells *c, rmpcd_rng *r, double t
     bool buckets = holds(shape, mean);
     const int cap = bucket_cap(mean);
     if (buckets) rc = ensure_buckets<R>(p, c->S, c->n_lut, cap, &buckets);
+    if (!rc && buckets) rc = ensure_bucket_map(c, &buckets);
     if (rc) return rc;
     if (buckets) return bulk_run_buckets<R>(p, c, r, tau, has_alpha, alpha, n_intervals, cap, shape);
     return bulk_run_fused<R>(p, c, r, tau, has_alpha, alpha, n_intervals);
