@@ -50,6 +50,7 @@
 
 #include "keys.cuh"
 #include "nlist_ops.cuh"
+#include "quotient.cuh"
 #include "rmpcd_common.cuh"
 #include "rng.cuh"
 #include "sortcore.cuh"
@@ -537,29 +538,6 @@ struct MdParts {
     __device__ int &num(int field, int s) const { return i[(size_t)field * cap + s]; }
 };
 
-// a / b rounded to nearest for a divisor used again: with y = 1 / b rounded to
-// nearest, two corrections by exact residuals give the correctly rounded
-// quotient (P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34(1), 1990); operands near the ends of the
-// exponent range, zeros and non-finite ones take the division itself.
-struct MdDiv {
-    double b, y;
-    bool safe;
-    __device__ void set(double d)
-    {
-        b = d;
-        y = 1.0 / d;
-        safe = fabs(d) > 1e-100 && fabs(d) < 1e100;
-    }
-    __device__ __forceinline__ double of(double a) const
-    {
-        if (!(safe && fabs(a) > 1e-180 && fabs(a) < 1e180)) return a / b;
-        double q = a * y;
-        q = __fma_rn(__fma_rn(-b, q, a), y, q);
-        return __fma_rn(__fma_rn(-b, q, a), y, q);
-    }
-};
-
 // What the steps need of the replica and the block
 template <typename R>
 struct MdBox {
@@ -582,7 +560,7 @@ struct MdBox {
 // root, each waiting for the one before.
 struct MdBead {
     double pos, vel, force, fold;
-    MdDiv vv, m, kk;       // 2 x own mass; own RATTLE mass; bond^2 (1/m1 + 1/m2)
+    Quotient vv, m, kk;  // 2 x own mass; own RATTLE mass; bond^2 (1/m1 + 1/m2)
     double dt_inv_mass;    // dt (1/m1 + 1/m2)
     double L;
     int i, k, sp0, sp1;
@@ -593,7 +571,7 @@ struct MdBead {
 // the beads' own force (compute_force_n2, src/neighbor_list.f90:227-264)
 struct MdPair {
     double s, rsq, f;
-    MdDiv g;
+    Quotient g;
     bool acts;
 };
 
