@@ -342,16 +342,16 @@ __global__ void __launch_bounds__(kBT)
     }
 }
 
-// *steps <- the first MD step at whose test the free particle i has moved
+// The first MD step before `best` at whose test the free particle i has moved
 // sqrt(d2) >= thr from pos_old (programs/single_dimer_pbc.f90:324-329,
-// src/particle_system.f90:357-378).  A particle's earliest possible step
+// src/particle_system.f90:357-378), or best.  A particle's earliest possible step
 // follows from its speed (reach bounds the distance of one addition, its
 // rounding included); only the particles that could be first -- a few per
 // replica -- go through their additions one by one.
 template <typename R>
-__device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &old, long long i, R vx, R vy, R vz,
+__device__ __forceinline__ int free_crossing(const PView<R> &v, const Vec3<R> &old, long long i, R vx, R vy, R vz,
                                               float reach, int fresh, R dt, double thr, int base, int n_rem,
-                                              int read_species, const int *aidx, int best, int *steps)
+                                              int read_species, const int *aidx, int best)
 {
     float left = (float)thr;
     if (fresh) {
@@ -362,12 +362,12 @@ __device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &
         reach += (sizeof(R) == 4 ? 2.4e-7f : 4.4e-16f) *
                  (fabsf((float)v.pos.x[i]) + fabsf((float)v.pos.y[i]) + fabsf((float)v.pos.z[i]));
     }
-    if (!(reach * (float)n_rem >= left)) return;
+    if (!(reach * (float)n_rem >= left)) return best;
     int lo = left > 0 ? (int)fminf(left / reach, 1e9f) - 1 : 1;  // no crossing before the lo-th addition
     if (lo < 1) lo = 1;
-    if (base + lo - 1 >= best) return;
-    if ((v.flags[i] & kActiveBits) || aidx[i] >= 0) return;
-    if (read_species && v.species[i] < 0) return;
+    if (base + lo - 1 >= best) return best;
+    if ((v.flags[i] & kActiveBits) || aidx[i] >= 0) return best;
+    if (read_species && v.species[i] < 0) return best;
     const R hx = dt * vx, hy = dt * vy, hz = dt * vz;
     R x = v.pos.x[i], y = v.pos.y[i], z = v.pos.z[i];
     const double ox = fresh ? (double)old.x[i] : (double)x, oy = fresh ? (double)old.y[i] : (double)y,
@@ -378,11 +378,9 @@ __device__ __forceinline__ void free_crossing(const PView<R> &v, const Vec3<R> &
         z = z + hz;
         if (j < lo) continue;
         const double d0 = (double)x - ox, d1 = (double)y - oy, d2 = (double)z - oz;
-        if (sqrt(d0 * d0 + d1 * d1 + d2 * d2) >= thr) {
-            atomicMin(steps, base + j - 1);
-            return;
-        }
+        if (sqrt(d0 * d0 + d1 * d1 + d2 * d2) >= thr) return min(best, base + j - 1);
     }
+    return best;
 }
 
 // After kb_claim: the first step at which a free particle forces a re-sort
@@ -413,7 +411,8 @@ __global__ void __launch_bounds__(kBT)
             constexpr int K = 4;
             for (long long i0 = t.begin + threadIdx.x; i0 < t.end; i0 += K * kBT) {
                 R vx[K], vy[K], vz[K];
-                const int best = *(volatile int *)(s_free + t.r);  // so far; it only falls
+                const int so_far = *(volatile int *)(s_free + t.r);  // it only falls
+                int best = so_far;
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     const long long i = i0 + k * kBT;
@@ -423,7 +422,7 @@ __global__ void __launch_bounds__(kBT)
                         vz[k] = v.vel.z[i];
                     }
                 }
-                const float steps = (float)(min(N_MD, best) - b0);
+                const float steps = (float)(min(N_MD, so_far) - b0);
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     const long long i = i0 + k * kBT;
@@ -432,9 +431,15 @@ __global__ void __launch_bounds__(kBT)
                     const float reach = (float)dt * sqrtf(ux * ux + uy * uy + uz * uz) * 1.001f + slack;
                     // (one step more: best is the step of the addition before it)
                     if (fr || reach * (steps + 1.0f) >= (float)thr)
-                        free_crossing<R>(v, old, i, vx[k], vy[k], vz[k], reach, fr, dt, thr, b0, N_MD - b0,
-                                         read_species, aidx, best, s_free + t.r);
+                        best = free_crossing<R>(v, old, i, vx[k], vy[k], vz[k], reach, fr, dt, thr, b0, N_MD - b0,
+                                                read_species, aidx, best);
                 }
+                // one atomic for the threads here, where there is a step to write at
+                // all (with a skin that many particles cross, 32^3 and skin 0.1, one
+                // per particle took 171 us, 11 so)
+                const unsigned here = __activemask();
+                best = __reduce_min_sync(here, best);
+                if (best < so_far && (int)(threadIdx.x & 31) == __ffs(here) - 1) atomicMin(s_free + t.r, best);
             }
         }
         return;
