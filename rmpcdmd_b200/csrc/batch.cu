@@ -46,6 +46,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "keys.cuh"
@@ -147,6 +148,9 @@ struct rmpcd_dimer_batch {
     rmpcd::MdTerm *over = nullptr, *terms = nullptr;
     unsigned long long *keys[2] = {nullptr, nullptr};
     int *n_over = nullptr;
+    // active particles beyond what kb_md holds in shared memory
+    unsigned char *far = nullptr;
+    int far_cap = 0;  // per replica
     int *nf = nullptr;         // per replica: flagged particles, listed in sol->key from the replica's first place
     int *s_free = nullptr;     // per replica: first MD step at which a free particle forces a re-sort
     int *adv = nullptr, *base = nullptr;  // per replica: md_pos steps done this interval, and those in memory
@@ -474,13 +478,13 @@ __global__ void __launch_bounds__(kBT)
 
 // kb_md's block: the warps that add up the pair forces and move the beads
 // (half of them per bead), then those that have the particles; and what it
-// holds of a step in shared memory (a list beyond kMdBits entries or more
-// terms than fit go through md_slow_sums)
+// holds of a step in shared memory (more terms than fit go to global memory; lists
+// of more entries than the map's largest size through md_slow_sums)
 constexpr int kMdSum = 256;
 constexpr int kMdThreads = kMdSum + 512;
 constexpr int kMdQueue = 1024;    // pairs of a particle and a bead that may reach it
 constexpr int kMdTerms = 512;     // pair forces per bead
-constexpr int kMdBits = 16384;    // list entries per bead covered by the bit map
+constexpr int kMdMapWords = 6144; // most words of the map of a bead's list entries
 constexpr size_t kMdSmem = 224 * 1024;  // dynamic shared memory
 // A particle is queued for the next step's pair forces before the beads have
 // moved: within this distance more than the cuts, which is far above a bead's
@@ -507,6 +511,8 @@ struct MdArgs {
     MdTerm *over, *terms;         // 2 * R * Nmax each: terms beyond the shared ones, terms to be put in order
     unsigned long long *keys[2];  // sort keys of the latter
     int *n_over;                  // per bead, one counter per step parity
+    unsigned char *far;           // room for far_cap active particles per replica (MdBox::far)
+    int far_cap;
     const int *s_free, *fresh;
     int *adv, *resort, *n_extra;
     ResortLists rl;
@@ -529,6 +535,11 @@ template <typename R>
 __host__ __device__ constexpr size_t md_part_bytes()
 {
     return 18 * sizeof(R) + 8 * sizeof(int);
+}
+template <typename R>
+__host__ __device__ constexpr size_t md_far_bytes()
+{
+    return 15 * sizeof(R) + 3 * sizeof(int);
 }
 
 // the fields of a block's particles in shared memory, cap of each
@@ -555,7 +566,15 @@ struct MdBox {
     int r, nl, na;        // replica; listed and active particles
     int run[2];           // entries per leaf of the tree, each bead's list
     int cur;              // buffer of the replica's current arrays
+    int words;            // of a bead's map (md_bits)
+    bool all_mapped;      // it covers both lists
     MdParts<R> parts;
+    // The active particles beyond parts.cap: the next far.cap in global memory, field
+    // by field by their place in act (p[3], v[3], o[3], g[3], the step's force; what
+    // the step has for the particle, flags, species), so that a warp reads whole lines,
+    // and any more where they are.  One dimer of sigma = 5 in 40^3 cells, ms per interval FP64, FP32:
+    // 13.2, 8.7 with all of them where they are, 9.5, 5.4 so
+    MdParts<R> far;
 };
 
 // The beads of a replica in warp 0 of its block 0: lane 3 i + k has component k of
@@ -582,7 +601,8 @@ struct MdPair {
 
 // The block's shared memory: the step's bead positions and decisions, the queue
 // of particles that need more than free flight; behind it the pair forces
-// (MdTotals) and the particles, field by field (MdParts).
+// (MdTotals), the maps of the lists' entries (md_bits, md_base) and the particles,
+// field by field (MdParts).
 //
 // What orders the words that both groups of warps use.  A step k has two points
 // between the groups: kBarForces, at which the particles' warps arrive without
@@ -607,7 +627,9 @@ struct MdShared {
     int stop, over[2];
     int last;               // this block is the launch's last
     int anew;               // a bead went farther than kMdWay (written like stop, read by the particles before kBarForces)
-    int spill;              // step + 1 of the last one with a term in global memory (written before kBarForces, read after it)
+    // step + 1 of the last one with a term in global memory, and with one whose place
+    // is beyond the map (written before kBarForces, read after it)
+    int spill, unmapped;
     // by step parity: particles queued for step k (counted by the particles after
     // kBarForces(k - 1), read by them before kBarForces(k), cleared by the beads
     // between that and kBarTurn(k)); pair forces per bead (counted before
@@ -622,10 +644,33 @@ struct MdShared {
 // it, and what puts them in order
 struct MdTotals {
     double f[2][3][kMdTerms], g[2][3][kMdTerms];  // as they come, and in order
-    int2 te[2][kMdTerms];                 // step + 1, place in the order of addition
-    unsigned bits[2][kMdBits / 32];       // places with a term in this step
-    unsigned short base[2][kMdBits / 32]; // terms before each word's places
+    int2 te[2][kMdTerms];                         // step + 1, place in the order of addition
 };
+
+template <typename R>
+__host__ __device__ constexpr size_t md_totals_at()
+{
+    return (sizeof(MdShared<R>) + 15) & ~(size_t)15;
+}
+template <typename R>
+__host__ __device__ constexpr size_t md_map_at()
+{
+    return (md_totals_at<R>() + sizeof(MdTotals) + 15) & ~(size_t)15;
+}
+// Bead i's map: the places in its order of addition that have a term in this step,
+// and the terms before each word's places (at offsets from the block's shared memory
+// itself, not through a pointer, which would make every access a generic one)
+template <typename R>
+__device__ __forceinline__ unsigned *md_bits(const MdBox<R> &B, int i)
+{
+    extern __shared__ __align__(16) unsigned char md_smem[];
+    return reinterpret_cast<unsigned *>(md_smem + md_map_at<R>()) + i * B.words;
+}
+template <typename R>
+__device__ __forceinline__ int *md_base(const MdBox<R> &B, int i)
+{
+    return reinterpret_cast<int *>(md_bits(B, 2 + i));
+}
 
 // the block's named barriers: of the summing warps, and between them and the
 // particles' warps (arrive: without waiting)
@@ -695,24 +740,19 @@ __device__ __forceinline__ int md_busy(const double *X, const MdBox<R> &B, const
     return (d[0] > reach_sq ? 0 : 1) | (d[1] > reach_sq ? 0 : 2) | ((f & kActiveBits) ? 4 : 0);
 }
 
+// where active particle i is kept during the launch
+constexpr int kShared = 0, kFar = 1, kInPlace = 2;
 template <typename R>
-__device__ __forceinline__ Part<R> md_read(const MdBox<R> &B, const MdArgs<R> &A, int i, int &idx, bool from_old)
+__device__ __forceinline__ int md_tier(const MdBox<R> &B, int i)
+{
+    return i < B.parts.cap ? kShared : i - B.parts.cap < B.far.cap ? kFar : kInPlace;
+}
+
+// from the particle arrays
+template <typename R>
+__device__ __forceinline__ Part<R> md_read_in_place(const MdBox<R> &B, const MdArgs<R> &A, int idx)
 {
     Part<R> q;
-    if (i < B.parts.cap && !from_old) {
-        idx = B.parts.num(0, i);
-        q.f = B.parts.num(1, i);
-        q.sp = B.parts.num(2, i);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            q.p[k] = B.parts.real(k, i);
-            q.v[k] = B.parts.real(3 + k, i);
-            q.o[k] = B.parts.real(6 + k, i);
-            q.g[k] = B.parts.real(9 + k, i);
-        }
-        return q;
-    }
-    idx = A.act[B.off + i];
     q.f = md_view(A, B).flags[idx];
     q.sp = md_view(A, B).species[idx];
     const bool forced = q.f & ((1 << MD_BIT) | (1 << PAST_MD_BIT));
@@ -725,23 +765,9 @@ __device__ __forceinline__ Part<R> md_read(const MdBox<R> &B, const MdArgs<R> &A
     }
     return q;
 }
-
-// in_place: to the particle arrays (those beyond the shared memory, and every
-// one at the end)
 template <typename R>
-__device__ __forceinline__ void md_write(const MdBox<R> &B, const MdArgs<R> &A, int i, int idx, const Part<R> &q, bool in_place)
+__device__ __forceinline__ void md_write_in_place(const MdBox<R> &B, const MdArgs<R> &A, int idx, const Part<R> &q)
 {
-    if (i < B.parts.cap && !in_place) {
-        B.parts.num(1, i) = q.f;
-        B.parts.num(2, i) = q.sp;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            B.parts.real(k, i) = q.p[k];
-            B.parts.real(3 + k, i) = q.v[k];
-            B.parts.real(9 + k, i) = q.g[k];
-        }
-        return;
-    }
     md_view(A, B).flags[idx] = q.f;
     md_view(A, B).species[idx] = q.sp;
 #pragma unroll
@@ -749,6 +775,47 @@ __device__ __forceinline__ void md_write(const MdBox<R> &B, const MdArgs<R> &A, 
         md_view(A, B).pos[k][idx] = q.p[k];
         md_view(A, B).vel[k][idx] = q.v[k];
         md_view(A, B).force[k][idx] = q.g[k];
+    }
+}
+
+// from, and to, where particle i is kept
+template <int kTier, typename R>
+__device__ __forceinline__ Part<R> md_read(const MdBox<R> &B, const MdArgs<R> &A, int i)
+{
+    if constexpr (kTier == kInPlace) {
+        return md_read_in_place(B, A, A.act[B.off + i]);
+    } else {
+        const MdParts<R> &m = kTier == kShared ? B.parts : B.far;
+        const int s = kTier == kShared ? i : i - B.parts.cap;
+        Part<R> q;
+        q.f = m.num(1, s);
+        q.sp = m.num(2, s);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            q.p[k] = m.real(k, s);
+            q.v[k] = m.real(3 + k, s);
+            q.o[k] = m.real(6 + k, s);
+            q.g[k] = m.real(9 + k, s);
+        }
+        return q;
+    }
+}
+template <int kTier, typename R>
+__device__ __forceinline__ void md_write(const MdBox<R> &B, const MdArgs<R> &A, int i, const Part<R> &q)
+{
+    if constexpr (kTier == kInPlace) {
+        md_write_in_place(B, A, A.act[B.off + i], q);
+    } else {
+        const MdParts<R> &m = kTier == kShared ? B.parts : B.far;
+        const int s = kTier == kShared ? i : i - B.parts.cap;
+        m.num(1, s) = q.f;
+        m.num(2, s) = q.sp;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            m.real(k, s) = q.p[k];
+            m.real(3 + k, s) = q.v[k];
+            m.real(9 + k, s) = q.g[k];
+        }
     }
 }
 
@@ -787,20 +854,23 @@ __device__ __forceinline__ void md_push(MdShared<R> &sh, const MdBox<R> &B, cons
     const int par = k & 1;
     for (int t = 0; t < times; t++) {
         const int s = atomicAdd(&sh.cnt[par][i], 1), o = md_order<R>(e, B.run[i]);
-        if (s < kMdTerms && o < kMdBits) {
-            atomicOr(&tot.bits[i][o >> 5], 1u << (o & 31));
+        const bool mapped = (o >> 5) < B.words;
+        if (mapped) atomicOr(md_bits(B, i) + (o >> 5), 1u << (o & 31));
+        if (mapped && s < kMdTerms) {
             tot.te[i][s] = make_int2(k + 1, o);
             tot.f[i][0][s] = f0;
             tot.f[i][1][s] = f1;
             tot.f[i][2][s] = f2;
         } else {
             const int b = 2 * B.r + i;
-            MdTerm *g = A.over + (size_t)b * A.Nmax + atomicAdd(A.n_over + 2 * b + par, 1);
+            const int at = B.all_mapped ? s - kMdTerms : atomicAdd(A.n_over + 2 * b + par, 1);
+            MdTerm *g = A.over + (size_t)b * A.Nmax + at;
             g->e = o;
             g->f[0] = f0;
             g->f[1] = f1;
             g->f[2] = f2;
             sh.spill = k + 1;
+            if (!mapped) sh.unmapped = k + 1;
         }
         if (t + 1 < times) e = A.next[(size_t)(2 * B.r + i) * A.Nmax + e];
     }
@@ -925,10 +995,10 @@ __device__ __forceinline__ void md_tree_warp(MdShared<R> &sh, double3 leaf, int 
     }
 }
 
-// Pair forces that do not all fit in shared memory (beads larger than sigma = 4
-// at density 10): both beads' terms are put in order in global memory and added
-// from there, half of the summing warps per bead (FP32: up to the tree's warp
-// level).
+// A list whose entries the map does not cover (more than 196,608: beads of sigma = 12
+// at density 10): both beads' terms are put in order in global memory by their places
+// and added from there, half of the summing warps per bead (FP32: up to the tree's
+// warp level).
 template <typename R>
 __device__ __noinline__ void md_slow_sums(MdShared<R> &sh, const MdArgs<R> &A, const MdTotals &tt, int r, int k)
 {
@@ -1004,11 +1074,37 @@ __device__ __noinline__ void md_slow_sums(MdShared<R> &sh, const MdArgs<R> &A, c
     }
 }
 
+// acc and the m terms g[0, m) one after another
+__device__ __forceinline__ double md_chain(double acc, const double *g, int m)
+{
+    int j = 0;
+    if (m >= 8) {
+        double v[8], u[8];
+#pragma unroll
+        for (int c = 0; c < 8; c++) v[c] = g[c];
+        for (; j + 16 <= m; j += 8) {
+#pragma unroll
+            for (int c = 0; c < 8; c++) u[c] = g[j + 8 + c];
+#pragma unroll
+            for (int c = 0; c < 8; c++) acc = acc + v[c];
+#pragma unroll
+            for (int c = 0; c < 8; c++) v[c] = u[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 8; c++) acc = acc + v[c];
+        j += 8;
+    }
+    for (; j < m; j++) acc = acc + g[j];
+    return acc;
+}
+
 // sh.f[h] = the sum of bead h's pair forces (src/neighbor_list.f90:214-218), half
 // of the summing warps per bead.  The bit map gives every term its place among
 // the step's terms; the FP64 form adds them one after another in list order,
 // one thread per component, as the reference does; the FP32 form adds each
-// leaf's terms and then up colloid_tree_block's tree.
+// leaf's terms and then up colloid_tree_block's tree.  In order they stand in shared
+// memory, or in the bead's part of A.terms, component by component, in a step with
+// more of them (beads larger than sigma = 4 at density 10).
 template <typename R>
 __device__ __forceinline__ void md_colloid_sums(MdShared<R> &sh, MdTotals &tt, const MdArgs<R> &A, int r, int n0,
                                                 int n1, int k)
@@ -1016,16 +1112,20 @@ __device__ __forceinline__ void md_colloid_sums(MdShared<R> &sh, MdTotals &tt, c
     constexpr int H = kMdSum / 2;
     const int h = threadIdx.x / H, t = threadIdx.x % H, lane = t & 31, w = t >> 5;
     const int n = h ? n1 : n0;
-    if (sh.spill == k + 1) {
+    if (sh.unmapped == k + 1) {
         md_slow_sums<R>(sh, A, tt, r, k);
     } else {
         // terms before each word: a warp per bead, runs of words per lane
+        const unsigned *bits = md_bits(sh.box, h);
+        int *base = md_base(sh.box, h);
         const int places = sizeof(R) == 8 ? n : kNlBlockThreads * sh.box.run[h];
-        const int words = min((places + 31) / 32, kMdBits / 32), m = sh.cnt[k & 1][h];
+        const int words = min((places + 31) / 32, sh.box.words), m = sh.cnt[k & 1][h];
+        const bool spilled = sh.spill == k + 1;
+        double *far = (double *)(A.terms + (size_t)(2 * r + h) * A.Nmax);
         if (w == 0) {
             const int per = (words + 31) / 32, q0 = min(words, lane * per), q1 = min(words, q0 + per);
             int c = 0;
-            for (int q = q0; q < q1; q++) c += __popc(tt.bits[h][q]);
+            for (int q = q0; q < q1; q++) c += __popc(bits[q]);
             int inc = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -1034,47 +1134,48 @@ __device__ __forceinline__ void md_colloid_sums(MdShared<R> &sh, MdTotals &tt, c
             }
             int run = inc - c;
             for (int q = q0; q < q1; q++) {
-                tt.base[h][q] = (unsigned short)run;
-                run += __popc(tt.bits[h][q]);
+                base[q] = run;
+                run += __popc(bits[q]);
             }
         }
         md_sync(kBarSum, kMdSum);
-        // the terms before place o (none is beyond the map, or it would have
-        // gone to global memory)
-        auto before = [&](int o) {
-            return o >= kMdBits ? m : tt.base[h][o >> 5] + __popc(tt.bits[h][o >> 5] & ((1u << (o & 31)) - 1u));
-        };
+        // the terms before place o
+        auto before = [&](int o) { return (o >> 5) >= words ? m : base[o >> 5] + __popc(bits[o >> 5] & ((1u << (o & 31)) - 1u)); };
         // into order
-        for (int j = t; j < m; j += H) {
-            const int at = before(tt.te[h][j].y);
-            tt.g[h][0][at] = tt.f[h][0][j];
-            tt.g[h][1][at] = tt.f[h][1][j];
-            tt.g[h][2][at] = tt.f[h][2][j];
+        if (!spilled) {
+            for (int j = t; j < m; j += H) {
+                const int at = before(tt.te[h][j].y);
+                tt.g[h][0][at] = tt.f[h][0][j];
+                tt.g[h][1][at] = tt.f[h][1][j];
+                tt.g[h][2][at] = tt.f[h][2][j];
+            }
+        } else {
+            const MdTerm *over = A.over + (size_t)(2 * r + h) * A.Nmax;
+            for (int j = t; j < m; j += H) {
+                const bool in = j < kMdTerms;
+                const int at = before(in ? tt.te[h][j].y : __ldcg(&over[j - kMdTerms].e));
+                for (int c = 0; c < 3; c++)
+                    far[(size_t)c * A.Nmax + at] = in ? tt.f[h][c][j] : __ldcg(&over[j - kMdTerms].f[c]);
+            }
         }
         md_sync(kBarSum, kMdSum);
         if constexpr (sizeof(R) == 8) {
-            if (t < 3) {
-                const double *g = tt.g[h][t];
+            if (!spilled) {
+                if (t < 3) sh.f[h][t] = md_chain(0.0, tt.g[h][t], m);
+            } else {
+                // a part at a time into shared memory: the chain of adds is not to
+                // wait for a line from L2 every 16 terms
+                const int most = max(sh.cnt[k & 1][0], sh.cnt[k & 1][1]);
                 double acc = 0;
-                int j = 0;
-                if (m >= 8) {
-                    double v[8], u[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) v[c] = g[c];
-                    for (; j + 16 <= m; j += 8) {
-#pragma unroll
-                        for (int c = 0; c < 8; c++) u[c] = g[j + 8 + c];
-#pragma unroll
-                        for (int c = 0; c < 8; c++) acc = acc + v[c];
-#pragma unroll
-                        for (int c = 0; c < 8; c++) v[c] = u[c];
-                    }
-#pragma unroll
-                    for (int c = 0; c < 8; c++) acc = acc + v[c];
-                    j += 8;
+                for (int c0 = 0; c0 < most; c0 += kMdTerms) {
+                    const int mc = min(kMdTerms, m - c0);
+                    for (int j = t; j < mc; j += H)
+                        for (int c = 0; c < 3; c++) tt.g[h][c][j] = far[(size_t)c * A.Nmax + c0 + j];
+                    md_sync(kBarSum, kMdSum);
+                    if (t < 3) acc = md_chain(acc, tt.g[h][t], mc);
+                    md_sync(kBarSum, kMdSum);
                 }
-                for (; j < m; j++) acc = acc + g[j];
-                sh.f[h][t] = acc;
+                if (t < 3) sh.f[h][t] = acc;
             }
         } else {
             const int run = sh.box.run[h];
@@ -1082,10 +1183,18 @@ __device__ __forceinline__ void md_colloid_sums(MdShared<R> &sh, MdTotals &tt, c
                 const int l = t + q * H;
                 const int lo = run ? before(l * run) : 0, hi = run && l < kNlBlockThreads - 1 ? before((l + 1) * run) : m;
                 double3 leaf = make_double3(0, 0, 0);
-                for (int j = lo; j < hi; j++) {
-                    leaf.x = leaf.x + tt.g[h][0][j];
-                    leaf.y = leaf.y + tt.g[h][1][j];
-                    leaf.z = leaf.z + tt.g[h][2][j];
+                if (!spilled) {
+                    for (int j = lo; j < hi; j++) {
+                        leaf.x = leaf.x + tt.g[h][0][j];
+                        leaf.y = leaf.y + tt.g[h][1][j];
+                        leaf.z = leaf.z + tt.g[h][2][j];
+                    }
+                } else {
+                    for (int j = lo; j < hi; j++) {
+                        leaf.x = leaf.x + far[j];
+                        leaf.y = leaf.y + far[(size_t)A.Nmax + j];
+                        leaf.z = leaf.z + far[2 * (size_t)A.Nmax + j];
+                    }
                 }
                 md_tree_warp(sh, leaf, h, l);
             }
@@ -1214,10 +1323,9 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
 {
     extern __shared__ __align__(16) unsigned char md_smem[];
     MdShared<R> &sh = *reinterpret_cast<MdShared<R> *>(md_smem);
-    constexpr size_t kHead = (sizeof(MdShared<R>) + 15) & ~(size_t)15;
-    constexpr size_t kParts = (kHead + sizeof(MdTotals) + 15) & ~(size_t)15;
-    static_assert(kParts + 64 * 1024 <= kMdSmem, "room for particles");
-    MdTotals &totals = *reinterpret_cast<MdTotals *>(md_smem + kHead);
+    constexpr size_t kMap = md_map_at<R>();
+    static_assert(kMap + 16 * (size_t)kMdMapWords + 32 * 1024 <= kMdSmem, "room for particles");
+    MdTotals &totals = *reinterpret_cast<MdTotals *>(md_smem + md_totals_at<R>());
     const int r = blockIdx.x;
     const int t = threadIdx.x;
     const int all = blockDim.x;
@@ -1243,20 +1351,28 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
             W.nl = A.nl[r];
             W.na = W.nl + A.nx[r];
             for (int h = 0; h < 2; h++) W.run[h] = (A.n[2 * r + h] + kNlBlockThreads - 1) / kNlBlockThreads;
-            W.parts.cap = (int)((kMdSmem - kParts) / md_part_bytes<R>());
-            W.parts.r = reinterpret_cast<R *>(md_smem + kParts);
+            // (the FP32 form's leaves are of whole runs)
+            const int places = kNlBlockThreads * max(W.run[0], W.run[1]);
+            W.words = min(kMdMapWords, places / 32);
+            W.all_mapped = 32 * W.words == places;
+            const size_t parts = kMap + 16 * (size_t)W.words;
+            W.parts.cap = (int)((kMdSmem - parts) / md_part_bytes<R>());
+            W.parts.r = reinterpret_cast<R *>(md_smem + parts);
+            W.far.cap = A.far_cap;
+            W.far.r = reinterpret_cast<R *>(A.far + (size_t)r * A.far_cap * md_far_bytes<R>());
+            W.far.i = reinterpret_cast<int *>(W.far.r + 15 * (size_t)A.far_cap);
             W.parts.i = reinterpret_cast<int *>(W.parts.r + 18 * (size_t)W.parts.cap);
-            sh.stop = sh.over[0] = sh.over[1] = sh.spill = 0;
+            sh.stop = sh.over[0] = sh.over[1] = sh.spill = sh.unmapped = 0;
             sh.anew = 1;
             for (int p = 0; p < 2; p++) {
                 sh.nq[p] = sh.cnt[p][0] = sh.cnt[p][1] = 0;
                 A.n_over[4 * r + 2 * p] = A.n_over[4 * r + 2 * p + 1] = 0;
             }
         }
-        for (int q = t; q < 2 * (kMdBits / 32); q += all) (&totals.bits[0][0])[q] = 0;
         for (int q = t; q < 2 * kMdTerms; q += all) (&totals.te[0][0])[q] = make_int2(0, 0);
         __syncthreads();
         const MdBox<R> &B = sh.box;
+        for (int q = t; q < 2 * B.words; q += all) md_bits(B, 0)[q] = 0;  // used after kBarReady
         const int s_free = A.s_free[r];
         int k = A.start ? 0 : A.adv[r] - 1;
         if (t < kMdSum) {
@@ -1306,9 +1422,7 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                     md_turn<R>(sh, b, pair, A, k + 1, s_free, true, !last);
                 } else {
                     // ready for the step after the next forces
-                    // (256 places more: the FP32 form's leaves are of whole runs)
-                    for (int q = t - 32; q < (max(n0, n1) + 287) / 32 && q < kMdBits / 32; q += kMdSum - 32)
-                        totals.bits[0][q] = totals.bits[1][q] = 0;
+                    for (int q = t - 32; q < 2 * B.words; q += kMdSum - 32) md_bits(B, 0)[q] = 0;
                     if (t < 34) {
                         sh.cnt[k & 1][t - 32] = 0;
                         A.n_over[2 * (2 * r + t - 32) + (k & 1)] = 0;
@@ -1344,12 +1458,12 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
             const float near_sq = 0.99f * (float)thr * (float)thr;
             const uint64_t step0 = *A.d_step;
             for (int i = me; i < B.na; i += threads) {
-                int idx;
-                Part<R> q = md_read(B, A, i, idx, true);
+                const int idx = A.act[B.off + i], tier = md_tier(B, i);
+                Part<R> q = md_read_in_place(B, A, idx);
                 if (!fresh)
                     for (int c = 0; c < 3; c++) {
                         q.o[c] = q.p[c];
-                        if (i >= B.parts.cap) md_old(A, B)[c][idx] = q.p[c];
+                        if (tier == kInPlace) md_old(A, B)[c][idx] = q.p[c];
                     }
                 if (A.start) {
                     // force_old of the last interval's end is no longer current
@@ -1370,8 +1484,13 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                     B.parts.num(4, i) = e[0];
                     B.parts.num(5, i) = e[1];
                     for (int c = 0; c < 3; c++) B.parts.real(6 + c, i) = q.o[c];
+                    md_write<kShared>(B, A, i, q);
+                } else if (tier == kFar) {
+                    for (int c = 0; c < 3; c++) B.far.real(6 + c, i - B.parts.cap) = q.o[c];
+                    md_write<kFar>(B, A, i, q);
+                } else {
+                    md_write_in_place(B, A, idx, q);
                 }
-                md_write(B, A, i, idx, q, false);
             }
             md_sync(kBarReady, all);
             while (!(sh.stop | sh.over[k & 1])) {
@@ -1396,11 +1515,26 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                         md_pair_force(sh, B, A, totals, e >> 1, e & 1, k);
                     }
                 }
-                // the particles that the shared memory does not hold: their
-                // forces wait in force_old, whose entry is written again below
-                for (int i = B.parts.cap + me; i < B.na; i += threads) {
-                    int idx;
-                    const Part<R> q = md_read(B, A, i, idx, false);
+                // the particles that the shared memory does not hold
+                const int beyond = min(B.na, B.parts.cap + B.far.cap);
+                for (int i = B.parts.cap + me; i < beyond; i += threads) {
+                    const int s = i - B.parts.cap;
+                    int m = B.far.num(0, s);
+                    if (sh.anew) {
+                        const R p[3] = {B.far.real(0, s), B.far.real(1, s), B.far.real(2, s)};
+                        B.far.num(0, s) = m = md_busy(X, B, p, B.far.num(1, s), B.queue_sq);
+                    }
+                    if (!m) continue;
+                    const R p[3] = {B.far.real(0, s), B.far.real(1, s), B.far.real(2, s)};
+                    R nf[3];
+                    B.far.num(1, s) = md_forces(sh, B, A, totals, i, k, p, B.far.num(2, s), B.far.num(1, s), nf);
+                    for (int c = 0; c < 3; c++) B.far.real(12 + c, s) = nf[c];
+                }
+                // (those in place: the forces wait in force_old, whose entry is written
+                // again below)
+                for (int i = beyond + me; i < B.na; i += threads) {
+                    const int idx = A.act[B.off + i];
+                    const Part<R> q = md_read_in_place(B, A, idx);
                     if (!md_busy(X, B, q.p, q.f, B.reach_sq)) continue;
                     R nf[3];
                     md_view(A, B).flags[idx] = md_forces(sh, B, A, totals, i, k, q.p, q.sp, q.f, nf);
@@ -1409,16 +1543,18 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                 md_arrive(kBarForces, all);
                 md_sync(kBarPart, threads);  // the forces are written
                 // every particle's end of step k and beginning of step k + 1
-                for (int i = me; i < B.na; i += threads) {
-                    const bool in = i < B.parts.cap;
-                    int idx;
-                    Part<R> q = md_read(B, A, i, idx, false);
+                auto advance = [&](int i, auto tier_of, Part<R> q, int busy) {
+                    constexpr int T = decltype(tier_of)::value;
+                    const int s = i - B.parts.cap;  // in far
                     const bool past = (q.f >> PAST_MD_BIT) & 1;
                     const R gl[3] = {past ? q.g[0] : (R)0, past ? q.g[1] : (R)0, past ? q.g[2] : (R)0};
-                    // (forces only add flags, so the test gives what it gave)
-                    if (in ? B.parts.num(6, i) : md_busy(X, B, q.p, q.f, B.reach_sq)) {
+                    auto idx = [&] {
+                        if constexpr (T == kShared) return B.parts.num(0, i);
+                        else return A.act[B.off + i];
+                    };
+                    if (busy) {
                         R nf[3] = {0, 0, 0};
-                        if (in) {
+                        if constexpr (T == kShared) {
                             const int came = B.parts.num(7, i), m = B.parts.num(3, i);
 #pragma unroll
                             for (int h = 0; h < 2; h++)
@@ -1428,43 +1564,57 @@ __global__ void __launch_bounds__(kMdThreads, 1) kb_md(const __grid_constant__ M
                                         for (int c = 0; c < 3; c++) nf[c] = nf[c] - B.parts.real(12 + 3 * h + c, i);
                                 }
                             if (came & 4) q.f |= 1 << REAC_BIT;
+                        } else if constexpr (T == kFar) {
+                            for (int c = 0; c < 3; c++) nf[c] = B.far.real(12 + c, s);
                         } else {
-                            for (int c = 0; c < 3; c++) nf[c] = md_view(A, B).force_old[c][idx];
+                            for (int c = 0; c < 3; c++) nf[c] = md_view(A, B).force_old[c][idx()];
                         }
-                        md_end(q, X, B, A, nf, idx, step0 + (uint64_t)k);
-                        if (!in && !last)
-                            for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = 0;
+                        md_end(q, X, B, A, nf, idx(), step0 + (uint64_t)k);
+                        if (T == kInPlace && !last)
+                            for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx()] = 0;
                     } else {
                         for (int c = 0; c < 3; c++) q.v[c] = md_vel_free(q.v[c], A.dt_r);
                     }
                     if (last) {
                         // the interval's last step leaves force_old behind
-                        for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx] = gl[c];
+                        for (int c = 0; c < 3; c++) md_view(A, B).force_old[c][idx()] = gl[c];
                     } else {
                         if (md_begin(q, A.dt_r, A.dt_sq_r, A.read_species, thr, near_sq)) sh.over[1 - par] = 1;
-                        if (in) {
+                        if constexpr (T != kInPlace) {
                             const int m = md_busy(X, B, q.p, q.f, B.queue_sq);
-                            B.parts.num(6, i) = m;
-                            B.parts.num(7, i) = 0;
-                            if (m & 3) {
-                                const int s = atomicAdd(&sh.nq[1 - par], (m & 1) + (m >> 1 & 1));
-                                const int e = 2 * i + (m & 1 ? 0 : 1);
-                                if (s < kMdQueue) sh.q[1 - par][s] = e;
-                                if ((m & 3) == 3 && s + 1 < kMdQueue) sh.q[1 - par][s + 1] = 2 * i + 1;
+                            if constexpr (T == kFar) {
+                                B.far.num(0, s) = m;
+                            } else {
+                                B.parts.num(6, i) = m;
+                                B.parts.num(7, i) = 0;
+                                if (m & 3) {
+                                    const int at = atomicAdd(&sh.nq[1 - par], (m & 1) + (m >> 1 & 1));
+                                    const int e = 2 * i + (m & 1 ? 0 : 1);
+                                    if (at < kMdQueue) sh.q[1 - par][at] = e;
+                                    if ((m & 3) == 3 && at + 1 < kMdQueue) sh.q[1 - par][at + 1] = 2 * i + 1;
+                                }
                             }
                         }
                     }
-                    md_write(B, A, i, idx, q, false);
+                    md_write<T>(B, A, i, q);
+                };
+                for (int i = me; i < shared; i += threads)
+                    advance(i, std::integral_constant<int, kShared>(), md_read<kShared>(B, A, i), B.parts.num(6, i));
+                for (int i = B.parts.cap + me; i < beyond; i += threads)
+                    advance(i, std::integral_constant<int, kFar>(), md_read<kFar>(B, A, i), B.far.num(0, i - B.parts.cap));
+                for (int i = beyond + me; i < B.na; i += threads) {
+                    const Part<R> q = md_read<kInPlace>(B, A, i);
+                    // (forces only add flags, so the test gives what it gave)
+                    advance(i, std::integral_constant<int, kInPlace>(), q, md_busy(X, B, q.p, q.f, B.reach_sq));
                 }
                 md_sync(kBarTurn, all);
                 k++;
                 if (last) break;
             }
-            for (int i = me; i < min(B.na, B.parts.cap); i += threads) {
-                int idx;
-                const Part<R> q = md_read(B, A, i, idx, false);
-                md_write(B, A, i, idx, q, true);
-            }
+            for (int i = me; i < min(B.na, B.parts.cap); i += threads)
+                md_write_in_place(B, A, B.parts.num(0, i), md_read<kShared>(B, A, i));
+            for (int i = B.parts.cap + me; i < min(B.na, B.parts.cap + B.far.cap); i += threads)
+                md_write_in_place(B, A, A.act[B.off + i], md_read<kFar>(B, A, i));
         }
         __syncthreads();
     }
@@ -2021,6 +2171,8 @@ static void md_launches(Batch *b, const int *flag, cudaStream_t st, cudaGraphCon
     a.keys[0] = b->keys[0];
     a.keys[1] = b->keys[1];
     a.n_over = b->n_over;
+    a.far = b->far;
+    a.far_cap = b->far_cap;
     a.reach = reach;
     a.s_free = b->s_free;
     a.fresh = b->fresh;
@@ -2150,7 +2302,7 @@ static void free_batch(Batch *b)
     rmpcd_particles_destroy(b->col);
     void *ptrs[] = {b->rep, b->ptile, b->stile, b->stile_first, b->stile_count, b->tile_sum, b->tile_off, b->count,
                     b->start, b->cursor, b->is_md, b->is_reac, b->stencil, b->list, b->nn, b->act, b->nl, b->nx,
-                    b->aidx, b->next, b->mult, b->ent, b->over, b->terms, b->keys[0], b->keys[1], b->n_over, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
+                    b->aidx, b->next, b->mult, b->ent, b->over, b->terms, b->keys[0], b->keys[1], b->n_over, b->far, b->nf, b->s_free, b->adv, b->base, b->fresh, b->resort,
                     b->n_extra, b->rattle[0], b->rattle[1], b->rattle[2], b->vv_mass, b->d_step,
                     b->done, b->ptile_first, b->ptile_count, b->act_p, b->act_s, b->n_act, b->all_p, b->all_s,
                     b->n_all, b->any};
@@ -2421,6 +2573,10 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     }
     b->order_slots = order_slots(densest);
     size_t ne = (size_t)2 * R * b->Nmax;
+    // every particle that two full lists could make active
+    int most = 0;
+    for (const BRep &p : b->rep_h) most = p.n > most ? p.n : most;
+    b->far_cap = (int)(2LL * b->Nmax < most ? 2LL * b->Nmax : most);
     bool ok = !dalloc(&b->rep, R) && !dalloc(&b->ptile, cap_p) && !dalloc(&b->stile, stl.size()) &&
               !dalloc(&b->stile_first, R) && !dalloc(&b->stile_count, R) && !dalloc(&b->tile_sum, stl.size()) &&
               !dalloc(&b->tile_off, stl.size()) && !dalloc(&b->count, soff) && !dalloc(&b->start, soff) &&
@@ -2430,6 +2586,7 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
               !dalloc(&b->next, ne) && !dalloc(&b->mult, ne) && !dalloc(&b->ent, 2 * ne) && !dalloc(&b->over, ne) &&
               !dalloc(&b->terms, ne) && !dalloc(&b->keys[0], ne) && !dalloc(&b->keys[1], ne) &&
               !dalloc(&b->n_over, 4 * (size_t)R) &&
+              !dalloc(&b->far, (size_t)R * b->far_cap * (b->precision == RMPCD_FP32 ? md_far_bytes<float>() : md_far_bytes<double>())) &&
               !dalloc(&b->nf, R) && !dalloc(&b->s_free, R) && !dalloc(&b->adv, R) && !dalloc(&b->base, R) &&
               !dalloc(&b->fresh, R) && !dalloc(&b->resort, R) &&
               !dalloc(&b->n_extra, R) &&
