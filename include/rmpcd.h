@@ -396,8 +396,8 @@ int rmpcd_bulk_shapes(int precision, int *n_shapes, int *slots, int *min_blocks)
 int rmpcd_bulk_set_shape(int precision, int shape);
 int rmpcd_bulk_get_shape(int precision, int *shape);
 /* Autotuner: builds a synthetic bulk fluid of box L at density 10 (seeded
- * placement, Maxwell kT = 1/3), times n_intervals intervals with every
- * shape, puts the fastest in use for `precision` and returns its index in
+ * placement, Maxwell kT = 1/3), times n_intervals intervals of a long run with
+ * every shape, puts the fastest in use for `precision` and returns its index in
  * *best; ms_per_shape (may be NULL) receives each shape's time. */
 int rmpcd_bulk_autotune(const int L[3], int precision, double tau, int n_intervals, int *best,
                         float *ms_per_shape);
