@@ -10,9 +10,10 @@
 //
 // MD steps touch only the solvent that can interact.  A particle that is in
 // neither bead's neighbor list and carries no MD, PAST_MD, REAC or WALL flag, or
-// whose way stays clear of the beads, flies freely until the next re-sort: no
-// force can reach it before the list is rebuilt, so its md_pos steps depend on nothing but its own position and
-// velocity.  Such particles stay where they are in memory; the re-sort (or the
+// which has no force still to act and whose way stays clear of the beads, flies
+// freely until the next re-sort: no force can reach it before the list is rebuilt, so
+// its md_pos steps depend on nothing but its own position and velocity.  Such particles
+// stay where they are in memory; the re-sort (or the
 // interval's end) advances each by its pending md_pos steps in one pass, adding
 // dt * v once per step so that every rounding is that of the steps one by one.
 // The others -- the active particles, some 800 per dimer at sigma = 2: those
@@ -35,7 +36,7 @@
 //
 // Moving every particle in every MD step costs 56 B (FP32) per particle and
 // step: 121 us per step at 96^3 (4.1 TB/s) and 237 us for 48 replicas in boxes
-// of 16..48 cells, against 5 us per step for kb_md.
+// of 16..48 cells, against 6 us per step for kb_md.
 //
 // Arithmetic per particle is that of the single-system kernels
 // (stepops.cuh, nlist_ops.cuh), so replica r reproduces, bit for bit, the

@@ -575,8 +575,8 @@ __device__ __forceinline__ void bucket_drained(BucketTile<R, S> &sh, bool arrive
 }
 
 // Bound by the round trips of each particle (cell table, counting atomic), the
-// load/store pipe (69 % of its cycles at 96^3 FP32) and issue (66 %), not by HBM
-// (3.3 TB/s at 128^3), so occupancy decides: one particle per thread in flight,
+// load/store pipe (69 % of its cycles at 128x64x64 FP32) and issue (67 %), not by HBM
+// (3.4 TB/s at 128^3), so occupancy decides: one particle per thread in flight,
 // 40 registers, 48 warps per SM (two per thread with 32 warps: 128^3 FP32 566 us
 // for 531).  With the cell's collision on one thread per cell, copies by cp.async
 // and the moved records put back in shared memory, 64^3 FP32 took 94 us for 78,

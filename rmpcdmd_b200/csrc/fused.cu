@@ -749,7 +749,8 @@ static bool holds(const ShapeEntry<R> &e, double mean)
 // warps waiting at each barrier, are best for a large box; and a box just above one
 // wave of those (56,832 cells on 148 SMs) takes the 72-cell tiles if it is one wave
 // of them (63,936).  Between one and two waves the small blocks are best again, since
-// blocks of a second wave start as the first ones end.  us per interval by cells,
+// blocks of a second wave start as the first ones end.  us per interval of a run of 40,
+// pack and unpack included, by cells,
 // FP32 with 16 x 6 x 256 (cells x blocks per SM x threads), 24 x 16 x 96, 72 x 6 x 256:
 //   4,096  8.8 11.2 13.1    13,824 11.2 13.0 13.6    15,000 13.3 13.3 13.8    32,768 19.2 14.6 15.8
 //   54,872 37.5 20.8 20.7   59,280 39.5 23.2 20.9    61,500 32.1 23.0 20.7    62,400 40.5 24.4 21.6

@@ -76,8 +76,8 @@ struct rmpcd_particles {
     int *d_ints = nullptr;           // small integer scratch (64 ints)
     void *stage = nullptr;           // (3,N) layout staging for host transfers, 24 B/particle
     size_t stage_bytes = 0;
-    // packed particle records of the fused bulk schedule (double-buffered):
-    // 6 reals (pos, vel) + 6 ints (image, id, species, flags) per particle
+    // packed particle records of the bulk schedule's gather (double-buffered):
+    // pos, vel, species and the particle's index when the run started, 32 / 56 B
     unsigned char *rec[2] = {nullptr, nullptr};
     size_t rec_bytes = 0;
     unsigned char *buckets = nullptr;  // bucket arrays of the bulk schedule

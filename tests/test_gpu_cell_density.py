@@ -1,6 +1,6 @@
 """The collision kernels from thin to very dense fluids: their tiles have the slots
 that 832 particles in shared memory hold at the fluid's mean density (64 up to
-11.5 per cell, 4 at 177), beyond 178 a thread per slot on global memory; and uneven
+11.3 per cell, 4 at 177), beyond 178 a thread per slot on global memory; and uneven
 fluids, whose crowded tiles go run by run or on global memory."""
 import numpy as np
 import pytest

@@ -1,5 +1,5 @@
 """The ordering inside the sorts' gathers away from density 10: tiles of fewer slots
-for denser fluids (one from 1,630 particles per cell on), crowded tiles in runs of
+for denser fluids (one from 816 particles per cell on), crowded tiles in runs of
 cells, by rank (up to 64 particles per cell) or by merging, and cells too large for
 shared memory."""
 import numpy as np
