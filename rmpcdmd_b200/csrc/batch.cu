@@ -540,7 +540,7 @@ __host__ __device__ constexpr size_t md_part_bytes()
 template <typename R>
 __host__ __device__ constexpr size_t md_far_bytes()
 {
-    return 15 * sizeof(R) + 3 * sizeof(int);
+    return 15 * sizeof(R) + 3 * sizeof(int);  // times an even number: a multiple of sizeof(double)
 }
 
 // the fields of a block's particles in shared memory, cap of each
@@ -2577,10 +2577,11 @@ static int create(Batch **out, int R, rmpcd_particles *const *sol, rmpcd_particl
     }
     b->order_slots = order_slots(densest);
     size_t ne = (size_t)2 * R * b->Nmax;
-    // every particle that two full lists could make active
-    int most = 0;
+    // every particle that two full lists could make active; an even number, so that
+    // each replica's part (132 B per particle in FP64) begins at a multiple of 8 B
+    long long most = 0;
     for (const BRep &p : b->rep_h) most = p.n > most ? p.n : most;
-    b->far_cap = (int)(2LL * b->Nmax < most ? 2LL * b->Nmax : most);
+    b->far_cap = (int)(((2LL * b->Nmax < most ? 2LL * b->Nmax : most) + 1) & ~1LL);
     bool ok = !dalloc(&b->rep, R) && !dalloc(&b->ptile, cap_p) && !dalloc(&b->stile, stl.size()) &&
               !dalloc(&b->stile_first, R) && !dalloc(&b->stile_count, R) && !dalloc(&b->tile_sum, stl.size()) &&
               !dalloc(&b->tile_off, stl.size()) && !dalloc(&b->count, soff) && !dalloc(&b->start, soff) &&
